@@ -132,7 +132,10 @@ enum {
      kernel can be timed alone.  The workspace must have been prepared by an earlier full call;
      results of such partial calls are not meaningful. */
   FMHA_FLAG_BWD_SKIP_PREPARE = 2,
-  FMHA_FLAG_BWD_SKIP_FINISH = 4
+  FMHA_FLAG_BWD_SKIP_FINISH = 4,
+  /* FMHA_MASK_CU_SEQLENS: write zeros to the rows of o (forward) / dq, dk, dv (backward) that belong to no
+     sequence or lie past S_q = max_seqlen of theirs.  Without the flag such rows are not touched. */
+  FMHA_FLAG_ZERO_UNCOVERED = 8
 };
 
 typedef struct {

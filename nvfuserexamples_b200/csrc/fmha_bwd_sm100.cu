@@ -94,6 +94,7 @@ struct PrepArgs {
   float* dq_accum;  // [B*H, S_q_pad, D]
   int* work_counter;  // the main kernel's work-item counter, cleared here
   const int* cu_seqlens;  // packed batch: row offsets into the [total_rows, H, D] tensors (o_sb / do_sb unused), else null
+  UncoveredRows zero;
 };
 
 template <bool BF16>
@@ -120,6 +121,11 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const PrepArgs a) {
   if (a.cu_seqlens != nullptr) {
     const int base = a.cu_seqlens[b];
     q_limit = min(a.cu_seqlens[b + 1] - base, a.S_q);   // rows past the stated maximum length take no part
+    if (blockIdx.y == 0 && a.zero.grad[0].ptr != nullptr) {
+      for (int t = 0; t < 3; ++t)
+        zero_uncovered_rows(a.zero.grad[t].ptr, a.zero.grad[t].stride_s, a.zero.grad[t].stride_h, h, b, a.B, a.cu_seqlens, a.S_q,
+                            a.zero.total_rows, a.D, threadIdx.x, blockDim.x);
+    }
     row_o = static_cast<int64_t>(base + r) * a.o_ss;
     row_do = static_cast<int64_t>(base + r) * a.do_ss;
   }
@@ -962,14 +968,15 @@ int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream) {
 }
 
 int launch_bwd_prepare(const void* o, const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad,
-                       int D, int dtype, float* delta, float* dq_accum, int* work_counter, const int* cu_seqlens, cudaStream_t stream) {
+                       int D, int dtype, float* delta, float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero,
+                       cudaStream_t stream) {
   PrepArgs p;
   p.o = ot.ptr; p.d_o = dot.ptr;
   (void)o;
   p.o_sb = ot.stride_b; p.o_sh = ot.stride_h; p.o_ss = ot.stride_s;
   p.do_sb = dot.stride_b; p.do_sh = dot.stride_h; p.do_ss = dot.stride_s;
   p.B = B; p.H = H; p.S_q = S_q; p.S_q_pad = S_q_pad; p.D = D;
-  p.delta = delta; p.dq_accum = dq_accum; p.work_counter = work_counter; p.cu_seqlens = cu_seqlens;
+  p.delta = delta; p.dq_accum = dq_accum; p.work_counter = work_counter; p.cu_seqlens = cu_seqlens; p.zero = zero;
   const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q_pad + 31) / 32));
   const cudaError_t e = launch_overlapped(dtype == FMHA_DTYPE_BF16 ? bwd_prepare_kernel<true> : bwd_prepare_kernel<false>, grid,
                                           dim3(256), 0, stream, p);

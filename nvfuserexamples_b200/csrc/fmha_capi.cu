@@ -228,6 +228,7 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
   if ((rc = make_tmap(&a.tm_v, sanitized(p->v, mB, p->H, mSk, p->D), p->dtype, mB, p->H, mSk, p->D, kv_rows))) return rc;
   if ((rc = make_tmap(&a.tm_o, sanitized(p->o, mB, p->H, mSq, p->D), p->dtype, mB, p->H, mSq, p->D, kTileM))) return rc;
   a.total_rows = p->total_rows;
+  a.zero_uncovered = (p->flags & FMHA_FLAG_ZERO_UNCOVERED) != 0;
   a.o_ptr = p->o.ptr; a.o_ss = p->o.stride_s; a.o_sh = p->o.stride_h;
   a.o_sb = sanitized(p->o, mB, p->H, mSq, p->D).stride_b;
   a.o_sh = sanitized(p->o, mB, p->H, mSq, p->D).stride_h;
@@ -385,8 +386,10 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
 
   int e = 0;
   if (!(p->flags & FMHA_FLAG_BWD_SKIP_PREPARE)) {
+    UncoveredRows zero = {};
+    if (packed && (p->flags & FMHA_FLAG_ZERO_UNCOVERED)) zero = {{tdq, tdk, tdv}, p->total_rows};
     e = launch_bwd_prepare(nullptr, to, tdo, p->B, p->H, p->S_q, s_q_pad, p->D, p->dtype, delta, dq_accum, work_counter, cu_seqlens,
-                           stream);
+                           zero, stream);
     if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   } else {
     // the caller prepared delta and the accumulator itself; the work counter is still ours to clear

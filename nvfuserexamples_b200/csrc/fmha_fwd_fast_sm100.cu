@@ -174,6 +174,8 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     k_limit = len;
     q_limit = len;
     tb = 0;
+    if (blockIdx.x == 0 && a.zero_uncovered)
+      zero_uncovered_rows(a.o_ptr, a.o_ss, a.o_sh, h, b, a.B, cu, a.S_q, a.total_rows, D, threadIdx.x, blockDim.x);
     if (q0 >= len) return;   // this sequence has no such query tile (whole CTA, before any barrier)
   }
   const int n_kv = (k_limit + TN - 1) / TN;

@@ -35,6 +35,7 @@ struct FwdArgs {
   // FMHA_MASK_CU_SEQLENS (production kernel): mask = int32 [B+1] row offsets into the packed [total_rows, H, D]
   // tensors; o_ptr / strides serve the row-wise stores of a sequence's last, partial query tile
   int total_rows;
+  int zero_uncovered;         // FMHA_FLAG_ZERO_UNCOVERED
   void* o_ptr;
   int64_t o_ss, o_sh, o_sb;   // strides in elements (o_sb: dense-mask kernel, which stores O row by row)
   int B, H, S_q, S_k;
@@ -94,6 +95,12 @@ struct BwdArgs {
   int* status;
 };
 
+// FMHA_FLAG_ZERO_UNCOVERED of the backward pass: the three gradients whose uncovered rows are zeroed (ptr null: none).
+struct UncoveredRows {
+  fmha_tensor4 grad[3];
+  int total_rows;
+};
+
 // Launchers (defined in the .cu files).  Return a cudaError_t as int.
 int launch_fwd(const FwdArgs& a, int D, int dtype, bool legacy, bool p_via_smem, cudaStream_t stream);
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
@@ -102,7 +109,8 @@ bool fwd_dense_applies(const FwdArgs& a, int D);
 int launch_fwd_dense(const FwdArgs& a, int dtype, cudaStream_t stream);
 int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream);
 int launch_bwd_prepare(const void* o, const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad,
-                       int D, int dtype, float* delta, float* dq_accum, int* work_counter, const int* cu_seqlens, cudaStream_t stream);
+                       int D, int dtype, float* delta, float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero,
+                       cudaStream_t stream);
 int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int D, int dtype,
                       float scale, const int* cu_seqlens, cudaStream_t stream);
 
