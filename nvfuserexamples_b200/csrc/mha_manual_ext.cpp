@@ -18,13 +18,19 @@
 // There is no CPU implementation: the operators are registered for the CUDA key only and
 // every failure of the kernel library surfaces as a RuntimeError.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
-#include <cmath>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
 
+#include <array>
+#include <cmath>
 #include <cstdlib>
+#include <functional>
 #include <mutex>
 #include <vector>
 
@@ -74,18 +80,33 @@ void finish_call(int rc, const char* what, int device) {
   }
 }
 
+// An uninitialised CUDA tensor straight from the caching allocator: at::empty goes through two dispatcher hops first,
+// which is most of its cost for the sizes where the host sets the pace.
+at::Tensor empty_on(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
+  return at::Tensor(at::detail::empty_cuda(sizes, type, like.device(), std::nullopt));
+}
+
 struct View4 {
   fmha_tensor4 t;
   int64_t B, H, S, D;
 };
 
-// Accepts [B,H,S,D] or [B*H,S,D] (then B := B*H, H := 1) with a contiguous last axis.
-View4 view4(const at::Tensor& x, const char* name) {
+void check_operand(const at::Tensor& x, const char* name) {
   TORCH_CHECK(x.is_cuda(), "mha_manual: ", name, " must be a CUDA tensor");
   TORCH_CHECK(x.dim() == 3 || x.dim() == 4, "mha_manual: ", name, " must be [B,H,S,D] or [B*H,S,D]");
   TORCH_CHECK(x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16, "mha_manual: ", name,
               " must be float16 or bfloat16");
   TORCH_CHECK(x.stride(-1) == 1, "mha_manual: ", name, " must be contiguous along the head dimension");
+}
+void check_addressing(const View4& v, const char* name) {
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(v.t.ptr) & 15) == 0, "mha_manual: ", name, " must be 16-byte aligned");
+  TORCH_CHECK(v.t.stride_s % 8 == 0 && (v.H == 1 || v.t.stride_h % 8 == 0) && (v.B == 1 || v.t.stride_b % 8 == 0),
+              "mha_manual: strides of ", name, " must be multiples of 8 elements");
+}
+
+// Accepts [B,H,S,D] or [B*H,S,D] (then B := B*H, H := 1) with a contiguous last axis.
+View4 view4(const at::Tensor& x, const char* name) {
+  check_operand(x, name);
   View4 v;
   v.t.ptr = x.data_ptr();
   if (x.dim() == 4) {
@@ -95,9 +116,28 @@ View4 view4(const at::Tensor& x, const char* name) {
     v.B = x.size(0); v.H = 1; v.S = x.size(1); v.D = x.size(2);
     v.t.stride_b = x.stride(0); v.t.stride_h = x.stride(0); v.t.stride_s = x.stride(1);
   }
-  TORCH_CHECK((reinterpret_cast<uintptr_t>(v.t.ptr) & 15) == 0, "mha_manual: ", name, " must be 16-byte aligned");
-  TORCH_CHECK(v.t.stride_s % 8 == 0 && (v.H == 1 || v.t.stride_h % 8 == 0) && (v.B == 1 || v.t.stride_b % 8 == 0),
-              "mha_manual: strides of ", name, " must be multiples of 8 elements");
+  check_addressing(v, name);
+  return v;
+}
+// A [B,S,H,D] tensor, read through its strides.
+View4 view4_bshd(const at::Tensor& x, const char* name) {
+  check_operand(x, name);
+  View4 v;
+  v.t.ptr = x.data_ptr();
+  v.B = x.size(0); v.S = x.size(1); v.H = x.size(2); v.D = x.size(3);
+  v.t.stride_b = x.stride(0); v.t.stride_s = x.stride(1); v.t.stride_h = x.stride(2);
+  check_addressing(v, name);
+  return v;
+}
+// Slice i of a contiguous [B,S,3,H,D] projection (no tensor object is made for it).
+View4 qkv_slice(const at::Tensor& qkv, int i, const char* name) {
+  TORCH_CHECK(qkv.scalar_type() == at::kHalf || qkv.scalar_type() == at::kBFloat16, "mha_manual: ", name,
+              " must be float16 or bfloat16");
+  View4 v;
+  v.B = qkv.size(0); v.S = qkv.size(1); v.H = qkv.size(3); v.D = qkv.size(4);
+  v.t.ptr = static_cast<char*>(qkv.data_ptr()) + 2 * i * v.H * v.D;
+  v.t.stride_h = v.D; v.t.stride_s = 3 * v.H * v.D; v.t.stride_b = v.S * v.t.stride_s;
+  check_addressing(v, name);
   return v;
 }
 
@@ -138,7 +178,7 @@ std::vector<at::Tensor> legacy_forward(const at::Tensor& q, const at::Tensor& k,
   at::Tensor mask_c = dense_3d(mask, q, bh, vq.S, vk.S, "mask");
   at::Tensor dm_c;
   if (dropout_mask) dm_c = dense_3d(*dropout_mask, q, bh, vq.S, vk.S, "dropout_mask");
-  at::Tensor o = at::empty(q.sizes(), q.options());
+  at::Tensor o = empty_on(q, q.sizes(), q.scalar_type());
   const View4 vo = view4(o, "o");
   std::vector<at::Tensor> outs{o};
   fmha_fwd_params p{};
@@ -156,8 +196,8 @@ std::vector<at::Tensor> legacy_forward(const at::Tensor& q, const at::Tensor& k,
     p.dropout_scale = 2.0f;  // 1 / dropout_prob with dropout_prob = 0.5, fmha_manual.cpp:421,478-479
   }
   if (save) {
-    at::Tensor sm = at::empty({bh, vq.S, vk.S}, q.options());
-    at::Tensor dr = at::empty({bh, vq.S, vk.S}, q.options());
+    at::Tensor sm = empty_on(q, {bh, vq.S, vk.S}, q.scalar_type());
+    at::Tensor dr = empty_on(q, {bh, vq.S, vk.S}, q.scalar_type());
     p.save_softmax = sm.data_ptr();
     p.save_dropout = dr.data_ptr();
     outs.push_back(sm);
@@ -200,14 +240,15 @@ MaskArg resolve_mask(const c10::optional<at::Tensor>& mask, const c10::optional<
     const at::Tensor& t = *mask;
     TORCH_CHECK(t.device() == q.device(), "mha_manual: mask is on a different device");
     TORCH_CHECK(t.numel() == B * S_k, "mha_manual: mask must be [B,S_k] (or [B,1,1,S_k]) additive");
-    m.holder = t.reshape({B, S_k}).to(at::kFloat).contiguous();
+    // already what the kernels read (every call of a training loop as a rule): no reshape, no conversion
+    m.holder = t.scalar_type() == at::kFloat && t.is_contiguous() ? t : t.reshape({B, S_k}).to(at::kFloat).contiguous();
     m.kind = FMHA_MASK_KEY_ADDITIVE;
     m.ptr = m.holder.data_ptr();
   } else if (seqlens.has_value()) {
     const at::Tensor& t = *seqlens;
     TORCH_CHECK(t.device() == q.device(), "mha_manual: seqlens is on a different device");
     TORCH_CHECK(t.numel() == B, "mha_manual: seqlens must be [B]");
-    m.holder = t.reshape({B}).to(at::kInt).contiguous();
+    m.holder = t.scalar_type() == at::kInt && t.is_contiguous() ? t : t.reshape({B}).to(at::kInt).contiguous();
     m.kind = FMHA_MASK_SEQLEN;
     m.ptr = m.holder.data_ptr();
   }
@@ -223,40 +264,50 @@ const int64_t* offset_tensor_ptr(const c10::optional<at::Tensor>& t, const at::T
   return t->data_ptr<int64_t>();
 }
 
-// Forward into a caller-allocated `o` (any strides with a contiguous last axis); returns lse.
-at::Tensor fwd_into(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
-                    const c10::optional<at::Tensor>& mask, const c10::optional<at::Tensor>& seqlens, double p_drop,
-                    int64_t seed, int64_t offset, c10::optional<double> scale, int64_t bh_offset,
-                    const c10::optional<at::Tensor>& offset_tensor, const char* what) {
-  const View4 vq = view4(q, "q"), vk = view4(k, "k"), vv = view4(v, "v");
-  check_same(q, k, "k");
-  check_same(q, v, "v");
-  check_qkv(vq, vk, vv);
-  const c10::cuda::CUDAGuard guard(q.device());
-  const int dev = q.get_device();
-  const MaskArg m = resolve_mask(mask, seqlens, vq.B, vk.S, q);
-  std::vector<int64_t> lse_shape{vq.B, vq.S};
-  if (q.dim() == 4) lse_shape = {vq.B, vq.H, vq.S};
-  at::Tensor lse = at::empty(lse_shape, q.options().dtype(at::kFloat));
-  const View4 vo = view4(o, "o");
-  fmha_fwd_params p{};
+// What every operator passes on: the dropout and scale arguments.
+struct CallArgs {
+  double p_drop;
+  int64_t seed, offset;
+  c10::optional<double> scale;
+  int64_t bh_offset;
+  const c10::optional<at::Tensor>& offset_tensor;
+};
+template <typename Params>
+void fill_common(Params& p, const CallArgs& c, const at::Tensor& q, int64_t D) {
+  p.scale = c.scale.has_value() ? static_cast<float>(*c.scale) : 1.0f / std::sqrt(static_cast<float>(D));
+  if (c.p_drop > 0.0) {
+    p.dropout_kind = FMHA_DROPOUT_PHILOX;
+    p.p_drop = static_cast<float>(c.p_drop);
+    p.philox_seed = static_cast<uint64_t>(c.seed);
+    p.philox_offset = static_cast<uint64_t>(c.offset);
+    p.philox_offset_dev = offset_tensor_ptr(c.offset_tensor, q);
+  }
+  p.philox_bh_offset = static_cast<int32_t>(c.bh_offset);
+}
+template <typename Params>
+void fill_sizes(Params& p, const at::Tensor& q, const View4& vq, const View4& vk) {
   p.struct_bytes = sizeof(p);
   p.dtype = dtype_code(q);
   p.B = static_cast<int32_t>(vq.B); p.H = static_cast<int32_t>(vq.H);
   p.S_q = static_cast<int32_t>(vq.S); p.S_k = static_cast<int32_t>(vk.S); p.D = static_cast<int32_t>(vq.D);
-  p.scale = scale.has_value() ? static_cast<float>(*scale) : 1.0f / std::sqrt(static_cast<float>(vq.D));
+}
+
+// Forward into a caller-allocated o; returns lse.  `q` gives device and dtype, the views say where the operands lie.
+at::Tensor fwd_into(const at::Tensor& q, const View4& vq, const View4& vk, const View4& vv, const View4& vo,
+                    at::IntArrayRef lse_shape, const c10::optional<at::Tensor>& mask,
+                    const c10::optional<at::Tensor>& seqlens, const CallArgs& c, const char* what) {
+  check_qkv(vq, vk, vv);
+  const c10::cuda::CUDAGuard guard(q.device());
+  const int dev = q.get_device();
+  const MaskArg m = resolve_mask(mask, seqlens, vq.B, vk.S, q);
+  at::Tensor lse = empty_on(q, lse_shape, at::kFloat);
+  fmha_fwd_params p{};
+  fill_sizes(p, q, vq, vk);
   p.q = vq.t; p.k = vk.t; p.v = vv.t; p.o = vo.t;
   p.lse = lse.data_ptr<float>();
   p.mask_kind = m.kind;
   p.mask = m.ptr;
-  if (p_drop > 0.0) {
-    p.dropout_kind = FMHA_DROPOUT_PHILOX;
-    p.p_drop = static_cast<float>(p_drop);
-    p.philox_seed = static_cast<uint64_t>(seed);
-    p.philox_offset = static_cast<uint64_t>(offset);
-    p.philox_offset_dev = offset_tensor_ptr(offset_tensor, q);
-  }
-  p.philox_bh_offset = static_cast<int32_t>(bh_offset);
+  fill_common(p, c, q, vq.D);
   p.status = status_block(dev).data_ptr<int32_t>();
   finish_call(fmha_sm100_fwd(&p, at::cuda::getCurrentCUDAStream(dev).stream()), what, dev);
   return lse;
@@ -267,12 +318,15 @@ std::tuple<at::Tensor, at::Tensor> fmha_fwd(const at::Tensor& q, const at::Tenso
                                             const c10::optional<at::Tensor>& seqlens, double p_drop, int64_t seed,
                                             int64_t offset, c10::optional<double> scale, int64_t bh_offset,
                                             const c10::optional<at::Tensor>& offset_tensor) {
-  TORCH_CHECK(q.is_cuda(), "mha_manual: q must be a CUDA tensor");
-  at::Tensor o = at::empty(q.sizes(), q.options());
-  at::Tensor lse = fwd_into(q, k, v, o, mask, seqlens, p_drop, seed, offset, scale, bh_offset, offset_tensor, "fmha_fwd");
+  const View4 vq = view4(q, "q"), vk = view4(k, "k"), vv = view4(v, "v");
+  check_same(q, k, "k");
+  check_same(q, v, "v");
+  at::Tensor o = empty_on(q, q.sizes(), q.scalar_type());
+  const int64_t lse4[3] = {vq.B, vq.H, vq.S}, lse3[2] = {vq.B, vq.S};
+  at::Tensor lse = fwd_into(q, vq, vk, vv, view4(o, "o"), q.dim() == 4 ? at::IntArrayRef(lse4) : at::IntArrayRef(lse3), mask,
+                            seqlens, {p_drop, seed, offset, scale, bh_offset, offset_tensor}, "fmha_fwd");
   return {o, lse};
 }
-
 
 // An incoming gradient may be any view (autograd hands out expanded, i.e. stride-0, tensors for a broadcast loss):
 // what the tensor maps cannot describe - a non-contiguous last axis, a zero, negative or non-multiple-of-8 outer
@@ -284,16 +338,19 @@ at::Tensor dense_if_needed(const at::Tensor& t) {
   return ok ? t : t.contiguous();
 }
 
-// Backward into caller-allocated dq, dk, dv (any strides with a contiguous last axis).
-void bwd_into(const at::Tensor& d_o, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
-              const at::Tensor& lse, const at::Tensor& dq, const at::Tensor& dk, const at::Tensor& dv,
-              const c10::optional<at::Tensor>& mask, const c10::optional<at::Tensor>& seqlens, double p_drop, int64_t seed,
-              int64_t offset, c10::optional<double> scale, int64_t bh_offset,
-              const c10::optional<at::Tensor>& offset_tensor, const char* what) {
-  const View4 vq = view4(q, "q"), vk = view4(k, "k"), vv = view4(v, "v"), vo = view4(o, "o");
-  at::Tensor d_o_c = dense_if_needed(d_o);
-  const View4 vdo = view4(d_o_c, "d_o");
-  check_same(q, k, "k"); check_same(q, v, "v"); check_same(q, o, "o"); check_same(q, d_o_c, "d_o");
+at::Tensor bwd_workspace(fmha_bwd_params& p, const at::Tensor& q) {
+  size_t bytes = 0;
+  raise_if(fmha_sm100_bwd_workspace_bytes(&p, &bytes), "fmha_bwd_workspace_bytes");
+  at::Tensor ws = empty_on(q, {static_cast<int64_t>(bytes)}, at::kByte);
+  p.workspace = ws.data_ptr();
+  p.workspace_bytes = bytes;
+  return ws;
+}
+
+// Backward into caller-allocated dq, dk, dv.
+void bwd_into(const at::Tensor& q, const View4& vdo, const View4& vq, const View4& vk, const View4& vv, const View4& vo,
+              const at::Tensor& lse, const View4& vdq, const View4& vdk, const View4& vdv, const c10::optional<at::Tensor>& mask,
+              const c10::optional<at::Tensor>& seqlens, const CallArgs& c, const char* what) {
   check_qkv(vq, vk, vv);
   TORCH_CHECK(vo.B == vq.B && vo.H == vq.H && vo.S == vq.S && vo.D == vq.D, "mha_manual: o must have the shape of q");
   TORCH_CHECK(vdo.B == vq.B && vdo.H == vq.H && vdo.S == vq.S && vdo.D == vq.D, "mha_manual: d_o must have the shape of q");
@@ -303,31 +360,15 @@ void bwd_into(const at::Tensor& d_o, const at::Tensor& q, const at::Tensor& k, c
   const int dev = q.get_device();
   const MaskArg m = resolve_mask(mask, seqlens, vq.B, vk.S, q);
   at::Tensor lse_c = lse.contiguous();
-  const View4 vdq = view4(dq, "dq"), vdk = view4(dk, "dk"), vdv = view4(dv, "dv");
   fmha_bwd_params p{};
-  p.struct_bytes = sizeof(p);
-  p.dtype = dtype_code(q);
-  p.B = static_cast<int32_t>(vq.B); p.H = static_cast<int32_t>(vq.H);
-  p.S_q = static_cast<int32_t>(vq.S); p.S_k = static_cast<int32_t>(vk.S); p.D = static_cast<int32_t>(vq.D);
-  p.scale = scale.has_value() ? static_cast<float>(*scale) : 1.0f / std::sqrt(static_cast<float>(vq.D));
+  fill_sizes(p, q, vq, vk);
   p.q = vq.t; p.k = vk.t; p.v = vv.t; p.o = vo.t; p.d_o = vdo.t;
   p.lse = lse_c.data_ptr<float>();
   p.dq = vdq.t; p.dk = vdk.t; p.dv = vdv.t;
   p.mask_kind = m.kind;
   p.mask = m.ptr;
-  if (p_drop > 0.0) {
-    p.dropout_kind = FMHA_DROPOUT_PHILOX;
-    p.p_drop = static_cast<float>(p_drop);
-    p.philox_seed = static_cast<uint64_t>(seed);
-    p.philox_offset = static_cast<uint64_t>(offset);
-    p.philox_offset_dev = offset_tensor_ptr(offset_tensor, q);
-  }
-  p.philox_bh_offset = static_cast<int32_t>(bh_offset);
-  size_t ws = 0;
-  raise_if(fmha_sm100_bwd_workspace_bytes(&p, &ws), "fmha_bwd_workspace_bytes");
-  at::Tensor workspace = at::empty({static_cast<int64_t>(ws)}, q.options().dtype(at::kByte));
-  p.workspace = workspace.data_ptr();
-  p.workspace_bytes = ws;
+  fill_common(p, c, q, vq.D);
+  at::Tensor workspace = bwd_workspace(p, q);
   p.status = status_block(dev).data_ptr<int32_t>();
   finish_call(fmha_sm100_bwd(&p, at::cuda::getCurrentCUDAStream(dev).stream()), what, dev);
 }
@@ -338,11 +379,15 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> fmha_bwd(const at::Tensor& d_o, c
                                                         const c10::optional<at::Tensor>& seqlens, double p_drop,
                                                         int64_t seed, int64_t offset, c10::optional<double> scale,
                                                         int64_t bh_offset, const c10::optional<at::Tensor>& offset_tensor) {
-  TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda(), "mha_manual: q, k, v must be CUDA tensors");
-  at::Tensor dq = at::empty(q.sizes(), q.options());
-  at::Tensor dk = at::empty(k.sizes(), k.options());
-  at::Tensor dv = at::empty(v.sizes(), v.options());
-  bwd_into(d_o, q, k, v, o, lse, dq, dk, dv, mask, seqlens, p_drop, seed, offset, scale, bh_offset, offset_tensor, "fmha_bwd");
+  const View4 vq = view4(q, "q"), vk = view4(k, "k"), vv = view4(v, "v"), vo = view4(o, "o");
+  at::Tensor d_o_c = dense_if_needed(d_o);
+  const View4 vdo = view4(d_o_c, "d_o");
+  check_same(q, k, "k"); check_same(q, v, "v"); check_same(q, o, "o"); check_same(q, d_o_c, "d_o");
+  at::Tensor dq = empty_on(q, q.sizes(), q.scalar_type());
+  at::Tensor dk = empty_on(k, k.sizes(), k.scalar_type());
+  at::Tensor dv = empty_on(v, v.sizes(), v.scalar_type());
+  bwd_into(q, vdo, vq, vk, vv, vo, lse, view4(dq, "dq"), view4(dk, "dk"), view4(dv, "dv"), mask, seqlens,
+           {p_drop, seed, offset, scale, bh_offset, offset_tensor}, "fmha_bwd");
   return {dq, dk, dv};
 }
 
@@ -356,17 +401,15 @@ void check_qkvpacked(const at::Tensor& qkv) {
   TORCH_CHECK(qkv.dim() == 5 && qkv.size(2) == 3, "mha_manual: qkv must be [B,S,3,H,D]");
   TORCH_CHECK(qkv.is_contiguous(), "mha_manual: qkv must be contiguous");
 }
-// [B,S,3,H,D] -> the [B,H,S,D] view of slice i
-at::Tensor qkv_slice(const at::Tensor& qkv, int64_t i) { return qkv.select(2, i).permute({0, 2, 1, 3}); }
-
 std::tuple<at::Tensor, at::Tensor> fmha_qkvpacked_fwd(const at::Tensor& qkv, const c10::optional<at::Tensor>& mask,
                                                       const c10::optional<at::Tensor>& seqlens, double p_drop, int64_t seed,
                                                       int64_t offset, c10::optional<double> scale, int64_t bh_offset,
                                                       const c10::optional<at::Tensor>& offset_tensor) {
   check_qkvpacked(qkv);
-  at::Tensor o = at::empty({qkv.size(0), qkv.size(1), qkv.size(3), qkv.size(4)}, qkv.options());   // [B,S,H,D]
-  at::Tensor lse = fwd_into(qkv_slice(qkv, 0), qkv_slice(qkv, 1), qkv_slice(qkv, 2), o.permute({0, 2, 1, 3}), mask, seqlens,
-                            p_drop, seed, offset, scale, bh_offset, offset_tensor, "fmha_qkvpacked_fwd");
+  at::Tensor o = empty_on(qkv, {qkv.size(0), qkv.size(1), qkv.size(3), qkv.size(4)}, qkv.scalar_type());   // [B,S,H,D]
+  at::Tensor lse = fwd_into(qkv, qkv_slice(qkv, 0, "q"), qkv_slice(qkv, 1, "k"), qkv_slice(qkv, 2, "v"), view4_bshd(o, "o"),
+                            {qkv.size(0), qkv.size(3), qkv.size(1)}, mask, seqlens,
+                            {p_drop, seed, offset, scale, bh_offset, offset_tensor}, "fmha_qkvpacked_fwd");
   return {o, lse};
 }
 
@@ -378,10 +421,12 @@ at::Tensor fmha_qkvpacked_bwd(const at::Tensor& d_o, const at::Tensor& qkv, cons
   TORCH_CHECK(d_o.dim() == 4 && o.dim() == 4 && d_o.sizes() == o.sizes() && o.size(0) == qkv.size(0) &&
                   o.size(1) == qkv.size(1) && o.size(2) == qkv.size(3) && o.size(3) == qkv.size(4),
               "mha_manual: o and d_o must be [B,S,H,D]");
-  at::Tensor dqkv = at::empty(qkv.sizes(), qkv.options());
-  bwd_into(d_o.permute({0, 2, 1, 3}), qkv_slice(qkv, 0), qkv_slice(qkv, 1), qkv_slice(qkv, 2), o.permute({0, 2, 1, 3}), lse,
-           qkv_slice(dqkv, 0), qkv_slice(dqkv, 1), qkv_slice(dqkv, 2), mask, seqlens, p_drop, seed, offset, scale, bh_offset,
-           offset_tensor, "fmha_qkvpacked_bwd");
+  at::Tensor dqkv = empty_on(qkv, qkv.sizes(), qkv.scalar_type());
+  at::Tensor d_o_c = dense_if_needed(d_o);
+  check_same(qkv, o, "o"); check_same(qkv, d_o_c, "d_o");
+  bwd_into(qkv, view4_bshd(d_o_c, "d_o"), qkv_slice(qkv, 0, "q"), qkv_slice(qkv, 1, "k"), qkv_slice(qkv, 2, "v"),
+           view4_bshd(o, "o"), lse, qkv_slice(dqkv, 0, "dq"), qkv_slice(dqkv, 1, "dk"), qkv_slice(dqkv, 2, "dv"), mask, seqlens,
+           {p_drop, seed, offset, scale, bh_offset, offset_tensor}, "fmha_qkvpacked_bwd");
   return dqkv;
 }
 
@@ -410,7 +455,7 @@ Packed packed3(const at::Tensor& x, const char* name) {
 at::Tensor check_cu_seqlens(const at::Tensor& cu, const at::Tensor& q) {
   TORCH_CHECK(cu.device() == q.device(), "mha_manual: cu_seqlens is on a different device");
   TORCH_CHECK(cu.dim() == 1 && cu.numel() >= 2, "mha_manual: cu_seqlens must be [B+1]");
-  return cu.to(at::kInt).contiguous();
+  return cu.scalar_type() == at::kInt && cu.is_contiguous() ? cu : cu.to(at::kInt).contiguous();
 }
 void check_packed_qkv(const Packed& q, const Packed& k, const Packed& v, int64_t max_seqlen) {
   TORCH_CHECK(q.D == 64 || q.D == 128, "mha_manual: head dimension must be 64 or 128, got ", q.D);
@@ -419,37 +464,44 @@ void check_packed_qkv(const Packed& q, const Packed& k, const Packed& v, int64_t
   TORCH_CHECK(max_seqlen > 0, "mha_manual: max_seqlen must be positive");
 }
 
-// Packed forward into a caller-allocated `o` ([total_rows, H, D] with any row / head strides); returns lse.
-at::Tensor varlen_fwd_into(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
-                           const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop, int64_t seed, int64_t offset,
-                           c10::optional<double> scale, const c10::optional<at::Tensor>& offset_tensor, const char* what) {
-  const Packed vq = packed3(q, "q"), vk = packed3(k, "k"), vv = packed3(v, "v");
-  check_same(q, k, "k");
-  check_same(q, v, "v");
-  check_packed_qkv(vq, vk, vv, max_seqlen);
-  const c10::cuda::CUDAGuard guard(q.device());
-  const int dev = q.get_device();
-  const at::Tensor cu = check_cu_seqlens(cu_seqlens, q);
-  at::Tensor lse = at::empty({vq.H, vq.total}, q.options().dtype(at::kFloat));
-  if (vq.total == 0) return lse;
-  fmha_fwd_params p{};
+// Slice i of a contiguous [total_rows, 3, H, D] projection.
+Packed varlen_slice(const at::Tensor& qkv, int i, const char* name) {
+  TORCH_CHECK(qkv.scalar_type() == at::kHalf || qkv.scalar_type() == at::kBFloat16, "mha_manual: ", name,
+              " must be float16 or bfloat16");
+  Packed v;
+  v.total = qkv.size(0); v.H = qkv.size(2); v.D = qkv.size(3);
+  v.t.ptr = static_cast<char*>(qkv.data_ptr()) + 2 * i * v.H * v.D;
+  v.t.stride_b = 0; v.t.stride_h = v.D; v.t.stride_s = 3 * v.H * v.D;
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(v.t.ptr) & 15) == 0, "mha_manual: ", name, " must be 16-byte aligned");
+  return v;
+}
+template <typename Params>
+void fill_packed_sizes(Params& p, const at::Tensor& q, const Packed& vq, const at::Tensor& cu, int64_t max_seqlen) {
   p.struct_bytes = sizeof(p);
   p.dtype = dtype_code(q);
   p.B = static_cast<int32_t>(cu.numel() - 1); p.H = static_cast<int32_t>(vq.H);
   p.S_q = p.S_k = static_cast<int32_t>(max_seqlen); p.D = static_cast<int32_t>(vq.D);
-  p.scale = scale.has_value() ? static_cast<float>(*scale) : 1.0f / std::sqrt(static_cast<float>(vq.D));
-  p.q = vq.t; p.k = vk.t; p.v = vv.t; p.o = packed3(o, "o").t;
-  p.lse = lse.data_ptr<float>();
   p.mask_kind = FMHA_MASK_CU_SEQLENS;
   p.mask = cu.data_ptr();
   p.total_rows = static_cast<int32_t>(vq.total);
-  if (p_drop > 0.0) {
-    p.dropout_kind = FMHA_DROPOUT_PHILOX;
-    p.p_drop = static_cast<float>(p_drop);
-    p.philox_seed = static_cast<uint64_t>(seed);
-    p.philox_offset = static_cast<uint64_t>(offset);
-    p.philox_offset_dev = offset_tensor_ptr(offset_tensor, q);
-  }
+  // rows of a sequence beyond max_seqlen (where the kernels cut it) are returned as zeros
+  p.flags = FMHA_FLAG_ZERO_UNCOVERED;
+}
+
+// Packed forward into a caller-allocated o; returns lse.  `q` gives device and dtype.
+at::Tensor varlen_fwd_into(const at::Tensor& q, const Packed& vq, const Packed& vk, const Packed& vv, const Packed& vo,
+                           const at::Tensor& cu_seqlens, int64_t max_seqlen, const CallArgs& c, const char* what) {
+  check_packed_qkv(vq, vk, vv, max_seqlen);
+  const c10::cuda::CUDAGuard guard(q.device());
+  const int dev = q.get_device();
+  const at::Tensor cu = check_cu_seqlens(cu_seqlens, q);
+  at::Tensor lse = empty_on(q, {vq.H, vq.total}, at::kFloat);
+  if (vq.total == 0) return lse;
+  fmha_fwd_params p{};
+  fill_packed_sizes(p, q, vq, cu, max_seqlen);
+  p.q = vq.t; p.k = vk.t; p.v = vv.t; p.o = vo.t;
+  p.lse = lse.data_ptr<float>();
+  fill_common(p, c, q, vq.D);
   p.status = status_block(dev).data_ptr<int32_t>();
   finish_call(fmha_sm100_fwd(&p, at::cuda::getCurrentCUDAStream(dev).stream()), what, dev);
   return lse;
@@ -459,24 +511,20 @@ std::tuple<at::Tensor, at::Tensor> fmha_varlen_fwd(const at::Tensor& q, const at
                                                    const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop,
                                                    int64_t seed, int64_t offset, c10::optional<double> scale,
                                                    const c10::optional<at::Tensor>& offset_tensor) {
-  TORCH_CHECK(q.is_cuda(), "mha_manual: q must be a CUDA tensor");
-  // zero-filled: rows of a sequence beyond max_seqlen (where the kernels cut it) are never written
-  at::Tensor o = at::zeros(q.sizes(), q.options());
-  at::Tensor lse = varlen_fwd_into(q, k, v, o, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor, "fmha_varlen_fwd");
+  const Packed vq = packed3(q, "q"), vk = packed3(k, "k"), vv = packed3(v, "v");
+  check_same(q, k, "k");
+  check_same(q, v, "v");
+  at::Tensor o = empty_on(q, q.sizes(), q.scalar_type());
+  at::Tensor lse = varlen_fwd_into(q, vq, vk, vv, packed3(o, "o"), cu_seqlens, max_seqlen,
+                                   {p_drop, seed, offset, scale, 0, offset_tensor}, "fmha_varlen_fwd");
   return {o, lse};
 }
 
-// Packed backward into caller-allocated dq, dk, dv ([total_rows, H, D] with any row / head strides).
-void varlen_bwd_into(const at::Tensor& d_o, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o,
-                     const at::Tensor& lse, const at::Tensor& dq, const at::Tensor& dk, const at::Tensor& dv,
-                     const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop, int64_t seed, int64_t offset,
-                     c10::optional<double> scale, const c10::optional<at::Tensor>& offset_tensor, const char* what) {
-  const Packed vq = packed3(q, "q"), vk = packed3(k, "k"), vv = packed3(v, "v"), vo = packed3(o, "o");
-  at::Tensor d_o_c = dense_if_needed(d_o);
-  const Packed vdo = packed3(d_o_c, "d_o");
-  check_same(q, k, "k"); check_same(q, v, "v"); check_same(q, o, "o"); check_same(q, d_o_c, "d_o");
+// Packed backward into caller-allocated dq, dk, dv.
+void varlen_bwd_into(const at::Tensor& q, const Packed& vdo, const Packed& vq, const Packed& vk, const Packed& vv,
+                     const Packed& vo, const at::Tensor& lse, const Packed& vdq, const Packed& vdk, const Packed& vdv,
+                     const at::Tensor& cu_seqlens, int64_t max_seqlen, const CallArgs& c, const char* what) {
   check_packed_qkv(vq, vk, vv, max_seqlen);
-  TORCH_CHECK(o.sizes() == q.sizes() && d_o_c.sizes() == q.sizes(), "mha_manual: o and d_o must have the shape of q");
   TORCH_CHECK(lse.device() == q.device() && lse.scalar_type() == at::kFloat && lse.numel() == vq.H * vq.total,
               "mha_manual: lse must be float32 [H, total_rows] on the device of q");
   const c10::cuda::CUDAGuard guard(q.device());
@@ -485,29 +533,12 @@ void varlen_bwd_into(const at::Tensor& d_o, const at::Tensor& q, const at::Tenso
   at::Tensor lse_c = lse.contiguous();
   if (vq.total == 0) return;
   fmha_bwd_params p{};
-  p.struct_bytes = sizeof(p);
-  p.dtype = dtype_code(q);
-  p.B = static_cast<int32_t>(cu.numel() - 1); p.H = static_cast<int32_t>(vq.H);
-  p.S_q = p.S_k = static_cast<int32_t>(max_seqlen); p.D = static_cast<int32_t>(vq.D);
-  p.scale = scale.has_value() ? static_cast<float>(*scale) : 1.0f / std::sqrt(static_cast<float>(vq.D));
+  fill_packed_sizes(p, q, vq, cu, max_seqlen);
   p.q = vq.t; p.k = vk.t; p.v = vv.t; p.o = vo.t; p.d_o = vdo.t;
   p.lse = lse_c.data_ptr<float>();
-  p.dq = packed3(dq, "dq").t; p.dk = packed3(dk, "dk").t; p.dv = packed3(dv, "dv").t;
-  p.mask_kind = FMHA_MASK_CU_SEQLENS;
-  p.mask = cu.data_ptr();
-  p.total_rows = static_cast<int32_t>(vq.total);
-  if (p_drop > 0.0) {
-    p.dropout_kind = FMHA_DROPOUT_PHILOX;
-    p.p_drop = static_cast<float>(p_drop);
-    p.philox_seed = static_cast<uint64_t>(seed);
-    p.philox_offset = static_cast<uint64_t>(offset);
-    p.philox_offset_dev = offset_tensor_ptr(offset_tensor, q);
-  }
-  size_t ws = 0;
-  raise_if(fmha_sm100_bwd_workspace_bytes(&p, &ws), "fmha_bwd_workspace_bytes");
-  at::Tensor workspace = at::empty({static_cast<int64_t>(ws)}, q.options().dtype(at::kByte));
-  p.workspace = workspace.data_ptr();
-  p.workspace_bytes = ws;
+  p.dq = vdq.t; p.dk = vdk.t; p.dv = vdv.t;
+  fill_common(p, c, q, vq.D);
+  at::Tensor workspace = bwd_workspace(p, q);
   p.status = status_block(dev).data_ptr<int32_t>();
   finish_call(fmha_sm100_bwd(&p, at::cuda::getCurrentCUDAStream(dev).stream()), what, dev);
 }
@@ -517,13 +548,16 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> fmha_varlen_bwd(const at::Tensor&
                                                                const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop,
                                                                int64_t seed, int64_t offset, c10::optional<double> scale,
                                                                const c10::optional<at::Tensor>& offset_tensor) {
-  TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda(), "mha_manual: q, k, v must be CUDA tensors");
-  // zero-filled: rows of a sequence beyond max_seqlen (where the kernels cut it) are never written
-  at::Tensor dq = at::zeros(q.sizes(), q.options());
-  at::Tensor dk = at::zeros(k.sizes(), k.options());
-  at::Tensor dv = at::zeros(v.sizes(), v.options());
-  varlen_bwd_into(d_o, q, k, v, o, lse, dq, dk, dv, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor,
-                  "fmha_varlen_bwd");
+  const Packed vq = packed3(q, "q"), vk = packed3(k, "k"), vv = packed3(v, "v"), vo = packed3(o, "o");
+  at::Tensor d_o_c = dense_if_needed(d_o);
+  const Packed vdo = packed3(d_o_c, "d_o");
+  check_same(q, k, "k"); check_same(q, v, "v"); check_same(q, o, "o"); check_same(q, d_o_c, "d_o");
+  TORCH_CHECK(o.sizes() == q.sizes() && d_o_c.sizes() == q.sizes(), "mha_manual: o and d_o must have the shape of q");
+  at::Tensor dq = empty_on(q, q.sizes(), q.scalar_type());
+  at::Tensor dk = empty_on(k, k.sizes(), k.scalar_type());
+  at::Tensor dv = empty_on(v, v.sizes(), v.scalar_type());
+  varlen_bwd_into(q, vdo, vq, vk, vv, vo, lse, packed3(dq, "dq"), packed3(dk, "dk"), packed3(dv, "dv"), cu_seqlens, max_seqlen,
+                  {p_drop, seed, offset, scale, 0, offset_tensor}, "fmha_varlen_bwd");
   return {dq, dk, dv};
 }
 
@@ -539,9 +573,10 @@ std::tuple<at::Tensor, at::Tensor> fmha_varlen_qkvpacked_fwd(const at::Tensor& q
                                                              c10::optional<double> scale,
                                                              const c10::optional<at::Tensor>& offset_tensor) {
   check_varlen_qkvpacked(qkv);
-  at::Tensor o = at::zeros({qkv.size(0), qkv.size(2), qkv.size(3)}, qkv.options());
-  at::Tensor lse = varlen_fwd_into(qkv.select(1, 0), qkv.select(1, 1), qkv.select(1, 2), o, cu_seqlens, max_seqlen, p_drop, seed,
-                                   offset, scale, offset_tensor, "fmha_varlen_qkvpacked_fwd");
+  at::Tensor o = empty_on(qkv, {qkv.size(0), qkv.size(2), qkv.size(3)}, qkv.scalar_type());
+  at::Tensor lse = varlen_fwd_into(qkv, varlen_slice(qkv, 0, "q"), varlen_slice(qkv, 1, "k"), varlen_slice(qkv, 2, "v"),
+                                   packed3(o, "o"), cu_seqlens, max_seqlen, {p_drop, seed, offset, scale, 0, offset_tensor},
+                                   "fmha_varlen_qkvpacked_fwd");
   return {o, lse};
 }
 at::Tensor fmha_varlen_qkvpacked_bwd(const at::Tensor& d_o, const at::Tensor& qkv, const at::Tensor& o, const at::Tensor& lse,
@@ -549,10 +584,16 @@ at::Tensor fmha_varlen_qkvpacked_bwd(const at::Tensor& d_o, const at::Tensor& qk
                                      int64_t offset, c10::optional<double> scale,
                                      const c10::optional<at::Tensor>& offset_tensor) {
   check_varlen_qkvpacked(qkv);
-  at::Tensor dqkv = at::zeros(qkv.sizes(), qkv.options());
-  varlen_bwd_into(d_o, qkv.select(1, 0), qkv.select(1, 1), qkv.select(1, 2), o, lse, dqkv.select(1, 0), dqkv.select(1, 1),
-                  dqkv.select(1, 2), cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor,
-                  "fmha_varlen_qkvpacked_bwd");
+  const Packed vo = packed3(o, "o");
+  at::Tensor d_o_c = dense_if_needed(d_o);
+  const Packed vdo = packed3(d_o_c, "d_o");
+  check_same(qkv, o, "o"); check_same(qkv, d_o_c, "d_o");
+  TORCH_CHECK(o.size(0) == qkv.size(0) && o.size(1) == qkv.size(2) && o.size(2) == qkv.size(3) && d_o_c.sizes() == o.sizes(),
+              "mha_manual: o and d_o must have the shape of q");
+  at::Tensor dqkv = empty_on(qkv, qkv.sizes(), qkv.scalar_type());
+  varlen_bwd_into(qkv, vdo, varlen_slice(qkv, 0, "q"), varlen_slice(qkv, 1, "k"), varlen_slice(qkv, 2, "v"), vo, lse,
+                  varlen_slice(dqkv, 0, "dq"), varlen_slice(dqkv, 1, "dk"), varlen_slice(dqkv, 2, "dv"), cu_seqlens, max_seqlen,
+                  {p_drop, seed, offset, scale, 0, offset_tensor}, "fmha_varlen_qkvpacked_bwd");
   return dqkv;
 }
 
@@ -587,210 +628,184 @@ void check_status() {
 }
 
 // ---------------------------------------------------------------------------------------
-// autograd: fmha = fmha_fwd + fmha_bwd
+// autograd: fmha = fmha_fwd + fmha_bwd, and the same for the three other layouts.
+//
+// Written as graph nodes of their own instead of torch::autograd::Function: at the sizes where the host sets the pace
+// (a B=2, H=4, S=128 step takes 17 us of GPU time) that template's argument vectors, saved-value dictionary and output
+// wrapping cost more than the kernels.
 // ---------------------------------------------------------------------------------------
-class FmhaFunction : public torch::autograd::Function<FmhaFunction> {
- public:
-  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k,
-                            const at::Tensor& v, const c10::optional<at::Tensor>& mask,
-                            const c10::optional<at::Tensor>& seqlens, double p_drop, int64_t seed, int64_t offset,
-                            c10::optional<double> scale, const c10::optional<at::Tensor>& offset_tensor) {
-    at::AutoDispatchBelowADInplaceOrView guard;
-    // through the dispatcher, so that fake / meta tensors reach the shape-only kernels
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_fwd", "")
-                         .typed<std::tuple<at::Tensor, at::Tensor>(const at::Tensor&, const at::Tensor&, const at::Tensor&,
-                                                                   const c10::optional<at::Tensor>&,
-                                                                   const c10::optional<at::Tensor>&, double, int64_t, int64_t,
-                                                                   c10::optional<double>, int64_t,
-                                                                   const c10::optional<at::Tensor>&)>();
-    auto [o, lse] = op.call(q, k, v, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor);
-    // The backward pass must see the value the forward pass saw, even if the caller advances the tensor in
-    // between: it gets a private copy.
-    ctx->save_for_backward({q, k, v, o, lse, mask.has_value() ? *mask : at::Tensor(),
-                            seqlens.has_value() ? *seqlens : at::Tensor(),
-                            offset_tensor.has_value() ? offset_tensor->clone() : at::Tensor()});
-    ctx->saved_data["p_drop"] = p_drop;
-    ctx->saved_data["seed"] = seed;
-    ctx->saved_data["offset"] = offset;
-    ctx->saved_data["has_scale"] = scale.has_value();
-    ctx->saved_data["scale"] = scale.has_value() ? *scale : 0.0;
-    return o;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using OptTensor = c10::optional<at::Tensor>;
+
+struct AttnNode : public torch::autograd::Node {
+  SavedVariable in[3], o, lse, mask, lens, offset_tensor;   // lens: valid lengths or cu_seqlens
+  bool has_mask = false, has_lens = false, has_offset_tensor = false;
+  int64_t max_seqlen = 0;
+  double p_drop = 0.0;
+  int64_t seed = 0, offset = 0;
+  c10::optional<double> scale;
+
+  void release_variables() override {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable& s : in) s.reset_data();
+    for (SavedVariable* s : {&o, &lse, &mask, &lens, &offset_tensor}) s->reset_data();
   }
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
-                                                 torch::autograd::variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    c10::optional<at::Tensor> mask, seqlens;
-    if (saved[5].defined()) mask = saved[5];
-    if (saved[6].defined()) seqlens = saved[6];
-    c10::optional<at::Tensor> offset_tensor;
-    if (saved[7].defined()) offset_tensor = saved[7];
-    c10::optional<double> scale;
-    if (ctx->saved_data["has_scale"].toBool()) scale = ctx->saved_data["scale"].toDouble();
-    static auto op =
-        c10::Dispatcher::singleton()
-            .findSchemaOrThrow("mha_manual::fmha_bwd", "")
-            .typed<std::tuple<at::Tensor, at::Tensor, at::Tensor>(
-                const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
-                const c10::optional<at::Tensor>&, const c10::optional<at::Tensor>&, double, int64_t, int64_t,
-                c10::optional<double>, int64_t, const c10::optional<at::Tensor>&)>();
-    auto [dq, dk, dv] = op.call(grads[0], saved[0], saved[1], saved[2], saved[3], saved[4], mask, seqlens,
-                                ctx->saved_data["p_drop"].toDouble(), ctx->saved_data["seed"].toInt(),
-                                ctx->saved_data["offset"].toInt(), scale, 0, offset_tensor);
-    return {dq, dk, dv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+  OptTensor opt(const SavedVariable& s, bool has) const { return has ? OptTensor(s.unpack()) : OptTensor(); }
+  // The gradients of this node's inputs, given everything saved.
+  virtual variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) = 0;
+
+  variable_list apply(variable_list&& grads) override {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    const at::Tensor out = o.unpack(shared_from_this());
+    const at::Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(out);
+    variable_list g;
+    if (at::GradMode::is_enabled()) {   // create_graph: the backward operator says itself that it has no derivative
+      g = gradients(d_o, out);
+    } else {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      g = gradients(d_o, out);
+    }
+    g.resize(num_outputs());   // mask, lengths and offset take no gradient
+    return g;
   }
 };
 
-class FmhaVarlenFunction : public torch::autograd::Function<FmhaVarlenFunction> {
- public:
-  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k,
-                            const at::Tensor& v, const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop,
-                            int64_t seed, int64_t offset, c10::optional<double> scale,
-                            const c10::optional<at::Tensor>& offset_tensor) {
-    at::AutoDispatchBelowADInplaceOrView guard;
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_varlen_fwd", "")
-                         .typed<std::tuple<at::Tensor, at::Tensor>(const at::Tensor&, const at::Tensor&, const at::Tensor&,
-                                                                   const at::Tensor&, int64_t, double, int64_t, int64_t,
-                                                                   c10::optional<double>, const c10::optional<at::Tensor>&)>();
-    auto [o, lse] = op.call(q, k, v, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor);
-    ctx->save_for_backward({q, k, v, o, lse, cu_seqlens, offset_tensor.has_value() ? offset_tensor->clone() : at::Tensor()});
-    ctx->saved_data["max_seqlen"] = max_seqlen;
-    ctx->saved_data["p_drop"] = p_drop;
-    ctx->saved_data["seed"] = seed;
-    ctx->saved_data["offset"] = offset;
-    ctx->saved_data["has_scale"] = scale.has_value();
-    ctx->saved_data["scale"] = scale.has_value() ? *scale : 0.0;
-    return o;
-  }
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
-                                                 torch::autograd::variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    c10::optional<double> scale;
-    if (ctx->saved_data["has_scale"].toBool()) scale = ctx->saved_data["scale"].toDouble();
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_varlen_bwd", "")
-                         .typed<std::tuple<at::Tensor, at::Tensor, at::Tensor>(
-                             const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
-                             const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
-                             const c10::optional<at::Tensor>&)>();
-    c10::optional<at::Tensor> offset_tensor;
-    if (saved[6].defined()) offset_tensor = saved[6];
-    auto [dq, dk, dv] = op.call(grads[0], saved[0], saved[1], saved[2], saved[3], saved[4], saved[5],
-                                ctx->saved_data["max_seqlen"].toInt(), ctx->saved_data["p_drop"].toDouble(),
-                                ctx->saved_data["seed"].toInt(), ctx->saved_data["offset"].toInt(), scale, offset_tensor);
-    return {dq, dk, dv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
-  }
-};
-
-class FmhaVarlenQkvPackedFunction : public torch::autograd::Function<FmhaVarlenQkvPackedFunction> {
- public:
-  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& qkv, const at::Tensor& cu_seqlens,
-                            int64_t max_seqlen, double p_drop, int64_t seed, int64_t offset, c10::optional<double> scale,
-                            const c10::optional<at::Tensor>& offset_tensor) {
-    at::AutoDispatchBelowADInplaceOrView guard;
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_varlen_qkvpacked_fwd", "")
-                         .typed<std::tuple<at::Tensor, at::Tensor>(const at::Tensor&, const at::Tensor&, int64_t, double, int64_t,
-                                                                   int64_t, c10::optional<double>,
-                                                                   const c10::optional<at::Tensor>&)>();
-    auto [o, lse] = op.call(qkv, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor);
-    ctx->save_for_backward({qkv, o, lse, cu_seqlens, offset_tensor.has_value() ? offset_tensor->clone() : at::Tensor()});
-    ctx->saved_data["max_seqlen"] = max_seqlen;
-    ctx->saved_data["p_drop"] = p_drop;
-    ctx->saved_data["seed"] = seed;
-    ctx->saved_data["offset"] = offset;
-    ctx->saved_data["has_scale"] = scale.has_value();
-    ctx->saved_data["scale"] = scale.has_value() ? *scale : 0.0;
-    return o;
-  }
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
-                                                 torch::autograd::variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    c10::optional<double> scale;
-    if (ctx->saved_data["has_scale"].toBool()) scale = ctx->saved_data["scale"].toDouble();
-    c10::optional<at::Tensor> offset_tensor;
-    if (saved[4].defined()) offset_tensor = saved[4];
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_varlen_qkvpacked_bwd", "")
-                         .typed<at::Tensor(const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
-                                           const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
-                                           const c10::optional<at::Tensor>&)>();
-    at::Tensor dqkv = op.call(grads[0].contiguous(), saved[0], saved[1], saved[2], saved[3],
-                              ctx->saved_data["max_seqlen"].toInt(), ctx->saved_data["p_drop"].toDouble(),
-                              ctx->saved_data["seed"].toInt(), ctx->saved_data["offset"].toInt(), scale, offset_tensor);
-    return {dqkv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
-  }
-};
-
-at::Tensor fmha_varlen_qkvpacked_autograd(const at::Tensor& qkv, const at::Tensor& cu_seqlens, int64_t max_seqlen,
-                                          double p_drop, int64_t seed, int64_t offset, c10::optional<double> scale,
-                                          const c10::optional<at::Tensor>& offset_tensor) {
-  return FmhaVarlenQkvPackedFunction::apply(qkv, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor);
+template <typename Ret, typename... Args>
+c10::TypedOperatorHandle<Ret(Args...)> find_op(const char* name) {
+  return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Ret(Args...)>();
 }
 
+// Runs `forward` (which returns {o, lse}) below the autograd keys and, if a gradient will be wanted, records a NodeT.
+// `inputs`: the differentiable operands; offset_tensor: the backward pass must see the value the forward pass saw, even
+// if the caller advances the tensor in between, so it gets a private copy.
+template <typename NodeT, size_t N, typename Forward>
+at::Tensor record(const std::array<std::reference_wrapper<const at::Tensor>, N>& inputs, const OptTensor& mask,
+                  const OptTensor& lens, const OptTensor& offset_tensor, int64_t max_seqlen, double p_drop, int64_t seed,
+                  int64_t offset, c10::optional<double> scale, Forward forward) {
+  bool wanted = mask.has_value() && mask->requires_grad();
+  for (const at::Tensor& t : inputs) {
+    wanted = wanted || t.requires_grad();
+    TORCH_CHECK(!t._fw_grad(0).defined(), "mha_manual: forward-mode derivatives are not implemented");
+  }
+  wanted = wanted && at::GradMode::is_enabled();
+  std::shared_ptr<NodeT> node;
+  if (wanted) {
+    node = std::shared_ptr<NodeT>(new NodeT(), torch::autograd::deleteNode);
+    torch::autograd::edge_list edges;
+    edges.reserve(N + 1);
+    for (const at::Tensor& t : inputs) edges.push_back(torch::autograd::impl::gradient_edge(t));
+    if (mask.has_value()) edges.push_back(torch::autograd::impl::gradient_edge(*mask));
+    node->set_next_edges(std::move(edges));
+  }
+  at::Tensor o, lse;
+  {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    std::tie(o, lse) = forward();
+    if (wanted && offset_tensor.has_value()) {
+      node->offset_tensor = SavedVariable(offset_tensor->clone(), false);
+      node->has_offset_tensor = true;
+    }
+  }
+  if (wanted) {
+    torch::autograd::set_history(o, node);
+    for (size_t i = 0; i < N; ++i) node->in[i] = SavedVariable(inputs[i].get(), false);
+    node->o = SavedVariable(o, true);
+    node->lse = SavedVariable(lse, false);
+    if ((node->has_mask = mask.has_value())) node->mask = SavedVariable(*mask, false);
+    if ((node->has_lens = lens.has_value())) node->lens = SavedVariable(*lens, false);
+    node->max_seqlen = max_seqlen;
+    node->p_drop = p_drop;
+    node->seed = seed;
+    node->offset = offset;
+    node->scale = scale;
+  }
+  return o;
+}
+
+using Pair = std::tuple<at::Tensor, at::Tensor>;
+using Triple = std::tuple<at::Tensor, at::Tensor, at::Tensor>;
+using TensorRef = std::reference_wrapper<const at::Tensor>;
+
+struct FmhaBackward final : AttnNode {
+  std::string name() const override { return "FmhaBackward"; }
+  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+    static auto op = find_op<Triple, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                             const at::Tensor&, const OptTensor&, const OptTensor&, double, int64_t, int64_t,
+                             c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_bwd");
+    auto [dq, dk, dv] = op.call(d_o, in[0].unpack(), in[1].unpack(), in[2].unpack(), out, lse.unpack(), opt(mask, has_mask),
+                                opt(lens, has_lens), p_drop, seed, offset, scale, 0, opt(offset_tensor, has_offset_tensor));
+    return {dq, dk, dv};
+  }
+};
+at::Tensor fmha_autograd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const OptTensor& mask,
+                         const OptTensor& seqlens, double p_drop, int64_t seed, int64_t offset, c10::optional<double> scale,
+                         const OptTensor& offset_tensor) {
+  // through the dispatcher, so that fake / meta tensors reach the shape-only kernels
+  static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, const at::Tensor&, const OptTensor&, const OptTensor&,
+                           double, int64_t, int64_t, c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_fwd");
+  return record<FmhaBackward, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset,
+                                 scale, [&] { return op.call(q, k, v, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor); });
+}
+
+struct FmhaQkvPackedBackward final : AttnNode {
+  std::string name() const override { return "FmhaQkvPackedBackward"; }
+  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+    static auto op = find_op<at::Tensor, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                             const OptTensor&, const OptTensor&, double, int64_t, int64_t, c10::optional<double>, int64_t,
+                             const OptTensor&>("mha_manual::fmha_qkvpacked_bwd");
+    return {op.call(d_o, in[0].unpack(), out, lse.unpack(), opt(mask, has_mask), opt(lens, has_lens), p_drop, seed, offset, scale, 0,
+                    opt(offset_tensor, has_offset_tensor))};
+  }
+};
+at::Tensor fmha_qkvpacked_autograd(const at::Tensor& qkv, const OptTensor& mask, const OptTensor& seqlens, double p_drop,
+                                   int64_t seed, int64_t offset, c10::optional<double> scale, const OptTensor& offset_tensor) {
+  static auto op = find_op<Pair, const at::Tensor&, const OptTensor&, const OptTensor&, double, int64_t, int64_t,
+                           c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_qkvpacked_fwd");
+  return record<FmhaQkvPackedBackward, 1>({TensorRef(qkv)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset, scale, [&] {
+    return op.call(qkv, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor);
+  });
+}
+
+struct FmhaVarlenBackward final : AttnNode {
+  std::string name() const override { return "FmhaVarlenBackward"; }
+  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+    static auto op = find_op<Triple, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                             const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
+                             const OptTensor&>("mha_manual::fmha_varlen_bwd");
+    auto [dq, dk, dv] = op.call(d_o, in[0].unpack(), in[1].unpack(), in[2].unpack(), out, lse.unpack(), lens.unpack(), max_seqlen,
+                                p_drop, seed, offset, scale, opt(offset_tensor, has_offset_tensor));
+    return {dq, dk, dv};
+  }
+};
 at::Tensor fmha_varlen_autograd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_seqlens,
                                 int64_t max_seqlen, double p_drop, int64_t seed, int64_t offset, c10::optional<double> scale,
-                                const c10::optional<at::Tensor>& offset_tensor) {
-  return FmhaVarlenFunction::apply(q, k, v, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor);
+                                const OptTensor& offset_tensor) {
+  static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t, double,
+                           int64_t, int64_t, c10::optional<double>, const OptTensor&>("mha_manual::fmha_varlen_fwd");
+  return record<FmhaVarlenBackward, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen,
+                                       p_drop, seed, offset, scale,
+                                       [&] { return op.call(q, k, v, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor); });
 }
 
-class FmhaQkvPackedFunction : public torch::autograd::Function<FmhaQkvPackedFunction> {
- public:
-  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& qkv,
-                            const c10::optional<at::Tensor>& mask, const c10::optional<at::Tensor>& seqlens, double p_drop,
-                            int64_t seed, int64_t offset, c10::optional<double> scale,
-                            const c10::optional<at::Tensor>& offset_tensor) {
-    at::AutoDispatchBelowADInplaceOrView guard;
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_qkvpacked_fwd", "")
-                         .typed<std::tuple<at::Tensor, at::Tensor>(const at::Tensor&, const c10::optional<at::Tensor>&,
-                                                                   const c10::optional<at::Tensor>&, double, int64_t, int64_t,
-                                                                   c10::optional<double>, int64_t,
-                                                                   const c10::optional<at::Tensor>&)>();
-    auto [o, lse] = op.call(qkv, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor);
-    ctx->save_for_backward({qkv, o, lse, mask.has_value() ? *mask : at::Tensor(),
-                            seqlens.has_value() ? *seqlens : at::Tensor(),
-                            offset_tensor.has_value() ? offset_tensor->clone() : at::Tensor()});
-    ctx->saved_data["p_drop"] = p_drop;
-    ctx->saved_data["seed"] = seed;
-    ctx->saved_data["offset"] = offset;
-    ctx->saved_data["has_scale"] = scale.has_value();
-    ctx->saved_data["scale"] = scale.has_value() ? *scale : 0.0;
-    return o;
-  }
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
-                                                 torch::autograd::variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    c10::optional<at::Tensor> mask, seqlens, offset_tensor;
-    if (saved[3].defined()) mask = saved[3];
-    if (saved[4].defined()) seqlens = saved[4];
-    if (saved[5].defined()) offset_tensor = saved[5];
-    c10::optional<double> scale;
-    if (ctx->saved_data["has_scale"].toBool()) scale = ctx->saved_data["scale"].toDouble();
-    static auto op = c10::Dispatcher::singleton()
-                         .findSchemaOrThrow("mha_manual::fmha_qkvpacked_bwd", "")
-                         .typed<at::Tensor(const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
-                                           const c10::optional<at::Tensor>&, const c10::optional<at::Tensor>&, double, int64_t,
-                                           int64_t, c10::optional<double>, int64_t, const c10::optional<at::Tensor>&)>();
-    at::Tensor dqkv = op.call(grads[0].contiguous(), saved[0], saved[1], saved[2], mask, seqlens,
-                              ctx->saved_data["p_drop"].toDouble(), ctx->saved_data["seed"].toInt(),
-                              ctx->saved_data["offset"].toInt(), scale, 0, offset_tensor);
-    return {dqkv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+struct FmhaVarlenQkvPackedBackward final : AttnNode {
+  std::string name() const override { return "FmhaVarlenQkvPackedBackward"; }
+  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+    static auto op = find_op<at::Tensor, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
+                             const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>, const OptTensor&>(
+        "mha_manual::fmha_varlen_qkvpacked_bwd");
+    return {op.call(d_o, in[0].unpack(), out, lse.unpack(), lens.unpack(), max_seqlen, p_drop, seed, offset, scale,
+                    opt(offset_tensor, has_offset_tensor))};
   }
 };
-
-at::Tensor fmha_qkvpacked_autograd(const at::Tensor& qkv, const c10::optional<at::Tensor>& mask,
-                                   const c10::optional<at::Tensor>& seqlens, double p_drop, int64_t seed, int64_t offset,
-                                   c10::optional<double> scale, const c10::optional<at::Tensor>& offset_tensor) {
-  return FmhaQkvPackedFunction::apply(qkv, mask, seqlens, p_drop, seed, offset, scale, offset_tensor);
-}
-
-at::Tensor fmha_autograd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
-                         const c10::optional<at::Tensor>& mask, const c10::optional<at::Tensor>& seqlens, double p_drop,
-                         int64_t seed, int64_t offset, c10::optional<double> scale,
-                         const c10::optional<at::Tensor>& offset_tensor) {
-  return FmhaFunction::apply(q, k, v, mask, seqlens, p_drop, seed, offset, scale, offset_tensor);
+at::Tensor fmha_varlen_qkvpacked_autograd(const at::Tensor& qkv, const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop,
+                                          int64_t seed, int64_t offset, c10::optional<double> scale,
+                                          const OptTensor& offset_tensor) {
+  static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
+                           const OptTensor&>("mha_manual::fmha_varlen_qkvpacked_fwd");
+  return record<FmhaVarlenQkvPackedBackward, 1>({TensorRef(qkv)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen, p_drop, seed,
+                                                offset, scale,
+                                                [&] { return op.call(qkv, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor); });
 }
 
 // The same four operators below the autograd keys (torch.inference_mode(), a redispatch from another autograd

@@ -242,3 +242,32 @@ def test_sequence_longer_than_max_seqlen_is_cut_not_spilled(cuda_device):
     g = ops.fmha_varlen_bwd(d_o, q, k, v, o2, lse2, cu, max_len)
     assert (o2[406:450] == 0).all() and all((t[406:450] == 0).all() for t in g)
     helpers.assert_close(g[0][keep_rows], ref["dq"], "dq (operator)", dtype)
+
+
+@pytest.mark.parametrize("lens,gap,tail,max_len", [([150, 300, 90], 0, 0, 256), ([40, 130], 7, 33, 128), ([128], 1, 0, 128), ([0, 5], 0, 9, 64)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_operators_zero_the_rows_no_tile_covers(cuda_device, lens, gap, tail, max_len, D):
+    """Rows past max_seqlen of their sequence and rows outside all sequences are zeros whatever the memory held before
+    (blocks of NaN are handed back to the caching allocator first); every other row is finite."""
+    import mha_manual  # noqa: F401
+    H, total = 3, gap + sum(lens) + tail
+    q, k, v, d_o = (torch.randn(total, H, D, device=cuda_device).half() for _ in range(4))
+    cu = [gap]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    covered = torch.zeros(total, dtype=torch.bool)
+    for i, n in enumerate(lens):
+        covered[cu[i]:cu[i] + min(n, max_len)] = True
+    cu = torch.tensor(cu, dtype=torch.int32, device=cuda_device)
+    ops = torch.ops.mha_manual
+
+    def poison():
+        x = [torch.full_like(q, float("nan")) for _ in range(8)]
+        del x
+
+    poison()
+    o, lse = ops.fmha_varlen_fwd(q, k, v, cu, max_len)
+    poison()
+    for t in (o, *ops.fmha_varlen_bwd(d_o, q, k, v, o, lse, cu, max_len)):
+        t = t.cpu()
+        assert (t[~covered] == 0).all() and torch.isfinite(t[covered]).all()
