@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "../../include/fmha_sm100.h"
@@ -45,6 +46,8 @@ constexpr int kThreadsSplit = 192, kThreadsMerged = 160;
 template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged : kThreadsSplit; }
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr float kLn2F = 0.6931471805599453f;
+
+constexpr int kMaxKeySplit = 8;   // portable cluster size
 
 enum FastWaitSite {
   kFQFull = 111, kFKEmpty = 112, kFVEmpty = 113, kFKFull = 114, kFVFull = 115, kFPFull = 116, kFSFull = 117,
@@ -116,7 +119,10 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t (&r)[32], int cbase
 
 // PACKED: the batch is one [total_rows, H, D] tensor per operand with row offsets (FMHA_MASK_CU_SEQLENS); a
 // template parameter so that the padded kernels carry none of its bookkeeping in registers.
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
+// SPLIT: the keys of a query tile are dealt out over the CTAs of a cluster (see fwd_key_split); each runs its share of
+// the key steps and leaves its unnormalised O, row maximum and row sum in its own shared memory, and the cluster
+// combines them through distributed shared memory.
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool SPLIT = false>
 __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPerSm) fmha_fwd_fast_kernel(const __grid_constant__ FwdArgs a) {
   griddep_wait();
   constexpr bool MERGED = (D == 64);          // one warp issues the loads and the MMAs
@@ -156,7 +162,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   const int lane = threadIdx.x & 31;
   const int h = blockIdx.y;
   const int b = blockIdx.z;
-  const int q0 = blockIdx.x * kTileM;
+  const int n_split = SPLIT ? static_cast<int>(cluster_size()) : 1;
+  const int split = SPLIT ? static_cast<int>(cluster_rank()) : 0;
+  const int q0 = (SPLIT ? blockIdx.x / n_split : blockIdx.x) * kTileM;
   const int bh = b * a.H + h;
 
   int k_limit = a.S_k;
@@ -178,7 +186,10 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       zero_uncovered_rows(a.o_ptr, a.o_ss, a.o_sh, h, b, a.B, cu, a.S_q, a.total_rows, D, threadIdx.x, blockDim.x);
     if (q0 >= len) return;   // this sequence has no such query tile (whole CTA, before any barrier)
   }
-  const int n_kv = (k_limit + TN - 1) / TN;
+  const int n_kv_all = (k_limit + TN - 1) / TN;
+  // key steps of this CTA: [j0, j0 + n_kv); with SPLIT possibly none
+  const int j0 = SPLIT ? n_kv_all * split / n_split : 0;
+  const int n_kv = SPLIT ? n_kv_all * (split + 1) / n_split - j0 : n_kv_all;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -221,12 +232,12 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
         mbar_arrive_expect_tx(k_full + s, L::kTileBytes);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c)
-          tma_load_4d(sK + s * L::kTileBytes + c * L::kSubTile, &a.tm_k, k_full + s, c * 64, row_base + j * TN, h, tb);
+          tma_load_4d(sK + s * L::kTileBytes + c * L::kSubTile, &a.tm_k, k_full + s, c * 64, row_base + (j0 + j) * TN, h, tb);
         if (j >= ST) mbar_wait(v_empty + s, ((j / ST) - 1) & 1, wctx, kFVEmpty);
         mbar_arrive_expect_tx(v_full + s, L::kTileBytes);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c)
-          tma_load_4d(sV + s * L::kTileBytes + c * L::kSubTile, &a.tm_v, v_full + s, c * 64, row_base + j * TN, h, tb);
+          tma_load_4d(sV + s * L::kTileBytes + c * L::kSubTile, &a.tm_v, v_full + s, c * 64, row_base + (j0 + j) * TN, h, tb);
       }
     }
   } else if (warp == 0 && MERGED) {
@@ -246,12 +257,12 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       auto load_k = [&](int j) {
         const int s = j % ST;
         mbar_arrive_expect_tx(k_full + s, L::kTileBytes);
-        tma_load_4d(sK + s * L::kTileBytes, &a.tm_k, k_full + s, 0, row_base + j * TN, h, tb);
+        tma_load_4d(sK + s * L::kTileBytes, &a.tm_k, k_full + s, 0, row_base + (j0 + j) * TN, h, tb);
       };
       auto load_v = [&](int j) {
         const int s = j % ST;
         mbar_arrive_expect_tx(v_full + s, L::kTileBytes);
-        tma_load_4d(sV + s * L::kTileBytes, &a.tm_v, v_full + s, 0, row_base + j * TN, h, tb);
+        tma_load_4d(sV + s * L::kTileBytes, &a.tm_v, v_full + s, 0, row_base + (j0 + j) * TN, h, tb);
       };
       if (elect_one()) {
         mbar_arrive_expect_tx(q_full, L::kQBytes);
@@ -361,11 +372,15 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     const float sl2 = a.scale_log2;
     const uint32_t gbh = static_cast<uint32_t>(a.philox_bh_offset + bh);
 
+    // Rows past the end are never stored, so a warp that has only such rows (a ragged last tile; a handful of query
+    // rows against long keys) leaves P and O undefined instead of spending special-function time on them.
+    const bool warp_idle = q0 + quad * 32 >= q_limit;
+
     float m_ref = -INFINITY;
     float2 sum2 = make_float2(0.f, 0.f);  // running sum of exp2(t - m_ref), two interleaved partial sums
 
     for (int j = 0; j < n_kv; ++j) {
-      const int col0 = j * TN;
+      const int col0 = (j0 + j) * TN;
       const int n_cols = min(TN, k_limit - col0);
       const float* mask_stage = sMask + (j & 1) * TN;
       if constexpr (KEYADD) {
@@ -374,6 +389,11 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           sMask[(j & 1) * TN + tid] =
               (c < a.S_k) ? reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(b) * a.S_k + c] * kLog2eF : 0.f;
         named_bar_sync(1, 128);
+      }
+      if (warp_idle) {   // no query row of this warp exists: only keep the step's barriers in phase
+        mbar_wait(s_full, j & 1, wctx, kFSFull, 32);
+        mbar_arrive(p_full);
+        continue;
       }
       // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
       // before they are awaited, while the tensor core is still busy with Q K^T.
@@ -478,6 +498,29 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     mbar_wait(o_full, 0, wctx, kFOFull, 32);
     tc_fence_after_sync();
     const float l_sum = sum2.x + sum2.y;
+    if constexpr (SPLIT) {
+      // this CTA's share of the row: [128][D] fp32 over the K and V buffers (every load has been consumed) with the
+      // 16-byte chunks of a row XORed by the row, so that the 32 rows of a warp spread over the banks; statistics
+      // where Q was
+      float2* stats = reinterpret_cast<float2*>(sQ);
+      stats[row] = make_float2(m_ref, l_sum);
+      uint8_t* part = sK + row * (D * 4);
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t r[32];
+        if (n_kv > 0) {   // with no key step nothing has been accumulated
+          tmem_ld32(tO + c * 32, r);
+          tmem_wait_ld_dep(r);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) r[k] = 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<uint4*>(part + (((c * 8 + q) ^ (row & 7)) << 4)) =
+              make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
+      }
+    } else {
     const float out_scale = (DROP ? a.dropout_scale : 1.0f) / l_sum;
     if (a.lse != nullptr && row_ok) {
       const size_t li = packed ? static_cast<size_t>(h) * a.total_rows + row_base + q_row   // [H, total_rows]
@@ -519,10 +562,60 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       }
       tma_store_wait_read();  // the shared-memory source must outlive the copy; the writes finish on their own
     }
+    }
   }
 
   tc_fence_before_sync();
   __syncthreads();
+  if constexpr (SPLIT) {
+    // ============================ combine the cluster's shares ======================
+    // Work: (query row, 8 columns) pairs, dealt out over all threads of the cluster; every thread reads the row's
+    // statistics and its 8 columns of every share.  No wait precedes the cluster barriers that is not bounded, so
+    // every CTA arrives, also after a wait was given up.
+    cluster_sync();
+    const int rows = min(kTileM, q_limit - q0);
+    const int items = *abort_flag ? 0 : rows * (D / 8);
+    const uint32_t stats_addr = smem_u32(sQ), part_addr = smem_u32(sK);
+    for (int i = split * blockDim.x + threadIdx.x; i < items; i += n_split * blockDim.x) {
+      const int row = i / (D / 8), ch = i % (D / 8);
+      float m[kMaxKeySplit], l[kMaxKeySplit];
+      float m_all = -INFINITY, l_all = 0.f;
+#pragma unroll
+      for (int k = 0; k < kMaxKeySplit; ++k) {
+        const float2 st = k < n_split ? dsmem_ld2(dsmem_map(stats_addr + row * 8, k)) : make_float2(-INFINITY, 0.f);
+        m[k] = st.x;
+        l[k] = st.y;
+        m_all = fmaxf(m_all, m[k]);
+      }
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < kMaxKeySplit; ++k) {
+        if (k >= n_split) break;
+        const float w = fast_exp2(m[k] - m_all);   // 0 for a share without key steps
+        l_all = fmaf(w, l[k], l_all);
+        const uint32_t src = dsmem_map(part_addr + row * (D * 4), k);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float4 x = dsmem_ld4(src + (((ch * 2 + q) ^ (row & 7)) << 4));
+          acc[q * 4 + 0] = fmaf(w, x.x, acc[q * 4 + 0]);
+          acc[q * 4 + 1] = fmaf(w, x.y, acc[q * 4 + 1]);
+          acc[q * 4 + 2] = fmaf(w, x.z, acc[q * 4 + 2]);
+          acc[q * 4 + 3] = fmaf(w, x.w, acc[q * 4 + 3]);
+        }
+      }
+      const float out_scale = (DROP ? a.dropout_scale : 1.0f) / l_all;
+      uint4 w4;
+      w4.x = pack2<BF16>(acc[0] * out_scale, acc[1] * out_scale);
+      w4.y = pack2<BF16>(acc[2] * out_scale, acc[3] * out_scale);
+      w4.z = pack2<BF16>(acc[4] * out_scale, acc[5] * out_scale);
+      w4.w = pack2<BF16>(acc[6] * out_scale, acc[7] * out_scale);
+      *reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.o_ptr) + b * a.o_sb + h * a.o_sh +
+                                static_cast<int64_t>(q0 + row) * a.o_ss + ch * 8) = w4;
+      if (ch == 0 && a.lse != nullptr)
+        a.lse[static_cast<size_t>(bh) * a.S_q + q0 + row] = (m_all + fast_log2(l_all)) * kLn2F;
+    }
+    cluster_sync();   // no CTA leaves while another one reads its shared memory
+  }
   if (*abort_flag) {
     for (int k = 0; k < 20; ++k) __nanosleep(1000000);
     __syncthreads();
@@ -533,10 +626,38 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   }
 }
 
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
-static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream) {
+// Over how many CTAs of a cluster the keys of a query tile are split: the candidate (1, 2, 4, 8) of least modelled time,
+// in units of one key step of a CTA that has its SM to itself (1.1 us at D = 64, 1.9 us at D = 128, measured: there a
+// step is a chain of latencies, as long for one query row as for 128).  A step slows down in proportion to the CTAs per
+// SM once they compete for the special-function unit (`load`; a tile of at most 32 rows keeps one warp of four busy),
+// and a split adds the cluster launch, its barriers and the combination (`overhead`: measured 1.1 us for one query row,
+// 4 us for 128).  More than two CTAs per SM never paid.  Measured: B=2 H=16 S_q=1 S_k=4096 D=128 60.6 -> 17.3 us (8
+// shares), D=64 71.7 -> 15.6 us; B=8 H=8 S_q=20 S_k=1000 D=64 20.1 -> 10.9 us (4); B=1 H=12 S=1024 D=64 20.4 -> 17.9 us (2).
+static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, int sms) {
+  const bool few_rows = S_q <= 32;
+  const float overhead = D == 64 ? (few_rows ? 1.5f : 4.0f) : (few_rows ? 1.0f : 2.2f);
+  const float load = few_rows ? 0.5f : D == 64 ? 0.95f : 1.3f;
+  int best = 1;
+  float best_cost = static_cast<float>(steps) * std::max(1.0f, load * ctas / sms);
+  for (int s = 2; s <= kMaxKeySplit && ctas * s <= 2 * static_cast<int64_t>(sms) && s < 2 * steps; s *= 2) {
+    const float cost = static_cast<float>((steps + s - 1) / s) * std::max(1.0f, load * ctas * s / sms) + overhead;
+    if (cost < best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool SPLIT = false>
+static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream, int n_split = 1) {
   using L = FastSmem<D>;
-  auto kfn = fmha_fwd_fast_kernel<D, BF16, KEYADD, DROP, PACKED>;
+  if constexpr (!PACKED && !SPLIT) {
+    const int s = fwd_key_split(static_cast<int64_t>((a.S_q + kTileM - 1) / kTileM) * a.H * a.B, (a.S_k + L::TN - 1) / L::TN, a.S_q, D,
+                                sm_count());
+    if (s > 1) return launch_fast_impl<D, BF16, KEYADD, DROP, false, true>(a, stream, s);
+  }
+  auto kfn = fmha_fwd_fast_kernel<D, BF16, KEYADD, DROP, PACKED, SPLIT>;
   static std::atomic<bool> configured[64] = {};   // per device; set after the attribute call succeeded
   int dev = 0;
   cudaGetDevice(&dev);
@@ -545,8 +666,8 @@ static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  dim3 grid((a.S_q + kTileM - 1) / kTileM, a.H, a.B);
-  const cudaError_t e = launch_overlapped(kfn, grid, dim3(fast_threads<D>()), L::kDynBytes, stream, a);
+  dim3 grid((a.S_q + kTileM - 1) / kTileM * n_split, a.H, a.B);
+  const cudaError_t e = launch_overlapped(kfn, grid, dim3(fast_threads<D>()), L::kDynBytes, stream, a, SPLIT ? n_split : 0);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/fmha_sm100.h"
 #include "philox.cuh"
 
@@ -114,22 +116,40 @@ int launch_bwd_prepare(const void* o, const fmha_tensor4& ot, const fmha_tensor4
 int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int D, int dtype,
                       float scale, const int* cu_seqlens, cudaStream_t stream);
 
+// Multiprocessors of the current device, asked for once per device.
+inline int sm_count() {
+  static std::atomic<int> count[64] = {};
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && (n = count[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev >= 0 && dev < 64) count[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // Launches `kernel` with programmatic stream serialization: its CTAs may be scheduled while the previous
 // kernel of the stream drains (which hides the launch latency between the kernels of a training step); the
 // kernel itself calls griddep_wait() before it touches global memory, so stream order is preserved.
 template <typename Arg>
 inline cudaError_t launch_overlapped(void (*kernel)(Arg), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream,
-                                     const Arg& arg) {
+                                     const Arg& arg, int cluster_x = 0) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (cluster_x > 0) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster_x);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, arg);
 }
 

@@ -159,6 +159,43 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
 }
 
 // ------------------------------------------------------------------------------------
+// thread-block clusters and distributed shared memory
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctaid.x;" : "=r"(r));
+  return r;
+}
+// Barrier over all threads of the cluster; shared-memory writes before it are visible to the cluster after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile(
+      "barrier.cluster.arrive.release.aligned;\n\t"
+      "barrier.cluster.wait.acquire.aligned;"
+      ::: "memory");
+}
+// Address of this CTA's shared-memory location `saddr` in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t dsmem_map(uint32_t saddr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float2 dsmem_ld2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 dsmem_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// ------------------------------------------------------------------------------------
 // TMA: 4-D tiled loads and stores. coordinates are (c0 innermost .. c3 outermost)
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {

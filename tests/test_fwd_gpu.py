@@ -188,3 +188,33 @@ def test_bounded_wait_reports_instead_of_hanging(cuda_device):
     o, _ = api.fmha_forward(q, k, v, status=status)
     ref, *_ = helpers.oracle_forward(q, k, v)
     helpers.assert_close(o, ref["o"], "o after timeout")
+
+
+@pytest.mark.parametrize("B,H,S_q,S_k,D,dtype", [
+    (1, 1, 1, 1024, 64, torch.float16),     # one query row, 8 shares of two 64-key steps
+    (1, 2, 31, 1000, 64, torch.bfloat16),   # one warp of rows, a ragged last step
+    (2, 2, 33, 900, 128, torch.bfloat16),   # the second warp has a single row
+    (1, 1, 1, 300, 128, torch.float16),     # more shares than key steps: one of them is empty
+    (1, 2, 130, 1536, 128, torch.float16),  # two query tiles, the second with two rows
+    (1, 3, 128, 2048, 64, torch.float16),   # a full tile
+])
+@pytest.mark.parametrize("mask,p_drop", [("none", 0.0), ("seqlen", 0.1), ("key", 0.0), ("key", 0.1)])
+def test_keys_split_over_a_cluster(cuda_device, B, H, S_q, S_k, D, dtype, mask, p_drop):
+    """Few CTAs against long keys: the keys of a query tile are dealt out over a cluster whose CTAs combine their
+    shares.  Valid lengths down to a single key leave shares without any key step.  (bf16: 130 keys, two to three steps;
+    a result of one key is that key's value rounded once, up to 2^-8 of it off, which is outside assert_close's bf16 bar of
+    2e-3 on 99.5 % of the elements: it presumes sums of at least 128 keys.)"""
+    q, k, v, _, _ = helpers.randn_like_config(B, H, S_q, S_k, D, dtype, seed=S_q + S_k, device=cuda_device)
+    lens = torch.tensor([1 if dtype == torch.float16 else 130, S_k // 2 + 3][:B], dtype=torch.int32, device=cuda_device)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    kw, okw = {}, {}
+    if mask == "seqlen":
+        kw["seqlens"], okw["lens"] = lens, lens
+    elif mask == "key":
+        add = torch.randn(B, S_k, generator=torch.Generator().manual_seed(3)).to(cuda_device)
+        kw["mask"], okw["add_mask"] = add, add
+    o, lse = api.fmha_forward(q, k, v, p_drop=p_drop, seed=21, offset=4, status=status, **kw)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    ref, *_ = helpers.oracle_forward(q, k, v, p_drop=p_drop, seed=21, offset=4, **okw)
+    helpers.assert_close(o, ref["o"], "o", dtype)
+    helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
