@@ -47,6 +47,11 @@ template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged 
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr float kLn2F = 0.6931471805599453f;
 
+// Additive key mask, in the log2 domain: a key at or above kDeadMask may matter (scores of N(0,1) rows are a few units,
+// a padding mask is -10000 * log2e), a step with only keys below it is looked at for a shortcut; exp2(x) is zero in fp32,
+// flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.
+constexpr float kDeadMask = -1000.0f;
+constexpr float kZeroExp = -200.0f;
 constexpr int kMaxKeySplit = 8;   // portable cluster size
 
 enum FastWaitSite {
@@ -77,28 +82,18 @@ struct FastSmem {
   static constexpr int kDynBytes = kBytes + 1024;
 };
 
-// One 32-column chunk of the second sweep: r holds raw accumulators of columns
-// [cbase, cbase+32); produces 16 packed 16-bit pairs of exp2(t - m_ref) (dropout applied) and
+// 32 columns of a row: t holds their scores; produces 16 packed 16-bit pairs of exp2(t - m_ref) (dropout applied) and
 // adds the undropped values to sum2.
-template <bool BF16, bool KEYADD, bool DROP, bool BOUNDARY>
-__device__ __forceinline__ void softmax_chunk(const uint32_t (&r)[32], int cbase, int n_cols, float sl2, float neg_m,
-                                              const float* mask_stage, float2& sum2, uint32_t (&packed)[16],
-                                              const uint32_t* keepw) {
+template <bool BF16, bool KEYADD, bool DROP>
+__device__ __forceinline__ void softmax_chunk(const uint32_t (&t)[32], float sl2, float neg_m, float2& sum2,
+                                              uint32_t (&packed)[16], const uint32_t* keepw) {
   const float2 sl22 = make_float2(sl2, sl2);
   const float2 negm2 = make_float2(neg_m, neg_m);
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
-    float2 x = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
-    if constexpr (KEYADD) {
-      const float2 mk = *reinterpret_cast<const float2*>(mask_stage + cbase + 2 * k);
-      x = __fadd2_rn(__ffma2_rn(x, sl22, mk), negm2);
-    } else {
-      x = __ffma2_rn(x, sl22, negm2);
-    }
-    if constexpr (BOUNDARY) {
-      if (cbase + 2 * k >= n_cols) x.x = -INFINITY;
-      if (cbase + 2 * k + 1 >= n_cols) x.y = -INFINITY;
-    }
+    float2 x = make_float2(__uint_as_float(t[2 * k]), __uint_as_float(t[2 * k + 1]));
+    if constexpr (KEYADD) x = __fadd2_rn(x, negm2);
+    else x = __ffma2_rn(x, sl22, negm2);
     float2 p;
     p.x = fast_exp2(x.x);
     p.y = fast_exp2(x.y);
@@ -106,7 +101,7 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t (&r)[32], int cbase
     packed[k] = pack2<BF16>(p.x, p.y);
   }
   if constexpr (DROP) {
-    // keepw[i]: bit 7 of byte e = keep decision of column cbase + 4*i + e; the permutes replicate it over a 16-bit lane
+    // keepw[i]: bit 7 of byte e = keep decision of column 4*i + e; the permutes replicate it over a 16-bit lane
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       packed[2 * i] &= prmt(keepw[i], 0u, 0x9988u);
@@ -372,9 +367,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     const float sl2 = a.scale_log2;
     const uint32_t gbh = static_cast<uint32_t>(a.philox_bh_offset + bh);
 
-    // Rows past the end are never stored, so a warp that has only such rows (a ragged last tile; a handful of query
-    // rows against long keys) leaves P and O undefined instead of spending special-function time on them.
-    const bool warp_idle = q0 + quad * 32 >= q_limit;
+    // Rows past the end are never stored, so with a handful of query rows against long keys a warp that has no row
+    // leaves P and O undefined instead of competing with the others.  (No gain at a ragged last tile of a full grid.)
+    const bool warp_idle = SPLIT && q0 + quad * 32 >= q_limit;
 
     float m_ref = -INFINITY;
     float2 sum2 = make_float2(0.f, 0.f);  // running sum of exp2(t - m_ref), two interleaved partial sums
@@ -383,12 +378,15 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       const int col0 = (j0 + j) * TN;
       const int n_cols = min(TN, k_limit - col0);
       const float* mask_stage = sMask + (j & 1) * TN;
+      bool live = true;   // additive mask: some key of this step is not masked away
       if constexpr (KEYADD) {
         const int c = col0 + tid;
-        if (tid < TN)
-          sMask[(j & 1) * TN + tid] =
-              (c < a.S_k) ? reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(b) * a.S_k + c] * kLog2eF : 0.f;
-        named_bar_sync(1, 128);
+        float mk = -INFINITY;
+        if (tid < TN) {
+          mk = c < a.S_k ? reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(b) * a.S_k + c] * kLog2eF : 0.f;
+          sMask[(j & 1) * TN + tid] = mk;
+        }
+        live = named_bar_or(1, 128, tid < TN && c < a.S_k && !(mk < kDeadMask));
       }
       if (warp_idle) {   // no query row of this warp exists: only keep the step's barriers in phase
         mbar_wait(s_full, j & 1, wctx, kFSFull, 32);
@@ -398,7 +396,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
       // before they are awaited, while the tensor core is still busy with Q K^T.
       [[maybe_unused]] uint32_t keepw[DROP ? TN / 4 : 1];
-      if constexpr (DROP) {
+      auto draw_keep_words = [&]() {
         const uint32_t kb0 = static_cast<uint32_t>(col0 / 16);
         const uint32_t poff = *philox_off;
 #pragma unroll
@@ -409,42 +407,68 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           keepw[d * 4 + 2] = (draw.z & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
           keepw[d * 4 + 3] = (draw.w & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
         }
+      };
+      if constexpr (DROP) {
+        if (live) draw_keep_words();
       }
       mbar_wait(s_full, j & 1, wctx, kFSFull, 32);
       tc_fence_after_sync();
 
-      // ---- sweep 1: row maximum --------------------------------------------------------
+      // ---- scores into registers (raw, or scaled and masked with an additive mask), row maximum --------------------
+      uint32_t sv[TN / 32][32];
+#pragma unroll
+      for (int c = 0; c < TN / 32; ++c) tmem_ld32(tS + c * 32, sv[c]);
+#pragma unroll
+      for (int c = 0; c < TN / 32; ++c) tmem_wait_ld_dep(sv[c]);
+      if constexpr (KEYADD) {
+#pragma unroll
+        for (int c = 0; c < TN / 32; ++c)
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const float2 mk = *reinterpret_cast<const float2*>(mask_stage + c * 32 + 2 * k);
+            const float2 t = __ffma2_rn(make_float2(__uint_as_float(sv[c][2 * k]), __uint_as_float(sv[c][2 * k + 1])),
+                                        make_float2(sl2, sl2), mk);
+            sv[c][2 * k] = __float_as_uint(t.x);
+            sv[c][2 * k + 1] = __float_as_uint(t.y);
+          }
+      }
+      if (n_cols < TN) {   // keys past the end: exp2 makes them zero
+#pragma unroll
+        for (int c = 0; c < TN / 32; ++c)
+#pragma unroll
+          for (int k = 0; k < 32; ++k)
+            if (c * 32 + k >= n_cols) sv[c][k] = __float_as_uint(-INFINITY);
+      }
       float tile_max = -INFINITY;
-      {
-        uint32_t sv[TN / 32][32];
 #pragma unroll
-        for (int c = 0; c < TN / 32; ++c) tmem_ld32(tS + c * 32, sv[c]);
+      for (int c = 0; c < TN / 32; ++c) {
+        auto v = [&](int k) { return __uint_as_float(sv[c][k]); };
+        float m0 = fmax3(v(0), v(1), v(2));
+        float m1 = fmax3(v(3), v(4), v(5));
 #pragma unroll
-        for (int c = 0; c < TN / 32; ++c) tmem_wait_ld_dep(sv[c]);
-#pragma unroll
-        for (int c = 0; c < TN / 32; ++c) {
-          const int cbase = c * 32;
-          float v[32];
-#pragma unroll
-          for (int k = 0; k < 32; ++k) {
-            v[k] = __uint_as_float(sv[c][k]);
-            if constexpr (KEYADD) v[k] = fmaf(v[k], sl2, mask_stage[cbase + k]);
-          }
-          if (n_cols < TN) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k)
-              if (cbase + k >= n_cols) v[k] = -INFINITY;
-          }
-          float m0 = fmax3(v[0], v[1], v[2]);
-          float m1 = fmax3(v[3], v[4], v[5]);
-#pragma unroll
-          for (int k = 6; k + 3 < 32; k += 4) {
-            m0 = fmax3(m0, v[k], v[k + 1]);
-            m1 = fmax3(m1, v[k + 2], v[k + 3]);
-          }
-          tile_max = fmax3(tile_max, fmax3(m0, m1, v[30]), v[31]);
+        for (int k = 6; k + 3 < 32; k += 4) {
+          m0 = fmax3(m0, v(k), v(k + 1));
+          m1 = fmax3(m1, v(k + 2), v(k + 3));
         }
-        if constexpr (!KEYADD) tile_max *= sl2;  // scale > 0: the maximum commutes with it
+        tile_max = fmax3(tile_max, fmax3(m0, m1, v(30)), v(31));
+      }
+      if constexpr (!KEYADD) tile_max *= sl2;  // scale > 0: the maximum commutes with it
+      // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
+      // the reference maximum that its exponential is zero in fp32, P is zero and nothing else changes.  Decided on the
+      // scores themselves, so the result is the same bits; a third of the steps of a batch with lengths in [S/3, S].
+      if constexpr (KEYADD) {
+        if (!live && __all_sync(0xffffffffu, tile_max - m_ref < kZeroExp)) {
+          const uint32_t zero[16] = {};
+#pragma unroll
+          for (int c = 0; c < TN / 32; ++c) tmem_st16(tS + c * 16, zero);
+          tmem_wait_st();
+          tc_fence_before_sync();
+          mbar_arrive(p_full);
+          continue;
+        }
+        if constexpr (DROP) {
+          if (!live) draw_keep_words();
+        }
       }
       // ---- running reference maximum, lazy rescale of O ------------------------------------
       {
@@ -454,40 +478,25 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
         const float alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - m_new);
         if (j > 0 && __any_sync(0xffffffffu, moved)) {
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld32(tO + c * 32, r);
-            tmem_wait_ld_dep(r);
+          for (int c = 0; c < D / 8; ++c) {   // eight columns at a time: the scores of the step stay in registers meanwhile
+            uint32_t r[8];
+            tmem_ld8(tO + c * 8, r);
+            tmem_wait_ld_dep8(r);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * alpha);
-            tmem_st32(tO + c * 32, r);
+            for (int k = 0; k < 8; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * alpha);
+            tmem_st8(tO + c * 8, r);
           }
         }
         sum2.x *= alpha;
         sum2.y *= alpha;
         m_ref = m_new;
       }
-      // ---- sweep 2: exponentials, dropout, P (next chunk's load in flight) ----------------------
-      {
-        const float neg_m = -m_ref;
-        uint32_t ra[32], rb[32], packed[16];
-        tmem_ld32(tS + 0, ra);
-        auto run = [&](const uint32_t (&r)[32], int c) {
-          if (n_cols >= TN)
-            softmax_chunk<BF16, KEYADD, DROP, false>(r, c * 32, n_cols, sl2, neg_m, mask_stage, sum2, packed, keepw + (DROP ? c * 8 : 0));
-          else
-            softmax_chunk<BF16, KEYADD, DROP, true>(r, c * 32, n_cols, sl2, neg_m, mask_stage, sum2, packed, keepw + (DROP ? c * 8 : 0));
-          tmem_st16(tS + c * 16, packed);
-        };
+      // ---- exponentials, dropout, P over S ---------------------------------------------------------------------
 #pragma unroll
-        for (int c = 0; c < TN / 32; c += 2) {   // chunk c+1 (then c+2) is in flight while chunk c (c+1) is processed
-          tmem_wait_ld_dep(ra);
-          tmem_ld32(tS + (c + 1) * 32, rb);
-          run(ra, c);
-          tmem_wait_ld_dep(rb);
-          if (c + 2 < TN / 32) tmem_ld32(tS + (c + 2) * 32, ra);
-          run(rb, c + 1);
-        }
+      for (int c = 0; c < TN / 32; ++c) {
+        uint32_t packed[16];
+        softmax_chunk<BF16, KEYADD, DROP>(sv[c], sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
+        tmem_st16(tS + c * 16, packed);
       }
       tmem_wait_st();
       tc_fence_before_sync();
