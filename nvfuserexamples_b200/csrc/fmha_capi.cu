@@ -223,7 +223,8 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
   // tensor-map extents: [B, H, S, D], or one "batch" of total_rows rows for a packed batch
   const int mB = packed ? 1 : p->B, mSq = packed ? p->total_rows : p->S_q, mSk = packed ? p->total_rows : p->S_k;
   if ((rc = make_tmap(&a.tm_q, sanitized(p->q, mB, p->H, mSq, p->D), p->dtype, mB, p->H, mSq, p->D, kTileM))) return rc;
-  const int kv_rows = fwd_key_tile(p->D, legacy);
+  const bool rows = !legacy && !packed && fwd_rows_applies(p->S_q);
+  const int kv_rows = rows ? kRowsKeyStep : fwd_key_tile(p->D, legacy);
   if ((rc = make_tmap(&a.tm_k, sanitized(p->k, mB, p->H, mSk, p->D), p->dtype, mB, p->H, mSk, p->D, kv_rows))) return rc;
   if ((rc = make_tmap(&a.tm_v, sanitized(p->v, mB, p->H, mSk, p->D), p->dtype, mB, p->H, mSk, p->D, kv_rows))) return rc;
   if ((rc = make_tmap(&a.tm_o, sanitized(p->o, mB, p->H, mSq, p->D), p->dtype, mB, p->H, mSq, p->D, kTileM))) return rc;
@@ -232,6 +233,8 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
   a.o_ptr = p->o.ptr; a.o_ss = p->o.stride_s; a.o_sh = p->o.stride_h;
   a.o_sb = sanitized(p->o, mB, p->H, mSq, p->D).stride_b;
   a.o_sh = sanitized(p->o, mB, p->H, mSq, p->D).stride_h;
+  const fmha_tensor4 tq = sanitized(p->q, mB, p->H, mSq, p->D);
+  a.q_ptr = tq.ptr; a.q_ss = tq.stride_s; a.q_sh = tq.stride_h; a.q_sb = tq.stride_b;
   a.B = p->B; a.H = p->H; a.S_q = p->S_q; a.S_k = p->S_k;
   a.scale_log2 = p->scale * 1.4426950408889634f;
   a.scale = p->scale;
@@ -283,7 +286,8 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
     a.dmask_tiles = 1;
   }
 
-  const int e = launch_fwd(a, p->D, p->dtype, legacy, p_via_smem, static_cast<cudaStream_t>(stream));
+  const int e = rows ? launch_fwd_rows(a, p->D, p->dtype, static_cast<cudaStream_t>(stream))
+                     : launch_fwd(a, p->D, p->dtype, legacy, p_via_smem, static_cast<cudaStream_t>(stream));
   if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   return FMHA_OK;
 }

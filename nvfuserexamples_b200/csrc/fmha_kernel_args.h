@@ -16,6 +16,7 @@ constexpr int kTileM = 128;  // query rows per CTA tile
 constexpr int kTileN = 128;  // keys per step (general forward kernel, backward kernel)
 // Keys per step of the forward kernel that will run: the production kernel walks the keys in
 // 64-key steps at head dimension 64 (see fmha_fwd_fast_sm100.cu); the TMA box of K and V follows.
+constexpr int kRowsKeyStep = 64;   // keys per step of the kernel for a handful of query rows
 constexpr int fwd_key_tile(int D, bool legacy) { return (!legacy && D == 64) ? 64 : 128; }
 
 struct FwdArgs {
@@ -38,6 +39,8 @@ struct FwdArgs {
   // tensors; o_ptr / strides serve the row-wise stores of a sequence's last, partial query tile
   int total_rows;
   int zero_uncovered;         // FMHA_FLAG_ZERO_UNCOVERED
+  const void* q_ptr;          // the kernel for a handful of query rows reads Q with plain loads
+  int64_t q_ss, q_sh, q_sb;
   void* o_ptr;
   int64_t o_ss, o_sh, o_sb;   // strides in elements (o_sb: dense-mask kernel, which stores O row by row)
   int B, H, S_q, S_k;
@@ -106,6 +109,9 @@ struct UncoveredRows {
 // Launchers (defined in the .cu files).  Return a cudaError_t as int.
 int launch_fwd(const FwdArgs& a, int D, int dtype, bool legacy, bool p_via_smem, cudaStream_t stream);
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
+// the kernel for a handful of query rows per head (fmha_fwd_rows_sm100.cu): compact masks, not packed
+bool fwd_rows_applies(int S_q);
+int launch_fwd_rows(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
 // the persistent kernel of the dense-mask operators at head dimension 64 (fmha_fwd_dense_sm100.cu)
 bool fwd_dense_applies(const FwdArgs& a, int D);
 int launch_fwd_dense(const FwdArgs& a, int dtype, cudaStream_t stream);

@@ -218,3 +218,34 @@ def test_keys_split_over_a_cluster(cuda_device, B, H, S_q, S_k, D, dtype, mask, 
     ref, *_ = helpers.oracle_forward(q, k, v, p_drop=p_drop, seed=21, offset=4, **okw)
     helpers.assert_close(o, ref["o"], "o", dtype)
     helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("B,H,S_q,S_k,D,dtype", [
+    (2, 2, 1, 700, 64, torch.float16),       # one row; shares of a head over a cluster
+    (1, 3, 16, 1000, 128, torch.bfloat16),   # a full 16-row tile, a ragged last step
+    (2, 1, 9, 2049, 128, torch.float16),     # second half of the tile has one row; the last step has one key
+    (1, 1, 15, 130, 64, torch.bfloat16),     # too few steps for shares
+    (160, 1, 3, 200, 64, torch.float16),     # more heads than multiprocessors: no cluster
+])
+@pytest.mark.parametrize("mask,p_drop", [("none", 0.0), ("seqlen", 0.1), ("key", 0.0), ("key", 0.3)])
+def test_a_handful_of_query_rows(cuda_device, B, H, S_q, S_k, D, dtype, mask, p_drop):
+    """At most 16 query rows per head run on their own kernel.  (bf16: at least 130 keys, see
+    test_keys_split_over_a_cluster.)  Strided operands: Q and O as [B,S,H,D], K and V as slices of one tensor."""
+    g = torch.Generator().manual_seed(S_q * 7 + S_k)
+    q = torch.randn(B, S_q, H, D, generator=g).to(dtype).to(cuda_device).permute(0, 2, 1, 3)
+    kv = torch.randn(B, S_k, 2, H, D, generator=g).to(dtype).to(cuda_device)
+    k, v = kv[:, :, 0].permute(0, 2, 1, 3), kv[:, :, 1].permute(0, 2, 1, 3)
+    lens = torch.randint(1 if dtype == torch.float16 else 130, S_k + 1, (B,), generator=g, dtype=torch.int32).to(cuda_device)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    kw, okw = {}, {}
+    if mask == "seqlen":
+        kw["seqlens"], okw["lens"] = lens, lens
+    elif mask == "key":
+        add = torch.randn(B, S_k, generator=g).to(cuda_device)
+        kw["mask"], okw["add_mask"] = add, add
+    out = torch.empty(B, S_q, H, D, dtype=dtype, device=cuda_device).permute(0, 2, 1, 3)
+    o, lse = api.fmha_forward(q, k, v, p_drop=p_drop, seed=33, offset=6, bh_offset=5, status=status, out=out, **kw)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    ref, *_ = helpers.oracle_forward(q, k, v, p_drop=p_drop, seed=33, offset=6, bh_offset=5, **okw)
+    helpers.assert_close(o, ref["o"], "o", dtype)
+    helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
