@@ -43,40 +43,42 @@ namespace {
 #endif
 constexpr uint32_t kComputeSleepNs = FMHA_BWD_POLL_SLEEP_NS;  // pause between barrier polls of the compute warps
 constexpr int kComputeThreads = 512;               // 16 compute warps
-constexpr int kBwdThreads = 64 + kComputeThreads;   // + producer warp + MMA warp
+constexpr int kBwdStatWarp = 2 + kComputeThreads / 32;   // the warp that fetches lse and delta
+constexpr int kBwdThreads = 64 + kComputeThreads + 32;   // + producer warp + MMA warp + statistics warp
 constexpr float kLog2eB = 1.4426950408889634f;
 
 enum BwdWaitSite {
-  kSiteKvFull = 201, kSiteQdoFull = 202, kSiteQdoEmpty = 203, kSiteSdpFull = 204, kSitePdsFull = 205,
-  kSiteDqFull = 206, kSiteDqFree = 207, kSiteAccFull = 208, kSiteSdpFree = 209, kSiteKvEmpty = 210,
-  kSiteItemFull = 211, kSiteItemEmpty = 212
+  kSiteKvFull = 201, kSiteQFull = 202, kSiteQEmpty = 203, kSiteSFull = 204, kSitePFull = 205, kSiteDqFull = 206,
+  kSiteDqFree = 207, kSiteAccFull = 208, kSiteDpFull = 209, kSiteKvEmpty = 210, kSiteItemFull = 211, kSiteItemEmpty = 212,
+  kSiteDoFull = 213, kSiteDoEmpty = 214, kSiteDsFull = 215, kSiteStatFull = 216, kSiteStatEmpty = 217, kSiteSmemBase = 218
 };
 
 template <int D>
 struct BwdSmem {
-  // D = 64: two K/V buffers (the next work item's K and V arrive while this one finishes) and two
-  // Q/dO stages.  D = 128 fills shared memory with one of each.
+  // D = 64: two K/V buffers (the next work item's K and V arrive while this one finishes), two stages of Q and of dO
+  // and two dS buffers.  D = 128: one K/V buffer, two stages of Q, one of dO (dV is its last reader and comes early in a
+  // tile's MMAs; Q is needed by dK, the last but one) and one dS buffer.
   static constexpr int kKvBufs = (D == 64) ? 2 : 1;
-  static constexpr int kStages = (D == 64) ? 2 : 1;   // Q / dO stages
-  static constexpr int kPdsBufs = 1;                  // P / dS buffers
-  // dQ tiles leave through shared memory + TMA reduce-add.  D = 64 has a dedicated 32 KB staging area
-  // (2 KB per compute warp); at D = 128 the 64 KB fp32 tile is staged in the P/dS buffers (4 KB per
-  // compute warp), which are idle between the completion of a tile's MMAs and the next tile's P/dS write.
-  static constexpr bool kDqStageOwn = (D == 64);
+  static constexpr int kQStages = 2;
+  static constexpr int kDoStages = (D == 64) ? 2 : 1;
+  static constexpr int kDsBufs = (D == 64) ? 2 : 1;
   static constexpr int kTileBytes = kTileM * D * 2;
+  static constexpr int kDsBytes = kTileM * kTileN * 2;
   static constexpr int kOffK = 0;
   static constexpr int kOffV = kOffK + kKvBufs * kTileBytes;
   static constexpr int kOffQ = kOffV + kKvBufs * kTileBytes;
-  static constexpr int kOffdO = kOffQ + kStages * kTileBytes;
-  static constexpr int kOffP = kOffdO + kStages * kTileBytes;
-  static constexpr int kOffdS = kOffP + kPdsBufs * kTileM * kTileN * 2;
-  static constexpr int kOffDQ = kOffdS + kPdsBufs * kTileM * kTileN * 2;    // fp32 staging of dQ
-  static constexpr int kOffMask = kOffDQ + (kDqStageOwn ? kTileM * D * 4 : 0);   // 2 x 128 floats
-  static constexpr int kOffBar = kOffMask + 2 * kTileN * 4;
-  static constexpr int kNumBars = 6 + 2 * kKvBufs + 2 * kStages + 4;
+  static constexpr int kOffdO = kOffQ + kQStages * kTileBytes;
+  static constexpr int kOffdS = kOffdO + kDoStages * kTileBytes;
+  // Staging of dK and dV on their way out, 2 KB per compute warp.
+  static constexpr int kOffStage = kOffdS + kDsBufs * kDsBytes;
+  static constexpr int kOffStats = kOffStage + 32768;         // 2 slots x (128 of -lse*log2e, 128 of delta/c)
+  static constexpr int kOffBar = kOffStats + 2 * 2 * kTileM * 4;
+  static constexpr int kNumBars = 7 + 2 * kKvBufs + 2 * kQStages + 2 * kDoStages + 8;
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;
   static constexpr int kBytes = kOffMisc + 32;
-  static constexpr int kDynBytes = kBytes + 1024;
+  // The tiles need a 1024-byte aligned base.  Dynamic shared memory of a kernel without static shared memory begins at
+  // such an address; the kernel checks it and gives up if that should ever not hold.
+  static constexpr int kDynBytes = kBytes;
   static_assert(kDynBytes <= 232448, "shared memory budget of one CTA exceeded");
 };
 
@@ -163,32 +165,48 @@ struct FinishArgs {
   const int* cu_seqlens;  // packed batch: row offsets into the [total_rows, H, D] dQ (sb unused), else null
 };
 
-template <bool BF16>
+// A block converts 8192 elements, whole rows of a head: coalesced 16-byte reads of the accumulator (eight in flight per thread),
+// through shared memory to coalesced 16-byte writes of the rows.
+constexpr int kFinishElems = 8192;   // per block
+template <int D, bool BF16>
 __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
   griddep_wait();
-  // grid = (B*H, row blocks); one thread converts 8 consecutive elements, D/8 threads per row
-  const int per_row = a.D / 8;
-  const int part = threadIdx.x % per_row;
-  const int r = blockIdx.y * (256 / per_row) + threadIdx.x / per_row;
-  if (r >= a.S_q) return;
+  constexpr int R = kFinishElems / D;   // 128 or 64 rows
+  constexpr int kStride = D * 2 + 8;    // bytes; 8-byte accesses of consecutive rows hit different banks
+  __shared__ __align__(16) uint8_t tile[R * kStride];
   const int bh = blockIdx.x;
   const int h = bh % a.H;
   const int b = bh / a.H;
-  int64_t row_dq = static_cast<int64_t>(b) * a.sb + static_cast<int64_t>(r) * a.ss;
+  const int r0 = blockIdx.y * R;
+  int64_t base = static_cast<int64_t>(b) * a.sb;
+  int q_limit = a.S_q;
   if (a.cu_seqlens != nullptr) {
-    const int base = a.cu_seqlens[b];
-    if (r >= min(a.cu_seqlens[b + 1] - base, a.S_q)) return;   // rows past the stated maximum length take no part
-    row_dq = static_cast<int64_t>(base + r) * a.ss;
+    const int first = a.cu_seqlens[b];
+    q_limit = min(a.cu_seqlens[b + 1] - first, a.S_q);   // rows past the stated maximum length take no part
+    base = static_cast<int64_t>(first) * a.ss;
   }
-  const float4* src = reinterpret_cast<const float4*>(a.dq_accum + (static_cast<int64_t>(bh) * a.S_q_pad + r) * a.D + part * 8);
-  const float4 x = src[0], y = src[1];
-  uint4 w;
-  w.x = pack2<BF16>(x.x * a.scale, x.y * a.scale);
-  w.y = pack2<BF16>(x.z * a.scale, x.w * a.scale);
-  w.z = pack2<BF16>(y.x * a.scale, y.y * a.scale);
-  w.w = pack2<BF16>(y.z * a.scale, y.w * a.scale);
-  unsigned short* dst = reinterpret_cast<unsigned short*>(a.dq) + row_dq + h * a.sh + part * 8;
-  *reinterpret_cast<uint4*>(dst) = w;
+  if (r0 >= q_limit) return;
+  const float4* src = reinterpret_cast<const float4*>(a.dq_accum + (static_cast<int64_t>(bh) * a.S_q_pad + r0) * D);
+  float4 x[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) x[k] = src[k * 256 + threadIdx.x];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int i = k * 256 + threadIdx.x;   // see dq_accum_index
+    const int row = (i / (8 * D)) * 32 + (i & 31), c4 = (i / 32) % (D / 4);
+    *reinterpret_cast<uint2*>(tile + row * kStride + c4 * 8) =
+        make_uint2(pack2<BF16>(x[k].x * a.scale, x[k].y * a.scale), pack2<BF16>(x[k].z * a.scale, x[k].w * a.scale));
+  }
+  __syncthreads();
+  unsigned short* dst = reinterpret_cast<unsigned short*>(a.dq) + base + h * a.sh;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = k * 256 + threadIdx.x;
+    const int row = i / (D / 8), ch = i % (D / 8);
+    const uint2 lo = *reinterpret_cast<const uint2*>(tile + row * kStride + ch * 16);
+    const uint2 hi = *reinterpret_cast<const uint2*>(tile + row * kStride + ch * 16 + 8);
+    if (r0 + row < q_limit) *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r0 + row) * a.ss + ch * 8) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -200,14 +218,28 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
 // overlaps the neighbouring items instead of leaving the SM idle (it was ~30 % of a CTA's life when
 // every item was its own CTA).  Items whose key tile lies wholly past the valid length write zeros.
 //
+// Layout.  Scores are formed transposed, S^T = K Q^T and dP^T = V dO^T with keys along the tensor-memory lanes, so that
+// P^T, written back to tensor memory by the thread that computed it, is the A operand of dV += P^T dO: it is neither
+// written to shared memory nor read from it.  What limits this kernel is shared-memory bandwidth: with P and dS both
+// staged there a D = 64 tile moved 2 944 cycles' worth of shared-memory data (MMA operands 1 664, P/dS 512, TMA in and out
+// 768), now 2 432; and the freed 32 KB is a second dS buffer (D = 64) or a second Q stage (D = 128), without which every
+// tile waited for the previous tile's MMAs (D = 64) or for the reload of Q and dO (D = 128).
+// In this layout a thread is a key: lse and delta vary along its columns and come from shared memory (broadcast reads;
+// a helper warp fetches them one to two tiles ahead), the additive key mask is one value per thread, and the dropout
+// draws, which give 16 keys of one query row each, are made by the thread of that row and transposed in the warp.
+//
 // Schedule inside the stream of (item, query tile) pairs, numbered t = 0, 1, ...:
-//   compute warps:  S,dP(t) -> registers, release the columns (sdp_free) -> P, dS in registers ->
-//                   [first tile of an item: dK, dV of the previous item -> global memory] ->
-//                   P,dS(t) -> shared memory (pds_full) -> dQ(t-1) -> staging -> TMA reduce-add
-//   MMA warp:       S,dP(t+1) as soon as sdp_free(t), also across an item boundary (D = 64: the next
-//                   item's K and V are already in the second buffer) -> dV,dK(t) -> dQ(t)
-// At D = 128 shared and tensor memory are full: one K/V buffer, dQ shares the dP columns and is read
-// out at the end of its own iteration, S/dP(t+1) follow dQ(t).
+//   compute warps:  S(t) -> P(t) -> tensor memory (p_full) -> [D = 128: dQ(t-1) out] -> dP(t) -> dS(t) -> shared memory
+//                   (ds_full) -> [D = 64: dQ(t-1) out]; dK and dV of an item leave when the next item's first P is ready.
+//   MMA warp:       on p_full(t): dV(t), S(t+1); on ds_full(t): [D = 64: dP(t+1)], dK(t), dQ(t), [D = 128: dP(t+1), whose
+//                   columns dQ(t) shares, when dQ(t) has been read out].  S(t+1) and dP(t+1) may belong to the next item.
+// Position of element (row, col) of a 128-row tile of the fp32 dQ accumulator: 32-row groups, in them groups of four
+// columns, in them the 32 rows with their four values each.
+template <int D>
+__device__ __forceinline__ int dq_accum_index(int row, int col) {
+  return (((row >> 5) * (D / 4) + (col >> 2)) * 32 + (row & 31)) * 4 + (col & 3);
+}
+
 struct BwdItem {
   int id;      // < 0: no more work
   int b, h, bh, k0, n_cols;   // n_cols <= 0: key tile wholly masked out
@@ -217,45 +249,66 @@ struct BwdItem {
   int tb;        // batch coordinate of the tensor maps (0 for a packed batch)
 };
 
+// Transposes the 32 x 32 bit matrix a warp holds as one row per lane: afterwards bit L of lane p is what bit p of lane L
+// was.  Five exchanges of half-blocks: 16 and 8 bits as byte permutes, 4, 2 and 1 as a rotation and a bit select.
+__device__ __forceinline__ uint32_t warp_bit_transpose(uint32_t x, int lane) {
+  uint32_t y = __shfl_xor_sync(0xffffffffu, x, 16);
+  x = prmt(x, y, (lane & 16) ? 0x3276u : 0x5410u);
+  y = __shfl_xor_sync(0xffffffffu, x, 8);
+  x = prmt(x, y, (lane & 8) ? 0x3715u : 0x6240u);
+#pragma unroll
+  for (int s = 4; s >= 1; s >>= 1) {
+    const uint32_t low = s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
+    const bool up = lane & s;
+    y = __shfl_xor_sync(0xffffffffu, x, s);
+    y = __funnelshift_l(y, y, up ? 32 - s : s);
+    const uint32_t own = up ? ~low : low;
+    x = (x & own) | (y & ~own);
+  }
+  return x;
+}
+
 // PACKED: FMHA_MASK_CU_SEQLENS; a template parameter so that the padded kernels carry none of its bookkeeping.
 template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
   griddep_wait();
   using L = BwdSmem<D>;
-  constexpr int ST = L::kStages;
-  constexpr int KV = L::kKvBufs;
-  constexpr bool OWNSTAGE = L::kDqStageOwn;
-  constexpr bool EARLY = (D == 64);  // S/dP of the next tile are issued before dV/dK/dQ of this one
+  constexpr int QS = L::kQStages, OS = L::kDoStages, DS = L::kDsBufs, KV = L::kKvBufs;
   constexpr int kTmemCols = 512;
   constexpr uint32_t kColS = 0, kColdP = 128, kColdV = 256, kColdK = 256 + D;
-  constexpr uint32_t kColdQ = (D == 64) ? 384 : kColdP;
+  constexpr uint32_t kColdQ = (D == 64) ? 384 : kColdP;   // D = 128: dQ takes the columns dP has been read from
+  // P^T, 16 columns per 32 query rows: beside everything else (D = 64), or over the thread's own columns of S (D = 128)
+  constexpr uint32_t kColP = (D == 64) ? 448 : kColS, kPStride = (D == 64) ? 16 : 32;
   constexpr int kFmt = BF16 ? 1 : 0;
   constexpr uint32_t kIdescS = make_idesc_f16(128, 128, kFmt, false, false);
-  constexpr uint32_t kIdescT = make_idesc_f16(128, D, kFmt, true, true);    // dV, dK: A and B MN-major
-  constexpr uint32_t kIdescQ = make_idesc_f16(128, D, kFmt, false, true);   // dQ: A K-major, B MN-major
+  constexpr uint32_t kIdescMN = make_idesc_f16(128, D, kFmt, true, true);    // dQ: A and B MN-major
+  constexpr uint32_t kIdescKN = make_idesc_f16(128, D, kFmt, false, true);   // dV, dK: A K-major (dV: tensor memory), B MN-major
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem + L::kOffK;
   uint8_t* sV = smem + L::kOffV;
   uint8_t* sQ = smem + L::kOffQ;
   uint8_t* sdO = smem + L::kOffdO;
-  uint8_t* sP = smem + L::kOffP;
   uint8_t* sdS = smem + L::kOffdS;
-  uint8_t* sDQ = OWNSTAGE ? smem + L::kOffDQ : smem + L::kOffP;   // fp32 dQ staging
-  float* sMask = reinterpret_cast<float*>(smem + L::kOffMask);     // [2][128], by work-item parity
+  uint8_t* sStage = smem + L::kOffStage;
+  float* sStats = reinterpret_cast<float*>(smem + L::kOffStats);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
-  uint64_t* sdp_full = bars + 0;   // S and dP of a tile are in tensor memory
-  uint64_t* sdp_free = bars + 1;   // ... and have been copied to registers (all compute threads arrive)
-  uint64_t* pds_full = bars + 2;   // P and dS are in shared memory (all compute threads arrive)
-  uint64_t* dq_full = bars + 3;    // dQ tile is in tensor memory; dV/dK/dQ of that tile are complete
-  uint64_t* dq_free = bars + 4;    // dQ tile has been read out (all compute threads arrive)
-  uint64_t* acc_full = bars + 5;   // dK / dV of a work item are complete
-  uint64_t* kv_full = bars + 6;
+  uint64_t* s_full = bars + 0;     // S of a tile is in tensor memory
+  uint64_t* p_full = bars + 1;     // ... and P of it as well; S has been read (all compute threads arrive)
+  uint64_t* dp_full = bars + 2;    // dP of a tile is in tensor memory
+  uint64_t* ds_full = bars + 3;    // dS is in shared memory; dP has been read (all compute threads arrive)
+  uint64_t* dq_full = bars + 4;    // dQ tile is in tensor memory; dV/dK/dQ of that tile are complete
+  uint64_t* dq_free = bars + 5;    // dQ tile has been read out (all compute threads arrive)
+  uint64_t* acc_full = bars + 6;   // dK / dV of a work item are complete
+  uint64_t* kv_full = bars + 7;
   uint64_t* kv_empty = kv_full + KV;
-  uint64_t* qdo_full = kv_empty + KV;
-  uint64_t* qdo_empty = qdo_full + ST;
-  uint64_t* item_full = qdo_empty + ST;   // [2] ring of work-item ids
+  uint64_t* q_full = kv_empty + KV;
+  uint64_t* q_empty = q_full + QS;
+  uint64_t* do_full = q_empty + QS;
+  uint64_t* do_empty = do_full + OS;      // dV of the tile has completed (so P may be overwritten, too)
+  uint64_t* stat_full = do_empty + OS;    // [2] lse and delta of a tile's rows are in shared memory
+  uint64_t* stat_empty = stat_full + 2;   // [2] ... and have been read (every compute warp arrives)
+  uint64_t* item_full = stat_empty + 2;   // [2] ring of work-item ids
   uint64_t* item_empty = item_full + 2;
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 4);
@@ -263,6 +316,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   // Philox offset of this launch (launch parameter + optional device-resident value), read where a draw starts
   volatile uint32_t* philox_off = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 16);
 
+  if (smem_u32(smem) & 1023) {   // see kDynBytes
+    if (threadIdx.x == 0 && a.status != nullptr) atomicCAS(a.status, 0, kSiteSmemBase);
+    return;
+  }
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int kv_tiles = (a.S_k + kTileN - 1) / kTileN;
@@ -273,9 +330,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     *philox_off = a.philox_offset + (a.philox_offset_dev != nullptr ? static_cast<uint32_t>(*a.philox_offset_dev) : 0u);
-    mbar_init(sdp_full, 1);
-    mbar_init(sdp_free, kComputeThreads);
-    mbar_init(pds_full, kComputeThreads);
+    mbar_init(s_full, 1);
+    mbar_init(p_full, kComputeThreads);
+    mbar_init(dp_full, 1);
+    mbar_init(ds_full, kComputeThreads);
     mbar_init(dq_full, 1);
     mbar_init(dq_free, kComputeThreads);
     mbar_init(acc_full, 1);
@@ -283,13 +341,19 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       mbar_init(kv_full + s, 1);
       mbar_init(kv_empty + s, 1);
     }
-    for (int s = 0; s < ST; ++s) {
-      mbar_init(qdo_full + s, 1);
-      mbar_init(qdo_empty + s, 1);
+    for (int s = 0; s < QS; ++s) {
+      mbar_init(q_full + s, 1);
+      mbar_init(q_empty + s, 1);
+    }
+    for (int s = 0; s < OS; ++s) {
+      mbar_init(do_full + s, 1);
+      mbar_init(do_empty + s, 1);
     }
     for (int s = 0; s < 2; ++s) {
+      mbar_init(stat_full + s, 1);
+      mbar_init(stat_empty + s, kComputeThreads / 32);
       mbar_init(item_full + s, 1);
-      mbar_init(item_empty + s, 1 + kComputeThreads / 32);   // the MMA warp and every compute warp
+      mbar_init(item_empty + s, 2 + kComputeThreads / 32);   // MMA warp, statistics warp, every compute warp
     }
     mbar_fence_init();
     tma_prefetch_desc(&a.tm_q);
@@ -298,7 +362,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     tma_prefetch_desc(&a.tm_do);
     tma_prefetch_desc(&a.tm_dk);
     tma_prefetch_desc(&a.tm_dv);
-    tma_prefetch_desc(&a.tm_dq);
   }
   if (warp == 1) {
     tmem_alloc(tmem_base_slot, kTmemCols);
@@ -379,14 +442,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           tma_load_4d(sV + kvb * L::kTileBytes + c * 16384, &a.tm_v, kv_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
         }
         for (int i = 0; i < it.n_q; ++i, ++g) {
-          const int s = g % ST;
-          if (g >= ST) mbar_wait(qdo_empty + s, ((g / ST) - 1) & 1, wctx, kSiteQdoEmpty);
-          mbar_arrive_expect_tx(qdo_full + s, 2 * L::kTileBytes);
+          const int qs = g % QS, os = g % OS;
+          if (g >= QS) mbar_wait(q_empty + qs, ((g / QS) - 1) & 1, wctx, kSiteQEmpty);
+          mbar_arrive_expect_tx(q_full + qs, L::kTileBytes);
 #pragma unroll
-          for (int c = 0; c < D / 64; ++c) {
-            tma_load_4d(sQ + s * L::kTileBytes + c * 16384, &a.tm_q, qdo_full + s, c * 64, it.row_base + i * kTileM, it.h, it.tb);
-            tma_load_4d(sdO + s * L::kTileBytes + c * 16384, &a.tm_do, qdo_full + s, c * 64, it.row_base + i * kTileM, it.h, it.tb);
-          }
+          for (int c = 0; c < D / 64; ++c)
+            tma_load_4d(sQ + qs * L::kTileBytes + c * 16384, &a.tm_q, q_full + qs, c * 64, it.row_base + i * kTileM, it.h, it.tb);
+          if (g >= OS) mbar_wait(do_empty + os, ((g / OS) - 1) & 1, wctx, kSiteDoEmpty);
+          mbar_arrive_expect_tx(do_full + os, L::kTileBytes);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c)
+            tma_load_4d(sdO + os * L::kTileBytes + c * 16384, &a.tm_do, do_full + os, c * 64, it.row_base + i * kTileM, it.h, it.tb);
         }
         ++w;
       }
@@ -396,165 +462,188 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     // The whole warp runs this loop convergently; the MMAs go out in bursts of 4 or 8 from one
     // elected lane with descriptors prepared beforehand as warp-uniform values (see umma_ss_x4).
     // A loop in which a single lane computes each descriptor and then issues was starved by the
-    // compute warps' arithmetic: ~150 cycles per MMA during their exp/Philox phase, which put the
-    // tensor core's work on the critical path of every tile.
+    // compute warps' arithmetic: ~150 cycles per MMA during their exp/Philox phase.
     constexpr int KS = D / 16;      // k-steps of S and dP
     const uint32_t tS = tmem_base + kColS, tdP = tmem_base + kColdP, tdV = tmem_base + kColdV,
-                   tdK = tmem_base + kColdK, tdQ = tmem_base + kColdQ;
-    auto issue_s = [&](int stage, int kvb) {
-      const uint64_t dq = make_smem_desc_sw128(smem_u32(sQ + stage * L::kTileBytes), 16, 1024);
-      const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + kvb * L::kTileBytes), 16, 1024);   // K as K-major B
-      uint64_t aq[KS], bk[KS];
+                   tdK = tmem_base + kColdK, tdQ = tmem_base + kColdQ, tP = tmem_base + kColP;
+    // [128 x 128] = A (rows of D values, K-major) * B (likewise)^T
+    auto issue_kk = [&](uint32_t d, const uint8_t* a_tile, const uint8_t* b_tile) {
+      const uint64_t da = make_smem_desc_sw128(smem_u32(a_tile), 16, 1024), db = make_smem_desc_sw128(smem_u32(b_tile), 16, 1024);
+      uint64_t x[KS], y[KS];
 #pragma unroll
       for (int kk = 0; kk < KS; ++kk) {
-        aq[kk] = dq + kmajor_step(kk, 16384);
-        bk[kk] = dk + kmajor_step(kk, 16384);
+        x[kk] = da + kmajor_step(kk, 16384);
+        y[kk] = db + kmajor_step(kk, 16384);
       }
-      if constexpr (KS == 4) umma_ss_x4(tS, aq, bk, kIdescS, 0u);
-      else umma_ss_x8(tS, aq, bk, kIdescS, 0u);
+      if constexpr (KS == 4) umma_ss_x4(d, x, y, kIdescS, 0u);
+      else umma_ss_x8(d, x, y, kIdescS, 0u);
     };
-    auto issue_dp = [&](int stage, int kvb) {
-      const uint64_t dd = make_smem_desc_sw128(smem_u32(sdO + stage * L::kTileBytes), 16, 1024);
-      const uint64_t dv = make_smem_desc_sw128(smem_u32(sV + kvb * L::kTileBytes), 16, 1024);   // V as K-major B
-      uint64_t ad[KS], bv[KS];
-#pragma unroll
-      for (int kk = 0; kk < KS; ++kk) {
-        ad[kk] = dd + kmajor_step(kk, 16384);
-        bv[kk] = dv + kmajor_step(kk, 16384);
-      }
-      if constexpr (KS == 4) umma_ss_x4(tdP, ad, bv, kIdescS, 0u);
-      else umma_ss_x8(tdP, ad, bv, kIdescS, 0u);
-      umma_commit_elect(sdp_full);
+    // S^T of tile tt (its Q stage) with the K buffer kvb
+    auto issue_s = [&](int tt, int kvb) {
+      mbar_wait(q_full + tt % QS, (tt / QS) & 1, wctx, kSiteQFull);
+      tc_fence_after_sync();
+      issue_kk(tS, sK + kvb * L::kTileBytes, sQ + (tt % QS) * L::kTileBytes);
+      umma_commit_elect(s_full);
+    };
+    auto issue_dp = [&](int tt, int kvb) {
+      mbar_wait(do_full + tt % OS, (tt / OS) & 1, wctx, kSiteDoFull);
+      tc_fence_after_sync();
+      issue_kk(tdP, sV + kvb * L::kTileBytes, sdO + (tt % OS) * L::kTileBytes);
+      umma_commit_elect(dp_full);
     };
 
     int n = 0, w = 0, t = 0;   // items fetched, items with work, query tiles so far
-    bool ahead = false;         // S and dP of the current item's first tile were issued during the previous item
-    BwdItem cur = fetch_item(n++, 0);
+    auto next_work = [&]() {   // the next item with keys
+      BwdItem it = fetch_item(n++, 0);
+      while (it.id >= 0 && it.n_cols <= 0) it = fetch_item(n++, 0);
+      return it;
+    };
+    BwdItem cur = next_work();
+    if (cur.id >= 0) {
+      mbar_wait(kv_full, 0, wctx, kSiteKvFull);
+      issue_s(0, 0);
+      issue_dp(0, 0);
+    }
     while (cur.id >= 0) {
-      if (cur.n_cols <= 0) {
-        cur = fetch_item(n++, 0);
-        continue;
-      }
       const int kvb = w % KV;
-      if (!ahead) {
-        mbar_wait(kv_full + kvb, (w / KV) & 1, wctx, kSiteKvFull);
-        if (t > 0) {
-          mbar_wait(sdp_free, (t - 1) & 1, wctx, kSiteSdpFree);
-          if constexpr (!EARLY) mbar_wait(dq_free, (t - 1) & 1, wctx, kSiteDqFree);   // dQ shares the dP columns
-        }
-        mbar_wait(qdo_full + (t % ST), (t / ST) & 1, wctx, kSiteQdoFull);
-        tc_fence_after_sync();
-        issue_s(t % ST, kvb);
-        issue_dp(t % ST, kvb);
-      }
-      ahead = false;
-      BwdItem nxt = cur;
-      bool have_nxt = false;
-      const uint64_t dK_m = make_smem_desc_sw128(smem_u32(sK + kvb * L::kTileBytes), 16384, 1024);   // K as MN-major B (dQ)
       const int n_q = cur.n_q;
+      const uint64_t dK_m = make_smem_desc_sw128(smem_u32(sK + kvb * L::kTileBytes), 16384, 1024);   // K as MN-major B (dQ)
+      BwdItem nxt = cur;
       for (int i = 0; i < n_q; ++i, ++t) {
-        const int s = t % ST;
-        if constexpr (EARLY) {
-          if (i + 1 < n_q) {
-            mbar_wait(sdp_free, t & 1, wctx, kSiteSdpFree);
-            mbar_wait(qdo_full + ((t + 1) % ST), ((t + 1) / ST) & 1, wctx, kSiteQdoFull);
-            tc_fence_after_sync();
-            issue_s((t + 1) % ST, kvb);
-            issue_dp((t + 1) % ST, kvb);
-          } else {
-            // last tile of this item: look at the next item and start its first tile now
-            nxt = fetch_item(n++, 0);
-            have_nxt = true;
-            if (nxt.id >= 0 && nxt.n_cols > 0) {
-              const int nkvb = (w + 1) % KV;
-              mbar_wait(kv_full + nkvb, ((w + 1) / KV) & 1, wctx, kSiteKvFull);
-              mbar_wait(sdp_free, t & 1, wctx, kSiteSdpFree);
-              mbar_wait(qdo_full + ((t + 1) % ST), ((t + 1) / ST) & 1, wctx, kSiteQdoFull);
-              tc_fence_after_sync();
-              issue_s((t + 1) % ST, nkvb);
-              issue_dp((t + 1) % ST, nkvb);
-              ahead = true;
-            }
+        const bool last = i + 1 == n_q;
+        const int qs = t % QS, os = t % OS;
+        const uint8_t* ds_tile = sdS + (t % DS) * L::kDsBytes;
+        const uint32_t acc0 = (i > 0) ? 1u : 0u;
+        // ---- dV += P^T dO: A from tensor memory, dO read MN-major (16 query rows = 2048 B per k-step) ----------------
+        const uint64_t ddO_m = make_smem_desc_sw128(smem_u32(sdO + os * L::kTileBytes), 16384, 1024);
+        mbar_wait(p_full, t & 1, wctx, kSitePFull);
+        tc_fence_after_sync();
+        {
+          uint64_t y[4];
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) y[kk] = ddO_m + mnmajor_step(hf * 4 + kk);
+            const uint32_t p0 = tP + 2 * hf * kPStride;
+            umma_ts_2x2(tdV, p0, p0 + kPStride, 8u, y, kIdescKN, hf == 0 ? acc0 : 1u);
           }
         }
-        // MN-major views of this tile's operands (16 rows = 2048 B per k-step, 64-wide halves 16 KB apart)
-        const uint64_t dQ_m = make_smem_desc_sw128(smem_u32(sQ + s * L::kTileBytes), 16384, 1024);
-        const uint64_t ddO_m = make_smem_desc_sw128(smem_u32(sdO + s * L::kTileBytes), 16384, 1024);
-        const uint64_t dP_m = make_smem_desc_sw128(smem_u32(sP), 16384, 1024);
-        const uint64_t ddS_m = make_smem_desc_sw128(smem_u32(sdS), 16384, 1024);
-        const uint64_t ddS_k = make_smem_desc_sw128(smem_u32(sdS), 16, 1024);
-        mbar_wait(pds_full, t & 1, wctx, kSitePdsFull);
+        umma_commit_elect(do_empty + os);   // dP(t) came before, so dO(t) is not read again
+        // ---- S of the next tile: S(t) has been read (D = 128: and P(t), which lies over it) --------------------------------
+        // At the end of an item the next one is looked up here only where its K can be there already (D = 64); the compute
+        // warps finish tile t, and any items without keys that follow, without another MMA at D = 64, but not at D = 128.
+        if (D == 64 && last) nxt = next_work();
+        const int nkvb = last ? (w + 1) % KV : kvb;
+        if (!last || (D == 64 && nxt.id >= 0)) {
+          if (last) mbar_wait(kv_full + nkvb, ((w + 1) / KV) & 1, wctx, kSiteKvFull);
+          issue_s(t + 1, nkvb);
+        }
+        // ---- dK += dS^T Q, dQ tile = dS K -----------------------------------------------------------------------------------
+        const uint64_t dQ_m = make_smem_desc_sw128(smem_u32(sQ + qs * L::kTileBytes), 16384, 1024);
+        const uint64_t ddS_k = make_smem_desc_sw128(smem_u32(ds_tile), 16, 1024);       // dS^T as K-major A (keys x queries)
+        const uint64_t ddS_m = make_smem_desc_sw128(smem_u32(ds_tile), 16384, 1024);    // dS as MN-major A (queries x keys)
+        mbar_wait(ds_full, t & 1, wctx, kSiteDsFull);
         tc_fence_after_sync();
-        // dV += P^T dO ; dK += dS^T Q : A is the [q x keys] tile read MN-major (keys contiguous),
-        // 16 query rows (2048 B) per k-step, the two 64-key halves 16 KB apart.
-        const uint32_t acc0 = (i > 0) ? 1u : 0u;
-        {
+        if constexpr (D == 64) {
+          if (!last || nxt.id >= 0) issue_dp(t + 1, nkvb);   // dP(t) has been read
+        }
+        auto issue_dk = [&]() {
           uint64_t x[8], y[8];
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
-            x[kk] = dP_m + mnmajor_step(kk);
-            y[kk] = ddO_m + mnmajor_step(kk);
+            x[kk] = ddS_k + kmajor_step(kk, 16384);
+            y[kk] = dQ_m + mnmajor_step(kk);
           }
-          umma_ss_x8(tdV, x, y, kIdescT, acc0);
+          umma_ss_x8(tdK, x, y, kIdescKN, acc0);
+          umma_commit_elect(q_empty + qs);
+          if (last) umma_commit_elect(acc_full);
+        };
+        if constexpr (D == 64) issue_dk();
+        if (D == 64 && t > 0) {
+          mbar_wait(dq_free, (t - 1) & 1, wctx, kSiteDqFree);
+          tc_fence_after_sync();
         }
         {
           uint64_t x[8], y[8];
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             x[kk] = ddS_m + mnmajor_step(kk);
-            y[kk] = dQ_m + mnmajor_step(kk);
-          }
-          umma_ss_x8(tdK, x, y, kIdescT, acc0);
-        }
-        umma_commit_elect(qdo_empty + s);  // Q and dO of this stage are not read again (dQ needs dS and K only)
-        if (i == n_q - 1) umma_commit_elect(acc_full);
-        if (t > 0) {
-          mbar_wait(dq_free, (t - 1) & 1, wctx, kSiteDqFree);
-          tc_fence_after_sync();
-        }
-        // dQ tile = dS K : A K-major (keys along the row), B = K tile read MN-major
-        {
-          uint64_t x[8], y[8];
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            x[kk] = ddS_k + kmajor_step(kk, 16384);
             y[kk] = dK_m + mnmajor_step(kk);
           }
-          umma_ss_x8(tdQ, x, y, kIdescQ, 0u);
+          umma_ss_x8(tdQ, x, y, kIdescMN, 0u);
         }
         umma_commit_elect(dq_full);
-        if (i == n_q - 1) umma_commit_elect(kv_empty + kvb);   // K and V of this item are not read again
-        if constexpr (!EARLY) {
-          if (i + 1 < n_q) {
-            mbar_wait(qdo_full + ((t + 1) % ST), ((t + 1) / ST) & 1, wctx, kSiteQdoFull);
-            tc_fence_after_sync();
-            issue_s((t + 1) % ST, kvb);                          // S columns were released before pds_full(t)
+        if constexpr (D == 128) issue_dk();   // under the read-out of dQ, which dP(t+1) waits for
+        if (last) umma_commit_elect(kv_empty + kvb);   // K and V of this item are not read again
+        if constexpr (D == 128) {
+          if (last) nxt = next_work();
+          if (!last || nxt.id >= 0) {
+            if (last) {   // the single K/V buffer has been reloaded
+              mbar_wait(kv_full, (w + 1) & 1, wctx, kSiteKvFull);
+              issue_s(t + 1, 0);
+            }
             mbar_wait(dq_free, t & 1, wctx, kSiteDqFree);        // dQ shares the dP columns
-            tc_fence_after_sync();
-            issue_dp((t + 1) % ST, kvb);
+            issue_dp(t + 1, nkvb);
           }
         }
       }
       ++w;
-      cur = have_nxt ? nxt : fetch_item(n++, 0);
+      cur = nxt;
+    }
+  } else if (warp == kBwdStatWarp) {
+    // ============================ row statistics =====================================
+    // lse and delta of a tile's 128 query rows, in the form the compute warps use them, one to two tiles ahead.
+    const float inv_c = DROP ? 1.0f / a.dropout_scale : 1.0f;
+    int n = 0, t = 0;
+    while (true) {
+      const BwdItem cur = fetch_item(n++, 0);
+      if (cur.id < 0) break;
+      if (cur.n_cols <= 0) continue;
+      // logsumexp rows: [B*H, S_q], or [H, total_rows] for a packed batch; delta is always [B*H, S_q]
+      const float* lse = a.lse + (packed ? static_cast<int64_t>(cur.h) * a.total_rows + cur.row_base : static_cast<int64_t>(cur.bh) * a.S_q);
+      const float* delta = a.delta + static_cast<int64_t>(cur.bh) * a.S_q;
+      for (int i = 0; i < cur.n_q; ++i, ++t) {
+        float x[4], d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int r = i * kTileM + k * 32 + lane;
+          x[k] = INFINITY;   // rows past the end: their probabilities are zero
+          d[k] = 0.f;
+          if (r < cur.q_limit) {
+            x[k] = lse[r];
+            d[k] = delta[r];
+          }
+        }
+        const int slot = t & 1;
+        if (t >= 2) mbar_wait(stat_empty + slot, ((t >> 1) - 1) & 1, wctx, kSiteStatEmpty);
+        float* st = sStats + slot * 2 * kTileM;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          st[k * 32 + lane] = -x[k] * kLog2eB;
+          st[kTileM + k * 32 + lane] = d[k] * inv_c;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(stat_full + slot);
+      }
     }
   } else {
     // ============================ compute warps =====================================
-    // 16 warps: warp (quad, cq) owns rows [32*quad, +32) (its tensor-memory lane quarter) and the
-    // 32 columns [32*cq, +32) of every 128 x 128 tile.
+    // 16 warps: warp (quad, cq) owns keys [32*quad, +32) (its tensor-memory lane quarter, one key per thread) and the
+    // query columns [32*cq, +32) of every 128 x 128 tile.
     const int cw = warp - 2;             // 0..15
     const int quad = warp & 3;           // tensor-memory lane quarter of this warp
     const int cq = cw >> 2;              // which 32 columns of the tile
-    const int row = quad * 32 + lane;
-    const int tid = threadIdx.x - 64;    // 0..511
+    const int row = quad * 32 + lane;    // key within the tile
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float sl2 = a.scale_log2;
-    // With dropout dS is formed as keep*P*dP - P*delta/c and the factor c = 1/(1-p) moves into the
+    // With dropout dS is formed as P*(keep*dP - delta/c) and the factor c = 1/(1-p) moves into the
     // final scaling of dQ and dK (and of dV, whose P operand is unscaled as well).
-    const float inv_c = DROP ? 1.0f / a.dropout_scale : 1.0f;
     const float dscale = DROP ? a.dropout_scale : 1.0f;
-    const int cbase = cq * 32;           // first column of this thread within the tile
     constexpr int DQ = D / 4;            // columns of a [128 x D] accumulator handled by one thread
+    // The lane that draws for query column c of the warp's 32, chosen so that after the transposition the keep bits of
+    // columns 4j..4j+3 of a thread's key are the top bits of the four bytes of (word << j).
+    const int draw_col = 4 * (7 - (lane & 7)) + (lane >> 3);
+    uint8_t* stage = sStage + cw * 2048;   // this warp's staging tile for dK and dV
 
     // Every warp polls the mbarrier itself: funnelling the wait through one warp and a named barrier
     // was measured 8 % slower (it removes the skew between warps that lets their phases overlap).
@@ -562,12 +651,16 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       mbar_wait(bar, parity, wctx, site, kComputeSleepNs);
       tc_fence_after_sync();
     };
-
-    // D = 128: every warp stages its own 32 rows x 32 columns of dQ tile `tt` (4 KB, 128-byte swizzle)
-    // in the idle P/dS buffers and its lane 0 issues one TMA reduce-add for it.  The additions are
-    // performed line by line by the TMA unit instead of 2048 scattered 16-byte atomics per tile, which
-    // occupied the compute warps for ~1500 cycles per tile, and no warp waits for another one here.
-    auto dq_readout_tma = [&](int tt, int row0) {
+    // Frees the warp's staging tile (its previous TMA copies have been read).
+    auto stage_free = [&]() {
+      if (lane == 0) tma_store_wait_read();
+      __syncwarp();
+    };
+    // dQ tile `tt` (rows = queries): tensor memory -> registers -> fp32 accumulator, 16 bytes per reduction.  The
+    // accumulator is laid out so that a warp's instruction covers 512 consecutive bytes (dq_accum_index), which keeps the
+    // tile out of shared memory: staged there for TMA reduce-adds it cost 32 (D = 64) or 64 KB written and read again per
+    // tile, a fifth of all shared-memory traffic.
+    auto dq_readout = [&](int tt, int64_t row0) {
       wait_all(dq_full, tt & 1, kSiteDqFull);
       uint32_t r[DQ];
 #pragma unroll
@@ -576,52 +669,19 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       tmem_wait_ld();
       tc_fence_before_sync();
       mbar_arrive(dq_free);                          // the dQ columns may be overwritten
-      uint8_t* stage = sDQ + cw * 4096;
-      const uint32_t rowaddr = smem_u32(stage) + lane * 128;
-      const uint32_t sw = lane & 7;                  // 128-byte swizzle: 16-byte chunk ^= row mod 8
+      float* dst = a.dq_accum + row0 * D + dq_accum_index<D>(row, cq * DQ);
 #pragma unroll
       for (int q = 0; q < DQ / 4; ++q)
-        sts128(rowaddr + ((q ^ sw) << 4), r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0 && *abort_flag == 0) {
-        tma_reduce_add_2d(&a.tm_dq, stage, cq * DQ, row0 + quad * 32);
-        tma_store_commit();
-      }
-    };
-    // D = 64: every warp stages its own 32 rows x 16 columns (2 KB, 64-byte swizzle) and its lane 0
-    // issues the reduce, so the warps never wait for one another here.
-    auto dq_readout_warp = [&](int tt, int row0) {
-      wait_all(dq_full, tt & 1, kSiteDqFull);
-      uint32_t t16[16];
-      tmem_ld16(tmem_base + lane_addr + kColdQ + cq * 16, t16);
-      tmem_wait_ld();
-      tc_fence_before_sync();
-      mbar_arrive(dq_free);                          // the dQ columns may be overwritten
-      if (lane == 0) tma_store_wait_read();          // this warp's previous reduce has read its staging tile
-      __syncwarp();
-      uint8_t* stage = sDQ + cw * 2048;
-      const uint32_t rowaddr = smem_u32(stage) + lane * 64;
-      const uint32_t sw = (lane >> 1) & 3;           // 64-byte swizzle: 16-byte chunk ^= bits 7..8 of the offset
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        sts128(rowaddr + ((q ^ sw) << 4), t16[q * 4], t16[q * 4 + 1], t16[q * 4 + 2], t16[q * 4 + 3]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0 && *abort_flag == 0) {
-        tma_reduce_add_2d(&a.tm_dq, stage, cq * 16, row0 + quad * 32);
-        tma_store_commit();
-      }
+        red_add_v4(dst + q * 128, __uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]), __uint_as_float(r[q * 4 + 2]),
+                   __uint_as_float(r[q * 4 + 3]));
     };
     // dK and dV of a finished item: tensor memory -> registers -> this warp's staging tile -> two TMA
     // stores issued by its lane 0.  Warp (quad, cq) holds key rows [32*quad, +32) x columns [cq*DQ, +DQ)
-    // of both accumulators: 32 rows of DQ*2 bytes each, dV first, dK behind it.  The staging tile is the
-    // warp's dQ staging slot (D = 64) or its 4 KB share of the idle P/dS buffers (D = 128).  Rows past
-    // S_k are clipped by the TMA unit.  The caller orders this against other users of the tile.
+    // of both accumulators: 32 rows of DQ*2 bytes each.  The staging tile holds one of them at D = 128, both at D = 64
+    // (dV first).  Rows past S_k are clipped by the TMA unit.
     constexpr int kDkvRowBytes = DQ * 2;
     auto store_dkdv = [&](int item_id, bool from_tmem) {
       const BwdItem it = decode(item_id);
-      uint8_t* stage = OWNSTAGE ? sDQ + cw * 2048 : sP + cw * 4096;
       // Packed batch: a slice that reaches past the end of the sequence would overwrite the next sequence's
       // rows, so its rows are written one by one from registers.
       const int key = it.k0 + quad * 32 + lane;
@@ -629,7 +689,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
         const float mul = (which == 0) ? dscale : a.scale * dscale;
-        const uint32_t rowaddr = smem_u32(stage) + which * 32 * kDkvRowBytes + lane * kDkvRowBytes;
+        uint8_t* tile = stage + (D == 64 ? which * 32 * kDkvRowBytes : 0);
+        const uint32_t rowaddr = smem_u32(tile) + lane * kDkvRowBytes;
+        if (D == 128 || which == 0) stage_free();
         unsigned short* grow = reinterpret_cast<unsigned short*>(which == 0 ? a.dv_ptr : a.dk_ptr) +
                                static_cast<int64_t>(it.row_base + key) * (which == 0 ? a.dv_ss : a.dk_ss) +
                                static_cast<int64_t>(it.h) * (which == 0 ? a.dv_sh : a.dk_sh) + cq * DQ;
@@ -657,229 +719,155 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
             }
           }
         }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && *abort_flag == 0 && !edge) {
+          tma_store_4d(which == 0 ? &a.tm_dv : &a.tm_dk, tile, cq * DQ, it.row_base + it.k0 + quad * 32, it.h, it.tb);
+          tma_store_commit();
+        }
       }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0 && *abort_flag == 0 && !edge) {
-        tma_store_4d(&a.tm_dv, stage, cq * DQ, it.row_base + it.k0 + quad * 32, it.h, it.tb);
-        tma_store_4d(&a.tm_dk, stage + 32 * kDkvRowBytes, cq * DQ, it.row_base + it.k0 + quad * 32, it.h, it.tb);
-        tma_store_commit();
-      }
-    };
-    // Frees the warp's staging tile for store_dkdv / the next dQ tile (D = 64 only: at D = 128 the
-    // tile lies in the P/dS buffers, whose users are ordered by the CTA-wide barrier 2).
-    auto own_stage_free = [&]() {
-      if (lane == 0) tma_store_wait_read();
-      __syncwarp();
     };
 
     int n = 0, w = 0, t = 0;      // items fetched, items with work, query tiles so far
     int prev_id = -1;             // >= 0: dK/dV of that item are still in tensor memory
-    int prev_row0 = 0;            // accumulator row of the tile whose dQ is still in tensor memory (D = 64)
+    int64_t prev_row0 = 0;        // accumulator row of tile t-1
+    bool dq_out = true;           // dQ of tile t-1 has been read out
 
     while (true) {
       const BwdItem cur = fetch_item(n++, kComputeSleepNs);
       if (cur.id < 0) break;
       if (cur.n_cols <= 0) {
         if (packed) continue;   // a packed sequence has no rows past its length
-        // key tile wholly past the valid length: its gradients are zero
-        if constexpr (OWNSTAGE) {
-          own_stage_free();
-          store_dkdv(cur.id, false);
-        } else {
-          // the P/dS buffers may still be read by the previous tile's MMAs and dQ reduce
-          if (t > 0) {
-            if (lane == 0) tma_store_wait_read();
-            named_bar_sync(2, kComputeThreads);
-          }
-          store_dkdv(cur.id, false);
-          if (lane == 0) tma_store_wait_read();
-          named_bar_sync(2, kComputeThreads);
-        }
+        store_dkdv(cur.id, false);   // key tile wholly past the valid length: its gradients are zero
         continue;
       }
-      const int k0 = cur.k0, n_cols = cur.n_cols, bh = cur.bh, n_q = cur.n_q, q_limit = cur.q_limit;
+      const int n_cols = cur.n_cols, bh = cur.bh, n_q = cur.n_q;
       const uint32_t gbh = static_cast<uint32_t>(a.philox_bh_offset + bh);
-      // logsumexp rows: [B*H, S_q], or [H, total_rows] for a packed batch; delta is always [B*H, S_q]
-      const int64_t lse_base = packed ? static_cast<int64_t>(cur.h) * a.total_rows + cur.row_base : static_cast<int64_t>(bh) * a.S_q;
-      const int64_t delta_base = static_cast<int64_t>(bh) * a.S_q;
-      const float* mask_row = sMask + (w & 1) * kTileN;
+      const bool key_ok = row < n_cols;     // keys past the valid length / tensor edge
+      float key_add = 0.f;
       if constexpr (KEYADD) {
-        // both barriers are needed: a slower warp may still read the other item's values (first),
-        // and every warp reads what the first four wrote (second)
-        named_bar_sync(1, kComputeThreads);
-        if (tid < kTileN) {
-          const int c = k0 + tid;
-          sMask[(w & 1) * kTileN + tid] =
-              (c < a.S_k) ? reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(cur.b) * a.S_k + c] * kLog2eB : 0.f;
-        }
-        named_bar_sync(1, kComputeThreads);
-      }
-
-      // Row statistics of the next tile are fetched one iteration ahead and kept RAW: any arithmetic
-      // on the loaded value here would make the warp wait for the load at once (~1000 cycles per tile).
-      float lse_next = INFINITY, delta_next = 0.f;
-      if (row < q_limit) {
-        lse_next = a.lse[lse_base + row];
-        delta_next = a.delta[delta_base + row];
+        const int c = cur.k0 + row;
+        if (c < a.S_k) key_add = reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(cur.b) * a.S_k + c] * kLog2eB;
       }
 
       for (int i = 0; i < n_q; ++i, ++t) {
-        const int q_row = i * kTileM + row;
-        // lse in the log2 domain; +inf for rows past the end makes their probabilities zero
-        const float neg_lse2 = -lse_next * kLog2eB;
-        const float delta = delta_next * inv_c;
-        {
-          const int nr = q_row + kTileM;  // prefetch the statistics of the next tile's row
-          const bool ok = (i + 1 < n_q) && nr < q_limit;
-          lse_next = INFINITY;
-          delta_next = 0.f;
-          if (ok) {
-            lse_next = a.lse[lse_base + nr];
-            delta_next = a.delta[delta_base + nr];
-          }
-        }
-
-        // keep decisions of the 32 columns: two Philox draws, computed together (their rounds
-        // interleave) and before S and dP are needed
-        [[maybe_unused]] uint32_t kw8[8];
+        // Keep decisions of this thread's key and 32 query columns: two Philox draws (16 keys of one query row each),
+        // made before S is needed, packed to one bit per key and transposed over the warp.
+        [[maybe_unused]] uint32_t keep = 0u;
         if constexpr (DROP) {
           const uint32_t poff = *philox_off;
+          const uint32_t q_row = static_cast<uint32_t>(i * kTileM + cq * 32 + draw_col);
 #pragma unroll
           for (int d = 0; d < 2; ++d) {
-            const U4 draw = dropout_draw_keys(a.philox_keys, poff, gbh, static_cast<uint32_t>(q_row),
-                                         static_cast<uint32_t>((k0 + cbase) / 16 + d));
-            kw8[d * 4 + 0] = (draw.x & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-            kw8[d * 4 + 1] = (draw.y & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-            kw8[d * 4 + 2] = (draw.z & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-            kw8[d * 4 + 3] = (draw.w & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-          }
-        }
-        wait_all(sdp_full, t & 1, kSiteSdpFull);
-        // The 32 columns are processed as two halves of 16: the second half of S and dP is fetched
-        // from tensor memory only after the first has been turned into packed P and dS, which keeps
-        // 32 fewer values live (the kernel is bound by the ALU pipe, and with all 64 values in
-        // registers the compiler spilled and shuffled registers in this loop).
-        uint32_t pk_p[16], pk_ds[16];  // 32 columns: 16 packed pairs each
-        auto half_chunk = [&](auto edge_tag, auto half_tag, const uint32_t (&rs)[16], const uint32_t (&rp)[16]) {
-          constexpr bool EDGE = decltype(edge_tag)::value;
-          constexpr int HALF = decltype(half_tag)::value;
-          const float2 sl22 = make_float2(sl2, sl2);
-          const float2 nl2 = make_float2(neg_lse2, neg_lse2);
-          const float2 nd2 = make_float2(-delta, -delta);
+            const U4 u = dropout_draw_keys(a.philox_keys, poff, gbh, q_row, static_cast<uint32_t>((cur.k0 + quad * 32) / 16 + d));
+            const uint32_t ws[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int col = cbase + HALF * 16 + 2 * k;       // column of the pair within the tile
-            float2 x = make_float2(__uint_as_float(rs[2 * k]), __uint_as_float(rs[2 * k + 1]));
-            if constexpr (KEYADD) {
-              const float2 mk = *reinterpret_cast<const float2*>(mask_row + col);
-              x = __fadd2_rn(__ffma2_rn(x, sl22, mk), nl2);
-            } else {
-              x = __ffma2_rn(x, sl22, nl2);
-            }
-            float2 p;
-            p.x = fast_exp2(x.x);
-            p.y = fast_exp2(x.y);
-            if constexpr (EDGE) {                            // keys past the valid length / tensor edge
-              if (col >= n_cols) p.x = 0.f;
-              if (col + 1 >= n_cols) p.y = 0.f;
-            }
-            const float2 dp = make_float2(__uint_as_float(rp[2 * k]), __uint_as_float(rp[2 * k + 1]));
-            float2 pkeep = p;
-            if constexpr (DROP) {
-              // bit 7 of byte e of the keep word decides element e; the permute smears it over 32 bits
-              const uint32_t kw = kw8[HALF * 4 + (k >> 1)];
-              const uint32_t m0 = prmt(kw, 0u, (k & 1) ? 0xAAAAu : 0x8888u);
-              const uint32_t m1 = prmt(kw, 0u, (k & 1) ? 0xBBBBu : 0x9999u);
-              pkeep.x = __uint_as_float(__float_as_uint(p.x) & m0);
-              pkeep.y = __uint_as_float(__float_as_uint(p.y) & m1);
-            }
-            const float2 ds = __ffma2_rn(pkeep, dp, __fmul2_rn(p, nd2));
-            pk_p[HALF * 8 + k] = pack2<BF16>(pkeep.x, pkeep.y);
-            pk_ds[HALF * 8 + k] = pack2<BF16>(ds.x, ds.y);
+            for (int k = 0; k < 4; ++k)   // the keep bit of key 16d + 4k + e ends as bit 8e + 4d + k
+              keep = (keep >> 1) | (((ws[k] & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u) & 0x80808080u);
           }
-        };
-        {
-          uint32_t rs[16], rp[16];
-          tmem_ld16(tmem_base + lane_addr + kColS + cbase, rs);
-          tmem_ld16(tmem_base + lane_addr + kColdP + cbase, rp);
-          tmem_wait_ld_dep16(rs, rp);
-          if (n_cols >= kTileN) half_chunk(std::false_type{}, std::integral_constant<int, 0>{}, rs, rp);
-          else half_chunk(std::true_type{}, std::integral_constant<int, 0>{}, rs, rp);
+          keep = warp_bit_transpose(keep, lane);
+          keep = __shfl_sync(0xffffffffu, keep, 8 * (lane & 3) + (lane >> 2));
         }
-        {
-          uint32_t rs[16], rp[16];
-          tmem_ld16(tmem_base + lane_addr + kColS + cbase + 16, rs);
-          tmem_ld16(tmem_base + lane_addr + kColdP + cbase + 16, rp);
-          tmem_wait_ld_dep16(rs, rp);
-          tc_fence_before_sync();
-          mbar_arrive(sdp_free);   // the tensor core may overwrite S and dP now
-          if (n_cols >= kTileN) half_chunk(std::false_type{}, std::integral_constant<int, 1>{}, rs, rp);
-          else half_chunk(std::true_type{}, std::integral_constant<int, 1>{}, rs, rp);
-        }
-
-        if constexpr (EARLY) {
-          // dQ of the previous tile is complete <=> the MMAs which read the single P/dS buffer have
-          // completed, so it can be overwritten below (the dQ tile itself is read out afterwards).
-          if (t > 0) wait_all(dq_full, (t - 1) & 1, kSiteDqFull);
-        } else {
-          // D = 128: the previous tile's dQ was staged in the P/dS buffers; the reduce must have read them.
-          if (t > 0) {
-            if (lane == 0) tma_store_wait_read();
-            named_bar_sync(2, kComputeThreads);
+        const uint32_t stats = smem_u32(sStats + (t & 1) * 2 * kTileM + cq * 32);
+        mbar_wait(stat_full + (t & 1), (t >> 1) & 1, wctx, kSiteStatFull, kComputeSleepNs);
+        wait_all(s_full, t & 1, kSiteSFull);
+        // ---- P ----------------------------------------------------------------------------------------------------------
+        uint32_t p[32];
+        tmem_ld32(tmem_base + lane_addr + kColS + cq * 32, p);
+        tmem_wait_ld_dep(p);
+        const float2 sl22 = make_float2(sl2, sl2);
+        const float2 add2 = make_float2(key_add, key_add);
+        uint32_t pk[16];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {   // four columns at a time
+          const uint4 nl = lds128(stats + j * 16);
+          float2 l0 = make_float2(__uint_as_float(nl.x), __uint_as_float(nl.y)), l1 = make_float2(__uint_as_float(nl.z), __uint_as_float(nl.w));
+          if constexpr (KEYADD) {
+            l0 = __fadd2_rn(l0, add2);
+            l1 = __fadd2_rn(l1, add2);
           }
+          const float2 x0 = __ffma2_rn(make_float2(__uint_as_float(p[4 * j]), __uint_as_float(p[4 * j + 1])), sl22, l0);
+          const float2 x1 = __ffma2_rn(make_float2(__uint_as_float(p[4 * j + 2]), __uint_as_float(p[4 * j + 3])), sl22, l1);
+          const float e0 = fast_exp2(x0.x), e1 = fast_exp2(x0.y), e2 = fast_exp2(x1.x), e3 = fast_exp2(x1.y);
+          p[4 * j] = __float_as_uint(e0);
+          p[4 * j + 1] = __float_as_uint(e1);
+          p[4 * j + 2] = __float_as_uint(e2);
+          p[4 * j + 3] = __float_as_uint(e3);
+          pk[2 * j] = pack2<BF16>(e0, e1);
+          pk[2 * j + 1] = pack2<BF16>(e2, e3);
+          if constexpr (DROP) {
+            pk[2 * j] &= prmt(keep << j, 0u, 0x9988u);
+            pk[2 * j + 1] &= prmt(keep << j, 0u, 0xBBAAu);
+          }
+        }
+        if (n_cols < kTileN && !key_ok) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) pk[k] = 0u;
         }
         if (i == 0 && prev_id >= 0) {
-          // dK and dV of the previous item: complete since its last dV/dK MMAs, and they must be out
-          // of tensor memory before this tile's P and dS let the tensor core overwrite them.
+          // dK and dV of the previous item must be out of tensor memory before this tile's P lets the tensor core
+          // overwrite dV.
           wait_all(acc_full, (w - 1) & 1, kSiteAccFull);
-          if constexpr (OWNSTAGE) {
-            own_stage_free();
-            store_dkdv(prev_id, true);
-          } else {
-            store_dkdv(prev_id, true);
-            if (lane == 0) tma_store_wait_read();   // every warp's slice must be read before P and dS land there
-            named_bar_sync(2, kComputeThreads);
-          }
-          tc_fence_before_sync();
+          store_dkdv(prev_id, true);
           prev_id = -1;
         }
-        {
-          // columns [32*cq, +32) of row `row`: 64 bytes = 16-byte chunks (cq%2)*4 .. +3 of sub-tile cq/2
-          const uint32_t bufP = smem_u32(sP + (cq >> 1) * 16384);
-          const uint32_t bufS = smem_u32(sdS + (cq >> 1) * 16384);
+        if (D == 64 && t > 0) mbar_wait(do_empty + (t - 1) % OS, ((t - 1) / OS) & 1, wctx, kSiteDoEmpty, kComputeSleepNs);   // dV(t-1) has read P
+        tmem_st16(tmem_base + lane_addr + kColP + cq * kPStride, pk);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(p_full);
+        if (D == 128 && !dq_out) dq_readout(t - 1, prev_row0);
+        // ---- dS -----------------------------------------------------------------------------------------------------------
+        wait_all(dp_full, t & 1, kSiteDpFull);
+        uint32_t dp[32];
+        tmem_ld32(tmem_base + lane_addr + kColdP + cq * 32, dp);
+        tmem_wait_ld_dep(dp);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t off = sw128_offset(row, (cq & 1) * 4 + q);
-            sts128(bufP + off, pk_p[q * 4], pk_p[q * 4 + 1], pk_p[q * 4 + 2], pk_p[q * 4 + 3]);
-            sts128(bufS + off, pk_ds[q * 4], pk_ds[q * 4 + 1], pk_ds[q * 4 + 2], pk_ds[q * 4 + 3]);
+        for (int j = 0; j < 8; ++j) {
+          const uint4 de = lds128(stats + kTileM * 4 + j * 16);
+          if constexpr (DROP) {
+            const uint32_t y = keep << j;
+            dp[4 * j] &= prmt(y, 0u, 0x8888u);
+            dp[4 * j + 1] &= prmt(y, 0u, 0x9999u);
+            dp[4 * j + 2] &= prmt(y, 0u, 0xAAAAu);
+            dp[4 * j + 3] &= prmt(y, 0u, 0xBBBBu);
           }
+          const float2 d0 = __fadd2_rn(make_float2(__uint_as_float(dp[4 * j]), __uint_as_float(dp[4 * j + 1])),
+                                       make_float2(-__uint_as_float(de.x), -__uint_as_float(de.y)));
+          const float2 d1 = __fadd2_rn(make_float2(__uint_as_float(dp[4 * j + 2]), __uint_as_float(dp[4 * j + 3])),
+                                       make_float2(-__uint_as_float(de.z), -__uint_as_float(de.w)));
+          const float2 s0 = __fmul2_rn(make_float2(__uint_as_float(p[4 * j]), __uint_as_float(p[4 * j + 1])), d0);
+          const float2 s1 = __fmul2_rn(make_float2(__uint_as_float(p[4 * j + 2]), __uint_as_float(p[4 * j + 3])), d1);
+          pk[2 * j] = pack2<BF16>(s0.x, s0.y);
+          pk[2 * j + 1] = pack2<BF16>(s1.x, s1.y);
+        }
+        if (n_cols < kTileN && !key_ok) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) pk[k] = 0u;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(stat_empty + (t & 1));
+        {
+          // query columns [32*cq, +32) of key `row`: 64 bytes = 16-byte chunks (cq%2)*4 .. +3 of sub-tile cq/2
+          const uint32_t buf = smem_u32(sdS + (t % DS) * L::kDsBytes + (cq >> 1) * 16384);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            sts128(buf + sw128_offset(row, (cq & 1) * 4 + q), pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
         }
         fence_proxy_async_smem();
-        mbar_arrive(pds_full);
-        const int row0 = bh * a.S_q_pad + i * kTileM;
-        if constexpr (EARLY) {
-          if (t > 0) dq_readout_warp(t - 1, prev_row0);
-          prev_row0 = row0;
-        } else {
-          dq_readout_tma(t, row0);   // D = 128: dQ shares columns with dP, it must be out before dP of tile t+1
-        }
+        tc_fence_before_sync();
+        mbar_arrive(ds_full);
+        if (D == 64 && !dq_out) dq_readout(t - 1, prev_row0);
+        dq_out = false;
+        prev_row0 = static_cast<int64_t>(bh) * a.S_q_pad + i * kTileM;
       }
       prev_id = cur.id;
       ++w;
     }
     // ---- drain: the last tile's dQ and the last item's dK, dV ------------------------------
-    if constexpr (EARLY) {
-      if (t > 0) dq_readout_warp(t - 1, prev_row0);
-    }
+    if (!dq_out) dq_readout(t - 1, prev_row0);
     if (prev_id >= 0) {
       wait_all(acc_full, (w - 1) & 1, kSiteAccFull);
-      if constexpr (OWNSTAGE) {
-        own_stage_free();
-      } else {
-        if (lane == 0) tma_store_wait_read();  // the last dQ reduces have read the P/dS buffers
-        named_bar_sync(2, kComputeThreads);
-      }
       store_dkdv(prev_id, true);
     }
     if (lane == 0) tma_store_wait_read();   // shared memory stays valid until the TMA unit has read it
@@ -989,10 +977,12 @@ int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int 
   f.dq_accum = dq_accum; f.dq = dq.ptr;
   f.sb = dq.stride_b; f.sh = dq.stride_h; f.ss = dq.stride_s;
   f.B = B; f.H = H; f.S_q = S_q; f.S_q_pad = S_q_pad; f.D = D; f.scale = scale; f.cu_seqlens = cu_seqlens;
-  const int rows_per_block = 256 / (D / 8);
-  const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q + rows_per_block - 1) / rows_per_block));
-  const cudaError_t e = launch_overlapped(dtype == FMHA_DTYPE_BF16 ? bwd_finish_kernel<true> : bwd_finish_kernel<false>, grid,
-                                          dim3(256), 0, stream, f);
+  const bool bf = dtype == FMHA_DTYPE_BF16;
+  const int rows = kFinishElems / D;
+  const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q + rows - 1) / rows));
+  auto kfn = D == 64 ? (bf ? bwd_finish_kernel<64, true> : bwd_finish_kernel<64, false>)
+                     : (bf ? bwd_finish_kernel<128, true> : bwd_finish_kernel<128, false>);
+  const cudaError_t e = launch_overlapped(kfn, grid, dim3(256), 0, stream, f);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 

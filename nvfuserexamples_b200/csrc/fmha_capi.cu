@@ -62,27 +62,6 @@ static int make_tmap(CUtensorMap* out, const fmha_tensor4& t, int dtype, int B, 
   return FMHA_OK;
 }
 
-// Tensor map of the fp32 dQ accumulator [rows, D].  One box per compute warp, so that no CTA-wide barrier is
-// needed around the staging buffer: its 32 rows x 16 columns with 64-byte swizzle at D = 64, its 32 rows x
-// 32 columns with 128-byte swizzle at D = 128.
-static int make_tmap_accum(CUtensorMap* out, float* ptr, uint64_t rows, int D) {
-  auto enc = get_encode_fn();
-  if (enc == nullptr) return FMHA_ERR_LAUNCH;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(D) * 4};
-  const bool per_warp = (D == 64);   // box = one warp's slice: 32 rows x 16 columns (D = 64) or x 32 (D = 128)
-  const cuuint32_t box[2] = {per_warp ? 16u : 32u, 32u};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   per_warp ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    g_last_cuda_error = static_cast<int>(r);
-    return FMHA_ERR_LAUNCH;
-  }
-  return FMHA_OK;
-}
-
 // Tensor map of a dense 16-bit [rows, cols] mask with {64 x 128} boxes and 128-byte swizzle.
 static int make_tmap_dense(CUtensorMap* out, const void* ptr, int dtype, uint64_t rows, uint64_t cols) {
   auto enc = get_encode_fn();
@@ -363,7 +342,6 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
   a.dk_ptr = tdk.ptr; a.dk_ss = tdk.stride_s; a.dk_sh = tdk.stride_h;
   a.dv_ptr = tdv.ptr; a.dv_ss = tdv.stride_s; a.dv_sh = tdv.stride_h;
   const int* cu_seqlens = packed ? reinterpret_cast<const int*>(p->mask) : nullptr;
-  if ((rc = make_tmap_accum(&a.tm_dq, dq_accum, static_cast<uint64_t>(bh) * s_q_pad, p->D))) return rc;
   a.B = p->B; a.H = p->H; a.S_q = p->S_q; a.S_k = p->S_k;
   a.scale = p->scale;
   a.scale_log2 = p->scale * 1.4426950408889634f;

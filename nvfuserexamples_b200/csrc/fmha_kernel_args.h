@@ -72,13 +72,12 @@ struct BwdArgs {
   alignas(64) CUtensorMap tm_do;
   alignas(64) CUtensorMap tm_dk;  // 16-bit outputs, {D/4 x 32} boxes (one per compute warp), no swizzle
   alignas(64) CUtensorMap tm_dv;
-  alignas(64) CUtensorMap tm_dq;  // fp32 dQ accumulator as [B*H*S_q_pad, D], 32-column boxes (TMA reduce-add)
   int B, H, S_q, S_k;
   float scale;       // softmax scale
   float scale_log2;  // softmax scale * log2(e)
   const float* lse;  // [B*H, S_q] natural log
   const float* delta;  // [B*H, S_q] rowsum(dO * O)
-  float* dq_accum;     // [B*H, S_q_pad, D] fp32, zero on entry
+  float* dq_accum;     // [B*H, S_q_pad, D] fp32 in the blocked order of dq_accum_index, zero on entry
   int* work_counter;   // zero on entry; the persistent CTAs draw their work items from it
   // FMHA_MASK_CU_SEQLENS: mask = int32 [B+1] row offsets into the packed [total_rows, H, D] tensors; the raw
   // dK / dV pointers serve the row-wise stores of a sequence's last, partial key tile

@@ -233,13 +233,9 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_
       ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-// Bulk reduction shared -> global: every element of the 2-D box is ADDED to the tensor in global
-// memory by the TMA unit (asynchronous, tracked by the same bulk groups as stores).
-__device__ __forceinline__ void tma_reduce_add_2d(const void* tmap, const void* smem_src, int c0, int c1) {
-  asm volatile(
-      "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-      ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
-      : "memory");
+// Adds four consecutive floats to global memory (no result), 16-byte aligned.
+__device__ __forceinline__ void red_add_v4(float* p, float x, float y, float z, float w) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 // First statement of every kernel that is launched with programmatic stream serialization (see
 // launch_overlapped): returns once the preceding kernels of the stream have completed and their
@@ -431,6 +427,26 @@ __device__ __forceinline__ void umma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uin
       "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], %6, %7, q;\n\t"
       "}\n"
       ::"r"(d_tmem), "r"(a_tmem), "r"(a_step), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "r"(idesc), "r"(acc_first)
+      : "memory");
+}
+// The same with the four A tiles in two pairs: MMAs 0 and 1 at a0 and a0 + a_step, 2 and 3 at a1 and a1 + a_step.
+__device__ __forceinline__ void umma_ts_2x2(uint32_t d_tmem, uint32_t a0, uint32_t a1, uint32_t a_step, const uint64_t (&b)[4],
+                                            uint32_t idesc, uint32_t acc_first) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q, pe;\n\t"
+      ".reg .b32 s0, s1;\n\t"
+      "setp.ne.b32 p, %9, 0;\n\t"
+      "setp.eq.b32 q, 0, 0;\n\t"
+      "add.u32 s0, %1, %3;\n\t"
+      "add.u32 s1, %2, %3;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %4, %8, p;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [s0], %5, %8, q;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %6, %8, q;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [s1], %7, %8, q;\n\t"
+      "}\n"
+      ::"r"(d_tmem), "r"(a0), "r"(a1), "r"(a_step), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "r"(idesc), "r"(acc_first)
       : "memory");
 }
 // tcgen05.commit by the elected lane of a converged warp.  elect.sync picks the same lane every
