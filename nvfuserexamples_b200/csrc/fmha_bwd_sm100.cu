@@ -5,21 +5,21 @@
 // (fmha/fmha_manual.cpp:891-897).  This backward needs neither: it recomputes the
 // probabilities from Q, K and the per-row logsumexp the forward kernel wrote.
 //
-// Three kernels per call:
+// Head dimension 64, three kernels per call:
 //   1. bwd_prepare : delta[row] = sum_d dO[row,d] * O[row,d]  and zero the fp32 dQ accumulator
 //   2. bwd_main    : persistent CTAs (one per SM) draw (128-key tile, head, batch) work items from a
 //                    counter and loop over the 128-row query tiles of each
-//                      S  = Q K^T            dP = dO V^T              (tcgen05.mma, fp32 in TMEM)
-//                      P  = exp2(S*scale*log2e + mask - lse*log2e)   (16 warps, thread = row, a quarter of the columns)
-//                      dS = P * (keep*c*dP - delta)                   c = 1/(1-p_drop)
+//                      S^T = K Q^T           dP^T = V dO^T            (tcgen05.mma, fp32 in TMEM)
+//                      P  = exp2(S*scale*log2e + mask - lse*log2e)   (16 warps, thread = key, a quarter of the queries)
+//                      dS = P * (keep*dP - delta/c)                   c = 1/(1-p_drop)
 //                      dV += (keep*P)^T dO     dK += dS^T Q     dQ_tile = dS K
-//                    P and dS go through shared memory (16-bit, 128-byte swizzle) and are read
-//                    by the tensor core both as K-major (dQ) and as MN-major (dV, dK) operands;
-//                    dQ tiles are staged in shared memory and added to the fp32 accumulator by TMA
-//                    reduce-add (cp.reduce.async.bulk.tensor ... .add);
-//                    dK and dV leave through per-warp staging tiles and TMA stores when the next item is
-//                    already under way.
+//                    P^T goes to tensor memory as the A operand of dV, dS^T to shared memory (16-bit, 128-byte swizzle),
+//                    where the tensor core reads it as K-major (dK) and as MN-major (dQ) operand; dQ tiles are added to
+//                    the fp32 accumulator from registers; dK and dV leave through per-warp staging tiles and TMA stores
+//                    when the next item is already under way.
 //   3. bwd_finish  : dQ = (scale * accumulator) rounded to the 16-bit dtype
+// Head dimension 128: the kernel in fmha_bwd_dq_sm100.cu writes dQ and delta, then bwd_main as above without dQ (dS^T stays
+// in tensor memory).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -48,20 +48,20 @@ constexpr int kBwdThreads = 64 + kComputeThreads + 32;   // + producer warp + MM
 constexpr float kLog2eB = 1.4426950408889634f;
 
 enum BwdWaitSite {
-  kSiteKvFull = 201, kSiteQFull = 202, kSiteQEmpty = 203, kSiteSFull = 204, kSitePFull = 205, kSiteDqFull = 206,
-  kSiteDqFree = 207, kSiteAccFull = 208, kSiteDpFull = 209, kSiteKvEmpty = 210, kSiteItemFull = 211, kSiteItemEmpty = 212,
-  kSiteDoFull = 213, kSiteDoEmpty = 214, kSiteDsFull = 215, kSiteStatFull = 216, kSiteStatEmpty = 217, kSiteSmemBase = 218
+  kSiteKFull = 201, kSiteQFull = 202, kSiteQEmpty = 203, kSiteSFull = 204, kSitePFull = 205, kSiteDqFull = 206,
+  kSiteDqFree = 207, kSiteAccFull = 208, kSiteDpFull = 209, kSiteKEmpty = 210, kSiteItemFull = 211, kSiteItemEmpty = 212,
+  kSiteDoFull = 213, kSiteDoEmpty = 214, kSiteDsFull = 215, kSiteStatFull = 216, kSiteStatEmpty = 217, kSiteSmemBase = 218,
+  kSiteVFull = 219, kSiteVEmpty = 220
 };
 
 template <int D>
 struct BwdSmem {
-  // D = 64: two K/V buffers (the next work item's K and V arrive while this one finishes), two stages of Q and of dO
-  // and two dS buffers.  D = 128: one K/V buffer, two stages of Q, one of dO (dV is its last reader and comes early in a
-  // tile's MMAs; Q is needed by dK, the last but one) and one dS buffer.
+  // Two stages of Q and of dO.  D = 64: two K/V buffers (the next work item's K and V arrive while this one finishes) and
+  // two dS buffers.  D = 128: one K/V buffer, read for the last time a tile before the item ends, and no dS buffers.
   static constexpr int kKvBufs = (D == 64) ? 2 : 1;
   static constexpr int kQStages = 2;
-  static constexpr int kDoStages = (D == 64) ? 2 : 1;
-  static constexpr int kDsBufs = (D == 64) ? 2 : 1;
+  static constexpr int kDoStages = 2;
+  static constexpr int kDsBufs = (D == 64) ? 2 : 0;
   static constexpr int kTileBytes = kTileM * D * 2;
   static constexpr int kDsBytes = kTileM * kTileN * 2;
   static constexpr int kOffK = 0;
@@ -73,7 +73,7 @@ struct BwdSmem {
   static constexpr int kOffStage = kOffdS + kDsBufs * kDsBytes;
   static constexpr int kOffStats = kOffStage + 32768;         // 2 slots x (128 of -lse*log2e, 128 of delta/c)
   static constexpr int kOffBar = kOffStats + 2 * 2 * kTileM * 4;
-  static constexpr int kNumBars = 7 + 2 * kKvBufs + 2 * kQStages + 2 * kDoStages + 8;
+  static constexpr int kNumBars = 7 + 4 * kKvBufs + 2 * kQStages + 2 * kDoStages + 8;
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;
   static constexpr int kBytes = kOffMisc + 32;
   // The tiles need a 1024-byte aligned base.  Dynamic shared memory of a kernel without static shared memory begins at
@@ -87,11 +87,12 @@ struct BwdSmem {
 // ---------------------------------------------------------------------------------------
 // 1. delta and accumulator clearing
 // ---------------------------------------------------------------------------------------
+constexpr int kAccumD = 64;   // the head dimension whose dQ goes through the fp32 accumulator
 struct PrepArgs {
   const void* o;
   const void* d_o;
   int64_t o_sb, o_sh, o_ss, do_sb, do_sh, do_ss;
-  int B, H, S_q, S_q_pad, D;
+  int B, H, S_q, S_q_pad;
   float* delta;     // [B*H, S_q]
   float* dq_accum;  // [B*H, S_q_pad, D]
   int* work_counter;  // the main kernel's work-item counter, cleared here
@@ -102,9 +103,9 @@ struct PrepArgs {
 template <bool BF16>
 __global__ void __launch_bounds__(256) bwd_prepare_kernel(const PrepArgs a) {
   griddep_wait();
-  // grid = (B*H, blocks of 32 rows); 8 threads per row (D = 64: 8 elements each; D = 128: 16 each).
+  // grid = (B*H, blocks of 32 rows); 8 threads per row, 8 elements each.
   // The head index comes from the grid, so no thread divides 64-bit indices.
-  const int per = a.D / 8;
+  constexpr int D = kAccumD, per = D / 8;
   const int part = threadIdx.x & 7;
   const int bh = blockIdx.x;
   const int h = bh % a.H;
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const PrepArgs a) {
   const bool in_range = r < a.S_q_pad;  // no early exit: the shuffles below need every lane
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && a.work_counter != nullptr) *a.work_counter = 0;
   if (in_range) {
-    float4* acc = reinterpret_cast<float4*>(a.dq_accum + (static_cast<int64_t>(bh) * a.S_q_pad + r) * a.D + part * per);
+    float4* acc = reinterpret_cast<float4*>(a.dq_accum + (static_cast<int64_t>(bh) * a.S_q_pad + r) * D + part * per);
     for (int i = 0; i < per / 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   // packed batch: row r of sequence b is row cu[b] + r of the tensors, and exists for r < cu[b+1] - cu[b]
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const PrepArgs a) {
     if (blockIdx.y == 0 && a.zero.grad[0].ptr != nullptr) {
       for (int t = 0; t < 3; ++t)
         zero_uncovered_rows(a.zero.grad[t].ptr, a.zero.grad[t].stride_s, a.zero.grad[t].stride_h, h, b, a.B, a.cu_seqlens, a.S_q,
-                            a.zero.total_rows, a.D, threadIdx.x, blockDim.x);
+                            a.zero.total_rows, D, threadIdx.x, blockDim.x);
     }
     row_o = static_cast<int64_t>(base + r) * a.o_ss;
     row_do = static_cast<int64_t>(base + r) * a.do_ss;
@@ -160,18 +161,18 @@ struct FinishArgs {
   const float* dq_accum;
   void* dq;
   int64_t sb, sh, ss;
-  int B, H, S_q, S_q_pad, D;
+  int B, H, S_q, S_q_pad;
   float scale;
   const int* cu_seqlens;  // packed batch: row offsets into the [total_rows, H, D] dQ (sb unused), else null
 };
 
-// A block converts 8192 elements, whole rows of a head: coalesced 16-byte reads of the accumulator (eight in flight per thread),
+// A block converts 128 rows of a head: coalesced 16-byte reads of the accumulator (eight in flight per thread),
 // through shared memory to coalesced 16-byte writes of the rows.
-constexpr int kFinishElems = 8192;   // per block
-template <int D, bool BF16>
+constexpr int kFinishRows = 128;
+template <bool BF16>
 __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
   griddep_wait();
-  constexpr int R = kFinishElems / D;   // 128 or 64 rows
+  constexpr int D = kAccumD, R = kFinishRows;
   constexpr int kStride = D * 2 + 8;    // bytes; 8-byte accesses of consecutive rows hit different banks
   __shared__ __align__(16) uint8_t tile[R * kStride];
   const int bh = blockIdx.x;
@@ -222,17 +223,17 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
 // P^T, written back to tensor memory by the thread that computed it, is the A operand of dV += P^T dO: it is neither
 // written to shared memory nor read from it.  What limits this kernel is shared-memory bandwidth: with P and dS both
 // staged there a D = 64 tile moved 2 944 cycles' worth of shared-memory data (MMA operands 1 664, P/dS 512, TMA in and out
-// 768), now 2 432; and the freed 32 KB is a second dS buffer (D = 64) or a second Q stage (D = 128), without which every
-// tile waited for the previous tile's MMAs (D = 64) or for the reload of Q and dO (D = 128).
+// 768).  At D = 128 dS^T stays in tensor memory in the same way, as the A operand of dK += dS^T Q, and dQ is another kernel's
+// (fmha_bwd_dq_sm100.cu); at D = 64 dS also feeds dQ = dS K and goes to shared memory.
 // In this layout a thread is a key: lse and delta vary along its columns and come from shared memory (broadcast reads;
 // a helper warp fetches them one to two tiles ahead), the additive key mask is one value per thread, and the dropout
 // draws, which give 16 keys of one query row each, are made by the thread of that row and transposed in the warp.
 //
 // Schedule inside the stream of (item, query tile) pairs, numbered t = 0, 1, ...:
-//   compute warps:  S(t) -> P(t) -> tensor memory (p_full) -> [D = 128: dQ(t-1) out] -> dP(t) -> dS(t) -> shared memory
-//                   (ds_full) -> [D = 64: dQ(t-1) out]; dK and dV of an item leave when the next item's first P is ready.
-//   MMA warp:       on p_full(t): dV(t), S(t+1); on ds_full(t): [D = 64: dP(t+1)], dK(t), dQ(t), [D = 128: dP(t+1), whose
-//                   columns dQ(t) shares, when dQ(t) has been read out].  S(t+1) and dP(t+1) may belong to the next item.
+//   compute warps:  S(t) -> P(t) -> tensor memory (p_full) -> dP(t) -> dS(t) -> shared / tensor memory (ds_full) ->
+//                   [D = 64: dQ(t-1) out]; dK and dV of an item leave when the next item's first P is ready.
+//   MMA warp:       on p_full(t): dV(t), S(t+1); on ds_full(t), D = 64: dP(t+1), dK(t), dQ(t); D = 128: dK(t), dP(t+1), which
+//                   overwrites dS(t).  S(t+1) and dP(t+1) may belong to the next item.
 // Position of element (row, col) of a 128-row tile of the fp32 dQ accumulator: 32-row groups, in them groups of four
 // columns, in them the 32 rows with their four values each.
 template <int D>
@@ -273,10 +274,10 @@ template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
   griddep_wait();
   using L = BwdSmem<D>;
-  constexpr int QS = L::kQStages, OS = L::kDoStages, DS = L::kDsBufs, KV = L::kKvBufs;
+  constexpr int QS = L::kQStages, OS = L::kDoStages, DS = L::kDsBufs > 0 ? L::kDsBufs : 1, KV = L::kKvBufs;
   constexpr int kTmemCols = 512;
   constexpr uint32_t kColS = 0, kColdP = 128, kColdV = 256, kColdK = 256 + D;
-  constexpr uint32_t kColdQ = (D == 64) ? 384 : kColdP;   // D = 128: dQ takes the columns dP has been read from
+  constexpr uint32_t kColdQ = 384;   // D = 64
   // P^T, 16 columns per 32 query rows: beside everything else (D = 64), or over the thread's own columns of S (D = 128)
   constexpr uint32_t kColP = (D == 64) ? 448 : kColS, kPStride = (D == 64) ? 16 : 32;
   constexpr int kFmt = BF16 ? 1 : 0;
@@ -300,9 +301,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   uint64_t* dq_full = bars + 4;    // dQ tile is in tensor memory; dV/dK/dQ of that tile are complete
   uint64_t* dq_free = bars + 5;    // dQ tile has been read out (all compute threads arrive)
   uint64_t* acc_full = bars + 6;   // dK / dV of a work item are complete
-  uint64_t* kv_full = bars + 7;
-  uint64_t* kv_empty = kv_full + KV;
-  uint64_t* q_full = kv_empty + KV;
+  uint64_t* k_full = bars + 7;
+  uint64_t* k_empty = k_full + KV;   // D = 64: the item's last dQ has completed; D = 128: its last S
+  uint64_t* v_full = k_empty + KV;
+  uint64_t* v_empty = v_full + KV;   // the item's last dP has completed
+  uint64_t* q_full = v_empty + KV;
   uint64_t* q_empty = q_full + QS;
   uint64_t* do_full = q_empty + QS;
   uint64_t* do_empty = do_full + OS;      // dV of the tile has completed (so P may be overwritten, too)
@@ -338,8 +341,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     mbar_init(dq_free, kComputeThreads);
     mbar_init(acc_full, 1);
     for (int s = 0; s < KV; ++s) {
-      mbar_init(kv_full + s, 1);
-      mbar_init(kv_empty + s, 1);
+      mbar_init(k_full + s, 1);
+      mbar_init(k_empty + s, 1);
+      mbar_init(v_full + s, 1);
+      mbar_init(v_empty + s, 1);
     }
     for (int s = 0; s < QS; ++s) {
       mbar_init(q_full + s, 1);
@@ -434,13 +439,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         const BwdItem it = decode(id);
         if (it.n_cols <= 0) continue;
         const int kvb = w % KV;
-        if (w >= KV) mbar_wait(kv_empty + kvb, ((w / KV) - 1) & 1, wctx, kSiteKvEmpty);
-        mbar_arrive_expect_tx(kv_full + kvb, 2 * L::kTileBytes);
+        const uint32_t kvp = (w / KV - 1) & 1;
+        if (w >= KV) mbar_wait(k_empty + kvb, kvp, wctx, kSiteKEmpty);
+        mbar_arrive_expect_tx(k_full + kvb, L::kTileBytes);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) {
-          tma_load_4d(sK + kvb * L::kTileBytes + c * 16384, &a.tm_k, kv_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
-          tma_load_4d(sV + kvb * L::kTileBytes + c * 16384, &a.tm_v, kv_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
-        }
+        for (int c = 0; c < D / 64; ++c)
+          tma_load_4d(sK + kvb * L::kTileBytes + c * 16384, &a.tm_k, k_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
         for (int i = 0; i < it.n_q; ++i, ++g) {
           const int qs = g % QS, os = g % OS;
           if (g >= QS) mbar_wait(q_empty + qs, ((g / QS) - 1) & 1, wctx, kSiteQEmpty);
@@ -448,6 +452,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 #pragma unroll
           for (int c = 0; c < D / 64; ++c)
             tma_load_4d(sQ + qs * L::kTileBytes + c * 16384, &a.tm_q, q_full + qs, c * 64, it.row_base + i * kTileM, it.h, it.tb);
+          if (i == 0) {   // V after the first Q: with one K/V buffer it comes free after K
+            if (w >= KV) mbar_wait(v_empty + kvb, kvp, wctx, kSiteVEmpty);
+            mbar_arrive_expect_tx(v_full + kvb, L::kTileBytes);
+#pragma unroll
+            for (int c = 0; c < D / 64; ++c)
+              tma_load_4d(sV + kvb * L::kTileBytes + c * 16384, &a.tm_v, v_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
+          }
           if (g >= OS) mbar_wait(do_empty + os, ((g / OS) - 1) & 1, wctx, kSiteDoEmpty);
           mbar_arrive_expect_tx(do_full + os, L::kTileBytes);
 #pragma unroll
@@ -478,18 +489,22 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       if constexpr (KS == 4) umma_ss_x4(d, x, y, kIdescS, 0u);
       else umma_ss_x8(d, x, y, kIdescS, 0u);
     };
-    // S^T of tile tt (its Q stage) with the K buffer kvb
-    auto issue_s = [&](int tt, int kvb) {
+    // S^T and dP^T of tile tt, which belongs to item number wi (with work) and is its first / last one
+    auto issue_s = [&](int tt, int wi, bool first, bool last) {
+      if (first) mbar_wait(k_full + wi % KV, (wi / KV) & 1, wctx, kSiteKFull);
       mbar_wait(q_full + tt % QS, (tt / QS) & 1, wctx, kSiteQFull);
       tc_fence_after_sync();
-      issue_kk(tS, sK + kvb * L::kTileBytes, sQ + (tt % QS) * L::kTileBytes);
+      issue_kk(tS, sK + (wi % KV) * L::kTileBytes, sQ + (tt % QS) * L::kTileBytes);
       umma_commit_elect(s_full);
+      if (D == 128 && last) umma_commit_elect(k_empty + wi % KV);
     };
-    auto issue_dp = [&](int tt, int kvb) {
+    auto issue_dp = [&](int tt, int wi, bool first, bool last) {
+      if (first) mbar_wait(v_full + wi % KV, (wi / KV) & 1, wctx, kSiteVFull);
       mbar_wait(do_full + tt % OS, (tt / OS) & 1, wctx, kSiteDoFull);
       tc_fence_after_sync();
-      issue_kk(tdP, sV + kvb * L::kTileBytes, sdO + (tt % OS) * L::kTileBytes);
+      issue_kk(tdP, sV + (wi % KV) * L::kTileBytes, sdO + (tt % OS) * L::kTileBytes);
       umma_commit_elect(dp_full);
+      if (last) umma_commit_elect(v_empty + wi % KV);
     };
 
     int n = 0, w = 0, t = 0;   // items fetched, items with work, query tiles so far
@@ -500,9 +515,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     };
     BwdItem cur = next_work();
     if (cur.id >= 0) {
-      mbar_wait(kv_full, 0, wctx, kSiteKvFull);
-      issue_s(0, 0);
-      issue_dp(0, 0);
+      issue_s(0, 0, true, cur.n_q == 1);
+      issue_dp(0, 0, true, cur.n_q == 1);
     }
     while (cur.id >= 0) {
       const int kvb = w % KV;
@@ -512,7 +526,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       for (int i = 0; i < n_q; ++i, ++t) {
         const bool last = i + 1 == n_q;
         const int qs = t % QS, os = t % OS;
-        const uint8_t* ds_tile = sdS + (t % DS) * L::kDsBytes;
         const uint32_t acc0 = (i > 0) ? 1u : 0u;
         // ---- dV += P^T dO: A from tensor memory, dO read MN-major (16 query rows = 2048 B per k-step) ----------------
         const uint64_t ddO_m = make_smem_desc_sw128(smem_u32(sdO + os * L::kTileBytes), 16384, 1024);
@@ -529,25 +542,21 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           }
         }
         umma_commit_elect(do_empty + os);   // dP(t) came before, so dO(t) is not read again
-        // ---- S of the next tile: S(t) has been read (D = 128: and P(t), which lies over it) --------------------------------
-        // At the end of an item the next one is looked up here only where its K can be there already (D = 64); the compute
-        // warps finish tile t, and any items without keys that follow, without another MMA at D = 64, but not at D = 128.
-        if (D == 64 && last) nxt = next_work();
-        const int nkvb = last ? (w + 1) % KV : kvb;
-        if (!last || (D == 64 && nxt.id >= 0)) {
-          if (last) mbar_wait(kv_full + nkvb, ((w + 1) / KV) & 1, wctx, kSiteKvFull);
-          issue_s(t + 1, nkvb);
-        }
+        // ---- S of the next tile: S(t) has been read (D = 128: and P(t), which lies over it, by dV(t)) ------------------------
+        if (last) nxt = next_work();   // the compute warps finish tile t, and any items without keys, without another MMA
+        const bool more = !last || nxt.id >= 0;
+        const int wn = last ? w + 1 : w;                                  // item of tile t+1, and whether t+1 is its last tile
+        const bool next_last = last ? nxt.n_q == 1 : i + 2 == n_q;
+        if (more) issue_s(t + 1, wn, last, next_last);
         // ---- dK += dS^T Q, dQ tile = dS K -----------------------------------------------------------------------------------
         const uint64_t dQ_m = make_smem_desc_sw128(smem_u32(sQ + qs * L::kTileBytes), 16384, 1024);
-        const uint64_t ddS_k = make_smem_desc_sw128(smem_u32(ds_tile), 16, 1024);       // dS^T as K-major A (keys x queries)
-        const uint64_t ddS_m = make_smem_desc_sw128(smem_u32(ds_tile), 16384, 1024);    // dS as MN-major A (queries x keys)
         mbar_wait(ds_full, t & 1, wctx, kSiteDsFull);
         tc_fence_after_sync();
         if constexpr (D == 64) {
-          if (!last || nxt.id >= 0) issue_dp(t + 1, nkvb);   // dP(t) has been read
-        }
-        auto issue_dk = [&]() {
+          const uint8_t* ds_tile = sdS + (t % DS) * L::kDsBytes;
+          const uint64_t ddS_k = make_smem_desc_sw128(smem_u32(ds_tile), 16, 1024);       // dS^T as K-major A (keys x queries)
+          const uint64_t ddS_m = make_smem_desc_sw128(smem_u32(ds_tile), 16384, 1024);    // dS as MN-major A (queries x keys)
+          if (more) issue_dp(t + 1, wn, last, next_last);   // dP(t) has been read
           uint64_t x[8], y[8];
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
@@ -557,34 +566,29 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           umma_ss_x8(tdK, x, y, kIdescKN, acc0);
           umma_commit_elect(q_empty + qs);
           if (last) umma_commit_elect(acc_full);
-        };
-        if constexpr (D == 64) issue_dk();
-        if (D == 64 && t > 0) {
-          mbar_wait(dq_free, (t - 1) & 1, wctx, kSiteDqFree);
-          tc_fence_after_sync();
-        }
-        {
-          uint64_t x[8], y[8];
+          if (t > 0) {
+            mbar_wait(dq_free, (t - 1) & 1, wctx, kSiteDqFree);
+            tc_fence_after_sync();
+          }
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             x[kk] = ddS_m + mnmajor_step(kk);
             y[kk] = dK_m + mnmajor_step(kk);
           }
           umma_ss_x8(tdQ, x, y, kIdescMN, 0u);
-        }
-        umma_commit_elect(dq_full);
-        if constexpr (D == 128) issue_dk();   // under the read-out of dQ, which dP(t+1) waits for
-        if (last) umma_commit_elect(kv_empty + kvb);   // K and V of this item are not read again
-        if constexpr (D == 128) {
-          if (last) nxt = next_work();
-          if (!last || nxt.id >= 0) {
-            if (last) {   // the single K/V buffer has been reloaded
-              mbar_wait(kv_full, (w + 1) & 1, wctx, kSiteKvFull);
-              issue_s(t + 1, 0);
-            }
-            mbar_wait(dq_free, t & 1, wctx, kSiteDqFree);        // dQ shares the dP columns
-            issue_dp(t + 1, nkvb);
+          umma_commit_elect(dq_full);
+          if (last) umma_commit_elect(k_empty + kvb);   // K of this item is not read again
+        } else {
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            uint64_t y[4];
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) y[kk] = dQ_m + mnmajor_step(hf * 4 + kk);
+            umma_ts_2x2(tdK, tdP + hf * 64, tdP + hf * 64 + 32, 8u, y, kIdescKN, hf == 0 ? acc0 : 1u);
           }
+          umma_commit_elect(q_empty + qs);
+          if (last) umma_commit_elect(acc_full);
+          if (more) issue_dp(t + 1, wn, last, next_last);   // over dS(t): the tensor core works in order
         }
       }
       ++w;
@@ -660,7 +664,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     // accumulator is laid out so that a warp's instruction covers 512 consecutive bytes (dq_accum_index), which keeps the
     // tile out of shared memory: staged there for TMA reduce-adds it cost 32 (D = 64) or 64 KB written and read again per
     // tile, a fifth of all shared-memory traffic.
-    auto dq_readout = [&](int tt, int64_t row0) {
+    [[maybe_unused]] auto dq_readout = [&](int tt, int64_t row0) {   // D = 64
       wait_all(dq_full, tt & 1, kSiteDqFull);
       uint32_t r[DQ];
 #pragma unroll
@@ -730,8 +734,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 
     int n = 0, w = 0, t = 0;      // items fetched, items with work, query tiles so far
     int prev_id = -1;             // >= 0: dK/dV of that item are still in tensor memory
-    int64_t prev_row0 = 0;        // accumulator row of tile t-1
-    bool dq_out = true;           // dQ of tile t-1 has been read out
+    [[maybe_unused]] int64_t prev_row0 = 0;   // D = 64: accumulator row of tile t-1,
+    [[maybe_unused]] bool dq_out = true;      // and whether its dQ has been read out
 
     while (true) {
       const BwdItem cur = fetch_item(n++, kComputeSleepNs);
@@ -816,7 +820,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(p_full);
-        if (D == 128 && !dq_out) dq_readout(t - 1, prev_row0);
         // ---- dS -----------------------------------------------------------------------------------------------------------
         wait_all(dp_full, t & 1, kSiteDpFull);
         uint32_t dp[32];
@@ -847,25 +850,32 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(stat_empty + (t & 1));
-        {
+        if constexpr (D == 64) {
           // query columns [32*cq, +32) of key `row`: 64 bytes = 16-byte chunks (cq%2)*4 .. +3 of sub-tile cq/2
           const uint32_t buf = smem_u32(sdS + (t % DS) * L::kDsBytes + (cq >> 1) * 16384);
 #pragma unroll
           for (int q = 0; q < 4; ++q)
             sts128(buf + sw128_offset(row, (cq & 1) * 4 + q), pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
+          fence_proxy_async_smem();
+        } else {
+          tmem_st16(tmem_base + lane_addr + kColdP + cq * 32, pk);   // over this thread's own columns of dP
+          tmem_wait_st();
         }
-        fence_proxy_async_smem();
         tc_fence_before_sync();
         mbar_arrive(ds_full);
-        if (D == 64 && !dq_out) dq_readout(t - 1, prev_row0);
-        dq_out = false;
-        prev_row0 = static_cast<int64_t>(bh) * a.S_q_pad + i * kTileM;
+        if constexpr (D == 64) {
+          if (!dq_out) dq_readout(t - 1, prev_row0);
+          dq_out = false;
+          prev_row0 = static_cast<int64_t>(bh) * a.S_q_pad + i * kTileM;
+        }
       }
       prev_id = cur.id;
       ++w;
     }
     // ---- drain: the last tile's dQ and the last item's dK, dV ------------------------------
-    if (!dq_out) dq_readout(t - 1, prev_row0);
+    if constexpr (D == 64) {
+      if (!dq_out) dq_readout(t - 1, prev_row0);
+    }
     if (prev_id >= 0) {
       wait_all(acc_full, (w - 1) & 1, kSiteAccFull);
       store_dkdv(prev_id, true);
@@ -955,15 +965,13 @@ int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream) {
   return static_cast<int>(cudaErrorInvalidValue);
 }
 
-int launch_bwd_prepare(const void* o, const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad,
-                       int D, int dtype, float* delta, float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero,
-                       cudaStream_t stream) {
+int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad, int dtype, float* delta,
+                       float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero, cudaStream_t stream) {
   PrepArgs p;
   p.o = ot.ptr; p.d_o = dot.ptr;
-  (void)o;
   p.o_sb = ot.stride_b; p.o_sh = ot.stride_h; p.o_ss = ot.stride_s;
   p.do_sb = dot.stride_b; p.do_sh = dot.stride_h; p.do_ss = dot.stride_s;
-  p.B = B; p.H = H; p.S_q = S_q; p.S_q_pad = S_q_pad; p.D = D;
+  p.B = B; p.H = H; p.S_q = S_q; p.S_q_pad = S_q_pad;
   p.delta = delta; p.dq_accum = dq_accum; p.work_counter = work_counter; p.cu_seqlens = cu_seqlens; p.zero = zero;
   const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q_pad + 31) / 32));
   const cudaError_t e = launch_overlapped(dtype == FMHA_DTYPE_BF16 ? bwd_prepare_kernel<true> : bwd_prepare_kernel<false>, grid,
@@ -971,17 +979,14 @@ int launch_bwd_prepare(const void* o, const fmha_tensor4& ot, const fmha_tensor4
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int D, int dtype,
-                      float scale, const int* cu_seqlens, cudaStream_t stream) {
+int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int dtype, float scale,
+                      const int* cu_seqlens, cudaStream_t stream) {
   FinishArgs f;
   f.dq_accum = dq_accum; f.dq = dq.ptr;
   f.sb = dq.stride_b; f.sh = dq.stride_h; f.ss = dq.stride_s;
-  f.B = B; f.H = H; f.S_q = S_q; f.S_q_pad = S_q_pad; f.D = D; f.scale = scale; f.cu_seqlens = cu_seqlens;
-  const bool bf = dtype == FMHA_DTYPE_BF16;
-  const int rows = kFinishElems / D;
-  const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q + rows - 1) / rows));
-  auto kfn = D == 64 ? (bf ? bwd_finish_kernel<64, true> : bwd_finish_kernel<64, false>)
-                     : (bf ? bwd_finish_kernel<128, true> : bwd_finish_kernel<128, false>);
+  f.B = B; f.H = H; f.S_q = S_q; f.S_q_pad = S_q_pad; f.scale = scale; f.cu_seqlens = cu_seqlens;
+  const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q + kFinishRows - 1) / kFinishRows));
+  auto kfn = dtype == FMHA_DTYPE_BF16 ? bwd_finish_kernel<true> : bwd_finish_kernel<false>;
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(256), 0, stream, f);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

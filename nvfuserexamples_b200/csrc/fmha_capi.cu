@@ -273,6 +273,9 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
 
 static size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
+// fp32 dQ accumulator: at head dimension 128 dQ is finished inside one kernel and needs none.
+static size_t bwd_accum_bytes(size_t bh, size_t s_q_pad, int D) { return D == 64 ? bh * s_q_pad * D * sizeof(float) : 0; }
+
 int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes) {
   if (p == nullptr || bytes == nullptr) return FMHA_ERR_BAD_ARG;
   int rc = validate_common(p->struct_bytes, sizeof(fmha_bwd_params), p->dtype, p->B, p->H, p->S_q, p->S_k, p->D, p->scale);
@@ -280,7 +283,7 @@ int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes) {
   const size_t bh = static_cast<size_t>(p->B) * p->H;
   const size_t s_q_pad = (static_cast<size_t>(p->S_q) + kTileM - 1) / kTileM * kTileM;
   // fp32 dQ accumulator, delta, and the work-item counter of the persistent main kernel
-  *bytes = align256(bh * s_q_pad * p->D * sizeof(float)) + align256(bh * p->S_q * sizeof(float)) + 256;
+  *bytes = align256(bwd_accum_bytes(bh, s_q_pad, p->D)) + align256(bh * p->S_q * sizeof(float)) + 256;
   return FMHA_OK;
 }
 
@@ -319,7 +322,7 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
   const int s_q_pad = (p->S_q + kTileM - 1) / kTileM * kTileM;
   const size_t bh = static_cast<size_t>(p->B) * p->H;
   float* dq_accum = reinterpret_cast<float*>(p->workspace);
-  float* delta = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p->workspace) + align256(bh * s_q_pad * p->D * sizeof(float)));
+  float* delta = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p->workspace) + align256(bwd_accum_bytes(bh, s_q_pad, p->D)));
   int* work_counter = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(delta) + align256(bh * p->S_q * sizeof(float)));
 
   BwdArgs a;
@@ -366,24 +369,31 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
   a.philox_bh_offset = p->philox_bh_offset;
   a.status = p->status;
 
+  UncoveredRows zero = {};
+  if (packed && (p->flags & FMHA_FLAG_ZERO_UNCOVERED)) zero = {{tdq, tdk, tdv}, p->total_rows};
+  const bool two_pass = p->D == 128;   // dQ (and delta) in a kernel of its own; see fmha_bwd_dq_sm100.cu
   int e = 0;
-  if (!(p->flags & FMHA_FLAG_BWD_SKIP_PREPARE)) {
-    UncoveredRows zero = {};
-    if (packed && (p->flags & FMHA_FLAG_ZERO_UNCOVERED)) zero = {{tdq, tdk, tdv}, p->total_rows};
-    e = launch_bwd_prepare(nullptr, to, tdo, p->B, p->H, p->S_q, s_q_pad, p->D, p->dtype, delta, dq_accum, work_counter, cu_seqlens,
-                           zero, stream);
-    if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
-  } else {
+  if (p->flags & FMHA_FLAG_BWD_SKIP_PREPARE) {
     // the caller prepared delta and the accumulator itself; the work counter is still ours to clear
     cudaError_t ce = cudaMemsetAsync(work_counter, 0, sizeof(int), stream);
     if (ce != cudaSuccess) return cuda_fail(ce);
+  } else if (two_pass) {
+    if ((rc = make_tmap(&a.tm_dq, tdq, p->dtype, mB, p->H, mSq, p->D, 32, 16))) return rc;
+    a.o_ptr = to.ptr; a.o_sb = to.stride_b; a.o_sh = to.stride_h; a.o_ss = to.stride_s;
+    a.do_ptr = tdo.ptr; a.do_sb = tdo.stride_b; a.do_sh = tdo.stride_h; a.do_ss = tdo.stride_s;
+    a.dq_ptr = tdq.ptr; a.dq_ss = tdq.stride_s; a.dq_sh = tdq.stride_h;
+    a.zero = zero;
+    e = launch_bwd_dq(a, p->dtype, stream);
+    if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
+  } else {
+    e = launch_bwd_prepare(to, tdo, p->B, p->H, p->S_q, s_q_pad, p->dtype, delta, dq_accum, work_counter, cu_seqlens, zero, stream);
+    if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   }
   e = launch_bwd(a, p->D, p->dtype, stream);
   if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
-  if (!(p->flags & FMHA_FLAG_BWD_SKIP_FINISH)) {
+  if (!two_pass && !(p->flags & FMHA_FLAG_BWD_SKIP_FINISH)) {
     // the main kernel leaves the dropout factor 1/(1-p) out of dS; it is applied here (and to dK, dV in its epilogue)
-    e = launch_bwd_finish(dq_accum, tdq, p->B, p->H, p->S_q, s_q_pad, p->D, p->dtype, p->scale * a.dropout_scale, cu_seqlens,
-                          stream);
+    e = launch_bwd_finish(dq_accum, tdq, p->B, p->H, p->S_q, s_q_pad, p->dtype, p->scale * a.dropout_scale, cu_seqlens, stream);
     if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   }
   return FMHA_OK;

@@ -65,6 +65,12 @@ struct FwdArgs {
   int* status;
 };
 
+// FMHA_FLAG_ZERO_UNCOVERED of the backward pass: the three gradients whose uncovered rows are zeroed (ptr null: none).
+struct UncoveredRows {
+  fmha_tensor4 grad[3];
+  int total_rows;
+};
+
 struct BwdArgs {
   alignas(64) CUtensorMap tm_q;
   alignas(64) CUtensorMap tm_k;
@@ -72,12 +78,21 @@ struct BwdArgs {
   alignas(64) CUtensorMap tm_do;
   alignas(64) CUtensorMap tm_dk;  // 16-bit outputs, {D/4 x 32} boxes (one per compute warp), no swizzle
   alignas(64) CUtensorMap tm_dv;
+  // Head dimension 128, dQ kernel (fmha_bwd_dq_sm100.cu): 16-bit dQ in {16 x 32} boxes; O and dO for the row term delta
+  alignas(64) CUtensorMap tm_dq;
+  const void* o_ptr;
+  const void* do_ptr;
+  int64_t o_sb, o_sh, o_ss, do_sb, do_sh, do_ss;
+  void* dq_ptr;
+  int64_t dq_ss, dq_sh;
+  UncoveredRows zero;
+  int persist;   // a CTA takes further work items of the grid when it has done its own
   int B, H, S_q, S_k;
   float scale;       // softmax scale
   float scale_log2;  // softmax scale * log2(e)
   const float* lse;  // [B*H, S_q] natural log
-  const float* delta;  // [B*H, S_q] rowsum(dO * O)
-  float* dq_accum;     // [B*H, S_q_pad, D] fp32 in the blocked order of dq_accum_index, zero on entry
+  float* delta;        // [B*H, S_q] rowsum(dO * O)
+  float* dq_accum;     // head dimension 64: [B*H, S_q_pad, D] fp32 in the blocked order of dq_accum_index, zero on entry
   int* work_counter;   // zero on entry; the persistent CTAs draw their work items from it
   // FMHA_MASK_CU_SEQLENS: mask = int32 [B+1] row offsets into the packed [total_rows, H, D] tensors; the raw
   // dK / dV pointers serve the row-wise stores of a sequence's last, partial key tile
@@ -99,12 +114,6 @@ struct BwdArgs {
   int* status;
 };
 
-// FMHA_FLAG_ZERO_UNCOVERED of the backward pass: the three gradients whose uncovered rows are zeroed (ptr null: none).
-struct UncoveredRows {
-  fmha_tensor4 grad[3];
-  int total_rows;
-};
-
 // Launchers (defined in the .cu files).  Return a cudaError_t as int.
 int launch_fwd(const FwdArgs& a, int D, int dtype, bool legacy, bool p_via_smem, cudaStream_t stream);
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
@@ -114,12 +123,13 @@ int launch_fwd_rows(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
 // the persistent kernel of the dense-mask operators at head dimension 64 (fmha_fwd_dense_sm100.cu)
 bool fwd_dense_applies(const FwdArgs& a, int D);
 int launch_fwd_dense(const FwdArgs& a, int dtype, cudaStream_t stream);
+int launch_bwd_dq(const BwdArgs& a, int dtype, cudaStream_t stream);   // head dimension 128: dQ, delta, work counter
 int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream);
-int launch_bwd_prepare(const void* o, const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad,
-                       int D, int dtype, float* delta, float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero,
-                       cudaStream_t stream);
-int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int D, int dtype,
-                      float scale, const int* cu_seqlens, cudaStream_t stream);
+// head dimension 64: the passes before and after the main kernel
+int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad, int dtype, float* delta,
+                       float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero, cudaStream_t stream);
+int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int dtype, float scale,
+                      const int* cu_seqlens, cudaStream_t stream);
 
 // Multiprocessors of the current device, asked for once per device.
 inline int sm_count() {

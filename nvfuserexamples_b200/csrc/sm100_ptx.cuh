@@ -196,6 +196,37 @@ __device__ __forceinline__ float4 dsmem_ld4(uint32_t addr) {
 }
 
 // ------------------------------------------------------------------------------------
+// cluster launch control: a running CTA takes over the index of a CTA of its grid that has not been launched yet
+// ------------------------------------------------------------------------------------
+// Writes the 16-byte answer to `slot` (shared memory) and completes 16 bytes of `bar`'s transaction count.  Not to be
+// called again once an answer has said that no CTA was left.
+__device__ __forceinline__ void clc_try_cancel(uint4* slot, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(slot)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// Whether the answer in `slot` holds a CTA index, and which.
+__device__ __forceinline__ bool clc_query(const uint4* slot, int& x, int& y, int& z) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .b128 answer;\n\t"
+      ".reg .pred p;\n\t"
+      "ld.shared.b128 answer, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, answer;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "mov.u32 %2, 0;\n\t"
+      "mov.u32 %3, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, answer;\n\t"
+      "}\n"
+      : "=r"(ok), "=r"(x), "=r"(y), "=r"(z)
+      : "r"(smem_u32(slot))
+      : "memory");
+  return ok != 0;
+}
+
+// ------------------------------------------------------------------------------------
 // TMA: 4-D tiled loads and stores. coordinates are (c0 innermost .. c3 outermost)
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
