@@ -10,8 +10,10 @@
 //
 // One CTA per SM walks (128-row query tile, head, batch) items handed out by cluster launch control (a running CTA takes
 // over the index of a CTA that has not been launched yet).  Per key tile: S = Q K^T, dP = dO V^T, dS = P (keep dP -
-// delta/c) -> tensor memory over dP, dQ += dS K.  Tensor memory: S 128 | dP 2 x 128 | dQ 128 columns: S and dP of
-// the next key tile (also of the next item) are formed while the current one is turned into dS.
+// delta/c) -> tensor memory, dQ += dS K.  Tensor memory: S 128 | dP 128 | dQ 128 | Q 64 | dS 64 columns.  S of the next
+// key tile (also of the next item) is formed while the current one is exponentiated, dP of it next to dQ of this one.  Q, the
+// A operand of every S of an item, is copied to tensor memory once: with both operands in shared memory a 128-column MMA
+// takes all of its bandwidth, and the loads of K and V (64 KB per tile) then cost S and dP half as much again.
 //   warp 0: TMA producer (and the additive mask row)   warp 1: MMA issuer   warps 2-17: thread = query row x 32 keys
 //   warps 18, 19: lse and delta of the item's rows, one item ahead
 #include <cuda_bf16.h>
@@ -55,7 +57,7 @@ struct DqSmem {
   static constexpr int kOffMask = kOffStats + 2 * 2 * kTileM * 4;   // additive mask (log2 domain) of a K stage
   static constexpr int kOffItems = kOffMask + kKStages * kTileN * 4;
   static constexpr int kOffBar = kOffItems + 32;
-  static constexpr int kNumBars = 4 + 3 * kKStages + 2 + 2 + 2 + 1 + 1 + 4 + 4;
+  static constexpr int kNumBars = 4 + 3 * kKStages + 2 + 2 + 1 + 1 + 1 + 4 + 4;
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;
   static constexpr int kDynBytes = kOffMisc + 16;   // 1024-byte aligned base: checked by the kernel
   static_assert(kDynBytes <= 232448, "shared memory budget of one CTA exceeded");
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   constexpr int D = 128;
   constexpr int KS = L::kKStages;
   constexpr int kTmemCols = 512;
-  constexpr uint32_t kColS = 0, kColdP = 128, kColdQ = 384;   // dP, and dS over it: [2] x 128 columns
+  constexpr uint32_t kColS = 0, kColdP = 128, kColdQ = 256, kColQ = 384, kColdS = 448;
   constexpr int kFmt = BF16 ? 1 : 0;
   constexpr uint32_t kIdescKK = make_idesc_f16(128, 128, kFmt, false, false);
   constexpr uint32_t kIdescKN = make_idesc_f16(128, D, kFmt, false, true);
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   uint4* items = reinterpret_cast<uint4*>(smem + L::kOffItems);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
   uint64_t* q_full = bars + 0;
-  uint64_t* q_empty = bars + 1;     // the item's last S has completed
+  uint64_t* q_empty = bars + 1;     // Q has been copied to tensor memory
   uint64_t* do_full = bars + 2;
   uint64_t* do_empty = bars + 3;    // the item's last dP has completed
   uint64_t* k_full = bars + 4;      // [KS]
@@ -103,8 +105,8 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   uint64_t* v_empty = v_full + 1;   // dP of the tile has completed
   uint64_t* s_full = v_empty + 1;
   uint64_t* s_free = s_full + 1;    // S has been read (all compute threads)
-  uint64_t* dp_full = s_free + 1;   // [2]
-  uint64_t* ds_full = dp_full + 2;  // dS is in tensor memory (all compute threads)
+  uint64_t* dp_full = s_free + 1;
+  uint64_t* ds_full = dp_full + 1;  // dS is in tensor memory, dP has been read (all compute threads)
   uint64_t* dq_full = ds_full + 1;  // dQ of an item is complete
   uint64_t* stat_full = dq_full + 1;    // [2] by item parity
   uint64_t* stat_empty = stat_full + 2; // [2]
@@ -210,10 +212,10 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
     mbar_init(v_empty, 1);
     mbar_init(s_full, 1);
     mbar_init(s_free, kDqCompute);
+    mbar_init(dp_full, 1);
     mbar_init(ds_full, kDqCompute);
     mbar_init(dq_full, 1);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(dp_full + s, 1);
       mbar_init(stat_full + s, 2);
       mbar_init(stat_empty + s, kDqCompute / 32);
       mbar_init(item_full + s, 1);
@@ -259,8 +261,9 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
           if (g >= 1) mbar_wait(v_empty, (g - 1) & 1, wctx, kDqsVEmpty);
           mbar_arrive_expect_tx(v_full, L::kTile);
           for (int c = 0; c < 2; ++c) tma_load_4d(sV + c * 16384, &a.tm_v, v_full, c * 64, it.row_base + j * kTileN, it.h, it.tb);
-          // Not earlier: on a chip that is still filling up, the CTA asked for may be about to start on an idle SM.
-          if (persist && j == max(it.n_kv - 2, 0)) request_item(n + 1);
+          // Early, for the statistics warps need the next item's rows in time; but the first time not at once: on a chip
+          // that is still filling up, the CTA asked for may be about to start on an idle SM.
+          if (persist && j == (w == 0 ? min(2, it.n_kv - 1) : 0)) request_item(n + 1);
         }
         __syncwarp();
         if constexpr (KEYADD) {   // the slot is free: its K stage was
@@ -277,57 +280,78 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
     }
   } else if (warp == 1) {
     // ============================ MMA issuer ========================================
-    // Convergent warp, bursts from one elected lane (see umma_ss_x4).  S and dP of tile t+1 are issued before dQ of tile t;
-    // dP(t+1) overwrites dS(t-1), which dQ(t-1), issued before, reads: the tensor core works in order.
-    const uint32_t tS = tmem_base + kColS, tdQ = tmem_base + kColdQ;
-    auto issue_kk = [&](uint32_t d, const uint8_t* a_tile, const uint8_t* b_tile) {
-      const uint64_t da = make_smem_desc_sw128(smem_u32(a_tile), 16, 1024), db = make_smem_desc_sw128(smem_u32(b_tile), 16, 1024);
+    // Convergent warp, bursts from one elected lane (see umma_ss_x4).  Per tile t: S(t+1) as soon as S(t) has been read; then,
+    // with dS(t) there and dP(t) read, dP(t+1) and dQ(t).  Every wait is for something that needs an MMA issued after the
+    // previous wait on the same barrier, so no barrier can be a phase ahead of this warp.
+    const uint32_t tS = tmem_base + kColS, tdP = tmem_base + kColdP, tdQ = tmem_base + kColdQ, tQ = tmem_base + kColQ,
+                   tdS = tmem_base + kColdS;
+    // S of key tile number t of this CTA; `first` of its item number w (with work): Q goes to tensor memory before (the copy
+    // is ordered behind the previous item's last S and before this one in the tensor core's pipe)
+    auto issue_s = [&](int t, int w, bool first) {
+      if (first) {
+        mbar_wait(q_full, w & 1, wctx, kDqsQ);
+        tc_fence_after_sync();
+        const uint64_t d = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
+        uint64_t x[8];
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) x[kk] = d + kmajor_step(kk, 16384);
+        tmem_cp_128x256b_x8(tQ, x);
+        umma_commit_elect(q_empty);
+      }
+      mbar_wait(k_full + t % KS, (t / KS) & 1, wctx, kDqsK);
+      tc_fence_after_sync();
+      const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + (t % KS) * L::kTile), 16, 1024);
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint64_t y[4];
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) y[kk] = dk + kmajor_step(hf * 4 + kk, 16384);
+        umma_ts_x4(tS, tQ + hf * 32, 8u, y, kIdescKK, hf);
+      }
+      umma_commit_elect(s_full);
+    };
+    auto issue_dp = [&](int t, int w, bool first, bool last) {
+      if (first) mbar_wait(do_full, w & 1, wctx, kDqsDo);
+      mbar_wait(v_full, t & 1, wctx, kDqsV);
+      tc_fence_after_sync();
+      const uint64_t da = make_smem_desc_sw128(smem_u32(sdO), 16, 1024), db = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
       uint64_t x[8], y[8];
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
         x[kk] = da + kmajor_step(kk, 16384);
         y[kk] = db + kmajor_step(kk, 16384);
       }
-      umma_ss_x8(d, x, y, kIdescKK, 0u);
-    };
-    // S and dP of key tile number t of this CTA, which belongs to its item number w (with work)
-    auto issue_s_dp = [&](int t, int w, bool first, bool last) {
-      if (first) mbar_wait(q_full, w & 1, wctx, kDqsQ);
-      mbar_wait(k_full + t % KS, (t / KS) & 1, wctx, kDqsK);
-      tc_fence_after_sync();
-      issue_kk(tS, sQ, sK + (t % KS) * L::kTile);
-      umma_commit_elect(s_full);
-      if (last) umma_commit_elect(q_empty);
-      if (first) mbar_wait(do_full, w & 1, wctx, kDqsDo);
-      mbar_wait(v_full, t & 1, wctx, kDqsV);
-      tc_fence_after_sync();
-      issue_kk(tmem_base + kColdP + (t & 1) * 128, sdO, sV);
-      umma_commit_elect(dp_full + (t & 1));
+      umma_ss_x8(tdP, x, y, kIdescKK, 0u);
+      umma_commit_elect(dp_full);
       umma_commit_elect(v_empty);
       if (last) umma_commit_elect(do_empty);
     };
     int n = 0, w = 0, t = 0;
     DqItem it = first_work(n, false);
-    if (it.state == kDqWork) issue_s_dp(0, 0, true, it.n_kv == 1);
+    if (it.state == kDqWork) {
+      issue_s(0, 0, true);
+      issue_dp(0, 0, true, it.n_kv == 1);
+    }
     while (it.state == kDqWork) {
       DqItem nxt = it;
       for (int j = 0; j < it.n_kv; ++j, ++t) {
         const bool last = j + 1 == it.n_kv;
         if (last) nxt = next_work(n, false);
-        if (!last || nxt.state == kDqWork) {
+        const bool more = !last || nxt.state == kDqWork;
+        if (more) {
           mbar_wait(s_free, t & 1, wctx, kDqsSFree);
-          issue_s_dp(t + 1, w + 1, last, last ? nxt.n_kv == 1 : j + 2 == it.n_kv);
+          issue_s(t + 1, w + 1, last);
         }
-        const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + (t % KS) * L::kTile), 16384, 1024);   // K as MN-major B
-        const uint32_t tdS = tmem_base + kColdP + (t & 1) * 128;
         mbar_wait(ds_full, t & 1, wctx, kDqsDs);
         tc_fence_after_sync();
+        if (more) issue_dp(t + 1, w + 1, last, last ? nxt.n_kv == 1 : j + 2 == it.n_kv);
+        const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + (t % KS) * L::kTile), 16384, 1024);   // K as MN-major B
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint64_t y[4];
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) y[kk] = dk + mnmajor_step(hf * 4 + kk);
-          umma_ts_2x2(tdQ, tdS + hf * 64, tdS + hf * 64 + 32, 8u, y, kIdescKN, (j > 0 || hf > 0) ? 1u : 0u);
+          umma_ts_x4(tdQ, tdS + hf * 32, 8u, y, kIdescKN, (j > 0 || hf > 0) ? 1u : 0u);
         }
         umma_commit_elect(k_empty + t % KS);
         if (last) umma_commit_elect(dq_full);
@@ -507,13 +531,12 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
           store_dq(w - 1, prev);
           prev.state = kDqEnd;
         }
-        mbar_wait(dp_full + (t & 1), (t >> 1) & 1, wctx, kDqsDp, kDqSleepNs);
+        mbar_wait(dp_full, t & 1, wctx, kDqsDp, kDqSleepNs);
         tc_fence_after_sync();
-        const uint32_t tdP = tmem_base + lane_addr + kColdP + (t & 1) * 128 + cq * 32;
         const float2 nd2 = make_float2(neg_delta, neg_delta);
         uint32_t pk[16];
         uint32_t dp[32];
-        tmem_ld32(tdP, dp);
+        tmem_ld32(tmem_base + lane_addr + kColdP + cq * 32, dp);
         tmem_wait_ld_dep(dp);
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
@@ -526,7 +549,8 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
           const float2 ds = __fmul2_rn(make_float2(__uint_as_float(p[2 * k]), __uint_as_float(p[2 * k + 1])), d);
           pk[k] = pack2<BF16>(ds.x, ds.y);
         }
-        tmem_st16(tdP, pk);
+        if (t > 0) mbar_wait(k_empty + (t - 1) % KS, ((t - 1) / KS) & 1, wctx, kDqsKEmpty, kDqSleepNs);   // dQ(t-1) has read dS
+        tmem_st16(tmem_base + lane_addr + kColdS + cq * 16, pk);
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(ds_full);

@@ -480,6 +480,28 @@ __device__ __forceinline__ void umma_ts_2x2(uint32_t d_tmem, uint32_t a0, uint32
       ::"r"(d_tmem), "r"(a0), "r"(a1), "r"(a_step), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "r"(idesc), "r"(acc_first)
       : "memory");
 }
+// Copies a K-major 128 x 128 16-bit tile (descriptors of its eight 16-column steps) to 64 tensor-memory columns, where it
+// can be the A operand of an MMA: row = lane, two elements per column.  Runs in the tensor core's pipe, in order with MMAs.
+__device__ __forceinline__ void tmem_cp_128x256b_x8(uint32_t taddr, const uint64_t (&s)[8]) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred pe;\n\t"
+      ".reg .b32 a1, a2, a3, a4, a5, a6, a7;\n\t"
+      "add.u32 a1, %0, 8;\n\tadd.u32 a2, %0, 16;\n\tadd.u32 a3, %0, 24;\n\tadd.u32 a4, %0, 32;\n\t"
+      "add.u32 a5, %0, 40;\n\tadd.u32 a6, %0, 48;\n\tadd.u32 a7, %0, 56;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [%0], %1;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a1], %2;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a2], %3;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a3], %4;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a4], %5;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a5], %6;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a6], %7;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a7], %8;\n\t"
+      "}\n"
+      ::"r"(taddr), "l"(s[0]), "l"(s[1]), "l"(s[2]), "l"(s[3]), "l"(s[4]), "l"(s[5]), "l"(s[6]), "l"(s[7])
+      : "memory");
+}
 // tcgen05.commit by the elected lane of a converged warp.  elect.sync picks the same lane every
 // time for a full mask, so the commit tracks the MMAs issued by the helpers above.
 __device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
