@@ -10,10 +10,11 @@
 //
 // One CTA per SM walks (128-row query tile, head, batch) items handed out by cluster launch control (a running CTA takes
 // over the index of a CTA that has not been launched yet).  Per key tile: S = Q K^T, dP = dO V^T, dS = P (keep dP -
-// delta/c) -> tensor memory, dQ += dS K.  Tensor memory: S 128 | dP 128 | dQ 128 | Q 64 | dS 64 columns.  S of the next
-// key tile (also of the next item) is formed while the current one is exponentiated, dP of it next to dQ of this one.  Q, the
-// A operand of every S of an item, is copied to tensor memory once: with both operands in shared memory a 128-column MMA
-// takes all of its bandwidth, and the loads of K and V (64 KB per tile) then cost S and dP half as much again.
+// delta/c) -> tensor memory over dP, dQ += dS K.  Tensor memory: S 128 | dP 128 | dQ 128 | Q 64 | dO 64 columns.  S of the
+// next key tile (also of the next item) is formed while the current one is exponentiated, dP of it behind dQ of this one.
+// Q and dO, the A operands of every S and dP of an item, are copied to tensor memory once: with both operands in shared
+// memory a 128-column MMA takes all of its bandwidth, the loads of K and V (64 KB per tile) then cost S and dP half as much
+// again, and a shared-memory read of another warp - a barrier poll, say - takes 330 cycles instead of 65 (measured).
 //   warp 0: TMA producer (and the additive mask row)   warp 1: MMA issuer   warps 2-17: thread = query row x 32 keys
 //   warps 18, 19: lse and delta of the item's rows, one item ahead
 #include <cuda_bf16.h>
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   constexpr int D = 128;
   constexpr int KS = L::kKStages;
   constexpr int kTmemCols = 512;
-  constexpr uint32_t kColS = 0, kColdP = 128, kColdQ = 256, kColQ = 384, kColdS = 448;
+  constexpr uint32_t kColS = 0, kColdP = 128, kColdQ = 256, kColQ = 384, kColdO = 448;
   constexpr int kFmt = BF16 ? 1 : 0;
   constexpr uint32_t kIdescKK = make_idesc_f16(128, 128, kFmt, false, false);
   constexpr uint32_t kIdescKN = make_idesc_f16(128, D, kFmt, false, true);
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   uint64_t* q_full = bars + 0;
   uint64_t* q_empty = bars + 1;     // Q has been copied to tensor memory
   uint64_t* do_full = bars + 2;
-  uint64_t* do_empty = bars + 3;    // the item's last dP has completed
+  uint64_t* do_empty = bars + 3;    // dO has been copied to tensor memory
   uint64_t* k_full = bars + 4;      // [KS]
   uint64_t* k_empty = k_full + KS;  // [KS] dQ += dS K of the tile has completed
   uint64_t* mask_full = k_empty + KS;   // [KS]
@@ -281,56 +282,55 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   } else if (warp == 1) {
     // ============================ MMA issuer ========================================
     // Convergent warp, bursts from one elected lane (see umma_ss_x4).  Per tile t: S(t+1) as soon as S(t) has been read; then,
-    // with dS(t) there and dP(t) read, dP(t+1) and dQ(t).  Every wait is for something that needs an MMA issued after the
-    // previous wait on the same barrier, so no barrier can be a phase ahead of this warp.
+    // with dS(t) there, dQ(t) and dP(t+1), which overwrites dS(t): the tensor core works in order.  Every wait is for
+    // something that needs an MMA issued after the previous wait on the same barrier, so no barrier can be a phase ahead
+    // of this warp.
     const uint32_t tS = tmem_base + kColS, tdP = tmem_base + kColdP, tdQ = tmem_base + kColdQ, tQ = tmem_base + kColQ,
-                   tdS = tmem_base + kColdS;
-    // S of key tile number t of this CTA; `first` of its item number w (with work): Q goes to tensor memory before (the copy
-    // is ordered behind the previous item's last S and before this one in the tensor core's pipe)
-    auto issue_s = [&](int t, int w, bool first) {
-      if (first) {
-        mbar_wait(q_full, w & 1, wctx, kDqsQ);
-        tc_fence_after_sync();
-        const uint64_t d = make_smem_desc_sw128(smem_u32(sQ), 16, 1024);
-        uint64_t x[8];
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) x[kk] = d + kmajor_step(kk, 16384);
-        tmem_cp_128x256b_x8(tQ, x);
-        umma_commit_elect(q_empty);
-      }
-      mbar_wait(k_full + t % KS, (t / KS) & 1, wctx, kDqsK);
+                   tdO = tmem_base + kColdO;
+    // Q or dO of an item to tensor memory; the copy is ordered behind the previous item's last use of these columns and
+    // before the MMAs issued after it.
+    auto copy_a = [&](uint32_t dst, const uint8_t* tile, uint64_t* full, uint64_t* empty, int w, int site) {
+      mbar_wait(full, w & 1, wctx, site);
       tc_fence_after_sync();
-      const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + (t % KS) * L::kTile), 16, 1024);
+      const uint64_t d = make_smem_desc_sw128(smem_u32(tile), 16, 1024);
+      uint64_t x[8];
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) x[kk] = d + kmajor_step(kk, 16384);
+      tmem_cp_128x256b_x8(dst, x);
+      umma_commit_elect(empty);
+    };
+    // [128 x 128] = A (tensor memory) * (rows of a K or V tile)^T
+    auto issue_kk = [&](uint32_t d, uint32_t a_tmem, const uint8_t* b_tile) {
+      const uint64_t db = make_smem_desc_sw128(smem_u32(b_tile), 16, 1024);
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
         uint64_t y[4];
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) y[kk] = dk + kmajor_step(hf * 4 + kk, 16384);
-        umma_ts_x4(tS, tQ + hf * 32, 8u, y, kIdescKK, hf);
+        for (int kk = 0; kk < 4; ++kk) y[kk] = db + kmajor_step(hf * 4 + kk, 16384);
+        umma_ts_x4(d, a_tmem + hf * 32, 8u, y, kIdescKK, hf);
       }
+    };
+    // S and dP of key tile number t of this CTA; `first` of its item number w (with work)
+    auto issue_s = [&](int t, int w, bool first) {
+      if (first) copy_a(tQ, sQ, q_full, q_empty, w, kDqsQ);
+      mbar_wait(k_full + t % KS, (t / KS) & 1, wctx, kDqsK);
+      tc_fence_after_sync();
+      issue_kk(tS, tQ, sK + (t % KS) * L::kTile);
       umma_commit_elect(s_full);
     };
-    auto issue_dp = [&](int t, int w, bool first, bool last) {
-      if (first) mbar_wait(do_full, w & 1, wctx, kDqsDo);
+    auto issue_dp = [&](int t, int w, bool first) {
+      if (first) copy_a(tdO, sdO, do_full, do_empty, w, kDqsDo);
       mbar_wait(v_full, t & 1, wctx, kDqsV);
       tc_fence_after_sync();
-      const uint64_t da = make_smem_desc_sw128(smem_u32(sdO), 16, 1024), db = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
-      uint64_t x[8], y[8];
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
-        x[kk] = da + kmajor_step(kk, 16384);
-        y[kk] = db + kmajor_step(kk, 16384);
-      }
-      umma_ss_x8(tdP, x, y, kIdescKK, 0u);
+      issue_kk(tdP, tdO, sV);
       umma_commit_elect(dp_full);
       umma_commit_elect(v_empty);
-      if (last) umma_commit_elect(do_empty);
     };
     int n = 0, w = 0, t = 0;
     DqItem it = first_work(n, false);
     if (it.state == kDqWork) {
       issue_s(0, 0, true);
-      issue_dp(0, 0, true, it.n_kv == 1);
+      issue_dp(0, 0, true);
     }
     while (it.state == kDqWork) {
       DqItem nxt = it;
@@ -344,17 +344,17 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
         }
         mbar_wait(ds_full, t & 1, wctx, kDqsDs);
         tc_fence_after_sync();
-        if (more) issue_dp(t + 1, w + 1, last, last ? nxt.n_kv == 1 : j + 2 == it.n_kv);
         const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + (t % KS) * L::kTile), 16384, 1024);   // K as MN-major B
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint64_t y[4];
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) y[kk] = dk + mnmajor_step(hf * 4 + kk);
-          umma_ts_x4(tdQ, tdS + hf * 32, 8u, y, kIdescKN, (j > 0 || hf > 0) ? 1u : 0u);
+          umma_ts_2x2(tdQ, tdP + hf * 64, tdP + hf * 64 + 32, 8u, y, kIdescKN, (j > 0 || hf > 0) ? 1u : 0u);
         }
         umma_commit_elect(k_empty + t % KS);
         if (last) umma_commit_elect(dq_full);
+        if (more) issue_dp(t + 1, w + 1, last);
       }
       ++w;
       it = nxt;
@@ -549,8 +549,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
           const float2 ds = __fmul2_rn(make_float2(__uint_as_float(p[2 * k]), __uint_as_float(p[2 * k + 1])), d);
           pk[k] = pack2<BF16>(ds.x, ds.y);
         }
-        if (t > 0) mbar_wait(k_empty + (t - 1) % KS, ((t - 1) / KS) & 1, wctx, kDqsKEmpty, kDqSleepNs);   // dQ(t-1) has read dS
-        tmem_st16(tmem_base + lane_addr + kColdS + cq * 16, pk);
+        tmem_st16(tmem_base + lane_addr + kColdP + cq * 32, pk);   // over this thread's own columns of dP
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(ds_full);
