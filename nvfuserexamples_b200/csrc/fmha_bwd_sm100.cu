@@ -221,10 +221,11 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
 //
 // Layout.  Scores are formed transposed, S^T = K Q^T and dP^T = V dO^T with keys along the tensor-memory lanes, so that
 // P^T, written back to tensor memory by the thread that computed it, is the A operand of dV += P^T dO: it is neither
-// written to shared memory nor read from it.  What limits this kernel is shared-memory bandwidth: with P and dS both
-// staged there a D = 64 tile moved 2 944 cycles' worth of shared-memory data (MMA operands 1 664, P/dS 512, TMA in and out
-// 768).  At D = 128 dS^T stays in tensor memory in the same way, as the A operand of dK += dS^T Q, and dQ is another kernel's
-// (fmha_bwd_dq_sm100.cu); at D = 64 dS also feeds dQ = dS K and goes to shared memory.
+// written to shared memory nor read from it, and dS^T likewise that of dK += dS^T Q.  At D = 128 dQ is another kernel's
+// (fmha_bwd_dq_sm100.cu); at D = 64 dS also feeds dQ = dS K and goes to shared memory as well, and K and V, the A operands of
+// S^T and dP^T, lie in tensor memory.  What is saved is shared-memory bandwidth: a 128 x 128 x 16 MMA with both operands in
+// shared memory takes all of it (64 cycles, 8 KB; with 64 columns 48 cycles instead of 32), and while such MMAs run a
+// shared-memory access of another warp - a barrier poll, a read of lse - takes 330 cycles instead of 65 (measured).
 // In this layout a thread is a key: lse and delta vary along its columns and come from shared memory (broadcast reads;
 // a helper warp fetches them one to two tiles ahead), the additive key mask is one value per thread, and the dropout
 // draws, which give 16 keys of one query row each, are made by the thread of that row and transposed in the warp.
@@ -232,8 +233,8 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
 // Schedule inside the stream of (item, query tile) pairs, numbered t = 0, 1, ...:
 //   compute warps:  S(t) -> P(t) -> tensor memory (p_full) -> dP(t) -> dS(t) -> shared / tensor memory (ds_full) ->
 //                   [D = 64: dQ(t-1) out]; dK and dV of an item leave when the next item's first P is ready.
-//   MMA warp:       on p_full(t): dV(t), S(t+1); on ds_full(t), D = 64: dP(t+1), dK(t), dQ(t); D = 128: dK(t), dP(t+1), which
-//                   overwrites dS(t).  S(t+1) and dP(t+1) may belong to the next item.
+//   MMA warp:       on p_full(t): dV(t), S(t+1), which overwrites P(t); on ds_full(t): dK(t), dP(t+1), which overwrites dS(t),
+//                   and (D = 64) dQ(t).  S(t+1) and dP(t+1) may belong to the next item.
 // Position of element (row, col) of a 128-row tile of the fp32 dQ accumulator: 32-row groups, in them groups of four
 // columns, in them the 32 rows with their four values each.
 template <int D>
@@ -278,8 +279,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   constexpr int kTmemCols = 512;
   constexpr uint32_t kColS = 0, kColdP = 128, kColdV = 256, kColdK = 256 + D;
   constexpr uint32_t kColdQ = 384;   // D = 64
-  // P^T, 16 columns per 32 query rows: beside everything else (D = 64), or over the thread's own columns of S (D = 128)
-  constexpr uint32_t kColP = (D == 64) ? 448 : kColS, kPStride = (D == 64) ? 16 : 32;
+  // P^T and dS^T lie over S and dP, a thread's 16 packed columns at the start of its own 32.  D = 64: K and V of an item, the
+  // A operands of S^T and dP^T, are copied to tensor memory once.
+  constexpr uint32_t kColP = kColS, kColdS = kColdP, kPStride = 32, kColK = 448, kColV = 480;
   constexpr int kFmt = BF16 ? 1 : 0;
   constexpr uint32_t kIdescS = make_idesc_f16(128, 128, kFmt, false, false);
   constexpr uint32_t kIdescMN = make_idesc_f16(128, D, kFmt, true, true);    // dQ: A and B MN-major
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   uint64_t* k_full = bars + 7;
   uint64_t* k_empty = k_full + KV;   // D = 64: the item's last dQ has completed; D = 128: its last S
   uint64_t* v_full = k_empty + KV;
-  uint64_t* v_empty = v_full + KV;   // the item's last dP has completed
+  uint64_t* v_empty = v_full + KV;   // D = 64: V is in tensor memory; D = 128: the item's last dP has completed
   uint64_t* q_full = v_empty + KV;
   uint64_t* q_empty = q_full + QS;
   uint64_t* do_full = q_empty + QS;
@@ -489,22 +491,49 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       if constexpr (KS == 4) umma_ss_x4(d, x, y, kIdescS, 0u);
       else umma_ss_x8(d, x, y, kIdescS, 0u);
     };
+    // D = 64: K or V tile to 32 tensor-memory columns (in the tensor core's pipe, in order with the MMAs), and
+    // [128 x 128] = A (there) * B (rows of 64 values, K-major)^T
+    auto copy_a = [&](uint32_t dst, const uint8_t* tile) {
+      const uint64_t d = make_smem_desc_sw128(smem_u32(tile), 16, 1024);
+      uint64_t x[4];
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) x[kk] = d + kmajor_step(kk, 16384);
+      tmem_cp_128x256b_x4(dst, x);
+    };
+    auto issue_tk = [&](uint32_t d, uint32_t a_tmem, const uint8_t* b_tile) {
+      const uint64_t db = make_smem_desc_sw128(smem_u32(b_tile), 16, 1024);
+      uint64_t y[4];
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) y[kk] = db + kmajor_step(kk, 16384);
+      umma_ts_x4(d, a_tmem, 8u, y, kIdescS, 0u);
+    };
     // S^T and dP^T of tile tt, which belongs to item number wi (with work) and is its first / last one
     auto issue_s = [&](int tt, int wi, bool first, bool last) {
-      if (first) mbar_wait(k_full + wi % KV, (wi / KV) & 1, wctx, kSiteKFull);
+      if (first) {
+        mbar_wait(k_full + wi % KV, (wi / KV) & 1, wctx, kSiteKFull);
+        if constexpr (D == 64) copy_a(tmem_base + kColK, sK + (wi % KV) * L::kTileBytes);
+      }
       mbar_wait(q_full + tt % QS, (tt / QS) & 1, wctx, kSiteQFull);
       tc_fence_after_sync();
-      issue_kk(tS, sK + (wi % KV) * L::kTileBytes, sQ + (tt % QS) * L::kTileBytes);
+      if constexpr (D == 64) issue_tk(tS, tmem_base + kColK, sQ + (tt % QS) * L::kTileBytes);
+      else issue_kk(tS, sK + (wi % KV) * L::kTileBytes, sQ + (tt % QS) * L::kTileBytes);
       umma_commit_elect(s_full);
       if (D == 128 && last) umma_commit_elect(k_empty + wi % KV);
     };
     auto issue_dp = [&](int tt, int wi, bool first, bool last) {
-      if (first) mbar_wait(v_full + wi % KV, (wi / KV) & 1, wctx, kSiteVFull);
+      if (first) {
+        mbar_wait(v_full + wi % KV, (wi / KV) & 1, wctx, kSiteVFull);
+        if constexpr (D == 64) {
+          copy_a(tmem_base + kColV, sV + (wi % KV) * L::kTileBytes);
+          umma_commit_elect(v_empty + wi % KV);
+        }
+      }
       mbar_wait(do_full + tt % OS, (tt / OS) & 1, wctx, kSiteDoFull);
       tc_fence_after_sync();
-      issue_kk(tdP, sV + (wi % KV) * L::kTileBytes, sdO + (tt % OS) * L::kTileBytes);
+      if constexpr (D == 64) issue_tk(tdP, tmem_base + kColV, sdO + (tt % OS) * L::kTileBytes);
+      else issue_kk(tdP, sV + (wi % KV) * L::kTileBytes, sdO + (tt % OS) * L::kTileBytes);
       umma_commit_elect(dp_full);
-      if (last) umma_commit_elect(v_empty + wi % KV);
+      if (D == 128 && last) umma_commit_elect(v_empty + wi % KV);
     };
 
     int n = 0, w = 0, t = 0;   // items fetched, items with work, query tiles so far
@@ -521,7 +550,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     while (cur.id >= 0) {
       const int kvb = w % KV;
       const int n_q = cur.n_q;
-      const uint64_t dK_m = make_smem_desc_sw128(smem_u32(sK + kvb * L::kTileBytes), 16384, 1024);   // K as MN-major B (dQ)
       BwdItem nxt = cur;
       for (int i = 0; i < n_q; ++i, ++t) {
         const bool last = i + 1 == n_q;
@@ -542,34 +570,37 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           }
         }
         umma_commit_elect(do_empty + os);   // dP(t) came before, so dO(t) is not read again
-        // ---- S of the next tile: S(t) has been read (D = 128: and P(t), which lies over it, by dV(t)) ------------------------
+        // ---- S of the next tile ------------------------------------------------------------------------------------------------
         if (last) nxt = next_work();   // the compute warps finish tile t, and any items without keys, without another MMA
         const bool more = !last || nxt.id >= 0;
         const int wn = last ? w + 1 : w;                                  // item of tile t+1, and whether t+1 is its last tile
         const bool next_last = last ? nxt.n_q == 1 : i + 2 == n_q;
         if (more) issue_s(t + 1, wn, last, next_last);
-        // ---- dK += dS^T Q, dQ tile = dS K -----------------------------------------------------------------------------------
+        // ---- dK += dS^T Q (A from tensor memory), dP of the next tile over dS(t), dQ tile = dS K ------------------------------
         const uint64_t dQ_m = make_smem_desc_sw128(smem_u32(sQ + qs * L::kTileBytes), 16384, 1024);
         mbar_wait(ds_full, t & 1, wctx, kSiteDsFull);
         tc_fence_after_sync();
-        if constexpr (D == 64) {
-          const uint8_t* ds_tile = sdS + (t % DS) * L::kDsBytes;
-          const uint64_t ddS_k = make_smem_desc_sw128(smem_u32(ds_tile), 16, 1024);       // dS^T as K-major A (keys x queries)
-          const uint64_t ddS_m = make_smem_desc_sw128(smem_u32(ds_tile), 16384, 1024);    // dS as MN-major A (queries x keys)
-          if (more) issue_dp(t + 1, wn, last, next_last);   // dP(t) has been read
-          uint64_t x[8], y[8];
+        {
+          const uint32_t tdS = tmem_base + kColdS;
+          uint64_t y[4];
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            x[kk] = ddS_k + kmajor_step(kk, 16384);
-            y[kk] = dQ_m + mnmajor_step(kk);
+          for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) y[kk] = dQ_m + mnmajor_step(hf * 4 + kk);
+            umma_ts_2x2(tdK, tdS + 2 * hf * kPStride, tdS + (2 * hf + 1) * kPStride, 8u, y, kIdescKN, hf == 0 ? acc0 : 1u);
           }
-          umma_ss_x8(tdK, x, y, kIdescKN, acc0);
-          umma_commit_elect(q_empty + qs);
-          if (last) umma_commit_elect(acc_full);
+        }
+        umma_commit_elect(q_empty + qs);
+        if (last) umma_commit_elect(acc_full);
+        if (more) issue_dp(t + 1, wn, last, next_last);
+        if constexpr (D == 64) {
+          const uint64_t ddS_m = make_smem_desc_sw128(smem_u32(sdS + (t % DS) * L::kDsBytes), 16384, 1024);   // MN-major A (queries x keys)
+          const uint64_t dK_m = make_smem_desc_sw128(smem_u32(sK + kvb * L::kTileBytes), 16384, 1024);        // MN-major B
           if (t > 0) {
             mbar_wait(dq_free, (t - 1) & 1, wctx, kSiteDqFree);
             tc_fence_after_sync();
           }
+          uint64_t x[8], y[8];
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             x[kk] = ddS_m + mnmajor_step(kk);
@@ -578,17 +609,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           umma_ss_x8(tdQ, x, y, kIdescMN, 0u);
           umma_commit_elect(dq_full);
           if (last) umma_commit_elect(k_empty + kvb);   // K of this item is not read again
-        } else {
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint64_t y[4];
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) y[kk] = dQ_m + mnmajor_step(hf * 4 + kk);
-            umma_ts_2x2(tdK, tdP + hf * 64, tdP + hf * 64 + 32, 8u, y, kIdescKN, hf == 0 ? acc0 : 1u);
-          }
-          umma_commit_elect(q_empty + qs);
-          if (last) umma_commit_elect(acc_full);
-          if (more) issue_dp(t + 1, wn, last, next_last);   // over dS(t): the tensor core works in order
         }
       }
       ++w;
@@ -815,7 +835,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           store_dkdv(prev_id, true);
           prev_id = -1;
         }
-        if (D == 64 && t > 0) mbar_wait(do_empty + (t - 1) % OS, ((t - 1) / OS) & 1, wctx, kSiteDoEmpty, kComputeSleepNs);   // dV(t-1) has read P
         tmem_st16(tmem_base + lane_addr + kColP + cq * kPStride, pk);
         tmem_wait_st();
         tc_fence_before_sync();
@@ -857,10 +876,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           for (int q = 0; q < 4; ++q)
             sts128(buf + sw128_offset(row, (cq & 1) * 4 + q), pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
           fence_proxy_async_smem();
-        } else {
-          tmem_st16(tmem_base + lane_addr + kColdP + cq * 32, pk);   // over this thread's own columns of dP
-          tmem_wait_st();
         }
+        tmem_st16(tmem_base + lane_addr + kColdS + cq * kPStride, pk);
+        tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(ds_full);
         if constexpr (D == 64) {

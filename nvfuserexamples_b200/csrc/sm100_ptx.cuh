@@ -502,6 +502,22 @@ __device__ __forceinline__ void tmem_cp_128x256b_x8(uint32_t taddr, const uint64
       ::"r"(taddr), "l"(s[0]), "l"(s[1]), "l"(s[2]), "l"(s[3]), "l"(s[4]), "l"(s[5]), "l"(s[6]), "l"(s[7])
       : "memory");
 }
+// The same for a 128 x 64 tile: 32 columns.
+__device__ __forceinline__ void tmem_cp_128x256b_x4(uint32_t taddr, const uint64_t (&s)[4]) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred pe;\n\t"
+      ".reg .b32 a1, a2, a3;\n\t"
+      "add.u32 a1, %0, 8;\n\tadd.u32 a2, %0, 16;\n\tadd.u32 a3, %0, 24;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [%0], %1;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a1], %2;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a2], %3;\n\t"
+      "@pe tcgen05.cp.cta_group::1.128x256b [a3], %4;\n\t"
+      "}\n"
+      ::"r"(taddr), "l"(s[0]), "l"(s[1]), "l"(s[2]), "l"(s[3])
+      : "memory");
+}
 // tcgen05.commit by the elected lane of a converged warp.  elect.sync picks the same lane every
 // time for a full mask, so the commit tracks the MMAs issued by the helpers above.
 __device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
