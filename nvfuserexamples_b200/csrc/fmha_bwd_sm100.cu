@@ -92,66 +92,111 @@ struct PrepArgs {
   const void* o;
   const void* d_o;
   int64_t o_sb, o_sh, o_ss, do_sb, do_sh, do_ss;
-  int B, H, S_q, S_q_pad;
-  float* delta;     // [B*H, S_q]
-  float* dq_accum;  // [B*H, S_q_pad, D]
-  int* work_counter;  // the main kernel's work-item counter, cleared here
-  const int* cu_seqlens;  // packed batch: row offsets into the [total_rows, H, D] tensors (o_sb / do_sb unused), else null
-  UncoveredRows zero;
+  BwdArgs m;   // the main kernel's arguments
 };
 
-template <bool BF16>
-__global__ void __launch_bounds__(256) bwd_prepare_kernel(const PrepArgs a) {
+// Transposes the 32 x 32 bit matrix a warp holds as one row per lane: afterwards bit L of lane p is what bit p of lane L
+// was.  Five exchanges of half-blocks: 16 and 8 bits as byte permutes, 4, 2 and 1 as a rotation and a bit select.
+__device__ __forceinline__ uint32_t warp_bit_transpose(uint32_t x, int lane) {
+  uint32_t y = __shfl_xor_sync(0xffffffffu, x, 16);
+  x = prmt(x, y, (lane & 16) ? 0x3276u : 0x5410u);
+  y = __shfl_xor_sync(0xffffffffu, x, 8);
+  x = prmt(x, y, (lane & 8) ? 0x3715u : 0x6240u);
+#pragma unroll
+  for (int s = 4; s >= 1; s >>= 1) {
+    const uint32_t low = s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
+    const bool up = lane & s;
+    y = __shfl_xor_sync(0xffffffffu, x, s);
+    y = __funnelshift_l(y, y, up ? 32 - s : s);
+    const uint32_t own = up ? ~low : low;
+    x = (x & own) | (y & ~own);
+  }
+  return x;
+}
+// Keep decisions of 32 query rows (from q0) x 32 keys (from 16*kb), by a whole warp: every lane makes the two Philox draws of
+// one row, the bits are transposed, and lane l gets key l's: those of rows 4j..4j+3 are the top bits of the four bytes of
+// (word << j).
+__device__ __forceinline__ uint32_t keep_word_32x32(const PhiloxKeys& keys, uint32_t offset, uint32_t bh, uint32_t q0, uint32_t kb,
+                                                    uint32_t thr, int lane) {
+  const uint32_t q_row = q0 + 4 * (7 - (lane & 7)) + (lane >> 3);
+  uint32_t keep = 0u;
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+    const U4 u = dropout_draw_keys(keys, offset, bh, q_row, kb + d);
+    const uint32_t ws[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)   // the keep bit of key 16d + 4k + e ends as bit 8e + 4d + k
+      keep = (keep >> 1) | (((ws[k] & 0x7F7F7F7Fu) + (0x80u - thr) * 0x01010101u) & 0x80808080u);
+  }
+  keep = warp_bit_transpose(keep, lane);
+  return __shfl_sync(0xffffffffu, keep, 8 * (lane & 3) + (lane >> 2));
+}
+
+// KEEP: also the keep bits of the block's 32 query rows.  The draws run at the multipliers' rate beside the memory traffic of
+// the rest; in the main kernel, where 16 warps wait for one another's phases, they took 1 000 of 4 900 cycles per tile.
+template <bool BF16, bool KEEP>
+__global__ void __launch_bounds__(256) bwd_prepare_kernel(const __grid_constant__ PrepArgs a) {
   griddep_wait();
   // grid = (B*H, blocks of 32 rows); 8 threads per row, 8 elements each.
   // The head index comes from the grid, so no thread divides 64-bit indices.
   constexpr int D = kAccumD, per = D / 8;
+  const BwdArgs& m = a.m;
   const int part = threadIdx.x & 7;
   const int bh = blockIdx.x;
-  const int h = bh % a.H;
-  const int b = bh / a.H;
-  const int r = blockIdx.y * 32 + (threadIdx.x >> 3);
-  const bool in_range = r < a.S_q_pad;  // no early exit: the shuffles below need every lane
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && a.work_counter != nullptr) *a.work_counter = 0;
-  if (in_range) {
-    float4* acc = reinterpret_cast<float4*>(a.dq_accum + (static_cast<int64_t>(bh) * a.S_q_pad + r) * D + part * per);
-    for (int i = 0; i < per / 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  const int h = bh % m.H;
+  const int b = bh / m.H;
+  const int r0 = blockIdx.y * 32;
+  const int r = r0 + (threadIdx.x >> 3);   // < S_q_pad
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *m.work_counter = 0;
   // packed batch: row r of sequence b is row cu[b] + r of the tensors, and exists for r < cu[b+1] - cu[b]
   int64_t row_o = static_cast<int64_t>(b) * a.o_sb + static_cast<int64_t>(r) * a.o_ss;
   int64_t row_do = static_cast<int64_t>(b) * a.do_sb + static_cast<int64_t>(r) * a.do_ss;
-  int q_limit = a.S_q;
-  if (a.cu_seqlens != nullptr) {
-    const int base = a.cu_seqlens[b];
-    q_limit = min(a.cu_seqlens[b + 1] - base, a.S_q);   // rows past the stated maximum length take no part
-    if (blockIdx.y == 0 && a.zero.grad[0].ptr != nullptr) {
+  int q_limit = m.S_q, k_limit = m.S_k;
+  if (m.mask_kind == FMHA_MASK_CU_SEQLENS) {
+    const int* cu = static_cast<const int*>(m.mask);
+    const int base = cu[b];
+    q_limit = k_limit = min(cu[b + 1] - base, m.S_q);   // rows past the stated maximum length take no part
+    if (blockIdx.y == 0 && m.zero.grad[0].ptr != nullptr) {
       for (int t = 0; t < 3; ++t)
-        zero_uncovered_rows(a.zero.grad[t].ptr, a.zero.grad[t].stride_s, a.zero.grad[t].stride_h, h, b, a.B, a.cu_seqlens, a.S_q,
-                            a.zero.total_rows, D, threadIdx.x, blockDim.x);
+        zero_uncovered_rows(m.zero.grad[t].ptr, m.zero.grad[t].stride_s, m.zero.grad[t].stride_h, h, b, m.B, cu, m.S_q, m.total_rows, D,
+                            threadIdx.x, blockDim.x);
     }
+    if (r0 >= q_limit) return;   // nothing of the accumulator there is added to or read
     row_o = static_cast<int64_t>(base + r) * a.o_ss;
     row_do = static_cast<int64_t>(base + r) * a.do_ss;
+  } else if (m.mask_kind == FMHA_MASK_SEQLEN) {
+    const int len = static_cast<const int*>(m.mask)[b];
+    if (len > 0 && len < m.S_k) k_limit = len;
   }
-  float sum = 0.f;
-  if (in_range && r < q_limit) {
-    const unsigned short* po = reinterpret_cast<const unsigned short*>(a.o) + row_o + h * a.o_sh + part * per;
-    const unsigned short* pd = reinterpret_cast<const unsigned short*>(a.d_o) + row_do + h * a.do_sh + part * per;
-    for (int i = 0; i < per / 8; ++i) {
-      const uint4 wo = __ldg(reinterpret_cast<const uint4*>(po) + i);
-      const uint4 wd = __ldg(reinterpret_cast<const uint4*>(pd) + i);
-      const uint32_t xo[4] = {wo.x, wo.y, wo.z, wo.w};
-      const uint32_t xd[4] = {wd.x, wd.y, wd.z, wd.w};
+  uint4 wo = make_uint4(0u, 0u, 0u, 0u), wd = wo;
+  if (r < q_limit) {
+    wo = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.o) + row_o + h * a.o_sh + part * per));
+    wd = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.d_o) + row_do + h * a.do_sh + part * per));
+  }
+  float4* acc = reinterpret_cast<float4*>(m.dq_accum + (static_cast<int64_t>(bh) * m.S_q_pad + r) * D + part * per);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        sum = fmaf(unpack_lo<BF16>(xo[k]), unpack_lo<BF16>(xd[k]), sum);
-        sum = fmaf(unpack_hi<BF16>(xo[k]), unpack_hi<BF16>(xd[k]), sum);
-      }
-    }
+  for (int i = 0; i < per / 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (KEEP) {   // while the loads are under way
+    const int lane = threadIdx.x & 31;
+    const uint32_t off = m.philox_offset + (m.philox_offset_dev != nullptr ? static_cast<uint32_t>(*m.philox_offset_dev) : 0u);
+    uint32_t* words = m.keep.words + (static_cast<int64_t>(bh) * (m.S_q_pad / 32) + blockIdx.y) * m.keep.k_stride;
+    if (r0 < q_limit)
+      for (int k0 = (threadIdx.x >> 5) * 32; k0 < k_limit; k0 += 256)
+        words[k0 + lane] = keep_word_32x32(m.philox_keys, off, static_cast<uint32_t>(m.philox_bh_offset + bh), static_cast<uint32_t>(r0),
+                                           static_cast<uint32_t>(k0 / 16), m.philox_thr, lane);
+  }
+  const uint32_t xo[4] = {wo.x, wo.y, wo.z, wo.w};
+  const uint32_t xd[4] = {wd.x, wd.y, wd.z, wd.w};
+  float sum = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    sum = fmaf(unpack_lo<BF16>(xo[k]), unpack_lo<BF16>(xd[k]), sum);
+    sum = fmaf(unpack_hi<BF16>(xo[k]), unpack_hi<BF16>(xd[k]), sum);
   }
   sum += __shfl_xor_sync(0xffffffffu, sum, 1);
   sum += __shfl_xor_sync(0xffffffffu, sum, 2);
   sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-  if (part == 0 && in_range && r < q_limit) a.delta[static_cast<int64_t>(bh) * a.S_q + r] = sum;
+  if (part == 0 && r < q_limit) m.delta[static_cast<int64_t>(bh) * m.S_q + r] = sum;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -251,27 +296,9 @@ struct BwdItem {
   int tb;        // batch coordinate of the tensor maps (0 for a packed batch)
 };
 
-// Transposes the 32 x 32 bit matrix a warp holds as one row per lane: afterwards bit L of lane p is what bit p of lane L
-// was.  Five exchanges of half-blocks: 16 and 8 bits as byte permutes, 4, 2 and 1 as a rotation and a bit select.
-__device__ __forceinline__ uint32_t warp_bit_transpose(uint32_t x, int lane) {
-  uint32_t y = __shfl_xor_sync(0xffffffffu, x, 16);
-  x = prmt(x, y, (lane & 16) ? 0x3276u : 0x5410u);
-  y = __shfl_xor_sync(0xffffffffu, x, 8);
-  x = prmt(x, y, (lane & 8) ? 0x3715u : 0x6240u);
-#pragma unroll
-  for (int s = 4; s >= 1; s >>= 1) {
-    const uint32_t low = s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
-    const bool up = lane & s;
-    y = __shfl_xor_sync(0xffffffffu, x, s);
-    y = __funnelshift_l(y, y, up ? 32 - s : s);
-    const uint32_t own = up ? ~low : low;
-    x = (x & own) | (y & ~own);
-  }
-  return x;
-}
-
 // PACKED: FMHA_MASK_CU_SEQLENS; a template parameter so that the padded kernels carry none of its bookkeeping.
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
+// BITS: the keep decisions come from the words the pass before wrote (KeepBits), else they are drawn here.
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool BITS = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
   griddep_wait();
   using L = BwdSmem<D>;
@@ -664,9 +691,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     // final scaling of dQ and dK (and of dV, whose P operand is unscaled as well).
     const float dscale = DROP ? a.dropout_scale : 1.0f;
     constexpr int DQ = D / 4;            // columns of a [128 x D] accumulator handled by one thread
-    // The lane that draws for query column c of the warp's 32, chosen so that after the transposition the keep bits of
-    // columns 4j..4j+3 of a thread's key are the top bits of the four bytes of (word << j).
-    const int draw_col = 4 * (7 - (lane & 7)) + (lane >> 3);
     uint8_t* stage = sStage + cw * 2048;   // this warp's staging tile for dK and dV
 
     // Every warp polls the mbarrier itself: funnelling the wait through one warp and a named barrier
@@ -774,23 +798,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         if (c < a.S_k) key_add = reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(cur.b) * a.S_k + c] * kLog2eB;
       }
 
+      [[maybe_unused]] const uint32_t* keep_words = nullptr;
+      [[maybe_unused]] uint32_t keep_next = 0u;
+      if constexpr (DROP && BITS) {
+        keep_words = a.keep.words + (static_cast<int64_t>(bh) * (a.S_q_pad / 32) + cq) * a.keep.k_stride + cur.k0 + row;
+        keep_next = *keep_words;
+      }
       for (int i = 0; i < n_q; ++i, ++t) {
-        // Keep decisions of this thread's key and 32 query columns: two Philox draws (16 keys of one query row each),
-        // made before S is needed, packed to one bit per key and transposed over the warp.
-        [[maybe_unused]] uint32_t keep = 0u;
-        if constexpr (DROP) {
-          const uint32_t poff = *philox_off;
-          const uint32_t q_row = static_cast<uint32_t>(i * kTileM + cq * 32 + draw_col);
-#pragma unroll
-          for (int d = 0; d < 2; ++d) {
-            const U4 u = dropout_draw_keys(a.philox_keys, poff, gbh, q_row, static_cast<uint32_t>((cur.k0 + quad * 32) / 16 + d));
-            const uint32_t ws[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k)   // the keep bit of key 16d + 4k + e ends as bit 8e + 4d + k
-              keep = (keep >> 1) | (((ws[k] & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u) & 0x80808080u);
-          }
-          keep = warp_bit_transpose(keep, lane);
-          keep = __shfl_sync(0xffffffffu, keep, 8 * (lane & 3) + (lane >> 2));
+        [[maybe_unused]] uint32_t keep = 0u;   // keep decisions of this thread's key and 32 query columns
+        if constexpr (DROP && BITS) {
+          keep = keep_next;
+          if (i + 1 < n_q) keep_next = keep_words[static_cast<int64_t>(4 * (i + 1)) * a.keep.k_stride];   // a tile ahead
+        } else if constexpr (DROP) {
+          keep = keep_word_32x32(a.philox_keys, *philox_off, gbh, static_cast<uint32_t>(i * kTileM + cq * 32),
+                                 static_cast<uint32_t>((cur.k0 + quad * 32) / 16), a.philox_thr, lane);
         }
         const uint32_t stats = smem_u32(sStats + (t & 1) * 2 * kTileM + cq * 32);
         mbar_wait(stat_full + (t & 1), (t >> 1) & 1, wctx, kSiteStatFull, kComputeSleepNs);
@@ -916,10 +937,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool BITS = false>
 static int launch_bwd_impl(const BwdArgs& a, cudaStream_t stream) {
   using L = BwdSmem<D>;
-  auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED>;
+  if constexpr (D == 64 && DROP && !BITS) {
+    if (a.keep.words != nullptr) return launch_bwd_impl<D, BF16, KEYADD, DROP, PACKED, true>(a, stream);
+  }
+  auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED, BITS>;
   static std::atomic<bool> configured[64] = {};   // per device; set after the attribute call succeeded
   static std::atomic<int> sm_count[64] = {};
   int dev = 0;
@@ -983,17 +1007,17 @@ int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream) {
   return static_cast<int>(cudaErrorInvalidValue);
 }
 
-int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad, int dtype, float* delta,
-                       float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero, cudaStream_t stream) {
+int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const BwdArgs& m, int dtype, cudaStream_t stream) {
   PrepArgs p;
   p.o = ot.ptr; p.d_o = dot.ptr;
   p.o_sb = ot.stride_b; p.o_sh = ot.stride_h; p.o_ss = ot.stride_s;
   p.do_sb = dot.stride_b; p.do_sh = dot.stride_h; p.do_ss = dot.stride_s;
-  p.B = B; p.H = H; p.S_q = S_q; p.S_q_pad = S_q_pad;
-  p.delta = delta; p.dq_accum = dq_accum; p.work_counter = work_counter; p.cu_seqlens = cu_seqlens; p.zero = zero;
-  const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q_pad + 31) / 32));
-  const cudaError_t e = launch_overlapped(dtype == FMHA_DTYPE_BF16 ? bwd_prepare_kernel<true> : bwd_prepare_kernel<false>, grid,
-                                          dim3(256), 0, stream, p);
+  p.m = m;
+  const dim3 grid(static_cast<unsigned>(m.B) * m.H, static_cast<unsigned>(m.S_q_pad / 32));
+  const bool bf = dtype == FMHA_DTYPE_BF16, keep = m.keep.words != nullptr;
+  auto kfn = keep ? (bf ? bwd_prepare_kernel<true, true> : bwd_prepare_kernel<false, true>)
+                  : (bf ? bwd_prepare_kernel<true, false> : bwd_prepare_kernel<false, false>);
+  const cudaError_t e = launch_overlapped(kfn, grid, dim3(256), 0, stream, p);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 

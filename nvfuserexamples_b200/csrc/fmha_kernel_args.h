@@ -65,6 +65,13 @@ struct FwdArgs {
   int* status;
 };
 
+// Head dimension 64 with dropout: the keep decisions as one bit per score, written by the pass before the main kernel.
+// Word ((bh * S_q_pad/32) + q/32) * k_stride + key holds 32 query rows of a key, in the order keep_word_32x32 makes them.
+struct KeepBits {
+  uint32_t* words;   // null: the main kernel draws for itself
+  int k_stride;      // keys rounded up to whole tiles
+};
+
 // FMHA_FLAG_ZERO_UNCOVERED of the backward pass: the three gradients whose uncovered rows are zeroed (ptr null: none).
 struct UncoveredRows {
   fmha_tensor4 grad[3];
@@ -111,6 +118,7 @@ struct BwdArgs {
   uint32_t philox_offset;
   const long long* philox_offset_dev;   // optional device value added to philox_offset
   int philox_bh_offset;
+  KeepBits keep;
   int* status;
 };
 
@@ -126,8 +134,8 @@ int launch_fwd_dense(const FwdArgs& a, int dtype, cudaStream_t stream);
 int launch_bwd_dq(const BwdArgs& a, int dtype, cudaStream_t stream);   // head dimension 128: dQ, delta, work counter
 int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream);
 // head dimension 64: the passes before and after the main kernel
-int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, int B, int H, int S_q, int S_q_pad, int dtype, float* delta,
-                       float* dq_accum, int* work_counter, const int* cu_seqlens, const UncoveredRows& zero, cudaStream_t stream);
+// `m`: the main kernel's arguments (sizes, mask, Philox, workspace)
+int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const BwdArgs& m, int dtype, cudaStream_t stream);
 int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int dtype, float scale,
                       const int* cu_seqlens, cudaStream_t stream);
 

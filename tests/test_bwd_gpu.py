@@ -262,3 +262,26 @@ def test_backward_accepts_a_broadcast_gradient(cuda_device):
     helpers.assert_close(qg.grad, rdq, "dq")
     helpers.assert_close(kg.grad, rdk, "dk")
     helpers.assert_close(vg.grad, rdv, "dv")
+
+
+@pytest.mark.parametrize("S_q,S_k", [(128, 128), (1, 33), (129, 127), (300, 513), (512, 64)])
+@pytest.mark.parametrize("mask", ["none", "seqlen", "key"])
+def test_keep_bits_and_draws_in_the_kernel_give_the_same_gradients(cuda_device, S_q, S_k, mask):
+    """Head dimension 64 with dropout: the keep decisions come from words an earlier pass wrote, or, where the workspace has
+    no room for them, from draws in the main kernel.  dK and dV have a fixed summation order: the same bits; dQ is summed
+    by atomics."""
+    B, H, p = 2, 3, 0.2
+    q, k, v, d_o, lens = helpers.randn_like_config(B, H, S_q, S_k, 64, torch.float16, seed=S_q + S_k, device=cuda_device)
+    kw = dict(mask_kind=capi.MASK_NONE, mask=None)
+    if mask == "seqlen":
+        kw = dict(mask_kind=capi.MASK_SEQLEN, mask=lens)
+    elif mask == "key":
+        kw = dict(mask_kind=capi.MASK_KEY_ADDITIVE, mask=torch.randn(B, S_k, device=cuda_device))
+    fwd = capi.fwd(q, k, v, dropout_kind=capi.DROPOUT_PHILOX, p_drop=p, seed=3, offset=8, bh_offset=2, **kw)
+    align = lambda x: (x + 255) // 256 * 256
+    least = align(B * H * ((S_q + 127) // 128 * 128) * 64 * 4) + align(B * H * S_q * 4) + 256
+    grads = []
+    for ws in (torch.full((least,), 0xFF, dtype=torch.uint8, device=cuda_device), None):   # None: the size the library asks for
+        grads.append(capi.bwd(d_o, q, k, v, fwd["o"], fwd["lse"], p_drop=p, seed=3, offset=8, bh_offset=2, workspace=ws, **kw))
+    assert torch.equal(grads[0][1], grads[1][1]) and torch.equal(grads[0][2], grads[1][2])
+    helpers.assert_close(grads[0][0], grads[1][0].float(), "dq", torch.float16)
