@@ -74,8 +74,10 @@ struct BwdSmem {
   static constexpr int kOffStats = kOffStage + 32768;         // 2 slots x (128 of -lse*log2e, 128 of delta/c)
   static constexpr int kOffBar = kOffStats + 2 * 2 * kTileM * 4;
   static constexpr int kNumBars = 7 + 4 * kKvBufs + 2 * kQStages + 2 * kDoStages + 8;
-  static constexpr int kOffMisc = kOffBar + kNumBars * 8;
-  static constexpr int kBytes = kOffMisc + 32;
+  static constexpr int kOffRing = (kOffBar + kNumBars * 8 + 15) / 16 * 16;   // 2 work items of 32 bytes
+  static constexpr int kOffRec = kOffRing + 64;   // two 16-byte item records per compute warp
+  static constexpr int kOffMisc = kOffRec + 512;
+  static constexpr int kBytes = kOffMisc + 16;
   // The tiles need a 1024-byte aligned base.  Dynamic shared memory of a kernel without static shared memory begins at
   // such an address; the kernel checks it and gives up if that should ever not hold.
   static constexpr int kDynBytes = kBytes;
@@ -289,11 +291,10 @@ __device__ __forceinline__ int dq_accum_index(int row, int col) {
 
 struct BwdItem {
   int id;      // < 0: no more work
-  int b, h, bh, k0, n_cols;   // n_cols <= 0: key tile wholly masked out
+  int b, h, k0, n_cols;   // n_cols <= 0: key tile wholly masked out
   int n_q;     // query tiles of this item
   int q_limit; // query rows [0, q_limit) exist
   int row_base;  // packed batch: first row of the sequence in the [total_rows, H, D] tensors (else 0)
-  int tb;        // batch coordinate of the tensor maps (0 for a packed batch)
 };
 
 // PACKED: FMHA_MASK_CU_SEQLENS; a template parameter so that the padded kernels carry none of its bookkeeping.
@@ -340,13 +341,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   uint64_t* do_empty = do_full + OS;      // dV of the tile has completed (so P may be overwritten, too)
   uint64_t* stat_full = do_empty + OS;    // [2] lse and delta of a tile's rows are in shared memory
   uint64_t* stat_empty = stat_full + 2;   // [2] ... and have been read (every compute warp arrives)
-  uint64_t* item_full = stat_empty + 2;   // [2] ring of work-item ids
+  uint64_t* item_full = stat_empty + 2;   // [2] ring of work items
   uint64_t* item_empty = item_full + 2;
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 4);
-  volatile int* ring = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 8);   // [2]
   // Philox offset of this launch (launch parameter + optional device-resident value), read where a draw starts
-  volatile uint32_t* philox_off = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 16);
+  volatile uint32_t* philox_off = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 8);
 
   if (smem_u32(smem) & 1023) {   // see kDynBytes
     if (threadIdx.x == 0 && a.status != nullptr) atomicCAS(a.status, 0, kSiteSmemBase);
@@ -407,21 +407,21 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
   const uint32_t tmem_base = *tmem_base_slot;
   const WaitCtx wctx{abort_flag, a.status};
 
+  // By the producer alone: the others get the result through shared memory (divisions and a read of the mask per item and
+  // warp stood in the way of every item's first tile).
   auto decode = [&](int id) {
     BwdItem it;
     it.id = id;
-    it.b = it.h = it.bh = it.k0 = 0;
+    it.b = it.h = it.k0 = 0;
     it.n_cols = 0;
     it.n_q = n_q_all;
     it.q_limit = a.S_q;
     it.row_base = 0;
-    it.tb = 0;
     if (id >= 0) {
       const int kv_tile = id % kv_tiles;
-      it.bh = id / kv_tiles;
-      it.h = it.bh % a.H;
-      it.b = it.bh / a.H;
-      it.tb = it.b;
+      const int bh = id / kv_tiles;
+      it.h = bh % a.H;
+      it.b = bh / a.H;
       it.k0 = kv_tile * kTileN;
       int k_limit = a.S_k;
       if (!packed && a.mask_kind == FMHA_MASK_SEQLEN) {
@@ -436,36 +436,48 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         k_limit = len;
         it.q_limit = len;
         it.n_q = (len + kTileM - 1) / kTileM;
-        it.tb = 0;
       }
       it.n_cols = min(kTileN, k_limit - it.k0);
     }
     return it;
   };
+  const uint32_t ring = smem_u32(smem + L::kOffRing);
   // Consumer side of the work-item ring (whole warp): item number `n` of this CTA.
   auto fetch_item = [&](int n, uint32_t sleep_ns) {
     const int slot = n & 1;
     mbar_wait(item_full + slot, (n >> 1) & 1, wctx, kSiteItemFull, sleep_ns);
-    int id = ring[slot];
-    if (*abort_flag) id = -1;
+    const uint4 x = lds128(ring + slot * 32), y = lds128(ring + slot * 32 + 16);
+    BwdItem it;
+    it.id = *abort_flag ? -1 : static_cast<int>(x.x);
+    it.b = static_cast<int>(x.y);
+    it.h = static_cast<int>(x.z);
+    it.k0 = static_cast<int>(x.w);
+    it.n_cols = static_cast<int>(y.x);
+    it.n_q = static_cast<int>(y.y);
+    it.q_limit = static_cast<int>(y.z);
+    it.row_base = static_cast<int>(y.w);
     __syncwarp();
     if (lane == 0) mbar_arrive(item_empty + slot);
-    return decode(id);
+    return it;
   };
 
   if (warp == 0) {
     // ============================ TMA producer ======================================
     if (lane == 0) {
       int w = 0, g = 0;   // work items with keys / query tiles loaded so far
+      int next = static_cast<int>(blockIdx.x);
       for (int n = 0;; ++n) {
         const int slot = n & 1;
+        const BwdItem it = decode(next < num_items && !*abort_flag ? next : -1);
         if (n >= 2) mbar_wait(item_empty + slot, ((n >> 1) - 1) & 1, wctx, kSiteItemEmpty);
-        int id = (n == 0) ? static_cast<int>(blockIdx.x) : atomicAdd(a.work_counter, 1) + static_cast<int>(gridDim.x);
-        if (id >= num_items || *abort_flag) id = -1;
-        ring[slot] = id;
+        sts128(ring + slot * 32, static_cast<uint32_t>(it.id), static_cast<uint32_t>(it.b), static_cast<uint32_t>(it.h),
+               static_cast<uint32_t>(it.k0));
+        sts128(ring + slot * 32 + 16, static_cast<uint32_t>(it.n_cols), static_cast<uint32_t>(it.n_q), static_cast<uint32_t>(it.q_limit),
+               static_cast<uint32_t>(it.row_base));
         mbar_arrive(item_full + slot);
-        if (id < 0) break;
-        const BwdItem it = decode(id);
+        if (it.id < 0) break;
+        next = atomicAdd(a.work_counter, 1) + static_cast<int>(gridDim.x);   // not looked at before this item's loads are out
+        const int tb = packed ? 0 : it.b;
         if (it.n_cols <= 0) continue;
         const int kvb = w % KV;
         const uint32_t kvp = (w / KV - 1) & 1;
@@ -473,26 +485,26 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         mbar_arrive_expect_tx(k_full + kvb, L::kTileBytes);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c)
-          tma_load_4d(sK + kvb * L::kTileBytes + c * 16384, &a.tm_k, k_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
+          tma_load_4d(sK + kvb * L::kTileBytes + c * 16384, &a.tm_k, k_full + kvb, c * 64, it.row_base + it.k0, it.h, tb);
         for (int i = 0; i < it.n_q; ++i, ++g) {
           const int qs = g % QS, os = g % OS;
           if (g >= QS) mbar_wait(q_empty + qs, ((g / QS) - 1) & 1, wctx, kSiteQEmpty);
           mbar_arrive_expect_tx(q_full + qs, L::kTileBytes);
 #pragma unroll
           for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(sQ + qs * L::kTileBytes + c * 16384, &a.tm_q, q_full + qs, c * 64, it.row_base + i * kTileM, it.h, it.tb);
+            tma_load_4d(sQ + qs * L::kTileBytes + c * 16384, &a.tm_q, q_full + qs, c * 64, it.row_base + i * kTileM, it.h, tb);
           if (i == 0) {   // V after the first Q: with one K/V buffer it comes free after K
             if (w >= KV) mbar_wait(v_empty + kvb, kvp, wctx, kSiteVEmpty);
             mbar_arrive_expect_tx(v_full + kvb, L::kTileBytes);
 #pragma unroll
             for (int c = 0; c < D / 64; ++c)
-              tma_load_4d(sV + kvb * L::kTileBytes + c * 16384, &a.tm_v, v_full + kvb, c * 64, it.row_base + it.k0, it.h, it.tb);
+              tma_load_4d(sV + kvb * L::kTileBytes + c * 16384, &a.tm_v, v_full + kvb, c * 64, it.row_base + it.k0, it.h, tb);
           }
           if (g >= OS) mbar_wait(do_empty + os, ((g / OS) - 1) & 1, wctx, kSiteDoEmpty);
           mbar_arrive_expect_tx(do_full + os, L::kTileBytes);
 #pragma unroll
           for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(sdO + os * L::kTileBytes + c * 16384, &a.tm_do, do_full + os, c * 64, it.row_base + i * kTileM, it.h, it.tb);
+            tma_load_4d(sdO + os * L::kTileBytes + c * 16384, &a.tm_do, do_full + os, c * 64, it.row_base + i * kTileM, it.h, tb);
         }
         ++w;
       }
@@ -540,7 +552,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         mbar_wait(k_full + wi % KV, (wi / KV) & 1, wctx, kSiteKFull);
         if constexpr (D == 64) copy_a(tmem_base + kColK, sK + (wi % KV) * L::kTileBytes);
       }
-      mbar_wait(q_full + tt % QS, (tt / QS) & 1, wctx, kSiteQFull);
+      if (first) mbar_wait(q_full + tt % QS, (tt / QS) & 1, wctx, kSiteQFull);   // else waited for already
       tc_fence_after_sync();
       if constexpr (D == 64) issue_tk(tS, tmem_base + kColK, sQ + (tt % QS) * L::kTileBytes);
       else issue_kk(tS, sK + (wi % KV) * L::kTileBytes, sQ + (tt % QS) * L::kTileBytes);
@@ -555,7 +567,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           umma_commit_elect(v_empty + wi % KV);
         }
       }
-      mbar_wait(do_full + tt % OS, (tt / OS) & 1, wctx, kSiteDoFull);
+      if (first) mbar_wait(do_full + tt % OS, (tt / OS) & 1, wctx, kSiteDoFull);
       tc_fence_after_sync();
       if constexpr (D == 64) issue_tk(tdP, tmem_base + kColV, sdO + (tt % OS) * L::kTileBytes);
       else issue_kk(tdP, sV + (wi % KV) * L::kTileBytes, sdO + (tt % OS) * L::kTileBytes);
@@ -582,6 +594,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         const bool last = i + 1 == n_q;
         const int qs = t % QS, os = t % OS;
         const uint32_t acc0 = (i > 0) ? 1u : 0u;
+        // (the next tile's Q and, below, dO are usually there: polled here, the answer does not hold up S and dP)
+        if (!last) mbar_wait(q_full + (t + 1) % QS, ((t + 1) / QS) & 1, wctx, kSiteQFull);
         // ---- dV += P^T dO: A from tensor memory, dO read MN-major (16 query rows = 2048 B per k-step) ----------------
         const uint64_t ddO_m = make_smem_desc_sw128(smem_u32(sdO + os * L::kTileBytes), 16384, 1024);
         mbar_wait(p_full, t & 1, wctx, kSitePFull);
@@ -605,6 +619,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         if (more) issue_s(t + 1, wn, last, next_last);
         // ---- dK += dS^T Q (A from tensor memory), dP of the next tile over dS(t), dQ tile = dS K ------------------------------
         const uint64_t dQ_m = make_smem_desc_sw128(smem_u32(sQ + qs * L::kTileBytes), 16384, 1024);
+        if (!last) mbar_wait(do_full + (t + 1) % OS, ((t + 1) / OS) & 1, wctx, kSiteDoFull);
         mbar_wait(ds_full, t & 1, wctx, kSiteDsFull);
         tc_fence_after_sync();
         {
@@ -651,8 +666,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       if (cur.id < 0) break;
       if (cur.n_cols <= 0) continue;
       // logsumexp rows: [B*H, S_q], or [H, total_rows] for a packed batch; delta is always [B*H, S_q]
-      const float* lse = a.lse + (packed ? static_cast<int64_t>(cur.h) * a.total_rows + cur.row_base : static_cast<int64_t>(cur.bh) * a.S_q);
-      const float* delta = a.delta + static_cast<int64_t>(cur.bh) * a.S_q;
+      const float* lse = a.lse + (packed ? static_cast<int64_t>(cur.h) * a.total_rows + cur.row_base : static_cast<int64_t>(cur.b * a.H + cur.h) * a.S_q);
+      const float* delta = a.delta + static_cast<int64_t>(cur.b * a.H + cur.h) * a.S_q;
       for (int i = 0; i < cur.n_q; ++i, ++t) {
         float x[4], d[4];
 #pragma unroll
@@ -708,7 +723,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     // accumulator is laid out so that a warp's instruction covers 512 consecutive bytes (dq_accum_index), which keeps the
     // tile out of shared memory: staged there for TMA reduce-adds it cost 32 (D = 64) or 64 KB written and read again per
     // tile, a fifth of all shared-memory traffic.
-    [[maybe_unused]] auto dq_readout = [&](int tt, int64_t row0) {   // D = 64
+    [[maybe_unused]] auto dq_readout = [&](int tt, int tile) {   // D = 64
       wait_all(dq_full, tt & 1, kSiteDqFull);
       uint32_t r[DQ];
 #pragma unroll
@@ -717,7 +732,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       tmem_wait_ld();
       tc_fence_before_sync();
       mbar_arrive(dq_free);                          // the dQ columns may be overwritten
-      float* dst = a.dq_accum + row0 * D + dq_accum_index<D>(row, cq * DQ);
+      float* dst = a.dq_accum + static_cast<int64_t>(tile) * (kTileM * D) + dq_accum_index<D>(row, cq * DQ);
 #pragma unroll
       for (int q = 0; q < DQ / 4; ++q)
         red_add_v4(dst + q * 128, __uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]), __uint_as_float(r[q * 4 + 2]),
@@ -728,21 +743,21 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     // of both accumulators: 32 rows of DQ*2 bytes each.  The staging tile holds one of them at D = 128, both at D = 64
     // (dV first).  Rows past S_k are clipped by the TMA unit.
     constexpr int kDkvRowBytes = DQ * 2;
-    auto store_dkdv = [&](int item_id, bool from_tmem) {
-      const BwdItem it = decode(item_id);
+    auto store_dkdv = [&](int h, int b, int k0, int row_base, int q_limit, bool from_tmem) {
       // Packed batch: a slice that reaches past the end of the sequence would overwrite the next sequence's
       // rows, so its rows are written one by one from registers.
-      const int key = it.k0 + quad * 32 + lane;
-      const bool edge = packed && (it.k0 + quad * 32 + 32 > it.q_limit);
+      const int key = k0 + quad * 32 + lane;
+      const bool edge = packed && (k0 + quad * 32 + 32 > q_limit);
+      stage_free();
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
         const float mul = (which == 0) ? dscale : a.scale * dscale;
         uint8_t* tile = stage + (D == 64 ? which * 32 * kDkvRowBytes : 0);
         const uint32_t rowaddr = smem_u32(tile) + lane * kDkvRowBytes;
-        if (D == 128 || which == 0) stage_free();
+        if (D == 128 && which == 1) stage_free();
         unsigned short* grow = reinterpret_cast<unsigned short*>(which == 0 ? a.dv_ptr : a.dk_ptr) +
-                               static_cast<int64_t>(it.row_base + key) * (which == 0 ? a.dv_ss : a.dk_ss) +
-                               static_cast<int64_t>(it.h) * (which == 0 ? a.dv_sh : a.dk_sh) + cq * DQ;
+                               static_cast<int64_t>(row_base + key) * (which == 0 ? a.dv_ss : a.dk_ss) +
+                               static_cast<int64_t>(h) * (which == 0 ? a.dv_sh : a.dk_sh) + cq * DQ;
 #pragma unroll
         for (int c = 0; c < DQ / 16; ++c) {
           uint32_t r[16];
@@ -761,24 +776,35 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
             w.z = pack2<BF16>(__uint_as_float(r[q * 8 + 4]) * mul, __uint_as_float(r[q * 8 + 5]) * mul);
             w.w = pack2<BF16>(__uint_as_float(r[q * 8 + 6]) * mul, __uint_as_float(r[q * 8 + 7]) * mul);
             if (edge) {
-              if (key < it.q_limit) *reinterpret_cast<uint4*>(grow + c * 16 + q * 8) = w;
+              if (key < q_limit) *reinterpret_cast<uint4*>(grow + c * 16 + q * 8) = w;
             } else {
               sts128(rowaddr + c * 32 + q * 16, w.x, w.y, w.z, w.w);
             }
           }
         }
+        if (D == 64 && which == 0) continue;   // one fence and one commit for both
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && *abort_flag == 0 && !edge) {
-          tma_store_4d(which == 0 ? &a.tm_dv : &a.tm_dk, tile, cq * DQ, it.row_base + it.k0 + quad * 32, it.h, it.tb);
+          const int row0 = row_base + k0 + quad * 32, tb = packed ? 0 : b;
+          if (D == 64 || which == 0) tma_store_4d(&a.tm_dv, stage, cq * DQ, row0, h, tb);
+          if (which == 1) tma_store_4d(&a.tm_dk, tile, cq * DQ, row0, h, tb);
           tma_store_commit();
         }
       }
     };
 
     int n = 0, w = 0, t = 0;      // items fetched, items with work, query tiles so far
-    int prev_id = -1;             // >= 0: dK/dV of that item are still in tensor memory
-    [[maybe_unused]] int64_t prev_row0 = 0;   // D = 64: accumulator row of tile t-1,
+    // What the write-out of an item's dK and dV, done during the next item, needs to know of it waits in shared memory.
+    const uint32_t rec = smem_u32(smem + L::kOffRec) + cw * 32;
+    bool pending = false;         // dK and dV of item number w-1 (with work) are still in tensor memory
+    auto store_pending = [&]() {
+      const uint4 r = lds128(rec + ((w - 1) & 1) * 16);
+      store_dkdv(static_cast<int>(r.x & 0xffffu), static_cast<int>(r.x >> 16), static_cast<int>(r.y), static_cast<int>(r.z),
+                 static_cast<int>(r.w), true);
+      pending = false;
+    };
+    [[maybe_unused]] int prev_tile = 0;       // D = 64: accumulator tile of tile t-1,
     [[maybe_unused]] bool dq_out = true;      // and whether its dQ has been read out
 
     while (true) {
@@ -786,10 +812,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       if (cur.id < 0) break;
       if (cur.n_cols <= 0) {
         if (packed) continue;   // a packed sequence has no rows past its length
-        store_dkdv(cur.id, false);   // key tile wholly past the valid length: its gradients are zero
+        store_dkdv(cur.h, cur.b, cur.k0, cur.row_base, cur.q_limit, false);   // key tile wholly past the valid length: its gradients are zero
         continue;
       }
-      const int n_cols = cur.n_cols, bh = cur.bh, n_q = cur.n_q;
+      if (lane == 0)   // h, b <= 65535
+        sts128(rec + (w & 1) * 16, static_cast<uint32_t>(cur.h) | static_cast<uint32_t>(cur.b) << 16, static_cast<uint32_t>(cur.k0),
+               static_cast<uint32_t>(cur.row_base), static_cast<uint32_t>(cur.q_limit));
+      const int n_cols = cur.n_cols, bh = cur.b * a.H + cur.h, n_q = cur.n_q;
       const uint32_t gbh = static_cast<uint32_t>(a.philox_bh_offset + bh);
       const bool key_ok = row < n_cols;     // keys past the valid length / tensor edge
       float key_add = 0.f;
@@ -798,24 +827,27 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         if (c < a.S_k) key_add = reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(cur.b) * a.S_k + c] * kLog2eB;
       }
 
-      [[maybe_unused]] const uint32_t* keep_words = nullptr;
-      [[maybe_unused]] uint32_t keep_next = 0u;
+      [[maybe_unused]] uint32_t keep_at = 0u, keep_next = 0u;   // at most 2^28 words
       if constexpr (DROP && BITS) {
-        keep_words = a.keep.words + (static_cast<int64_t>(bh) * (a.S_q_pad / 32) + cq) * a.keep.k_stride + cur.k0 + row;
-        keep_next = *keep_words;
+        keep_at = static_cast<uint32_t>((bh * n_q_all * 4 + cq) * a.keep.k_stride + cur.k0 + row);
+        keep_next = a.keep.words[keep_at];
       }
       for (int i = 0; i < n_q; ++i, ++t) {
         [[maybe_unused]] uint32_t keep = 0u;   // keep decisions of this thread's key and 32 query columns
         if constexpr (DROP && BITS) {
           keep = keep_next;
-          if (i + 1 < n_q) keep_next = keep_words[static_cast<int64_t>(4 * (i + 1)) * a.keep.k_stride];   // a tile ahead
+          if (i + 1 < n_q) keep_next = a.keep.words[keep_at += 4 * a.keep.k_stride];   // a tile ahead
         } else if constexpr (DROP) {
           keep = keep_word_32x32(a.philox_keys, *philox_off, gbh, static_cast<uint32_t>(i * kTileM + cq * 32),
                                  static_cast<uint32_t>((cur.k0 + quad * 32) / 16), a.philox_thr, lane);
         }
         const uint32_t stats = smem_u32(sStats + (t & 1) * 2 * kTileM + cq * 32);
-        mbar_wait(stat_full + (t & 1), (t >> 1) & 1, wctx, kSiteStatFull, kComputeSleepNs);
-        wait_all(s_full, t & 1, kSiteSFull);
+        {   // both polls go out before either answer is looked at
+          const bool st_ok = mbar_try_wait(stat_full + (t & 1), (t >> 1) & 1), s_ok = mbar_try_wait(s_full, t & 1);
+          if (!st_ok) mbar_wait(stat_full + (t & 1), (t >> 1) & 1, wctx, kSiteStatFull, kComputeSleepNs);
+          if (!s_ok) mbar_wait(s_full, t & 1, wctx, kSiteSFull, kComputeSleepNs);
+          tc_fence_after_sync();
+        }
         // ---- P ----------------------------------------------------------------------------------------------------------
         uint32_t p[32];
         tmem_ld32(tmem_base + lane_addr + kColS + cq * 32, p);
@@ -849,12 +881,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 #pragma unroll
           for (int k = 0; k < 16; ++k) pk[k] = 0u;
         }
-        if (i == 0 && prev_id >= 0) {
+        if (pending) {
           // dK and dV of the previous item must be out of tensor memory before this tile's P lets the tensor core
           // overwrite dV.
           wait_all(acc_full, (w - 1) & 1, kSiteAccFull);
-          store_dkdv(prev_id, true);
-          prev_id = -1;
+          store_pending();
         }
         tmem_st16(tmem_base + lane_addr + kColP + cq * kPStride, pk);
         tmem_wait_st();
@@ -903,21 +934,21 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         tc_fence_before_sync();
         mbar_arrive(ds_full);
         if constexpr (D == 64) {
-          if (!dq_out) dq_readout(t - 1, prev_row0);
+          if (!dq_out) dq_readout(t - 1, prev_tile);
           dq_out = false;
-          prev_row0 = static_cast<int64_t>(bh) * a.S_q_pad + i * kTileM;
+          prev_tile = bh * n_q_all + i;
         }
       }
-      prev_id = cur.id;
+      pending = true;
       ++w;
     }
     // ---- drain: the last tile's dQ and the last item's dK, dV ------------------------------
     if constexpr (D == 64) {
-      if (!dq_out) dq_readout(t - 1, prev_row0);
+      if (!dq_out) dq_readout(t - 1, prev_tile);
     }
-    if (prev_id >= 0) {
+    if (pending) {
       wait_all(acc_full, (w - 1) & 1, kSiteAccFull);
-      store_dkdv(prev_id, true);
+      store_pending();
     }
     if (lane == 0) tma_store_wait_read();   // shared memory stays valid until the TMA unit has read it
   }
