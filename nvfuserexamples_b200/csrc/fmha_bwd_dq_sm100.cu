@@ -37,6 +37,7 @@ constexpr int kDqCompute = 512;
 constexpr int kDqStatWarp = 2 + kDqCompute / 32;      // the first of two
 constexpr int kDqThreads = 64 + kDqCompute + 64;
 constexpr uint32_t kDqSleepNs = 32;
+constexpr int kDeltaPassKeys = 1024;   // up to here delta has a pass of its own, see launch_dq_impl
 constexpr float kDqLog2e = 1.4426950408889634f;
 
 enum DqWaitSite {
@@ -393,6 +394,13 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
           const int r = half * 64 + k * 32 + lane, q = it.q0 + r;
           st[r] = q < it.q_limit ? -lse[q] * kDqLog2e : -INFINITY;   // rows past the end: their probabilities are zero
         }
+        if (a.o_ptr == nullptr) {   // delta is there already (bwd_delta_kernel)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int r = half * 64 + k * 32 + lane, q = it.q0 + r;
+            st[kTileM + r] = q < it.q_limit ? delta[q] * inv_c : 0.f;
+          }
+        } else
         for (int r0 = half * 64; r0 < half * 64 + 64; r0 += 16) {
           uint4 wo[8], wd[8];
 #pragma unroll
@@ -404,22 +412,37 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
               wd[k] = __ldg(reinterpret_cast<const uint4*>(pd + q * a.do_ss));
             }
           }
+          float v[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const uint32_t xo[4] = {wo[k].x, wo[k].y, wo[k].z, wo[k].w}, xd[4] = {wd[k].x, wd[k].y, wd[k].z, wd[k].w};
-            float sum = 0.f;
+            v[k] = 0.f;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              sum = fmaf(unpack_lo<BF16>(xo[e]), unpack_lo<BF16>(xd[e]), sum);
-              sum = fmaf(unpack_hi<BF16>(xo[e]), unpack_hi<BF16>(xd[e]), sum);
+              v[k] = fmaf(unpack_lo<BF16>(xo[e]), unpack_lo<BF16>(xd[e]), v[k]);
+              v[k] = fmaf(unpack_hi<BF16>(xo[e]), unpack_hi<BF16>(xd[e]), v[k]);
             }
+          }
+          // Eight sums over 16 lanes: in each of three steps a lane keeps half of its values and gets the partner's other
+          // half; `idx` ends as the value it has kept.  (One sum after the other, four shuffles deep each, took 2 000
+          // cycles per batch and made items of few key tiles wait for their statistics.)
+          int idx = 0;
 #pragma unroll
-            for (int m = 1; m < 16; m *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, m);
-            const int r = r0 + 2 * k + (lane >> 4);
-            if (part == 0) {
-              st[kTileM + r] = sum * inv_c;
-              if (it.q0 + r < it.q_limit) delta[it.q0 + r] = sum;
-            }
+          for (int m = 8, cnt = 4; m >= 2; m /= 2, cnt /= 2) {
+            const bool up = part & m;
+            idx = idx * 2 + (up ? 1 : 0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (k < cnt) {
+                const float send = up ? v[k] : v[k + cnt], own = up ? v[k + cnt] : v[k];
+                v[k] = own + __shfl_xor_sync(0xffffffffu, send, m);
+              }
+          }
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+          const int r = r0 + 2 * idx + (lane >> 4);
+          if ((part & 1) == 0) {
+            st[kTileM + r] = v[0] * inv_c;
+            if (it.q0 + r < it.q_limit) delta[it.q0 + r] = v[0];
           }
         }
         __syncwarp();
@@ -574,6 +597,48 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
   }
 }
 
+// delta alone, in a pass of its own: 16 lanes per row, four rows per lane.
+template <bool BF16>
+__global__ void __launch_bounds__(256) bwd_delta_kernel(const __grid_constant__ BwdArgs a) {
+  griddep_wait();
+  const int bh = blockIdx.x, h = bh % a.H, b = bh / a.H;
+  const int part = threadIdx.x & 15;
+  int q_limit = a.S_q;
+  int64_t base_o = static_cast<int64_t>(b) * a.o_sb, base_do = static_cast<int64_t>(b) * a.do_sb;
+  if (a.mask_kind == FMHA_MASK_CU_SEQLENS) {
+    const int* cu = static_cast<const int*>(a.mask);
+    q_limit = min(cu[b + 1] - cu[b], a.S_q);
+    base_o = static_cast<int64_t>(cu[b]) * a.o_ss;
+    base_do = static_cast<int64_t>(cu[b]) * a.do_ss;
+  }
+  const unsigned short* po = static_cast<const unsigned short*>(a.o_ptr) + base_o + h * a.o_sh + part * 8;
+  const unsigned short* pd = static_cast<const unsigned short*>(a.do_ptr) + base_do + h * a.do_sh + part * 8;
+  uint4 wo[4], wd[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t q = blockIdx.y * 64 + k * 16 + (threadIdx.x >> 4);
+    wo[k] = wd[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (q < q_limit) {
+      wo[k] = __ldg(reinterpret_cast<const uint4*>(po + q * a.o_ss));
+      wd[k] = __ldg(reinterpret_cast<const uint4*>(pd + q * a.do_ss));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t xo[4] = {wo[k].x, wo[k].y, wo[k].z, wo[k].w}, xd[4] = {wd[k].x, wd[k].y, wd[k].z, wd[k].w};
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      sum = fmaf(unpack_lo<BF16>(xo[e]), unpack_lo<BF16>(xd[e]), sum);
+      sum = fmaf(unpack_hi<BF16>(xo[e]), unpack_hi<BF16>(xd[e]), sum);
+    }
+#pragma unroll
+    for (int m = 1; m < 16; m *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    const int q = blockIdx.y * 64 + k * 16 + (threadIdx.x >> 4);
+    if (part == 0 && q < q_limit) a.delta[static_cast<int64_t>(bh) * a.S_q + q] = sum;
+  }
+}
+
 template <bool BF16, bool KEYADD, bool DROP, bool PACKED>
 static int launch_dq_impl(const BwdArgs& a, cudaStream_t stream) {
   auto kfn = fmha_bwd_dq_kernel<BF16, KEYADD, DROP, PACKED>;
@@ -587,6 +652,15 @@ static int launch_dq_impl(const BwdArgs& a, cudaStream_t stream) {
   }
   const dim3 grid((a.S_q + kTileM - 1) / kTileM, a.H, a.B);
   BwdArgs args = a;
+  // The two statistics warps need 12 000 cycles for an item's delta, five key tiles' worth: with fewer tiles the compute
+  // warps wait (9 600 cycles per item at four), and a separate pass over O and dO is the cheaper way (B=16 H=16 S=512 with
+  // dropout: 162 us for the whole backward fused, 158 separate; from S_k = 2048 on it is hidden).
+  if (a.S_k <= kDeltaPassKeys) {
+    const cudaError_t e = launch_overlapped(bwd_delta_kernel<BF16>, dim3(static_cast<unsigned>(a.B) * a.H, (a.S_q + 63) / 64), dim3(256), 0,
+                                            stream, a);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    args.o_ptr = nullptr;
+  }
   args.persist = static_cast<int64_t>(grid.x) * grid.y * grid.z > sm_count();
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(kDqThreads), DqSmem::kDynBytes, stream, args);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());

@@ -264,6 +264,8 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_
       ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+// Brings the 128-byte line of a global address to the L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Adds four consecutive floats to global memory (no result), 16-byte aligned.
 __device__ __forceinline__ void red_add_v4(float* p, float x, float y, float z, float w) {
   asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
