@@ -415,30 +415,32 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       tc_fence_after_sync();
 
       // ---- scores into registers (raw, or scaled and masked with an additive mask), row maximum --------------------
+      // Without dropout they stay there until they are exponentiated.  With dropout the step's keep words are live as well:
+      // the scores are read a second time, 32 columns at a time, instead of being spilled.
+      constexpr bool HOLD = !DROP;
+      auto finish_scores = [&](int c, uint32_t (&v)[32]) {   // mask added, keys past the end to -inf (exp2 makes them zero)
+        if constexpr (KEYADD) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const float2 mk = *reinterpret_cast<const float2*>(mask_stage + c * 32 + 2 * k);
+            const float2 t = __ffma2_rn(make_float2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1])), make_float2(sl2, sl2), mk);
+            v[2 * k] = __float_as_uint(t.x);
+            v[2 * k + 1] = __float_as_uint(t.y);
+          }
+        }
+        if (n_cols < TN) {
+#pragma unroll
+          for (int k = 0; k < 32; ++k)
+            if (c * 32 + k >= n_cols) v[k] = __float_as_uint(-INFINITY);
+        }
+      };
       uint32_t sv[TN / 32][32];
 #pragma unroll
       for (int c = 0; c < TN / 32; ++c) tmem_ld32(tS + c * 32, sv[c]);
 #pragma unroll
       for (int c = 0; c < TN / 32; ++c) tmem_wait_ld_dep(sv[c]);
-      if constexpr (KEYADD) {
 #pragma unroll
-        for (int c = 0; c < TN / 32; ++c)
-#pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            const float2 mk = *reinterpret_cast<const float2*>(mask_stage + c * 32 + 2 * k);
-            const float2 t = __ffma2_rn(make_float2(__uint_as_float(sv[c][2 * k]), __uint_as_float(sv[c][2 * k + 1])),
-                                        make_float2(sl2, sl2), mk);
-            sv[c][2 * k] = __float_as_uint(t.x);
-            sv[c][2 * k + 1] = __float_as_uint(t.y);
-          }
-      }
-      if (n_cols < TN) {   // keys past the end: exp2 makes them zero
-#pragma unroll
-        for (int c = 0; c < TN / 32; ++c)
-#pragma unroll
-          for (int k = 0; k < 32; ++k)
-            if (c * 32 + k >= n_cols) sv[c][k] = __float_as_uint(-INFINITY);
-      }
+      for (int c = 0; c < TN / 32; ++c) finish_scores(c, sv[c]);
       float tile_max = -INFINITY;
 #pragma unroll
       for (int c = 0; c < TN / 32; ++c) {
@@ -492,11 +494,29 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
         m_ref = m_new;
       }
       // ---- exponentials, dropout, P over S ---------------------------------------------------------------------
+      if constexpr (HOLD) {
 #pragma unroll
-      for (int c = 0; c < TN / 32; ++c) {
-        uint32_t packed[16];
-        softmax_chunk<BF16, KEYADD, DROP>(sv[c], sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
-        tmem_st16(tS + c * 16, packed);
+        for (int c = 0; c < TN / 32; ++c) {
+          uint32_t packed[16];
+          softmax_chunk<BF16, KEYADD, DROP>(sv[c], sl2, -m_ref, sum2, packed, keepw);
+          tmem_st16(tS + c * 16, packed);
+        }
+      } else {
+        uint32_t ra[32], rb[32], packed[16];   // chunk c+1 (then c+2) is in flight while chunk c (c+1) is processed
+        tmem_ld32(tS, ra);
+#pragma unroll
+        for (int c = 0; c < TN / 32; c += 2) {
+          tmem_wait_ld_dep(ra);
+          finish_scores(c, ra);
+          tmem_ld32(tS + (c + 1) * 32, rb);
+          softmax_chunk<BF16, KEYADD, DROP>(ra, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
+          tmem_st16(tS + c * 16, packed);
+          tmem_wait_ld_dep(rb);
+          finish_scores(c + 1, rb);
+          if (c + 2 < TN / 32) tmem_ld32(tS + (c + 2) * 32, ra);
+          softmax_chunk<BF16, KEYADD, DROP>(rb, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 + 8 : 0));
+          tmem_st16(tS + c * 16 + 16, packed);
+        }
       }
       tmem_wait_st();
       tc_fence_before_sync();
