@@ -285,3 +285,30 @@ def test_keep_bits_and_draws_in_the_kernel_give_the_same_gradients(cuda_device, 
         grads.append(capi.bwd(d_o, q, k, v, fwd["o"], fwd["lse"], p_drop=p, seed=3, offset=8, bh_offset=2, workspace=ws, **kw))
     assert torch.equal(grads[0][1], grads[1][1]) and torch.equal(grads[0][2], grads[1][2])
     helpers.assert_close(grads[0][0], grads[1][0].float(), "dq", torch.float16)
+
+
+@pytest.mark.parametrize("B,H,S_q,S_k,mask,p", [(3, 2, 129, 1025, "key", 0.2), (1, 2, 1, 1100, "seqlen", 0.0), (2, 1, 260, 1024, "key", 0.1),
+                                                (5, 16, 300, 1030, "seqlen", 0.1), (2, 2, 640, 1281, "none", 0.3)])
+def test_head_dim_128_on_both_sides_of_the_delta_pass(cuda_device, B, H, S_q, S_k, mask, p):
+    """Head dimension 128: delta has a pass of its own up to 1024 keys and is formed by two warps of the dQ kernel beyond;
+    both sides of the limit, ragged rows and keys, each mask, and more work items than SMs (5 * 16 * 3 query tiles).  The
+    first and the last head against the oracle."""
+    dtype = torch.float16
+    q, k, v, d_o, lens = helpers.randn_like_config(B, H, S_q, S_k, 128, dtype, seed=S_q + S_k, device=cuda_device)
+    lens[0] = min(S_k, 150)   # whole key tiles without a valid key
+    kw, one = {}, lambda b: {}
+    if mask == "seqlen":
+        kw["seqlens"], one = lens, lambda b: dict(lens=lens[b:b + 1])
+    elif mask == "key":
+        add = composite.padding_add_mask(lens.cpu(), S_k).reshape(B, S_k).to(cuda_device)
+        kw["mask"], one = add, lambda b: dict(add_mask=add[b:b + 1])
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    o, lse = api.fmha_forward(q, k, v, p_drop=p, seed=6, offset=3, status=status, **kw)
+    dq, dk, dv = api.fmha_backward(d_o, q, k, v, o, lse, p_drop=p, seed=6, offset=3, status=status, **kw)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    for b, h in ((0, 0), (B - 1, H - 1)):
+        sl = (slice(b, b + 1), slice(h, h + 1))
+        ref, add_, keep, ks = helpers.oracle_forward(q[sl], k[sl], v[sl], p_drop=p, seed=6, offset=3, bh_offset=b * H + h, **one(b))
+        rdq, rdk, rdv = helpers.oracle_backward(q[sl], k[sl], v[sl], d_o[sl], add=add_, keep=keep, ks=ks)
+        for got, want, name in ((o, ref["o"], "o"), (dq, rdq, "dq"), (dk, rdk, "dk"), (dv, rdv, "dv")):
+            helpers.assert_close(got[sl], want, f"{name}[{b},{h}]", dtype)
