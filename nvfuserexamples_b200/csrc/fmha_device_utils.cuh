@@ -89,6 +89,24 @@ __device__ __forceinline__ void store_row32(void* base, size_t elem_off, int n_v
   }
 }
 
+// The batch element of a given rank when they are sorted by a class (0..7) each, highest first, ties in batch order; evaluated
+// by a whole warp, the same result in every lane.  Lane b holds the class of element b < B <= kMaxOrdered.  A descent over
+// the three bits: of the elements still in question, those with the bit set come first.
+constexpr int kMaxOrdered = 32;
+__device__ __forceinline__ int batch_of_rank(int rank, int B, uint32_t cls) {
+  const int lane = threadIdx.x & 31;
+  uint32_t in = 0xffffffffu >> (32 - B);
+#pragma unroll
+  for (int bit = 2; bit >= 0; --bit) {
+    const uint32_t set = in & __ballot_sync(0xffffffffu, (cls >> bit) & 1u);
+    const int n = __popc(set);
+    const bool among = rank < n;
+    rank -= among ? 0 : n;
+    in = among ? set : in & ~set;
+  }
+  return __ffs(__ballot_sync(0xffffffffu, (in >> lane & 1u) && __popc(in & ((1u << lane) - 1u)) == rank)) - 1;
+}
+
 // Packed batch, FMHA_FLAG_ZERO_UNCOVERED: zeroes, in head h of a [total_rows, H, D] tensor, the rows no tile of
 // sequence b covers: those past the stated maximum length, and (first and last sequence) those outside all sequences.
 // Called by all `nthreads` threads of the one CTA that stands for (b, h); as a rule there is no such row.

@@ -156,7 +156,16 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int h = blockIdx.y;
-  const int b = blockIdx.z;
+  int b = blockIdx.z;
+  if constexpr (D == 64 && !KEYADD && !SPLIT) {
+    if (a.length_class_shift >= 0) {
+      const int* len = reinterpret_cast<const int*>(a.mask);
+      int n = 0;
+      if (lane < a.B) n = PACKED ? len[lane + 1] - len[lane] : len[lane];
+      if (n > a.S_k || (!PACKED && n <= 0)) n = a.S_k;
+      b = batch_of_rank(b, a.B, static_cast<uint32_t>(max(n - 1, 0)) >> a.length_class_shift);
+    }
+  }
   const int n_split = SPLIT ? static_cast<int>(cluster_size()) : 1;
   const int split = SPLIT ? static_cast<int>(cluster_rank()) : 0;
   const int q0 = (SPLIT ? blockIdx.x / n_split : blockIdx.x) * kTileM;
@@ -678,6 +687,23 @@ static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, int sms) {
   return best;
 }
 
+// Longest sequences first: with valid lengths the CTAs of a batch differ in their number of key steps, and they start in grid
+// order.  The shift that puts the lengths into eight classes, or -1 for the order of the batch.  Each CTA finds its batch
+// element by itself (a load and some 200 cycles at its start), which pays at D = 64 up to four rounds of resident CTAs, where
+// the last ones to finish leave SMs idle (lengths U[S/2, S]: B=8 H=12 S=512 16.2 -> 14.9 us, B=16 H=8 S=640 with dropout
+// 35.2 -> 33.3, B=32 H=12 S=512 with dropout 57.0 -> 54.2); beyond it does not (B=64 H=16 S=384 62.3 -> 64.9 us, with two
+// elements per lane), nor at D = 128, where a CTA's start is the longer chain (B=16 H=12 S=512 37.1 -> 38.4 us), and with no
+// more CTAs than SMs the order does not matter.
+static int length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_lengths) {
+  const int64_t sms = sm_count();
+  if (no_lengths || D != 64 || (a.mask_kind != FMHA_MASK_SEQLEN && a.mask_kind != FMHA_MASK_CU_SEQLENS) || a.B < 2 ||
+      a.B > kMaxOrdered || ctas <= sms || ctas > 4 * FastSmem<64>::kCtasPerSm * sms)
+    return -1;
+  int shift = 0;
+  while ((a.S_k - 1) >> shift > 7) ++shift;
+  return shift;
+}
+
 template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool SPLIT = false>
 static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream, int n_split = 1) {
   using L = FastSmem<D>;
@@ -696,7 +722,9 @@ static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream, int n_split =
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   dim3 grid((a.S_q + kTileM - 1) / kTileM * n_split, a.H, a.B);
-  const cudaError_t e = launch_overlapped(kfn, grid, dim3(fast_threads<D>()), L::kDynBytes, stream, a, SPLIT ? n_split : 0);
+  FwdArgs args = a;
+  args.length_class_shift = length_class_shift(a, D, static_cast<int64_t>(grid.x) * grid.y * grid.z, KEYADD || SPLIT);
+  const cudaError_t e = launch_overlapped(kfn, grid, dim3(fast_threads<D>()), L::kDynBytes, stream, args, SPLIT ? n_split : 0);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 

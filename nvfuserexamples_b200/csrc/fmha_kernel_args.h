@@ -39,6 +39,7 @@ struct FwdArgs {
   // tensors; o_ptr / strides serve the row-wise stores of a sequence's last, partial query tile
   int total_rows;
   int zero_uncovered;         // FMHA_FLAG_ZERO_UNCOVERED
+  int length_class_shift;     // production kernel: -1, or the grid's last axis counts batch elements by (length - 1) >> shift
   const void* q_ptr;          // the kernel for a handful of query rows reads Q with plain loads
   int64_t q_ss, q_sh, q_sb;
   void* o_ptr;

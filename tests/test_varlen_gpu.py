@@ -271,3 +271,33 @@ def test_operators_zero_the_rows_no_tile_covers(cuda_device, lens, gap, tail, ma
     for t in (o, *ops.fmha_varlen_bwd(d_o, q, k, v, o, lse, cu, max_len)):
         t = t.cpu()
         assert (t[~covered] == 0).all() and torch.isfinite(t[covered]).all()
+
+
+@pytest.mark.parametrize("B,H,S", [(2, 25, 260), (31, 5, 65), (32, 3, 300), (32, 37, 128)])
+def test_sequences_taken_longest_first_give_the_same_bits(cuda_device, B, H, S):
+    """Up to 32 sequences in more CTAs than SMs are taken longest first, whatever their order in the batch; the same batch
+    with sequences added up to 33 is not.  Each CTA's arithmetic is the same: the same bits.  Lengths 0 (nothing masked),
+    past the end, 1, equal ones; packed: also an empty sequence."""
+    dtype = torch.float16
+    g = torch.Generator().manual_seed(B)
+    lens = torch.randint(1, S + 1, (33,), generator=g, dtype=torch.int32)
+    lens[:2] = torch.tensor([1, S])
+    if B > 8:
+        lens[2:8] = torch.tensor([0, S + 40, S // 2, S // 2, S // 2 + 1, S])
+    q, k, v = (torch.randn(33, H, S, 64, generator=g).to(dtype).to(cuda_device) for _ in range(3))
+    dev = lens.to(cuda_device)
+    few = capi.fwd(q[:B], k[:B], v[:B], mask_kind=capi.MASK_SEQLEN, mask=dev[:B].contiguous())
+    all33 = capi.fwd(q, k, v, mask_kind=capi.MASK_SEQLEN, mask=dev)
+    assert torch.equal(few["o"], all33["o"][:B]) and torch.equal(few["lse"].view(-1), all33["lse"].view(-1)[:B * H * S])
+    ops = torch.ops.mha_manual
+    n = [min(int(x), S) for x in lens]
+    cu = torch.tensor([0] + list(torch.tensor(n).cumsum(0)), dtype=torch.int32, device=cuda_device)
+    pq, pk, pv = (torch.cat([t[b, :, :n[b]].transpose(0, 1) for b in range(33)]).contiguous() for t in (q, k, v))
+    rows = int(cu[B])
+    o1, lse1 = ops.fmha_varlen_fwd(pq[:rows].contiguous(), pk[:rows].contiguous(), pv[:rows].contiguous(), cu[:B + 1].contiguous(), S)
+    o2, lse2 = ops.fmha_varlen_fwd(pq, pk, pv, cu, S)
+    assert torch.equal(o1, o2[:rows]) and torch.equal(lse1, lse2[:, :rows])
+    for b in (0, 1, B - 1):
+        if n[b] >= 128:   # sums long enough for the oracle's bar
+            ref, *_ = helpers.oracle_forward(q[b:b + 1], k[b:b + 1], v[b:b + 1], lens=lens[b:b + 1].clamp(max=S))
+            helpers.assert_close(few["o"][b:b + 1], ref["o"], f"o[{b}]", dtype)
