@@ -128,9 +128,10 @@ typedef struct {
 enum {
   FMHA_FLAG_P_VIA_SMEM = 1, /* forward: stage the probability tile through shared memory instead
                                of tensor memory for the second GEMM (slower; diagnostic) */
-  /* backward, measurement aids: launch only part of the three-kernel sequence so that the main
-     kernel can be timed alone.  The workspace must have been prepared by an earlier full call;
-     results of such partial calls are not meaningful. */
+  /* backward, measurement aids: launch only part of the kernel sequence so that the main kernel (dK and dV; at D = 64 also
+     dQ) can be timed alone: without what comes before it (D = 64: row statistics, accumulator clearing, keep bits; D = 128:
+     dQ and the row statistics), without the dQ conversion that follows it (D = 64).  The workspace must have been prepared by
+     an earlier full call; results of such partial calls are not meaningful. */
   FMHA_FLAG_BWD_SKIP_PREPARE = 2,
   FMHA_FLAG_BWD_SKIP_FINISH = 4,
   /* FMHA_MASK_CU_SEQLENS: write zeros to the rows of o (forward) / dq, dk, dv (backward) that belong to no
@@ -152,7 +153,7 @@ typedef struct {
   float p_drop;
   uint64_t philox_seed, philox_offset;
   int32_t philox_bh_offset;
-  void* workspace;            /* device scratch of fmha_sm100_bwd_workspace_bytes() bytes */
+  void* workspace;            /* device scratch, 256-byte aligned, of fmha_sm100_bwd_workspace_bytes() bytes */
   size_t workspace_bytes;
   int32_t flags;
   int32_t* status;
@@ -169,8 +170,9 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream);
 /* Backward: dQ, dK, dV from (Q, K, V, O, dO, LSE).  P is recomputed from LSE. */
 int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream);
 
-/* Bytes of device scratch fmha_sm100_bwd needs for these sizes (fp32 dQ accumulator and
-   the row term delta = rowsum(dO * O)). */
+/* Bytes of device scratch fmha_sm100_bwd uses for these sizes: the row term delta = rowsum(dO * O), at D = 64 an fp32 dQ
+   accumulator and, with dropout, one bit per score for the keep decisions where that is at most 1 GiB.  A workspace without
+   room for the bits is accepted too: the main kernel then draws for itself (slower, same results). */
 int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes);
 
 /* Backward for callers that cannot hand over a workspace (this entry point has no counterpart
@@ -179,12 +181,12 @@ int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes);
    gave every free byte to its own pool at start-up, a foreign runtime whose calling thread may
    not enter the CUDA allocator, a latency-critical loop for which the implicit device
    synchronisation of cudaMalloc/cudaFree is unacceptable.  For them this variant of
-   fmha_sm100_bwd takes its scratch (fp32 dQ accumulator + delta) from an array that is part of
+   fmha_sm100_bwd takes its scratch from an array that is part of
    the library image instead of p->workspace, which is ignored.  It calls no cudaMalloc, cudaFree
    or other allocating routine.
      - The array is FMHA_STATIC_SCRATCH_BYTES large on EVERY GPU that loads the library, from load
-       to process exit.  Sizes whose fmha_sm100_bwd_workspace_bytes() exceeds it are refused with
-       FMHA_ERR_TOO_LARGE and nothing is launched.
+       to process exit.  Sizes whose accumulator and delta do not fit are refused with FMHA_ERR_TOO_LARGE and nothing is
+       launched; the keep bits are used where they fit as well.
      - The first call on each device looks up the array's device address (once per device, with
        that device current); make that first call before any stream capture begins.
      - All calls share the one array and it keeps what the previous call left; the kernels clear

@@ -6,7 +6,8 @@
 // probabilities from Q, K and the per-row logsumexp the forward kernel wrote.
 //
 // Head dimension 64, three kernels per call:
-//   1. bwd_prepare : delta[row] = sum_d dO[row,d] * O[row,d]  and zero the fp32 dQ accumulator
+//   1. bwd_prepare : delta[row] = sum_d dO[row,d] * O[row,d], zero the fp32 dQ accumulator, and with dropout the keep
+//                    decisions as one bit per score
 //   2. bwd_main    : persistent CTAs (one per SM) draw (128-key tile, head, batch) work items from a
 //                    counter and loop over the 128-row query tiles of each
 //                      S^T = K Q^T           dP^T = V dO^T            (tcgen05.mma, fp32 in TMEM)

@@ -14,9 +14,12 @@
 //   * the row maximum is taken over the raw accumulators with 3-input max (the scale is
 //     positive), the exponent argument is one packed fma.rn.f32x2 per two elements, the row
 //     sum one packed add;
-//   * S is read twice from tensor memory (max, then exponentials) instead of being held in
-//     registers; in the second sweep the load of the next 32 columns is in flight while the
-//     current 32 are processed;
+//   * without dropout the scores of a step are read from tensor memory once and held in registers between the maximum and
+//     the exponentials; with dropout, whose keep words need those registers, they are read twice, the load of the next 32
+//     columns in flight while the current 32 are processed;
+//   * with an additive key mask a step whose keys are all masked away, and would add exact zeros, is skipped;
+//   * few CTAs against many keys: the key steps of a query tile are dealt out over a cluster (fwd_key_split); many CTAs of
+//     unequal length: the longest sequences first (length_class_shift);
 //   * Philox uses one 32x32->64 multiply per product, its keep words for a key step are
 //     computed before the step's scores are awaited (they do not depend on them), and the
 //     keep decision is applied to the packed 16-bit pairs with two byte permutes and two ANDs
