@@ -55,6 +55,10 @@ constexpr float kLn2F = 0.6931471805599453f;
 // flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.
 constexpr float kDeadMask = -1000.0f;
 constexpr float kZeroExp = -200.0f;
+// The row maximum before any score: the lowest float, not -inf, so that a step or a share whose scores are all -inf (an
+// additive mask of -inf, or of the lowest float, which becomes -inf times log2 e) gives exponentials of zero, not of
+// -inf - (-inf).  No finite score is below it.
+constexpr float kNoScore = -3.402823466e+38f;
 constexpr int kMaxKeySplit = 8;   // portable cluster size
 
 enum FastWaitSite {
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     // leaves P and O undefined instead of competing with the others.  (No gain at a ragged last tile of a full grid.)
     const bool warp_idle = SPLIT && q0 + quad * 32 >= q_limit;
 
-    float m_ref = -INFINITY;
+    float m_ref = kNoScore;
     float2 sum2 = make_float2(0.f, 0.f);  // running sum of exp2(t - m_ref), two interleaved partial sums
 
     for (int j = 0; j < n_kv; ++j) {
@@ -500,9 +504,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       // ---- running reference maximum, lazy rescale of O ------------------------------------
       {
         float m_new = fmaxf(m_ref, tile_max);
-        if (m_ref != -INFINITY && m_new - m_ref <= 8.0f) m_new = m_ref;  // exponentials stay below 2^8
-        const bool moved = (m_new != m_ref) && (m_ref != -INFINITY);
-        const float alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - m_new);
+        if (m_new - m_ref <= 8.0f) m_new = m_ref;  // exponentials stay below 2^8
+        const bool moved = m_new != m_ref;
+        const float alpha = fast_exp2(m_ref - m_new);
         if (j > 0 && __any_sync(0xffffffffu, moved)) {
 #pragma unroll
           for (int c = 0; c < D / 8; ++c) {   // eight columns at a time: the scores of the step stay in registers meanwhile
@@ -645,7 +649,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
 #pragma unroll
       for (int k = 0; k < kMaxKeySplit; ++k) {
         if (k >= n_split) break;
-        const float w = fast_exp2(m[k] - m_all);   // 0 for a share without key steps
+        const float w = fast_exp2(m[k] - m_all);   // 0 for a share without key steps, or with keys masked by -inf only
         l_all = fmaf(w, l[k], l_all);
         const uint32_t src = dsmem_map(part_addr + row * (D * 4), k);
 #pragma unroll

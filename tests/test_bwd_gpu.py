@@ -1,5 +1,7 @@
 """Backward parity on the GPU against autograd through the fp32 composite (the reference has
 no backward pass), through the C ABI."""
+import math
+
 import pytest
 import torch
 
@@ -312,3 +314,30 @@ def test_head_dim_128_on_both_sides_of_the_delta_pass(cuda_device, B, H, S_q, S_
         rdq, rdk, rdv = helpers.oracle_backward(q[sl], k[sl], v[sl], d_o[sl], add=add_, keep=keep, ks=ks)
         for got, want, name in ((o, ref["o"], "o"), (dq, rdq, "dq"), (dk, rdk, "dk"), (dv, rdv, "dv")):
             helpers.assert_close(got[sl], want, f"{name}[{b},{h}]", dtype)
+
+
+@pytest.mark.parametrize("B,H,S_q,S_k,D", [
+    (1, 2, 33, 1024, 64),     # keys split over a cluster, shares without a live key
+    (1, 3, 130, 1536, 128),   # ... two query tiles
+    (2, 2, 24, 1000, 64),     # ... one warp of rows
+    (2, 1, 9, 700, 128),      # the kernel for a handful of rows, shares over a cluster
+    (19, 16, 128, 256, 64),   # one CTA per query tile
+    (19, 8, 200, 384, 128),
+])
+@pytest.mark.parametrize("value", [-1e4, torch.finfo(torch.float32).min, -math.inf])
+@pytest.mark.parametrize("side,p_drop", [("right", 0.0), ("left", 0.0), ("right", 0.1)])
+def test_additive_mask_down_to_minus_infinity(cuda_device, B, H, S_q, S_k, D, value, side, p_drop):
+    """Padding as an additive row of any size, the lowest float and -inf included, at either end of the keys: whole key
+    steps, and whole shares where the keys are split, have no live key and contribute nothing."""
+    q, k, v, d_o, _ = helpers.randn_like_config(B, H, S_q, S_k, D, torch.float16, seed=S_q + S_k, device=cuda_device)
+    live = torch.arange(S_k) < 80 if side == "right" else torch.arange(S_k) >= S_k - 80
+    add = torch.where(live, 0.0, value).to(torch.float32).repeat(B, 1)
+    kw = dict(mask=add.to(cuda_device), p_drop=p_drop, seed=11, offset=2)
+    o, lse = api.fmha_forward(q, k, v, **kw)
+    grads = api.fmha_backward(d_o, q, k, v, o, lse, **kw)
+    ref, add_, keep, ks = helpers.oracle_forward(q, k, v, add_mask=add, p_drop=p_drop, seed=11, offset=2)
+    helpers.assert_close(o, ref["o"], "o", torch.float16)
+    helpers.assert_close(lse, ref["lse"], "lse", torch.float16, rtol=1e-4)
+    for got, want, name in zip(grads, helpers.oracle_backward(q, k, v, d_o, add=add_, keep=keep, ks=ks), ("dq", "dk", "dv")):
+        helpers.assert_close(got, want, name, torch.float16)
+    assert all((g[:, :, ~live.to(cuda_device)] == 0).all() for g in grads[1:])
