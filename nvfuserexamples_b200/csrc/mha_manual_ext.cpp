@@ -17,6 +17,7 @@
 //
 // There is no CPU implementation: the operators are registered for the CUDA key only and
 // every failure of the kernel library surfaces as a RuntimeError.
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -683,6 +684,8 @@ template <typename NodeT, size_t N, typename Forward>
 at::Tensor record(const std::array<std::reference_wrapper<const at::Tensor>, N>& inputs, const OptTensor& mask,
                   const OptTensor& lens, const OptTensor& offset_tensor, int64_t max_seqlen, double p_drop, int64_t seed,
                   int64_t offset, c10::optional<double> scale, Forward forward) {
+  // torch.func.grad, vjp and jvp are refused, as by torch::autograd::Function: the node knows nothing of their levels
+  if (const auto& transforms = at::functorch::functorchTLSAccessor()) transforms->checkSupportsCppAutogradFunction();
   bool wanted = mask.has_value() && mask->requires_grad();
   for (const at::Tensor& t : inputs) {
     wanted = wanted || t.requires_grad();

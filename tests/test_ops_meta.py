@@ -124,3 +124,20 @@ def test_torch_compile_traces_the_operator_as_one_graph(ops):
     assert o.shape == q.shape and o.requires_grad
     gq, gk, gv = torch.autograd.grad(o, (q, k, v), torch.empty_like(o))
     assert gq.shape == q.shape and gk.shape == k.shape and gv.shape == v.shape
+
+
+def every_differentiable_operator(ops):
+    """(call, operands) of the four: `call` takes the operands and keyword arguments."""
+    cu = torch.tensor([0, 16, 32], dtype=torch.int32, device="meta")
+    qkv = [meta(2, 3, 16, 64) for _ in range(3)]
+    return [(ops.fmha, qkv), (ops.fmha_qkvpacked, [meta(2, 16, 3, 4, 64)]),
+            (lambda q, k, v, **kw: ops.fmha_varlen(q, k, v, cu, 16, **kw), [meta(32, 3, 64) for _ in range(3)]),
+            (lambda qkv, **kw: ops.fmha_varlen_qkvpacked(qkv, cu, 16, **kw), [meta(32, 3, 4, 64)])]
+
+
+def test_function_transforms_are_refused(ops):
+    for call, x in every_differentiable_operator(ops):
+        for transform in (lambda f: torch.func.grad(lambda t: f(t).sum())(x[0]), lambda f: torch.func.vjp(f, x[0]),
+                          lambda f: torch.func.jvp(f, (x[0],), (x[0],))):
+            with pytest.raises(RuntimeError, match="functorch transforms"):
+                transform(lambda t: call(t, *x[1:]))
