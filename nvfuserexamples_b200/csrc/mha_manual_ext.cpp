@@ -686,19 +686,23 @@ at::Tensor record(const std::array<std::reference_wrapper<const at::Tensor>, N>&
                   int64_t offset, c10::optional<double> scale, Forward forward) {
   // torch.func.grad, vjp and jvp are refused, as by torch::autograd::Function: the node knows nothing of their levels
   if (const auto& transforms = at::functorch::functorchTLSAccessor()) transforms->checkSupportsCppAutogradFunction();
-  bool wanted = mask.has_value() && mask->requires_grad();
-  for (const at::Tensor& t : inputs) {
-    wanted = wanted || t.requires_grad();
+  bool wanted = false;
+  auto look_at = [&](const at::Tensor& t) {
     TORCH_CHECK(!t._fw_grad(0).defined(), "mha_manual: forward-mode derivatives are not implemented");
-  }
+    wanted = wanted || t.requires_grad();
+  };
+  for (const at::Tensor& t : inputs) look_at(t);
+  for (const OptTensor* t : {&mask, &lens, &offset_tensor})
+    if (t->has_value()) look_at(**t);
   wanted = wanted && at::GradMode::is_enabled();
   std::shared_ptr<NodeT> node;
   if (wanted) {
     node = std::shared_ptr<NodeT>(new NodeT(), torch::autograd::deleteNode);
     torch::autograd::edge_list edges;
-    edges.reserve(N + 1);
+    edges.reserve(N + 3);
     for (const at::Tensor& t : inputs) edges.push_back(torch::autograd::impl::gradient_edge(t));
-    if (mask.has_value()) edges.push_back(torch::autograd::impl::gradient_edge(*mask));
+    for (const OptTensor* t : {&mask, &lens, &offset_tensor})   // they take no gradient, but belong to the graph
+      if (t->has_value()) edges.push_back(torch::autograd::impl::gradient_edge(**t));
     node->set_next_edges(std::move(edges));
   }
   at::Tensor o, lse;

@@ -141,3 +141,21 @@ def test_function_transforms_are_refused(ops):
                           lambda f: torch.func.jvp(f, (x[0],), (x[0],))):
             with pytest.raises(RuntimeError, match="functorch transforms"):
                 transform(lambda t: call(t, *x[1:]))
+
+
+def test_every_tensor_argument_takes_part_in_autograd(ops):
+    """A forward-mode tangent is refused on the mask and the lengths as on the operands; an argument that requires a
+    gradient, if only the mask, gives an output that does (the mask's own gradient is undefined)."""
+    import torch.autograd.forward_ad as fw
+
+    qkv = [meta(2, 3, 16, 64) for _ in range(3)]
+    mask, lens = meta(2, 16, dtype=torch.float32), meta(2, dtype=torch.float32)
+    with fw.dual_level():
+        for args in ((fw.make_dual(qkv[0], meta(2, 3, 16, 64)), *qkv[1:], mask), (*qkv, fw.make_dual(mask, torch.empty_like(mask))),
+                     (*qkv, None, fw.make_dual(lens, torch.empty_like(lens)))):
+            with pytest.raises(RuntimeError, match="forward-mode"):
+                ops.fmha(*args)
+    for args in ((*qkv, mask.requires_grad_()), (*qkv, None, lens.requires_grad_())):
+        o = ops.fmha(*args)
+        assert o.requires_grad
+        assert torch.autograd.grad(o, [t for t in args if t is not None and t.requires_grad], torch.empty_like(o), allow_unused=True) == (None,)
