@@ -25,7 +25,6 @@
 
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <torch/csrc/autograd/functions/utils.h>
-#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 
 #include <array>
@@ -631,118 +630,125 @@ void check_status() {
 // ---------------------------------------------------------------------------------------
 // autograd: fmha = fmha_fwd + fmha_bwd, and the same for the three other layouts.
 //
-// Written as graph nodes of their own instead of torch::autograd::Function: at the sizes where the host sets the pace
-// (a B=2, H=4, S=128 step takes 17 us of GPU time) that template's argument vectors, saved-value dictionary and output
-// wrapping cost more than the kernels.
+// The backward functions are ordinary torch::autograd::Function ones, with the node type that goes with them (saved-tensor
+// hooks, compiled autograd and the errors for freed or modified tensors come with it).  Only the forward half of that template
+// is left out: at the sizes where the host sets the pace (a B=2, H=4, S=128 step takes 17 us of GPU time) its argument
+// vectors and output wrapping cost a good part of what the kernels take.
 // ---------------------------------------------------------------------------------------
-using torch::autograd::SavedVariable;
+using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 using OptTensor = c10::optional<at::Tensor>;
-
-struct AttnNode : public torch::autograd::Node {
-  SavedVariable in[3], o, lse, mask, lens, offset_tensor;   // lens: valid lengths or cu_seqlens
-  bool has_mask = false, has_lens = false, has_offset_tensor = false;
-  int64_t max_seqlen = 0;
-  double p_drop = 0.0;
-  int64_t seed = 0, offset = 0;
-  c10::optional<double> scale;
-
-  void release_variables() override {
-    const std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable& s : in) s.reset_data();
-    for (SavedVariable* s : {&o, &lse, &mask, &lens, &offset_tensor}) s->reset_data();
-  }
-  OptTensor opt(const SavedVariable& s, bool has) const { return has ? OptTensor(s.unpack()) : OptTensor(); }
-  // The gradients of this node's inputs, given everything saved.
-  virtual variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) = 0;
-
-  variable_list apply(variable_list&& grads) override {
-    const std::lock_guard<std::mutex> lock(mutex_);
-    const at::Tensor out = o.unpack(shared_from_this());
-    const at::Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(out);
-    variable_list g;
-    if (at::GradMode::is_enabled()) {   // create_graph: the backward operator says itself that it has no derivative
-      g = gradients(d_o, out);
-    } else {
-      at::AutoDispatchBelowADInplaceOrView guard;
-      g = gradients(d_o, out);
-    }
-    g.resize(num_outputs());   // mask, lengths and offset take no gradient
-    return g;
-  }
-};
+using Pair = std::tuple<at::Tensor, at::Tensor>;
+using Triple = std::tuple<at::Tensor, at::Tensor, at::Tensor>;
+using TensorRef = std::reference_wrapper<const at::Tensor>;
 
 template <typename Ret, typename... Args>
 c10::TypedOperatorHandle<Ret(Args...)> find_op(const char* name) {
   return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Ret(Args...)>();
 }
 
-// Runs `forward` (which returns {o, lse}) below the autograd keys and, if a gradient will be wanted, records a NodeT.
-// `inputs`: the differentiable operands; offset_tensor: the backward pass must see the value the forward pass saw, even
-// if the caller advances the tensor in between, so it gets a private copy.
-template <typename NodeT, size_t N, typename Forward>
-at::Tensor record(const std::array<std::reference_wrapper<const at::Tensor>, N>& inputs, const OptTensor& mask,
-                  const OptTensor& lens, const OptTensor& offset_tensor, int64_t max_seqlen, double p_drop, int64_t seed,
-                  int64_t offset, c10::optional<double> scale, Forward forward) {
-  // torch.func.grad, vjp and jvp are refused, as by torch::autograd::Function: the node knows nothing of their levels
+// Runs `forward` (which returns {o, lse}) below the autograd keys and, if a gradient will be wanted, records the node whose
+// backward function is F's.  `inputs`: the differentiable operands; lens: valid lengths or cu_seqlens; offset_tensor: the
+// backward pass must see the value the forward pass saw, even if the caller advances the tensor in between, so it gets a
+// private copy.
+template <typename F, size_t N, typename Forward>
+at::Tensor record(const std::array<TensorRef, N>& inputs, const OptTensor& mask, const OptTensor& lens, const OptTensor& offset_tensor,
+                  int64_t max_seqlen, double p_drop, int64_t seed, int64_t offset, c10::optional<double> scale, Forward forward) {
+  // torch.func.grad, vjp and jvp are refused, as by the template: the node knows nothing of their levels
   if (const auto& transforms = at::functorch::functorchTLSAccessor()) transforms->checkSupportsCppAutogradFunction();
   bool wanted = false;
-  auto look_at = [&](const at::Tensor& t) {
+  size_t n = 0;
+  auto each = [&](auto&& use) {   // only the operands get gradients, but all belong to the graph
+    for (const at::Tensor& t : inputs) use(t);
+    for (const OptTensor* t : {&mask, &lens, &offset_tensor})
+      if (t->has_value()) use(**t);
+  };
+  each([&](const at::Tensor& t) {
     TORCH_CHECK(!t._fw_grad(0).defined(), "mha_manual: forward-mode derivatives are not implemented");
     wanted = wanted || t.requires_grad();
-  };
-  for (const at::Tensor& t : inputs) look_at(t);
-  for (const OptTensor* t : {&mask, &lens, &offset_tensor})
-    if (t->has_value()) look_at(**t);
+    ++n;
+  });
   wanted = wanted && at::GradMode::is_enabled();
-  std::shared_ptr<NodeT> node;
+  std::shared_ptr<torch::autograd::CppNode<F>> node;
   if (wanted) {
-    node = std::shared_ptr<NodeT>(new NodeT(), torch::autograd::deleteNode);
+    node = std::shared_ptr<torch::autograd::CppNode<F>>(new torch::autograd::CppNode<F>(), torch::autograd::deleteNode);
     torch::autograd::edge_list edges;
-    edges.reserve(N + 3);
-    for (const at::Tensor& t : inputs) edges.push_back(torch::autograd::impl::gradient_edge(t));
-    for (const OptTensor* t : {&mask, &lens, &offset_tensor})   // they take no gradient, but belong to the graph
-      if (t->has_value()) edges.push_back(torch::autograd::impl::gradient_edge(**t));
+    edges.reserve(n);
+    each([&](const at::Tensor& t) { edges.push_back(torch::autograd::impl::gradient_edge(t)); });
     node->set_next_edges(std::move(edges));
+    node->is_variable_input_.assign(n, true);
   }
-  at::Tensor o, lse;
+  at::Tensor o, lse, offset_copy;
   {
     at::AutoDispatchBelowADInplaceOrView guard;
     std::tie(o, lse) = forward();
-    if (wanted && offset_tensor.has_value()) {
-      node->offset_tensor = SavedVariable(offset_tensor->clone(), false);
-      node->has_offset_tensor = true;
-    }
+    if (wanted && offset_tensor.has_value()) offset_copy = offset_tensor->clone();
   }
   if (wanted) {
     torch::autograd::set_history(o, node);
-    for (size_t i = 0; i < N; ++i) node->in[i] = SavedVariable(inputs[i].get(), false);
-    node->o = SavedVariable(o, true);
-    node->lse = SavedVariable(lse, false);
-    if ((node->has_mask = mask.has_value())) node->mask = SavedVariable(*mask, false);
-    if ((node->has_lens = lens.has_value())) node->lens = SavedVariable(*lens, false);
-    node->max_seqlen = max_seqlen;
-    node->p_drop = p_drop;
-    node->seed = seed;
-    node->offset = offset;
-    node->scale = scale;
+    node->output_info_.emplace_back(o);
+    node->set_ctx_grad_fn(node);
+    AutogradContext& ctx = node->ctx_;
+    variable_list save;
+    save.reserve(N + 5);
+    for (const at::Tensor& t : inputs) save.push_back(t);
+    save.insert(save.end(), {o, lse, mask.value_or(at::Tensor()), lens.value_or(at::Tensor()), offset_copy});
+    ctx.save_for_backward(std::move(save));
+    ctx.saved_data["max_seqlen"] = max_seqlen;
+    ctx.saved_data["p_drop"] = p_drop;
+    ctx.saved_data["seed"] = seed;
+    ctx.saved_data["offset"] = offset;
+    ctx.saved_data["scale"] = scale;
+    node->save_variables_to_ctx();
   }
   return o;
 }
 
-using Pair = std::tuple<at::Tensor, at::Tensor>;
-using Triple = std::tuple<at::Tensor, at::Tensor, at::Tensor>;
-using TensorRef = std::reference_wrapper<const at::Tensor>;
+// What `record` saved.
+template <size_t N>
+struct Recorded {
+  variable_list t;   // inputs, o, lse, mask, lens, offset_tensor
+  int64_t max_seqlen, seed, offset;
+  double p_drop;
+  c10::optional<double> scale;
+  explicit Recorded(AutogradContext* ctx)
+      : t(ctx->get_saved_variables()), max_seqlen(ctx->saved_data["max_seqlen"].toInt()), seed(ctx->saved_data["seed"].toInt()),
+        offset(ctx->saved_data["offset"].toInt()), p_drop(ctx->saved_data["p_drop"].toDouble()),
+        scale(ctx->saved_data["scale"].toOptional<double>()) {}
+  const at::Tensor& in(size_t i) const { return t[i]; }
+  const at::Tensor& o() const { return t[N]; }
+  const at::Tensor& lse() const { return t[N + 1]; }
+  OptTensor opt(size_t i) const { return t[i].defined() ? OptTensor(t[i]) : OptTensor(); }
+  OptTensor mask() const { return opt(N + 2); }
+  OptTensor lens() const { return opt(N + 3); }
+  OptTensor offset_tensor() const { return opt(N + 4); }
+  // The gradients of the recorded node's inputs: `call` gives those of the operands, the others take none.
+  template <typename Call>
+  variable_list gradients(Call call) const {
+    variable_list g;
+    if (at::GradMode::is_enabled()) {   // create_graph: the backward operator says itself that it has no derivative
+      g = call();
+    } else {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      g = call();
+    }
+    for (size_t i = N + 2; i < N + 5; ++i)
+      if (t[i].defined()) g.emplace_back();
+    return g;
+  }
+};
 
-struct FmhaBackward final : AttnNode {
-  std::string name() const override { return "FmhaBackward"; }
-  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+struct FmhaFunction : public torch::autograd::Function<FmhaFunction> {
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
     static auto op = find_op<Triple, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const at::Tensor&, const OptTensor&, const OptTensor&, double, int64_t, int64_t,
                              c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_bwd");
-    auto [dq, dk, dv] = op.call(d_o, in[0].unpack(), in[1].unpack(), in[2].unpack(), out, lse.unpack(), opt(mask, has_mask),
-                                opt(lens, has_lens), p_drop, seed, offset, scale, 0, opt(offset_tensor, has_offset_tensor));
-    return {dq, dk, dv};
+    const Recorded<3> r(ctx);
+    return r.gradients([&]() -> variable_list {
+      auto [dq, dk, dv] = op.call(grads[0], r.in(0), r.in(1), r.in(2), r.o(), r.lse(), r.mask(), r.lens(), r.p_drop, r.seed, r.offset,
+                                  r.scale, 0, r.offset_tensor());
+      return {dq, dk, dv};
+    });
   }
 };
 at::Tensor fmha_autograd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const OptTensor& mask,
@@ -751,38 +757,41 @@ at::Tensor fmha_autograd(const at::Tensor& q, const at::Tensor& k, const at::Ten
   // through the dispatcher, so that fake / meta tensors reach the shape-only kernels
   static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, const at::Tensor&, const OptTensor&, const OptTensor&,
                            double, int64_t, int64_t, c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_fwd");
-  return record<FmhaBackward, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset,
+  return record<FmhaFunction, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset,
                                  scale, [&] { return op.call(q, k, v, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor); });
 }
 
-struct FmhaQkvPackedBackward final : AttnNode {
-  std::string name() const override { return "FmhaQkvPackedBackward"; }
-  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+struct FmhaQkvPackedFunction : public torch::autograd::Function<FmhaQkvPackedFunction> {
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
     static auto op = find_op<at::Tensor, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const OptTensor&, const OptTensor&, double, int64_t, int64_t, c10::optional<double>, int64_t,
                              const OptTensor&>("mha_manual::fmha_qkvpacked_bwd");
-    return {op.call(d_o, in[0].unpack(), out, lse.unpack(), opt(mask, has_mask), opt(lens, has_lens), p_drop, seed, offset, scale, 0,
-                    opt(offset_tensor, has_offset_tensor))};
+    const Recorded<1> r(ctx);
+    return r.gradients([&]() -> variable_list {
+      return {op.call(grads[0], r.in(0), r.o(), r.lse(), r.mask(), r.lens(), r.p_drop, r.seed, r.offset, r.scale, 0, r.offset_tensor())};
+    });
   }
 };
 at::Tensor fmha_qkvpacked_autograd(const at::Tensor& qkv, const OptTensor& mask, const OptTensor& seqlens, double p_drop,
                                    int64_t seed, int64_t offset, c10::optional<double> scale, const OptTensor& offset_tensor) {
   static auto op = find_op<Pair, const at::Tensor&, const OptTensor&, const OptTensor&, double, int64_t, int64_t,
                            c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_qkvpacked_fwd");
-  return record<FmhaQkvPackedBackward, 1>({TensorRef(qkv)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset, scale, [&] {
+  return record<FmhaQkvPackedFunction, 1>({TensorRef(qkv)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset, scale, [&] {
     return op.call(qkv, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor);
   });
 }
 
-struct FmhaVarlenBackward final : AttnNode {
-  std::string name() const override { return "FmhaVarlenBackward"; }
-  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+struct FmhaVarlenFunction : public torch::autograd::Function<FmhaVarlenFunction> {
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
     static auto op = find_op<Triple, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
                              const OptTensor&>("mha_manual::fmha_varlen_bwd");
-    auto [dq, dk, dv] = op.call(d_o, in[0].unpack(), in[1].unpack(), in[2].unpack(), out, lse.unpack(), lens.unpack(), max_seqlen,
-                                p_drop, seed, offset, scale, opt(offset_tensor, has_offset_tensor));
-    return {dq, dk, dv};
+    const Recorded<3> r(ctx);
+    return r.gradients([&]() -> variable_list {
+      auto [dq, dk, dv] = op.call(grads[0], r.in(0), r.in(1), r.in(2), r.o(), r.lse(), *r.lens(), r.max_seqlen, r.p_drop, r.seed,
+                                  r.offset, r.scale, r.offset_tensor());
+      return {dq, dk, dv};
+    });
   }
 };
 at::Tensor fmha_varlen_autograd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_seqlens,
@@ -790,19 +799,20 @@ at::Tensor fmha_varlen_autograd(const at::Tensor& q, const at::Tensor& k, const 
                                 const OptTensor& offset_tensor) {
   static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t, double,
                            int64_t, int64_t, c10::optional<double>, const OptTensor&>("mha_manual::fmha_varlen_fwd");
-  return record<FmhaVarlenBackward, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen,
+  return record<FmhaVarlenFunction, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen,
                                        p_drop, seed, offset, scale,
                                        [&] { return op.call(q, k, v, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor); });
 }
 
-struct FmhaVarlenQkvPackedBackward final : AttnNode {
-  std::string name() const override { return "FmhaVarlenQkvPackedBackward"; }
-  variable_list gradients(const at::Tensor& d_o, const at::Tensor& out) override {
+struct FmhaVarlenQkvPackedFunction : public torch::autograd::Function<FmhaVarlenQkvPackedFunction> {
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
     static auto op = find_op<at::Tensor, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>, const OptTensor&>(
         "mha_manual::fmha_varlen_qkvpacked_bwd");
-    return {op.call(d_o, in[0].unpack(), out, lse.unpack(), lens.unpack(), max_seqlen, p_drop, seed, offset, scale,
-                    opt(offset_tensor, has_offset_tensor))};
+    const Recorded<1> r(ctx);
+    return r.gradients([&]() -> variable_list {
+      return {op.call(grads[0], r.in(0), r.o(), r.lse(), *r.lens(), r.max_seqlen, r.p_drop, r.seed, r.offset, r.scale, r.offset_tensor())};
+    });
   }
 };
 at::Tensor fmha_varlen_qkvpacked_autograd(const at::Tensor& qkv, const at::Tensor& cu_seqlens, int64_t max_seqlen, double p_drop,
@@ -810,7 +820,7 @@ at::Tensor fmha_varlen_qkvpacked_autograd(const at::Tensor& qkv, const at::Tenso
                                           const OptTensor& offset_tensor) {
   static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
                            const OptTensor&>("mha_manual::fmha_varlen_qkvpacked_fwd");
-  return record<FmhaVarlenQkvPackedBackward, 1>({TensorRef(qkv)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen, p_drop, seed,
+  return record<FmhaVarlenQkvPackedFunction, 1>({TensorRef(qkv)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen, p_drop, seed,
                                                 offset, scale,
                                                 [&] { return op.call(qkv, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor); });
 }

@@ -159,3 +159,37 @@ def test_every_tensor_argument_takes_part_in_autograd(ops):
         o = ops.fmha(*args)
         assert o.requires_grad
         assert torch.autograd.grad(o, [t for t in args if t is not None and t.requires_grad], torch.empty_like(o), allow_unused=True) == (None,)
+
+
+def test_backward_runs_under_compiled_autograd(ops):
+    from torch._dynamo import compiled_autograd
+
+    graphs = []
+    for call, x in every_differentiable_operator(ops):
+        x = [t.requires_grad_() for t in x]
+        with compiled_autograd._enable(lambda graph: graphs.append(graph) or graph):
+            call(*x, p_drop=0.1, scale=0.5, offset_tensor=torch.zeros(1, dtype=torch.int64, device="meta")).sum().backward()
+        assert all(t.grad.shape == t.shape for t in x)
+    assert len(graphs) == 4
+
+
+def test_saved_tensor_hooks_run_with_autograd_in_reach(ops):
+    """The hooks see the operands, o, lse, the mask and the offset, and what they compute may be differentiable: they run
+    outside the region below the autograd keys in which the kernels are called."""
+    packed, unpacked = [], []
+
+    def pack(t):
+        packed.append(tuple(t.shape))
+        return t
+
+    def unpack(t):
+        with torch.enable_grad():
+            unpacked.append((tuple(t.shape), (torch.zeros(1, requires_grad=True) * 2).requires_grad))
+        return t
+
+    q, k, v = (meta(2, 3, 16, 64).requires_grad_() for _ in range(3))
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        o = ops.fmha(q, k, v, meta(2, 16, dtype=torch.float32), None, 0.1, 1, 2, None, torch.zeros(1, dtype=torch.int64, device="meta"))
+    torch.autograd.backward(o, torch.empty_like(o))
+    assert packed == 4 * [(2, 3, 16, 64)] + [(2, 3, 16), (2, 16), (1,)]
+    assert unpacked == [(shape, True) for shape in packed]
