@@ -81,8 +81,12 @@ void finish_call(int rc, const char* what, int device) {
 }
 
 // An uninitialised CUDA tensor straight from the caching allocator: at::empty goes through two dispatcher hops first,
-// which is most of its cost for the sizes where the host sets the pace.
+// which is most of its cost for the sizes where the host sets the pace.  Where torch.use_deterministic_algorithms has new
+// memory filled (rows of a packed logsumexp that belong to no sequence are never written), at::empty does that.
 at::Tensor empty_on(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
+  const at::Context& context = at::globalContext();
+  if (context.deterministicAlgorithms() && context.deterministicFillUninitializedMemory())
+    return at::empty(sizes, like.options().dtype(type));
   return at::Tensor(at::detail::empty_cuda(sizes, type, like.device(), std::nullopt));
 }
 

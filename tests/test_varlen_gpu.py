@@ -301,3 +301,21 @@ def test_sequences_taken_longest_first_give_the_same_bits(cuda_device, B, H, S):
         if n[b] >= 128:   # sums long enough for the oracle's bar
             ref, *_ = helpers.oracle_forward(q[b:b + 1], k[b:b + 1], v[b:b + 1], lens=lens[b:b + 1].clamp(max=S))
             helpers.assert_close(few["o"][b:b + 1], ref["o"], f"o[{b}]", dtype)
+
+
+def test_deterministic_algorithms_fill_what_no_sequence_writes(cuda_device):
+    """torch.use_deterministic_algorithms fills new memory with NaN: the logsumexp rows outside all sequences."""
+    import mha_manual  # noqa: F401
+    x = torch.randn(3, 200, 2, 64, device=cuda_device).half()
+    cu = torch.tensor([10, 150], dtype=torch.int32, device=cuda_device)
+    lse = torch.zeros(2, 200, device=cuda_device)   # the block the operator's allocation is likely to get
+    del lse
+    before = torch.are_deterministic_algorithms_enabled(), torch.utils.deterministic.fill_uninitialized_memory
+    try:
+        torch.use_deterministic_algorithms(True, warn_only=True)
+        torch.utils.deterministic.fill_uninitialized_memory = True
+        lse = torch.ops.mha_manual.fmha_varlen_fwd(x[0], x[1], x[2], cu, 200)[1].cpu()
+    finally:
+        torch.use_deterministic_algorithms(before[0])
+        torch.utils.deterministic.fill_uninitialized_memory = before[1]
+    assert torch.isnan(lse[:, :10]).all() and torch.isnan(lse[:, 150:]).all() and torch.isfinite(lse[:, 10:150]).all()
