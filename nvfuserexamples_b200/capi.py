@@ -28,6 +28,7 @@ DROPOUT_NONE, DROPOUT_DENSE, DROPOUT_PHILOX = 0, 1, 2
 FLAG_P_VIA_SMEM = 1
 FLAG_BWD_SKIP_PREPARE = 2
 FLAG_BWD_SKIP_FINISH = 4
+FLAG_ZERO_UNCOVERED = 8
 STATIC_SCRATCH_BYTES = 32 << 20
 
 EXPORTS = [
@@ -293,7 +294,7 @@ def _t4_packed(x) -> Tensor4:
 
 
 def fwd_varlen(q, k, v, cu_seqlens, max_seqlen, *, p_drop=0.0, seed=0, offset=0, bh_offset=0, scale=None, status=None,
-               out=None):
+               out=None, flags=0):
     """Forward over a packed batch.  Returns {'o': [total,H,D], 'lse': [H,total]}."""
     import torch
     total, H, D = q.shape
@@ -310,17 +311,18 @@ def fwd_varlen(q, k, v, cu_seqlens, max_seqlen, *, p_drop=0.0, seed=0, offset=0,
     if p_drop > 0:
         p.dropout_kind, p.p_drop = DROPOUT_PHILOX, p_drop
     p.philox_seed, p.philox_offset, p.philox_bh_offset = seed, offset, bh_offset
+    p.flags = flags
     p.status = _ptr(status)
     _check(load().fmha_sm100_fwd(C.byref(p), _stream_ptr(q.device)), "fmha_sm100_fwd")
     return {"o": o, "lse": lse}
 
 
 def bwd_varlen(d_o, q, k, v, o, lse, cu_seqlens, max_seqlen, *, p_drop=0.0, seed=0, offset=0, bh_offset=0, scale=None,
-               status=None, workspace=None):
+               status=None, workspace=None, out=None, flags=0):
     """Backward over a packed batch.  Returns (dq, dk, dv), each [total,H,D]."""
     import torch
     total, H, D = q.shape
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    dq, dk, dv = out if out is not None else (torch.empty_like(q), torch.empty_like(k), torch.empty_like(v))
     p = BwdParams()
     p.struct_bytes = C.sizeof(BwdParams)
     p.dtype = _dtype_code(q)
@@ -335,6 +337,7 @@ def bwd_varlen(d_o, q, k, v, o, lse, cu_seqlens, max_seqlen, *, p_drop=0.0, seed
     p.dropout_kind = DROPOUT_PHILOX if p_drop > 0 else DROPOUT_NONE
     p.p_drop = p_drop
     p.philox_seed, p.philox_offset, p.philox_bh_offset = seed, offset, bh_offset
+    p.flags = flags
     p.status = _ptr(status)
     need = bwd_workspace_bytes(p)
     if workspace is None:

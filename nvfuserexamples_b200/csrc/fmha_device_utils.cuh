@@ -109,12 +109,15 @@ __device__ __forceinline__ int batch_of_rank(int rank, int B, uint32_t cls) {
 
 // Packed batch, FMHA_FLAG_ZERO_UNCOVERED: zeroes, in head h of a [total_rows, H, D] tensor, the rows no tile of
 // sequence b covers: those past the stated maximum length, and (first and last sequence) those outside all sequences.
-// Called by all `nthreads` threads of the one CTA that stands for (b, h); as a rule there is no such row.
+// Called by all `nthreads` threads of the one CTA that stands for (b, h); as a rule there is no such row.  Offsets outside the
+// tensor, which the host cannot see, are cut to its rows.
 __device__ __forceinline__ void zero_uncovered_rows(void* base, int64_t stride_s, int64_t stride_h, int h, int b, int B,
                                                     const int* cu, int max_len, int total_rows, int D, int tid, int nthreads) {
   const int lo = cu[b], hi = cu[b + 1];
   auto zero = [&](int r0, int r1) {
     const int per_row = D / 8;   // 16-byte pieces
+    r0 = max(r0, 0);
+    r1 = min(r1, total_rows);
     for (int64_t i = tid; i < static_cast<int64_t>(r1 - r0) * per_row; i += nthreads)
       *reinterpret_cast<uint4*>(static_cast<unsigned short*>(base) + (r0 + i / per_row) * stride_s + h * stride_h +
                                 (i % per_row) * 8) = make_uint4(0u, 0u, 0u, 0u);

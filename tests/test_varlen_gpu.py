@@ -319,3 +319,18 @@ def test_deterministic_algorithms_fill_what_no_sequence_writes(cuda_device):
         torch.use_deterministic_algorithms(before[0])
         torch.utils.deterministic.fill_uninitialized_memory = before[1]
     assert torch.isnan(lse[:, :10]).all() and torch.isnan(lse[:, 150:]).all() and torch.isfinite(lse[:, 10:150]).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_uncovered_rows_are_zeroed_inside_the_tensor_only(cuda_device, D):
+    """Offsets that reach past the rows the call states (a caller's mistake the host cannot see): the zeroing of uncovered
+    rows stops at the last of them.  The tensors are the first 200 rows of larger ones."""
+    H, total, room, max_len = 2, 200, 320, 64
+    q, k, v, d_o = (torch.randn(room, H, D, device=cuda_device).half() for _ in range(4))
+    cu = torch.tensor([0, 100, 300], dtype=torch.int32, device=cuda_device)   # covered: 0..63 and 100..163
+    outs = [torch.full((room, H, D), 7.0, dtype=torch.float16, device=cuda_device) for _ in range(4)]
+    r = capi.fwd_varlen(q[:total], k[:total], v[:total], cu, max_len, out=outs[0][:total], flags=capi.FLAG_ZERO_UNCOVERED)
+    capi.bwd_varlen(d_o[:total], q[:total], k[:total], v[:total], r["o"], r["lse"], cu, max_len,
+                    out=tuple(t[:total] for t in outs[1:]), flags=capi.FLAG_ZERO_UNCOVERED)
+    for t in outs:
+        assert (t[total:] == 7.0).all() and (t[164:total] == 0).all() and (t[64:100] == 0).all() and torch.isfinite(t).all()
