@@ -55,9 +55,10 @@ constexpr float kLn2F = 0.6931471805599453f;
 // flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.
 constexpr float kDeadMask = -1000.0f;
 constexpr float kZeroExp = -200.0f;
-// The row maximum before any score: the lowest float, not -inf, so that a step or a share whose scores are all -inf (an
-// additive mask of -inf, or of the lowest float, which becomes -inf times log2 e) gives exponentials of zero, not of
-// -inf - (-inf).  No finite score is below it.
+// Floor of a step's row maximum: the lowest float, not -inf, so that a step or a share whose scores are all -inf (an additive
+// mask of -inf, or of the lowest float, which becomes -inf times log2 e) gives exponentials of zero, not of -inf - (-inf).  No
+// finite score is below it.  (As the start of the running maximum it does the same, but the additive variant at D = 128 then
+// spills more: B=32 H=16 S=512 103.7 -> 107.8 us.)
 constexpr float kNoScore = -3.402823466e+38f;
 constexpr int kMaxKeySplit = 8;   // portable cluster size
 
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     // leaves P and O undefined instead of competing with the others.  (No gain at a ragged last tile of a full grid.)
     const bool warp_idle = SPLIT && q0 + quad * 32 >= q_limit;
 
-    float m_ref = kNoScore;
+    float m_ref = -INFINITY;
     float2 sum2 = make_float2(0.f, 0.f);  // running sum of exp2(t - m_ref), two interleaved partial sums
 
     for (int j = 0; j < n_kv; ++j) {
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
 #pragma unroll
         for (int c = 0; c < TN / 32; ++c) finish_scores(c, sv[c]);
       }
-      float tile_max = -INFINITY;
+      float tile_max = kNoScore;
 #pragma unroll
       for (int c = 0; c < TN / 32; ++c) {
         if constexpr (AHEAD) {
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
         }
       }
-      if constexpr (!KEYADD) tile_max *= sl2;  // scale > 0: the maximum commutes with it
+      if constexpr (!KEYADD) tile_max = fmaxf(tile_max * sl2, kNoScore);  // scale > 0: the maximum commutes with it
       // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
       // the reference maximum that its exponential is zero in fp32, P is zero and nothing else changes.  Decided on the
       // scores themselves, so the result is the same bits; a third of the steps of a batch with lengths in [S/3, S].
@@ -504,9 +505,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       // ---- running reference maximum, lazy rescale of O ------------------------------------
       {
         float m_new = fmaxf(m_ref, tile_max);
-        if (m_new - m_ref <= 8.0f) m_new = m_ref;  // exponentials stay below 2^8
-        const bool moved = m_new != m_ref;
-        const float alpha = fast_exp2(m_ref - m_new);
+        if (m_ref != -INFINITY && m_new - m_ref <= 8.0f) m_new = m_ref;  // exponentials stay below 2^8
+        const bool moved = (m_new != m_ref) && (m_ref != -INFINITY);
+        const float alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - m_new);
         if (j > 0 && __any_sync(0xffffffffu, moved)) {
 #pragma unroll
           for (int c = 0; c < D / 8; ++c) {   // eight columns at a time: the scores of the step stay in registers meanwhile
