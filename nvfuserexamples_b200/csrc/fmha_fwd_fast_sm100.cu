@@ -425,6 +425,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           keepw[d * 4 + 3] = (draw.w & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
         }
       };
+    draw_and_look:
       if constexpr (DROP) {
         if (live) draw_keep_words();
       }
@@ -453,9 +454,10 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       };
       uint32_t sv[TN / 32][32];
       // The maximum of 32 columns is taken while the next 32 are on their way (D = 128: B=16 H=16 S=1024 163.1 -> 161.6 us,
-      // S=512 with dropout 57.5 -> 56.1; D = 64: 0.5 %); with an additive mask that form spills (B=32 H=16 S=512 D=128
-      // 117 -> 121 us), there all are loaded first.
-      constexpr bool AHEAD = !KEYADD;
+      // S=512 with dropout 57.5 -> 56.1; D = 64: 0.5 %).  With an additive mask and the scores held that form spills (B=32 H=16
+      // S=512 D=128 117 -> 121 us), there all are loaded first; with dropout they are not held, and it spares spills (the same
+      // size with dropout: 134.2 -> 121.3 us, D = 64 93.7 -> 89.5).
+      constexpr bool AHEAD = !KEYADD || DROP;
 #pragma unroll
       for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_ld32(tS + c * 32, sv[c]);
 #pragma unroll
@@ -499,7 +501,10 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           continue;
         }
         if constexpr (DROP) {
-          if (!live) draw_keep_words();
+          if (!live) {   // rare, and a second copy of the draws costs every step (B=2 H=12 S=1024 37.2 -> 36.2 us without it)
+            live = true;
+            goto draw_and_look;
+          }
         }
       }
       // ---- running reference maximum, lazy rescale of O ------------------------------------

@@ -325,7 +325,7 @@ def test_head_dim_128_on_both_sides_of_the_delta_pass(cuda_device, B, H, S_q, S_
     (19, 8, 200, 384, 128),
 ])
 @pytest.mark.parametrize("value", [-1e4, torch.finfo(torch.float32).min, -math.inf])
-@pytest.mark.parametrize("side,p_drop", [("right", 0.0), ("left", 0.0), ("right", 0.1)])
+@pytest.mark.parametrize("side,p_drop", [("right", 0.0), ("left", 0.0), ("right", 0.1), ("left", 0.1)])
 def test_additive_mask_down_to_minus_infinity(cuda_device, B, H, S_q, S_k, D, value, side, p_drop):
     """Padding as an additive row of any size, the lowest float and -inf included, at either end of the keys: whole key
     steps, and whole shares where the keys are split, have no live key and contribute nothing."""
