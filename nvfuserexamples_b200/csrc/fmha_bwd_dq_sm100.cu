@@ -366,13 +366,14 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
     const int half = warp - kDqStatWarp;
     const float inv_c = DROP ? 1.0f / a.dropout_scale : 1.0f;
     const int part = lane & 15;       // 16-byte piece of a row; a warp instruction covers two rows
-    auto side_jobs = [&](const DqItem& x) {   // once per grid / per (b, h), whether the item has work or not
-      if (x.state == kDqEnd || x.q0 != 0) return;
-      if (x.bh == 0 && half == 0 && lane == 0) *a.work_counter = 0;   // the dK / dV kernel draws its items from it
-      if (packed && a.zero.grad[0].ptr != nullptr) {
+    auto side_jobs = [&](const DqItem& x) {   // for every item of the grid, whether it has work or not
+      if (x.state == kDqEnd) return;
+      if (x.bh == 0 && x.q0 == 0 && half == 0 && lane == 0) *a.work_counter = 0;   // the dK / dV kernel draws its items from it
+      if (packed && a.zero.grad[0].ptr != nullptr && (x.q0 + kTileM > x.q_limit || x.q_limit == a.S_q)) {
         for (int k = 0; k < 3; ++k)
           zero_uncovered_rows(a.zero.grad[k].ptr, a.zero.grad[k].stride_s, a.zero.grad[k].stride_h, x.h, x.b, a.B,
-                              reinterpret_cast<const int*>(a.mask), a.S_q, a.total_rows, D, half * 32 + lane, 64);
+                              reinterpret_cast<const int*>(a.mask), a.S_q, a.total_rows, D, x.q0, x.q0 + kTileM,
+                              a.zero.mode == kUncoveredAll, half * 32 + lane, 64);
       }
     };
     int n = 0, w = 0;

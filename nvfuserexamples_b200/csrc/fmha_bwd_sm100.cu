@@ -138,7 +138,9 @@ __device__ __forceinline__ uint32_t keep_word_32x32(const PhiloxKeys& keys, uint
 // KEEP: also the keep bits of the block's 32 query rows.  The draws run at the multipliers' rate beside the memory traffic of
 // the rest; in the main kernel, where 16 warps wait for one another's phases, they took 1 000 of 4 900 cycles per tile.
 template <bool BF16, bool KEEP>
-__global__ void __launch_bounds__(256) bwd_prepare_kernel(const __grid_constant__ PrepArgs a) {
+// Without draws 32 registers, so that eight blocks share an SM: the rare zeroing of uncovered rows had taken 48 (20.2 -> 24.6 us at
+// 16 384 rows, 16 heads).
+__global__ void __launch_bounds__(256, KEEP ? 5 : 8) bwd_prepare_kernel(const __grid_constant__ PrepArgs a) {
   griddep_wait();
   // grid = (B*H, blocks of 32 rows); 8 threads per row, 8 elements each.
   // The head index comes from the grid, so no thread divides 64-bit indices.
@@ -158,11 +160,12 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const __grid_constant_
   if (m.mask_kind == FMHA_MASK_CU_SEQLENS) {
     const int* cu = static_cast<const int*>(m.mask);
     const int base = cu[b];
-    q_limit = k_limit = min(cu[b + 1] - base, m.S_q);   // rows past the stated maximum length take no part
-    if (blockIdx.y == 0 && m.zero.grad[0].ptr != nullptr) {
+    const int len = cu[b + 1] - base;
+    q_limit = k_limit = min(len, m.S_q);   // rows past the stated maximum length take no part
+    if (m.zero.grad[0].ptr != nullptr && (r0 + 32 > q_limit || len > q_limit)) {
       for (int t = 0; t < 3; ++t)
         zero_uncovered_rows(m.zero.grad[t].ptr, m.zero.grad[t].stride_s, m.zero.grad[t].stride_h, h, b, m.B, cu, m.S_q, m.total_rows, D,
-                            threadIdx.x, blockDim.x);
+                            r0, r0 + 32, m.zero.mode == kUncoveredAll, threadIdx.x, blockDim.x);
     }
     if (r0 >= q_limit) return;   // nothing of the accumulator there is added to or read
     row_o = static_cast<int64_t>(base + r) * a.o_ss;

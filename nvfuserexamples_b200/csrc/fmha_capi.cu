@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -117,6 +118,40 @@ static fmha_tensor4 sanitized(const fmha_tensor4& t, int B, int H, int S, int D)
   return r;
 }
 
+// More rows than sequences of the stated length can have: the rows outside all sequences are zeroed by a kernel of their own.
+static int uncovered_mode(int B, int max_len, int total_rows) {
+  return static_cast<int64_t>(B) * max_len < total_rows ? kUncoveredCut : kUncoveredAll;
+}
+struct OutsideArgs {
+  UncoveredRows u;
+  int B, H, D;
+  const int* cu;
+};
+// Bound by its writes; kOutsideRows rows of all heads per block and step.
+constexpr int kOutsideRows = 8;
+__global__ void __launch_bounds__(256) zero_outside_rows_kernel(const __grid_constant__ OutsideArgs a) {
+  griddep_wait();
+  const UncoveredRows& u = a.u;
+  const int* cu = a.cu;
+  const int B = a.B, H = a.H, D = a.D;
+  const int first = min(max(cu[0], 0), u.total_rows), last = min(max(cu[B], first), u.total_rows), n = first + u.total_rows - last;
+  const int per_row = H * (D / 8);
+  for (int t = 0; t < 3 && u.grad[t].ptr != nullptr; ++t)
+    for (int k0 = blockIdx.x * kOutsideRows; k0 < n; k0 += gridDim.x * kOutsideRows)
+      for (int i = threadIdx.x; i < min(kOutsideRows, n - k0) * per_row; i += 256) {
+        const int k = k0 + i / per_row, piece = i % per_row;
+        unsigned short* row = static_cast<unsigned short*>(u.grad[t].ptr) + (k < first ? k : last + static_cast<int64_t>(k - first)) * u.grad[t].stride_s;
+        *reinterpret_cast<uint4*>(row + piece / (D / 8) * u.grad[t].stride_h + piece % (D / 8) * 8) = make_uint4(0u, 0u, 0u, 0u);
+      }
+}
+static int zero_outside_rows(const UncoveredRows& u, int B, int H, int D, const int* cu, cudaStream_t stream) {
+  if (u.mode != kUncoveredCut) return 0;
+  const OutsideArgs a = {u, B, H, D, cu};
+  const int blocks = std::min(u.total_rows / kOutsideRows + 1, 8 * sm_count());
+  const cudaError_t e = launch_overlapped(zero_outside_rows_kernel, dim3(blocks), dim3(256), 0, stream, a);
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+
 static int check_device() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -208,7 +243,12 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
   if ((rc = make_tmap(&a.tm_v, sanitized(p->v, mB, p->H, mSk, p->D), p->dtype, mB, p->H, mSk, p->D, kv_rows))) return rc;
   if ((rc = make_tmap(&a.tm_o, sanitized(p->o, mB, p->H, mSq, p->D), p->dtype, mB, p->H, mSq, p->D, kTileM))) return rc;
   a.total_rows = p->total_rows;
-  a.zero_uncovered = (p->flags & FMHA_FLAG_ZERO_UNCOVERED) != 0;
+  if (packed && (p->flags & FMHA_FLAG_ZERO_UNCOVERED)) {
+    const UncoveredRows u = {{sanitized(p->o, mB, p->H, mSq, p->D)}, p->total_rows, uncovered_mode(p->B, p->S_q, p->total_rows)};
+    a.zero_uncovered = u.mode;
+    if (const int e = zero_outside_rows(u, p->B, p->H, p->D, static_cast<const int*>(p->mask), static_cast<cudaStream_t>(stream)))
+      return cuda_fail(static_cast<cudaError_t>(e));
+  }
   a.o_ptr = p->o.ptr; a.o_ss = p->o.stride_s; a.o_sh = p->o.stride_h;
   a.o_sb = sanitized(p->o, mB, p->H, mSq, p->D).stride_b;
   a.o_sh = sanitized(p->o, mB, p->H, mSq, p->D).stride_h;
@@ -389,7 +429,10 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
   a.philox_bh_offset = p->philox_bh_offset;
   a.status = p->status;
 
-  if (packed && (p->flags & FMHA_FLAG_ZERO_UNCOVERED)) a.zero = {{tdq, tdk, tdv}, p->total_rows};
+  if (packed && (p->flags & FMHA_FLAG_ZERO_UNCOVERED)) {
+    a.zero = {{tdq, tdk, tdv}, p->total_rows, uncovered_mode(p->B, p->S_q, p->total_rows)};
+    if (const int e0 = zero_outside_rows(a.zero, p->B, p->H, p->D, cu_seqlens, stream)) return cuda_fail(static_cast<cudaError_t>(e0));
+  }
   const bool two_pass = p->D == 128;   // dQ (and delta) in a kernel of its own; see fmha_bwd_dq_sm100.cu
   int e = 0;
   if (p->flags & FMHA_FLAG_BWD_SKIP_PREPARE) {

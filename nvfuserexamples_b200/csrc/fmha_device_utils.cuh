@@ -107,24 +107,37 @@ __device__ __forceinline__ int batch_of_rank(int rank, int B, uint32_t cls) {
   return __ffs(__ballot_sync(0xffffffffu, (in >> lane & 1u) && __popc(in & ((1u << lane) - 1u)) == rank)) - 1;
 }
 
-// Packed batch, FMHA_FLAG_ZERO_UNCOVERED: zeroes, in head h of a [total_rows, H, D] tensor, the rows no tile of
-// sequence b covers: those past the stated maximum length, and (first and last sequence) those outside all sequences.
-// Called by all `nthreads` threads of the one CTA that stands for (b, h); as a rule there is no such row.  Offsets outside the
-// tensor, which the host cannot see, are cut to its rows.
+// Packed batch, FMHA_FLAG_ZERO_UNCOVERED: zeroes, in head h of a [total_rows, H, D] tensor, the caller's share of the rows that no
+// tile covers.  The caller stands for rows [r0, r1) of sequence b, as if every sequence had max_len rows; all callers together
+// stand for all of them.  A sequence past max_len: its callers share the rows it is cut by.  Rows outside all sequences (`outside`;
+// at most as many as the batch has rows of padding in this sense, else zero_outside_rows_kernel): the k-th row of padding, counted
+// through the batch, stands for the k-th such row, so that callers without padding have nothing to look up and no caller has more
+// rows than its own.  (One caller per head for all of them took three to four times as long as the fill of whole tensors that this
+// replaces where a buffer was far from full.)  Offsets outside the tensor, which the host cannot see, are cut to its rows.
+// Only callers with r1 > len or len > max_len can have a share.
 __device__ __forceinline__ void zero_uncovered_rows(void* base, int64_t stride_s, int64_t stride_h, int h, int b, int B,
-                                                    const int* cu, int max_len, int total_rows, int D, int tid, int nthreads) {
-  const int lo = cu[b], hi = cu[b + 1];
-  auto zero = [&](int r0, int r1) {
+                                                    const int* cu, int max_len, int total_rows, int D, int r0, int r1, bool outside,
+                                                    int tid, int nthreads) {
+  const int lo = cu[b], hi = cu[b + 1], len = hi - lo;
+  r1 = min(r1, max_len);
+  auto zero = [&](int64_t from, int64_t to) {
+    from = max(from, static_cast<int64_t>(0));
+    to = min(to, static_cast<int64_t>(total_rows));
     const int per_row = D / 8;   // 16-byte pieces
-    r0 = max(r0, 0);
-    r1 = min(r1, total_rows);
-    for (int64_t i = tid; i < static_cast<int64_t>(r1 - r0) * per_row; i += nthreads)
-      *reinterpret_cast<uint4*>(static_cast<unsigned short*>(base) + (r0 + i / per_row) * stride_s + h * stride_h +
+    for (int64_t i = tid; i < (to - from) * per_row; i += nthreads)
+      *reinterpret_cast<uint4*>(static_cast<unsigned short*>(base) + (from + i / per_row) * stride_s + h * stride_h +
                                 (i % per_row) * 8) = make_uint4(0u, 0u, 0u, 0u);
   };
-  if (hi - lo > max_len) zero(lo + max_len, hi);
-  if (b == 0 && lo > 0) zero(0, lo);
-  if (b == B - 1 && hi < total_rows) zero(hi, total_rows);
+  if (len > max_len) {
+    const int64_t cut = len - max_len, at = static_cast<int64_t>(lo) + max_len;
+    zero(at + cut * r0 / max_len, at + cut * r1 / max_len);
+  } else if (outside && r1 > len) {
+    const int64_t first = cu[0], last = cu[B], n = first + total_rows - last;
+    const int64_t pad0 = max(r0, len);
+    const int64_t k0 = static_cast<int64_t>(b) * max_len - (lo - first) + (pad0 - len), k1 = min(k0 + (r1 - pad0), n);
+    if (k0 < first) zero(k0, min(k1, first));
+    if (k1 > first) zero(last + max(k0, first) - first, last + k1 - first);
+  }
 }
 
 }  // namespace fmha

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   // Philox offset of this launch: the launch parameter plus the optional device-resident value.  Kept in shared
   // memory and read where a draw starts, so that it holds no register in between.
   volatile uint32_t* philox_off = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 8);
+  volatile int* uncovered = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 12);   // packed: rows may be left to zero
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -190,13 +191,18 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   } else if (packed) {
     const int* cu = reinterpret_cast<const int*>(a.mask);
     row_base = cu[b];
-    const int len = min(cu[b + 1] - row_base, a.S_q);   // a sequence longer than the stated maximum is cut there
+    const int all = cu[b + 1] - row_base;
+    const int len = min(all, a.S_q);   // a sequence longer than the stated maximum is cut there
     k_limit = len;
     q_limit = len;
     tb = 0;
-    if (blockIdx.x == 0 && a.zero_uncovered)
-      zero_uncovered_rows(a.o_ptr, a.o_ss, a.o_sh, h, b, a.B, cu, a.S_q, a.total_rows, D, threadIdx.x, blockDim.x);
-    if (q0 >= len) return;   // this sequence has no such query tile (whole CTA, before any barrier)
+    if (q0 >= len) {   // this sequence has no such query tile (whole CTA, before any barrier)
+      if (a.zero_uncovered)
+        zero_uncovered_rows(a.o_ptr, a.o_ss, a.o_sh, h, b, a.B, cu, a.S_q, a.total_rows, D, q0, q0 + kTileM,
+                            a.zero_uncovered == kUncoveredAll, threadIdx.x, blockDim.x);
+      return;
+    }
+    if (threadIdx.x == 0) *uncovered = a.zero_uncovered && (q0 + kTileM > len || all > len);
   }
   const int n_kv_all = (k_limit + TN - 1) / TN;
   // key steps of this CTA: [j0, j0 + n_kv); with SPLIT possibly none
@@ -629,6 +635,11 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     }
   }
 
+  if constexpr (PACKED) {   // last, so that no start of a CTA waits for the offsets
+    if (*uncovered)
+      zero_uncovered_rows(a.o_ptr, a.o_ss, a.o_sh, h, b, a.B, reinterpret_cast<const int*>(a.mask), a.S_q, a.total_rows, D, q0,
+                          q0 + kTileM, a.zero_uncovered == kUncoveredAll, threadIdx.x, blockDim.x);
+  }
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (SPLIT) {

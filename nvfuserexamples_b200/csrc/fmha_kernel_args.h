@@ -38,7 +38,7 @@ struct FwdArgs {
   // FMHA_MASK_CU_SEQLENS (production kernel): mask = int32 [B+1] row offsets into the packed [total_rows, H, D]
   // tensors; o_ptr / strides serve the row-wise stores of a sequence's last, partial query tile
   int total_rows;
-  int zero_uncovered;         // FMHA_FLAG_ZERO_UNCOVERED
+  int zero_uncovered;         // FMHA_FLAG_ZERO_UNCOVERED: 0, or an UncoveredMode
   int length_class_shift;     // production kernel: -1, or the grid's last axis counts batch elements by (length - 1) >> shift
   const void* q_ptr;          // the kernel for a handful of query rows reads Q with plain loads
   int64_t q_ss, q_sh, q_sb;
@@ -73,10 +73,14 @@ struct KeepBits {
   int k_stride;      // keys rounded up to whole tiles
 };
 
-// FMHA_FLAG_ZERO_UNCOVERED of the backward pass: the three gradients whose uncovered rows are zeroed (ptr null: none).
+// FMHA_FLAG_ZERO_UNCOVERED: the kernels zero the rows sequences are cut by, and those outside all sequences unless
+// zero_outside_rows_kernel has (there are more of them than rows of padding, see zero_uncovered_rows).
+enum UncoveredMode { kUncoveredAll = 1, kUncoveredCut = 2 };
+// The backward pass: the three gradients (ptr null: none).
 struct UncoveredRows {
   fmha_tensor4 grad[3];
   int total_rows;
+  int mode;
 };
 
 struct BwdArgs {

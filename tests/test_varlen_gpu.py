@@ -244,7 +244,9 @@ def test_sequence_longer_than_max_seqlen_is_cut_not_spilled(cuda_device):
     helpers.assert_close(g[0][keep_rows], ref["dq"], "dq (operator)", dtype)
 
 
-@pytest.mark.parametrize("lens,gap,tail,max_len", [([150, 300, 90], 0, 0, 256), ([40, 130], 7, 33, 128), ([128], 1, 0, 128), ([0, 5], 0, 9, 64)])
+@pytest.mark.parametrize("lens,gap,tail,max_len", [([150, 300, 90], 0, 0, 256), ([40, 130], 7, 33, 128), ([128], 1, 0, 128), ([0, 5], 0, 9, 64),
+                                                   ([40, 130], 700, 3001, 128), ([5], 0, 20000, 64), ([1500, 0, 20], 1, 400, 100),
+                                                   ([300, 10, 0, 64, 200], 5, 100, 256), ([100] * 9, 3, 30, 104)])
 @pytest.mark.parametrize("D", [64, 128])
 def test_operators_zero_the_rows_no_tile_covers(cuda_device, lens, gap, tail, max_len, D):
     """Rows past max_seqlen of their sequence and rows outside all sequences are zeros whatever the memory held before
