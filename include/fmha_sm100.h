@@ -129,7 +129,7 @@ enum {
   FMHA_FLAG_P_VIA_SMEM = 1, /* forward: stage the probability tile through shared memory instead
                                of tensor memory for the second GEMM (slower; diagnostic) */
   /* backward, measurement aids: launch only part of the kernel sequence so that the main kernel (dK and dV; at D = 64 also
-     dQ) can be timed alone: without what comes before it (D = 64: row statistics, accumulator clearing, keep bits; D = 128:
+     dQ) can be timed alone: without what comes before it (D = 64: row statistics, accumulator clearing; D = 128:
      dQ and the row statistics), without the dQ conversion that follows it (D = 64).  The workspace must have been prepared by
      an earlier full call; results of such partial calls are not meaningful. */
   FMHA_FLAG_BWD_SKIP_PREPARE = 2,
@@ -170,9 +170,8 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream);
 /* Backward: dQ, dK, dV from (Q, K, V, O, dO, LSE).  P is recomputed from LSE. */
 int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream);
 
-/* Bytes of device scratch fmha_sm100_bwd uses for these sizes: the row term delta = rowsum(dO * O), at D = 64 an fp32 dQ
-   accumulator and, with dropout, one bit per score for the keep decisions where that is at most 1 GiB.  A workspace without
-   room for the bits is accepted too: the main kernel then draws for itself (slower, same results). */
+/* Bytes of device scratch fmha_sm100_bwd needs for these sizes: the row term delta = rowsum(dO * O) and, at D = 64, an fp32 dQ
+   accumulator. */
 int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes);
 
 /* Backward for callers that cannot hand over a workspace (this entry point has no counterpart
@@ -185,8 +184,8 @@ int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes);
    the library image instead of p->workspace, which is ignored.  It calls no cudaMalloc, cudaFree
    or other allocating routine.
      - The array is FMHA_STATIC_SCRATCH_BYTES large on EVERY GPU that loads the library, from load
-       to process exit.  Sizes whose accumulator and delta do not fit are refused with FMHA_ERR_TOO_LARGE and nothing is
-       launched; the keep bits are used where they fit as well.
+       to process exit.  Sizes whose fmha_sm100_bwd_workspace_bytes() exceeds it are refused with
+       FMHA_ERR_TOO_LARGE and nothing is launched.
      - The first call on each device looks up the array's device address (once per device, with
        that device current); make that first call before any stream capture begins.
      - All calls share the one array and it keeps what the previous call left; the kernels clear

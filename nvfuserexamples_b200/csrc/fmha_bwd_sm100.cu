@@ -6,8 +6,7 @@
 // probabilities from Q, K and the per-row logsumexp the forward kernel wrote.
 //
 // Head dimension 64, three kernels per call:
-//   1. bwd_prepare : delta[row] = sum_d dO[row,d] * O[row,d], zero the fp32 dQ accumulator, and with dropout the keep
-//                    decisions as one bit per score
+//   1. bwd_prepare : delta[row] = sum_d dO[row,d] * O[row,d], and zero the fp32 dQ accumulator
 //   2. bwd_main    : persistent CTAs (one per SM) draw (128-key tile, head, batch) work items from a
 //                    counter and loop over the 128-row query tiles of each
 //                      S^T = K Q^T           dP^T = V dO^T            (tcgen05.mma, fp32 in TMEM)
@@ -135,12 +134,10 @@ __device__ __forceinline__ uint32_t keep_word_32x32(const PhiloxKeys& keys, uint
   return __shfl_sync(0xffffffffu, keep, 8 * (lane & 3) + (lane >> 2));
 }
 
-// KEEP: also the keep bits of the block's 32 query rows.  The draws run at the multipliers' rate beside the memory traffic of
-// the rest; in the main kernel, where 16 warps wait for one another's phases, they took 1 000 of 4 900 cycles per tile.
-template <bool BF16, bool KEEP>
-// Without draws 32 registers, so that eight blocks share an SM: the rare zeroing of uncovered rows had taken 48 (20.2 -> 24.6 us at
-// 16 384 rows, 16 heads).
-__global__ void __launch_bounds__(256, KEEP ? 5 : 8) bwd_prepare_kernel(const __grid_constant__ PrepArgs a) {
+// 32 registers, so that eight blocks share an SM: the rare zeroing of uncovered rows had taken 48 (20.2 -> 24.6 us at 16 384
+// rows, 16 heads).
+template <bool BF16>
+__global__ void __launch_bounds__(256, 8) bwd_prepare_kernel(const __grid_constant__ PrepArgs a) {
   griddep_wait();
   // grid = (B*H, blocks of 32 rows); 8 threads per row, 8 elements each.
   // The head index comes from the grid, so no thread divides 64-bit indices.
@@ -156,12 +153,12 @@ __global__ void __launch_bounds__(256, KEEP ? 5 : 8) bwd_prepare_kernel(const __
   // packed batch: row r of sequence b is row cu[b] + r of the tensors, and exists for r < cu[b+1] - cu[b]
   int64_t row_o = static_cast<int64_t>(b) * a.o_sb + static_cast<int64_t>(r) * a.o_ss;
   int64_t row_do = static_cast<int64_t>(b) * a.do_sb + static_cast<int64_t>(r) * a.do_ss;
-  int q_limit = m.S_q, k_limit = m.S_k;
+  int q_limit = m.S_q;
   if (m.mask_kind == FMHA_MASK_CU_SEQLENS) {
     const int* cu = static_cast<const int*>(m.mask);
     const int base = cu[b];
     const int len = cu[b + 1] - base;
-    q_limit = k_limit = min(len, m.S_q);   // rows past the stated maximum length take no part
+    q_limit = min(len, m.S_q);   // rows past the stated maximum length take no part
     if (m.zero.grad[0].ptr != nullptr && (r0 + 32 > q_limit || len > q_limit)) {
       for (int t = 0; t < 3; ++t)
         zero_uncovered_rows(m.zero.grad[t].ptr, m.zero.grad[t].stride_s, m.zero.grad[t].stride_h, h, b, m.B, cu, m.S_q, m.total_rows, D,
@@ -170,9 +167,6 @@ __global__ void __launch_bounds__(256, KEEP ? 5 : 8) bwd_prepare_kernel(const __
     if (r0 >= q_limit) return;   // nothing of the accumulator there is added to or read
     row_o = static_cast<int64_t>(base + r) * a.o_ss;
     row_do = static_cast<int64_t>(base + r) * a.do_ss;
-  } else if (m.mask_kind == FMHA_MASK_SEQLEN) {
-    const int len = static_cast<const int*>(m.mask)[b];
-    if (len > 0 && len < m.S_k) k_limit = len;
   }
   uint4 wo = make_uint4(0u, 0u, 0u, 0u), wd = wo;
   if (r < q_limit) {
@@ -182,15 +176,6 @@ __global__ void __launch_bounds__(256, KEEP ? 5 : 8) bwd_prepare_kernel(const __
   float4* acc = reinterpret_cast<float4*>(m.dq_accum + (static_cast<int64_t>(bh) * m.S_q_pad + r) * D + part * per);
 #pragma unroll
   for (int i = 0; i < per / 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  if constexpr (KEEP) {   // while the loads are under way
-    const int lane = threadIdx.x & 31;
-    const uint32_t off = m.philox_offset + (m.philox_offset_dev != nullptr ? static_cast<uint32_t>(*m.philox_offset_dev) : 0u);
-    uint32_t* words = m.keep.words + (static_cast<int64_t>(bh) * (m.S_q_pad / 32) + blockIdx.y) * m.keep.k_stride;
-    if (r0 < q_limit)
-      for (int k0 = (threadIdx.x >> 5) * 32; k0 < k_limit; k0 += 256)
-        words[k0 + lane] = keep_word_32x32(m.philox_keys, off, static_cast<uint32_t>(m.philox_bh_offset + bh), static_cast<uint32_t>(r0),
-                                           static_cast<uint32_t>(k0 / 16), m.philox_thr, lane);
-  }
   const uint32_t xo[4] = {wo.x, wo.y, wo.z, wo.w};
   const uint32_t xd[4] = {wd.x, wd.y, wd.z, wd.w};
   float sum = 0.f;
@@ -302,8 +287,7 @@ struct BwdItem {
 };
 
 // PACKED: FMHA_MASK_CU_SEQLENS; a template parameter so that the padded kernels carry none of its bookkeeping.
-// BITS: the keep decisions come from the words the pass before wrote (KeepBits), else they are drawn here.
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool BITS = false>
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
   griddep_wait();
   using L = BwdSmem<D>;
@@ -831,17 +815,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         if (c < a.S_k) key_add = reinterpret_cast<const float*>(a.mask)[static_cast<size_t>(cur.b) * a.S_k + c] * kLog2eB;
       }
 
-      [[maybe_unused]] uint32_t keep_at = 0u, keep_next = 0u;   // at most 2^28 words
-      if constexpr (DROP && BITS) {
-        keep_at = static_cast<uint32_t>((bh * n_q_all * 4 + cq) * a.keep.k_stride + cur.k0 + row);
-        keep_next = a.keep.words[keep_at];
-      }
       for (int i = 0; i < n_q; ++i, ++t) {
-        [[maybe_unused]] uint32_t keep = 0u;   // keep decisions of this thread's key and 32 query columns
-        if constexpr (DROP && BITS) {
-          keep = keep_next;
-          if (i + 1 < n_q) keep_next = a.keep.words[keep_at += 4 * a.keep.k_stride];   // a tile ahead
-        } else if constexpr (DROP) {
+        // Keep decisions of this thread's key and 32 query columns, drawn before S is needed.  (Measured and not better: after P
+        // or dS has been handed on, a tile ahead; among the exponentials; half of the warps ahead of the others; one bit per score
+        // from the pass before, whose draws cost there what they save here - B=16 H=16 S=1024 320 us for the backward against 319 -
+        // and take memory.)
+        [[maybe_unused]] uint32_t keep = 0u;
+        if constexpr (DROP) {
           keep = keep_word_32x32(a.philox_keys, *philox_off, gbh, static_cast<uint32_t>(i * kTileM + cq * 32),
                                  static_cast<uint32_t>((cur.k0 + quad * 32) / 16), a.philox_thr, lane);
         }
@@ -972,13 +952,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool BITS = false>
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
 static int launch_bwd_impl(const BwdArgs& a, cudaStream_t stream) {
   using L = BwdSmem<D>;
-  if constexpr (D == 64 && DROP && !BITS) {
-    if (a.keep.words != nullptr) return launch_bwd_impl<D, BF16, KEYADD, DROP, PACKED, true>(a, stream);
-  }
-  auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED, BITS>;
+  auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED>;
   static std::atomic<bool> configured[64] = {};   // per device; set after the attribute call succeeded
   static std::atomic<int> sm_count[64] = {};
   int dev = 0;
@@ -1049,9 +1026,7 @@ int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const Bw
   p.do_sb = dot.stride_b; p.do_sh = dot.stride_h; p.do_ss = dot.stride_s;
   p.m = m;
   const dim3 grid(static_cast<unsigned>(m.B) * m.H, static_cast<unsigned>(m.S_q_pad / 32));
-  const bool bf = dtype == FMHA_DTYPE_BF16, keep = m.keep.words != nullptr;
-  auto kfn = keep ? (bf ? bwd_prepare_kernel<true, true> : bwd_prepare_kernel<false, true>)
-                  : (bf ? bwd_prepare_kernel<true, false> : bwd_prepare_kernel<false, false>);
+  auto kfn = dtype == FMHA_DTYPE_BF16 ? bwd_prepare_kernel<true> : bwd_prepare_kernel<false>;
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(256), 0, stream, p);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

@@ -316,16 +316,7 @@ static size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255);
 // fp32 dQ accumulator: at head dimension 128 dQ is finished inside one kernel and needs none.
 static size_t bwd_accum_bytes(size_t bh, size_t s_q_pad, int D) { return D == 64 ? bh * s_q_pad * D * sizeof(float) : 0; }
 
-// Keep bits of the dropout at head dimension 64 (KeepBits).  Above 1 GiB they are not worth their memory: the main kernel
-// draws for itself then, and also where a caller's workspace (or the static one) has no room for them.
-static size_t bwd_keep_bytes(const fmha_bwd_params* p) {
-  if (p->D != 64 || p->dropout_kind != FMHA_DROPOUT_PHILOX || dropout_threshold(p->p_drop) == 0) return 0;
-  const size_t words = static_cast<size_t>(p->B) * p->H * ((p->S_q + kTileM - 1) / kTileM * (kTileM / 32)) *
-                       ((p->S_k + kTileN - 1) / kTileN * kTileN);
-  return words * 4 <= (size_t(1) << 30) ? words * 4 : 0;
-}
-// What the backward pass cannot do without.
-static int bwd_least_workspace(const fmha_bwd_params* p, size_t* bytes) {
+int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes) {
   if (p == nullptr || bytes == nullptr) return FMHA_ERR_BAD_ARG;
   int rc = validate_common(p->struct_bytes, sizeof(fmha_bwd_params), p->dtype, p->B, p->H, p->S_q, p->S_k, p->D, p->scale);
   if (rc != FMHA_OK) return rc;
@@ -334,12 +325,6 @@ static int bwd_least_workspace(const fmha_bwd_params* p, size_t* bytes) {
   // fp32 dQ accumulator, delta, and the work-item counter of the persistent main kernel
   *bytes = align256(bwd_accum_bytes(bh, s_q_pad, p->D)) + align256(bh * p->S_q * sizeof(float)) + 256;
   return FMHA_OK;
-}
-
-int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes) {
-  const int rc = bwd_least_workspace(p, bytes);
-  if (rc == FMHA_OK) *bytes += bwd_keep_bytes(p);
-  return rc;
 }
 
 int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
@@ -366,7 +351,7 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
       p->lse == nullptr)
     return FMHA_ERR_BAD_ARG;
   size_t need = 0;
-  rc = bwd_least_workspace(p, &need);
+  rc = fmha_sm100_bwd_workspace_bytes(p, &need);
   if (rc != FMHA_OK) return rc;
   if (p->workspace == nullptr || p->workspace_bytes < need || (reinterpret_cast<uintptr_t>(p->workspace) & 255))
     return FMHA_ERR_BAD_ARG;
@@ -382,11 +367,6 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
 
   BwdArgs a;
   std::memset(&a, 0, sizeof(a));
-  const size_t keep_bytes = bwd_keep_bytes(p);
-  if (keep_bytes > 0 && p->workspace_bytes >= need + keep_bytes) {
-    a.keep.words = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(work_counter) + 256);
-    a.keep.k_stride = (p->S_k + kTileN - 1) / kTileN * kTileN;
-  }
   // tensor-map extents: [B, H, S, D], or one "batch" of total_rows rows for a packed batch
   const int mB = packed ? 1 : p->B, mSq = packed ? p->total_rows : p->S_q, mSk = packed ? p->total_rows : p->S_k;
   const fmha_tensor4 tq = sanitized(p->q, mB, p->H, mSq, p->D), tk = sanitized(p->k, mB, p->H, mSk, p->D),
@@ -600,7 +580,7 @@ static int static_scratch_address(void** out) {
 extern "C" int fmha_sm100_bwd_static_scratch(const fmha_bwd_params* p, void* stream) {
   if (p == nullptr) return FMHA_ERR_BAD_ARG;
   size_t need = 0;
-  int rc = bwd_least_workspace(p, &need);  // also validates struct size, dtype, D, sizes
+  int rc = fmha_sm100_bwd_workspace_bytes(p, &need);  // also validates struct size, dtype, D, sizes
   if (rc != FMHA_OK) return rc;
   if (need > FMHA_STATIC_SCRATCH_BYTES) return FMHA_ERR_TOO_LARGE;
   rc = check_device();

@@ -66,13 +66,6 @@ struct FwdArgs {
   int* status;
 };
 
-// Head dimension 64 with dropout: the keep decisions as one bit per score, written by the pass before the main kernel.
-// Word ((bh * S_q_pad/32) + q/32) * k_stride + key holds 32 query rows of a key, in the order keep_word_32x32 makes them.
-struct KeepBits {
-  uint32_t* words;   // null: the main kernel draws for itself
-  int k_stride;      // keys rounded up to whole tiles
-};
-
 // FMHA_FLAG_ZERO_UNCOVERED: the kernels zero the rows sequences are cut by, and those outside all sequences unless
 // zero_outside_rows_kernel has (there are more of them than rows of padding, see zero_uncovered_rows).
 enum UncoveredMode { kUncoveredAll = 1, kUncoveredCut = 2 };
@@ -123,7 +116,6 @@ struct BwdArgs {
   uint32_t philox_offset;
   const long long* philox_offset_dev;   // optional device value added to philox_offset
   int philox_bh_offset;
-  KeepBits keep;
   int* status;
 };
 

@@ -268,10 +268,9 @@ def test_backward_accepts_a_broadcast_gradient(cuda_device):
 
 @pytest.mark.parametrize("S_q,S_k", [(128, 128), (1, 33), (129, 127), (300, 513), (512, 64)])
 @pytest.mark.parametrize("mask", ["none", "seqlen", "key"])
-def test_keep_bits_and_draws_in_the_kernel_give_the_same_gradients(cuda_device, S_q, S_k, mask):
-    """Head dimension 64 with dropout: the keep decisions come from words an earlier pass wrote, or, where the workspace has
-    no room for them, from draws in the main kernel.  dK and dV have a fixed summation order: the same bits; dQ is summed
-    by atomics."""
+def test_workspace_of_the_stated_size_whatever_it_holds(cuda_device, S_q, S_k, mask):
+    """Head dimension 64 with dropout: accumulator, delta and counter are all the scratch there is, and nothing that lies in it
+    is taken over.  dK and dV have a fixed summation order: the same bits; dQ is summed by atomics."""
     B, H, p = 2, 3, 0.2
     q, k, v, d_o, lens = helpers.randn_like_config(B, H, S_q, S_k, 64, torch.float16, seed=S_q + S_k, device=cuda_device)
     kw = dict(mask_kind=capi.MASK_NONE, mask=None)
