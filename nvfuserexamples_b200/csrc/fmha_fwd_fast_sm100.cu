@@ -701,21 +701,25 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   }
 }
 
-// Over how many CTAs of a cluster the keys of a query tile are split: the candidate (1, 2, 4, 8) of least modelled time,
-// in units of one key step of a CTA that has its SM to itself (1.1 us at D = 64, 1.9 us at D = 128, measured: there a
-// step is a chain of latencies, as long for one query row as for 128).  A step slows down in proportion to the CTAs per
-// SM once they compete for the special-function unit (`load`; a tile of at most 32 rows keeps one warp of four busy),
-// and a split adds the cluster launch, its barriers and the combination (`overhead`: measured 1.1 us for one query row,
-// 4 us for 128).  More than two CTAs per SM never paid.  Measured: B=2 H=16 S_q=1 S_k=4096 D=128 60.6 -> 17.3 us (8
-// shares), D=64 71.7 -> 15.6 us; B=8 H=8 S_q=20 S_k=1000 D=64 20.1 -> 10.9 us (4); B=1 H=12 S=1024 D=64 20.4 -> 17.9 us (2).
-static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, int sms) {
+// Over how many CTAs of a cluster the keys of a query tile are split: the candidate (1, 2, 4, 8) of least modelled time, in units
+// of one key step of a CTA that has its SM to itself (0.97 us at D = 64, 1.7 us at D = 128, measured: there a step is a chain of
+// latencies, as long for one query row as for 128; 1.2 units with an additive mask or dropout).  A split adds the cluster
+// launch, its barriers and the combination (`overhead`, from the times of 4 to 96 tiles over 128 to 2048 keys).  With more CTAs
+// than SMs a step takes 1.2 times as long and the start of a cluster longer, the more the larger it is; more than two CTAs per
+// SM never paid.  Measured, one share / the split chosen: 24 tiles of 20 rows, 1024 keys D=64 18.6 / 9.6 us (4), D=128 17.2 / 10.0
+// (4); 12 tiles of 128 rows 18.6 / 10.1 (8) and 17.6 / 13.2 (4); 48 tiles, 1024 keys 19.0 / 14.0 (4) and 17.6 / 15.8 (2), 512 keys
+// 11.2 / 11.0 (2) and 10.9 (1; 15.4 as 4 shares); 32 tiles, 384 keys D=64 9.1 (1; 14.6 as 8 shares).
+static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, bool long_step, int sms) {
+  static constexpr float kOverhead[2][2][3] = {{{1.9f, 2.4f, 3.2f}, {3.7f, 4.0f, 4.8f}},     // D = 64: up to 32 rows, more
+                                               {{1.05f, 1.5f, 2.2f}, {2.75f, 3.4f, 4.7f}}};  // D = 128
   const bool few_rows = S_q <= 32;
-  const float overhead = D == 64 ? (few_rows ? 1.5f : 4.0f) : (few_rows ? 1.0f : 2.2f);
-  const float load = few_rows ? 0.5f : D == 64 ? 0.95f : 1.3f;
+  const float step = long_step ? 1.2f : 1.0f;
   int best = 1;
-  float best_cost = static_cast<float>(steps) * std::max(1.0f, load * ctas / sms);
-  for (int s = 2; s <= kMaxKeySplit && ctas * s <= 2 * static_cast<int64_t>(sms) && s < 2 * steps; s *= 2) {
-    const float cost = static_cast<float>((steps + s - 1) / s) * std::max(1.0f, load * ctas * s / sms) + overhead;
+  float best_cost = static_cast<float>(steps) * step;
+  for (int s = 2, i = 0; s <= kMaxKeySplit && ctas * s <= 2 * static_cast<int64_t>(sms) && s < 2 * steps; s *= 2, ++i) {
+    const bool crowded = ctas * s > sms;
+    const float cost = static_cast<float>((steps + s - 1) / s) * step * (crowded ? 1.2f : 1.0f) + kOverhead[D == 64 ? 0 : 1][few_rows ? 0 : 1][i] +
+                       (crowded ? (few_rows ? 0.1f : 0.6f) * s : 0.f);
     if (cost < best_cost) {
       best = s;
       best_cost = cost;
@@ -746,7 +750,7 @@ static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream, int n_split =
   using L = FastSmem<D>;
   if constexpr (!PACKED && !SPLIT) {
     const int s = fwd_key_split(static_cast<int64_t>((a.S_q + kTileM - 1) / kTileM) * a.H * a.B, (a.S_k + L::TN - 1) / L::TN, a.S_q, D,
-                                sm_count());
+                                KEYADD || DROP, sm_count());
     if (s > 1) return launch_fast_impl<D, BF16, KEYADD, DROP, false, true>(a, stream, s);
   }
   auto kfn = fmha_fwd_fast_kernel<D, BF16, KEYADD, DROP, PACKED, SPLIT>;

@@ -191,10 +191,10 @@ def test_bounded_wait_reports_instead_of_hanging(cuda_device):
 
 
 @pytest.mark.parametrize("B,H,S_q,S_k,D,dtype", [
-    (1, 1, 1, 1024, 64, torch.float16),     # one query row, 8 shares of two 64-key steps
+    (1, 1, 17, 1024, 64, torch.float16),    # 8 shares of two 64-key steps
     (1, 2, 31, 1000, 64, torch.bfloat16),   # one warp of rows, a ragged last step
     (2, 2, 33, 900, 128, torch.bfloat16),   # the second warp has a single row
-    (1, 1, 1, 300, 128, torch.float16),     # more shares than key steps: one of them is empty
+    (1, 1, 17, 300, 128, torch.float16),    # more shares than key steps: one of them is empty
     (1, 2, 130, 1536, 128, torch.float16),  # two query tiles, the second with two rows
     (1, 3, 128, 2048, 64, torch.float16),   # a full tile
 ])
