@@ -237,7 +237,8 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream) {
   // tensor-map extents: [B, H, S, D], or one "batch" of total_rows rows for a packed batch
   const int mB = packed ? 1 : p->B, mSq = packed ? p->total_rows : p->S_q, mSk = packed ? p->total_rows : p->S_k;
   if ((rc = make_tmap(&a.tm_q, sanitized(p->q, mB, p->H, mSq, p->D), p->dtype, mB, p->H, mSq, p->D, kTileM))) return rc;
-  const bool rows = !legacy && !packed && fwd_rows_applies(p->S_q);
+  const bool rows = !legacy && !packed && fwd_rows_applies(p->S_q, p->S_k, p->D, static_cast<int64_t>(p->B) * p->H,
+                                                             p->dropout_kind == FMHA_DROPOUT_PHILOX);
   const int kv_rows = rows ? kRowsKeyStep : fwd_key_tile(p->D, legacy);
   if ((rc = make_tmap(&a.tm_k, sanitized(p->k, mB, p->H, mSk, p->D), p->dtype, mB, p->H, mSk, p->D, kv_rows))) return rc;
   if ((rc = make_tmap(&a.tm_v, sanitized(p->v, mB, p->H, mSk, p->D), p->dtype, mB, p->H, mSk, p->D, kv_rows))) return rc;

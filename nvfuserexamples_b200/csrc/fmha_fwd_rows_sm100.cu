@@ -342,7 +342,18 @@ __global__ void __launch_bounds__(kRwThreads, 2) fmha_fwd_rows_kernel(const __gr
   }
 }
 
-bool fwd_rows_applies(int S_q) { return S_q <= kRwRows; }
+// Up to 16 rows, but not where so many heads have so few keys that a CTA here is mostly start and end: at D = 64 four CTAs of the
+// tile kernel share an SM, two of this one.  The lines lie where the two cross (this kernel / the tile kernel, us): 16 rows, 64
+// keys 1024 heads 10.8 / 9.9, 2048 18.8 / 16.3, 8192 76.8 / 57.3; 128 keys 2048 heads 21.9 / 21.8, 4096 47.2 / 41.6; 256 keys 4096
+// heads 61.2 / 62.2; 8 rows, 64 keys 2048 heads 16.8 / 16.2; 4 rows 15.8 / 16.2, 8192 heads (more than the L2 cache) 68.1 / 57.8.
+// With dropout the tile kernel draws for 128 rows: 8 rows, 64 keys, 4096 heads 0.97 times its time, 16 rows 1.11 times.
+bool fwd_rows_applies(int S_q, int S_k, int D, int64_t heads, bool dropout) {
+  if (S_q > kRwRows) return false;
+  const int steps = (S_k + kRowsKeyStep - 1) / kRowsKeyStep;
+  const int64_t per_sm = heads / std::max(sm_count(), 1);
+  if (D != 64 || steps > (dropout ? 1 : 3)) return true;
+  return S_q <= (dropout ? 8 : 4) ? S_k <= 32 || per_sm < 32 || steps > 1 : per_sm < 8 * steps;
+}
 
 template <int D, bool BF16, bool KEYADD, bool DROP>
 static int launch_rows_impl(const FwdArgs& a, cudaStream_t stream) {

@@ -123,7 +123,7 @@ struct BwdArgs {
 int launch_fwd(const FwdArgs& a, int D, int dtype, bool legacy, bool p_via_smem, cudaStream_t stream);
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
 // the kernel for a handful of query rows per head (fmha_fwd_rows_sm100.cu): compact masks, not packed
-bool fwd_rows_applies(int S_q);
+bool fwd_rows_applies(int S_q, int S_k, int D, int64_t heads, bool dropout);
 int launch_fwd_rows(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
 // the persistent kernel of the dense-mask operators at head dimension 64 (fmha_fwd_dense_sm100.cu)
 bool fwd_dense_applies(const FwdArgs& a, int D);

@@ -226,6 +226,7 @@ def test_keys_split_over_a_cluster(cuda_device, B, H, S_q, S_k, D, dtype, mask, 
     (2, 1, 9, 2049, 128, torch.float16),     # second half of the tile has one row; the last step has one key
     (1, 1, 15, 130, 64, torch.bfloat16),     # too few steps for shares
     (160, 1, 3, 200, 64, torch.float16),     # more heads than multiprocessors: no cluster
+    (75, 16, 16, 60, 64, torch.float16),     # so many heads of so few keys that the tile kernel takes them
 ])
 @pytest.mark.parametrize("mask,p_drop", [("none", 0.0), ("seqlen", 0.1), ("key", 0.0), ("key", 0.3)])
 def test_a_handful_of_query_rows(cuda_device, B, H, S_q, S_k, D, dtype, mask, p_drop):
