@@ -65,6 +65,21 @@ struct DqSmem {
   static_assert(kDynBytes <= 232448, "shared memory budget of one CTA exceeded");
 };
 
+// The product of two rows of 128 values that 16 lanes hold, 16 bytes each; in every one of the lanes.
+template <bool BF16>
+__device__ __forceinline__ float row_dot16(const uint4& o, const uint4& d) {
+  const uint32_t xo[4] = {o.x, o.y, o.z, o.w}, xd[4] = {d.x, d.y, d.z, d.w};
+  float sum = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    sum = fmaf(unpack_lo<BF16>(xo[e]), unpack_lo<BF16>(xd[e]), sum);
+    sum = fmaf(unpack_hi<BF16>(xo[e]), unpack_hi<BF16>(xd[e]), sum);
+  }
+#pragma unroll
+  for (int m = 1; m < 16; m *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+  return sum;
+}
+
 enum DqItemState { kDqEnd, kDqEmpty, kDqWork };
 struct DqItem {
   int state;
@@ -395,7 +410,9 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
           const int r = half * 64 + k * 32 + lane, q = it.q0 + r;
           st[r] = q < it.q_limit ? -lse[q] * kDqLog2e : -INFINITY;   // rows past the end: their probabilities are zero
         }
-        if (a.o_ptr == nullptr) {   // delta is there already (bwd_delta_kernel)
+        if (!persist) {
+          // the compute warps form delta
+        } else if (a.o_ptr == nullptr) {   // delta is there already (bwd_delta_kernel)
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             const int r = half * 64 + k * 32 + lane, q = it.q0 + r;
@@ -506,6 +523,35 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
     DqItem prev;
     prev.state = kDqEnd;
     DqItem it = first_work(n, false);
+    if (!persist && it.state == kDqWork) {
+      // The CTA's only item: its delta while Q, K, dO and V are on their way, eight rows per warp, 16 lanes per row.  A pass of its
+      // own is on the critical path of so small a grid, and so are the two statistics warps (B=1 H=12 S=128, forward and backward,
+      // 22.0 -> 20.7 us; B=1 H=8 S=2048 95.7 -> 87.5).
+      const int64_t b_o = packed ? static_cast<int64_t>(it.row_base) * a.o_ss : static_cast<int64_t>(it.b) * a.o_sb;
+      const int64_t b_do = packed ? static_cast<int64_t>(it.row_base) * a.do_ss : static_cast<int64_t>(it.b) * a.do_sb;
+      const unsigned short* po = static_cast<const unsigned short*>(a.o_ptr) + b_o + it.h * a.o_sh + (lane & 15) * 8;
+      const unsigned short* pd = static_cast<const unsigned short*>(a.do_ptr) + b_do + it.h * a.do_sh + (lane & 15) * 8;
+      uint4 wo[4], wd[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int64_t q = it.q0 + cw * 8 + 2 * k + (lane >> 4);
+        wo[k] = wd[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (q < it.q_limit) {
+          wo[k] = __ldg(reinterpret_cast<const uint4*>(po + q * a.o_ss));
+          wd[k] = __ldg(reinterpret_cast<const uint4*>(pd + q * a.do_ss));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float sum = row_dot16<BF16>(wo[k], wd[k]);
+        const int r = cw * 8 + 2 * k + (lane >> 4);
+        if ((lane & 15) == 0) {
+          sStats[kTileM + r] = sum * (DROP ? 1.0f / a.dropout_scale : 1.0f);
+          if (it.q0 + r < it.q_limit) a.delta[static_cast<int64_t>(it.bh) * a.S_q + it.q0 + r] = sum;
+        }
+      }
+      named_bar_sync(1, kDqCompute);
+    }
     while (it.state == kDqWork) {
       const uint32_t gbh = static_cast<uint32_t>(a.philox_bh_offset + it.bh);
       mbar_wait(stat_full + (w & 1), (w >> 1) & 1, wctx, kDqsStat, kDqSleepNs);
@@ -626,15 +672,7 @@ __global__ void __launch_bounds__(256) bwd_delta_kernel(const __grid_constant__ 
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const uint32_t xo[4] = {wo[k].x, wo[k].y, wo[k].z, wo[k].w}, xd[4] = {wd[k].x, wd[k].y, wd[k].z, wd[k].w};
-    float sum = 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      sum = fmaf(unpack_lo<BF16>(xo[e]), unpack_lo<BF16>(xd[e]), sum);
-      sum = fmaf(unpack_hi<BF16>(xo[e]), unpack_hi<BF16>(xd[e]), sum);
-    }
-#pragma unroll
-    for (int m = 1; m < 16; m *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    const float sum = row_dot16<BF16>(wo[k], wd[k]);
     const int q = blockIdx.y * 64 + k * 16 + (threadIdx.x >> 4);
     if (part == 0 && q < q_limit) a.delta[static_cast<int64_t>(bh) * a.S_q + q] = sum;
   }
@@ -656,13 +694,13 @@ static int launch_dq_impl(const BwdArgs& a, cudaStream_t stream) {
   // The two statistics warps need 12 000 cycles for an item's delta, five key tiles' worth: with fewer tiles the compute
   // warps wait (9 600 cycles per item at four), and a separate pass over O and dO is the cheaper way (B=16 H=16 S=512 with
   // dropout: 162 us for the whole backward fused, 158 separate; from S_k = 2048 on it is hidden).
-  if (a.S_k <= kDeltaPassKeys) {
+  args.persist = static_cast<int64_t>(grid.x) * grid.y * grid.z > sm_count();
+  if (args.persist && a.S_k <= kDeltaPassKeys) {
     const cudaError_t e = launch_overlapped(bwd_delta_kernel<BF16>, dim3(static_cast<unsigned>(a.B) * a.H, (a.S_q + 63) / 64), dim3(256), 0,
                                             stream, a);
     if (e != cudaSuccess) return static_cast<int>(e);
     args.o_ptr = nullptr;
   }
-  args.persist = static_cast<int64_t>(grid.x) * grid.y * grid.z > sm_count();
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(kDqThreads), DqSmem::kDynBytes, stream, args);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

@@ -289,11 +289,12 @@ def test_workspace_of_the_stated_size_whatever_it_holds(cuda_device, S_q, S_k, m
 
 
 @pytest.mark.parametrize("B,H,S_q,S_k,mask,p", [(3, 2, 129, 1025, "key", 0.2), (1, 2, 1, 1100, "seqlen", 0.0), (2, 1, 260, 1024, "key", 0.1),
-                                                (5, 16, 300, 1030, "seqlen", 0.1), (2, 2, 640, 1281, "none", 0.3)])
+                                                (5, 16, 300, 1030, "seqlen", 0.1), (2, 2, 640, 1281, "none", 0.3),
+                                                (19, 4, 129, 1025, "key", 0.2), (19, 4, 129, 1024, "seqlen", 0.0), (160, 1, 77, 1000, "none", 0.1)])
 def test_head_dim_128_on_both_sides_of_the_delta_pass(cuda_device, B, H, S_q, S_k, mask, p):
-    """Head dimension 128: delta has a pass of its own up to 1024 keys and is formed by two warps of the dQ kernel beyond;
-    both sides of the limit, ragged rows and keys, each mask, and more work items than SMs (5 * 16 * 3 query tiles).  The
-    first and the last head against the oracle."""
+    """Head dimension 128: with no more query tiles than SMs the dQ kernel's compute warps form delta (the small sizes here);
+    with more (240, 152 and 160 tiles) it has a pass of its own up to 1024 keys and is formed by two warps of the dQ kernel
+    beyond.  Both sides of the limit, ragged rows and keys, each mask.  The first and the last head against the oracle."""
     dtype = torch.float16
     q, k, v, d_o, lens = helpers.randn_like_config(B, H, S_q, S_k, 128, dtype, seed=S_q + S_k, device=cuda_device)
     lens[0] = min(S_k, 150)   # whole key tiles without a valid key
