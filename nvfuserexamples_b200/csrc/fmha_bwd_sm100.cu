@@ -13,8 +13,8 @@
 //                      P  = exp2(S*scale*log2e + mask - lse*log2e)   (16 warps, thread = key, a quarter of the queries)
 //                      dS = P * (keep*dP - delta/c)                   c = 1/(1-p_drop)
 //                      dV += (keep*P)^T dO     dK += dS^T Q     dQ_tile = dS K
-//                    P^T goes to tensor memory as the A operand of dV, dS^T to shared memory (16-bit, 128-byte swizzle),
-//                    where the tensor core reads it as K-major (dK) and as MN-major (dQ) operand; dQ tiles are added to
+//                    P^T goes to tensor memory as the A operand of dV, dS^T there as that of dK and to shared memory (16-bit,
+//                    128-byte swizzle) as the MN-major operand of dQ; dQ tiles are added to
 //                    the fp32 accumulator from registers; dK and dV leave through per-warp staging tiles and TMA stores
 //                    when the next item is already under way.
 //   3. bwd_finish  : dQ = (scale * accumulator) rounded to the 16-bit dtype
@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include <cstring>
@@ -957,24 +958,15 @@ static int launch_bwd_impl(const BwdArgs& a, cudaStream_t stream) {
   using L = BwdSmem<D>;
   auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED>;
   static std::atomic<bool> configured[64] = {};   // per device; set after the attribute call succeeded
-  static std::atomic<int> sm_count[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  int sms = 0;
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynBytes);
     if (e != cudaSuccess) return static_cast<int>(e);
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    if (dev >= 0 && dev < 64) {
-      sm_count[dev] = sms;
-      configured[dev] = true;
-    }
-  } else {
-    sms = sm_count[dev];
+    if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   const int64_t items = static_cast<int64_t>((a.S_k + kTileN - 1) / kTileN) * a.H * a.B;
-  const int grid = static_cast<int>(items < sms ? items : sms);   // one persistent CTA per SM
+  const int grid = static_cast<int>(std::min<int64_t>(items, sm_count()));   // one persistent CTA per SM
   const cudaError_t e = launch_overlapped(kfn, dim3(grid), dim3(kBwdThreads), L::kDynBytes, stream, a);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

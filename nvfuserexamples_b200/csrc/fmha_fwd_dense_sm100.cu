@@ -22,6 +22,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "../../include/fmha_sm100.h"
@@ -601,23 +602,15 @@ template <bool BF16, bool KEEP, bool DROPMASK, bool SAVE>
 static int launch_dense_impl(const FwdArgs& a, cudaStream_t stream) {
   auto kfn = fmha_fwd_dense_kernel<BF16, KEEP, DROPMASK, SAVE>;
   static std::atomic<bool> configured[64] = {};   // per device; set after the attribute call succeeded
-  static std::atomic<int> sm_count[64] = {};
-  int dev = 0, sms = 0;
+  int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, DnSmem<DROPMASK>::kDynBytes);
     if (e != cudaSuccess) return static_cast<int>(e);
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    if (dev >= 0 && dev < 64) {
-      sm_count[dev] = sms;
-      configured[dev] = true;
-    }
-  } else {
-    sms = sm_count[dev];
+    if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   const int64_t items = static_cast<int64_t>((a.S_q + kTileM - 1) / kTileM) * a.H * a.B;
-  const int grid = static_cast<int>(items < sms ? items : sms);   // one persistent CTA per SM
+  const int grid = static_cast<int>(std::min<int64_t>(items, sm_count()));   // one persistent CTA per SM
   const cudaError_t e = launch_overlapped(kfn, dim3(grid), dim3(kDnThreads), DnSmem<DROPMASK>::kDynBytes, stream, a);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

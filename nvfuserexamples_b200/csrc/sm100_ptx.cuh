@@ -264,8 +264,6 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_
       ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-// Brings the 128-byte line of a global address to the L2.
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Adds four consecutive floats to global memory (no result), 16-byte aligned.
 __device__ __forceinline__ void red_add_v4(float* p, float x, float y, float z, float w) {
   asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
@@ -328,71 +326,6 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n, int fmt, boo
          (static_cast<uint32_t>(m >> 4) << 24);       // M / 16
 }
 
-// D[tmem] (+)= A[smem] * B[smem].  One thread issues.
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem].
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The issuing thread is a single lane, so every instruction between two tcgen05.mma counts
-// (a 128x64x16 MMA occupies the tensor core for only ~48 cycles).  These variants take the
-// descriptor as (low word, high word): the caller builds the descriptor of a tile once and per
-// k-step only adds a constant to the low word (the 16-byte-unit start address lives in its low
-// 14 bits and a tile never crosses the 256 KB field).
-struct DescWords {
-  uint32_t lo, hi;
-};
-__device__ __forceinline__ DescWords desc_words(uint64_t d) {
-  DescWords w;
-  w.lo = static_cast<uint32_t>(d);
-  w.hi = static_cast<uint32_t>(d >> 32);
-  return w;
-}
-__device__ __forceinline__ void umma_ss_w(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      ".reg .b64 da, db;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "mov.b64 da, {%1, %2};\n\t"
-      "mov.b64 db, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_ts_w(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      ".reg .b64 db;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
-      "}\n"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // ---- burst issue from a converged warp ---------------------------------------------------
 // The warp scheduler gives a warp whose next instruction is not ready no slot, and a warp that
 // competes with arithmetic-heavy warps waits tens of cycles for each slot it asks for.  An MMA loop
@@ -538,12 +471,6 @@ __device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
 __host__ __device__ constexpr uint32_t kmajor_step(int kk, int sub) { return static_cast<uint32_t>(((kk / 4) * sub + (kk % 4) * 32) >> 4); }
 __host__ __device__ constexpr uint32_t mnmajor_step(int kk) { return static_cast<uint32_t>((kk * 2048) >> 4); }
 
-// Arrive on `bar` when every tcgen05.mma issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
 // ------------------------------------------------------------------------------------
 // tensor memory loads / stores, shape 32x32b: thread i of the warp owns lane
 // (lane_base + i); register k holds column (col + k).
@@ -621,17 +548,6 @@ __device__ __forceinline__ void tmem_wait_ld_dep(uint32_t (&r)[32]) {
                  "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
                  "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
                  "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
-               :
-               : "memory");
-}
-
-// The wait for two 16-register loads at once.
-__device__ __forceinline__ void tmem_wait_ld_dep16(uint32_t (&r)[16], uint32_t (&q)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
-                 "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7]),
-                 "+r"(q[8]), "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15])
                :
                : "memory");
 }
