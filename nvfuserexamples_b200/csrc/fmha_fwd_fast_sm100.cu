@@ -480,14 +480,16 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           finish_scores(c, sv[c]);
         }
         auto v = [&](int k) { return __uint_as_float(sv[c][k]); };
-        float m0 = fmax3(v(0), v(1), v(2));
-        float m1 = fmax3(v(3), v(4), v(5));
+        // with an additive mask a NaN has to show in the maximum, or the shortcut below would step over it
+        auto max3 = [](float x, float y, float z) { return fmax3<KEYADD>(x, y, z); };
+        float m0 = max3(v(0), v(1), v(2));
+        float m1 = max3(v(3), v(4), v(5));
 #pragma unroll
         for (int k = 6; k + 3 < 32; k += 4) {
-          m0 = fmax3(m0, v(k), v(k + 1));
-          m1 = fmax3(m1, v(k + 2), v(k + 3));
+          m0 = max3(m0, v(k), v(k + 1));
+          m1 = max3(m1, v(k + 2), v(k + 3));
         }
-        tile_max = fmax3(tile_max, fmax3(m0, m1, v(30)), v(31));
+        tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
         if constexpr (AHEAD) {
           if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
         }

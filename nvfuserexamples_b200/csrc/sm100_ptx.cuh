@@ -555,10 +555,12 @@ __device__ __forceinline__ void tmem_wait_ld_dep(uint32_t (&r)[32]) {
 // ------------------------------------------------------------------------------------
 // math
 // ------------------------------------------------------------------------------------
-// Three-input maximum (one instruction on sm_100).
+// Three-input maximum (one instruction on sm_100).  NAN_WINS: a NaN among the operands is the result, else it is passed over.
+template <bool NAN_WINS = false>
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  if constexpr (NAN_WINS) asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  else asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
 __device__ __forceinline__ float fast_exp2(float x) {

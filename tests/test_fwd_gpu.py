@@ -250,3 +250,18 @@ def test_a_handful_of_query_rows(cuda_device, B, H, S_q, S_k, D, dtype, mask, p_
     ref, *_ = helpers.oracle_forward(q, k, v, p_drop=p_drop, seed=33, offset=6, bh_offset=5, **okw)
     helpers.assert_close(o, ref["o"], "o", dtype)
     helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("p_drop", [0.0, 0.1])
+def test_a_nan_among_masked_keys_is_not_stepped_over(cuda_device, D, p_drop):
+    """A key whose score is NaN makes its head's rows NaN, masked away or not: NaN + mask is NaN, as in the composite.  The
+    shortcut for steps whose keys are all masked away looks at the scores and must see it."""
+    B, H, S = 40, 8, 512   # one CTA per query tile
+    q, k, v, _, _ = helpers.randn_like_config(B, H, S, S, D, torch.float16, seed=5, device=cuda_device)
+    k[3, 2, 450] = float("nan")
+    mask = torch.where(torch.arange(S, device=cuda_device) < 150, 0.0, -1e4).repeat(B, 1)
+    o, lse = api.fmha_forward(q, k, v, mask=mask, p_drop=p_drop, seed=1)
+    assert torch.isnan(o[3, 2]).all() and torch.isnan(lse.view(B, H, S)[3, 2]).all()
+    o[3, 2] = 0
+    assert torch.isfinite(o).all()
