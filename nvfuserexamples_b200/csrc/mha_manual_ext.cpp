@@ -635,9 +635,10 @@ void check_status() {
 // autograd: fmha = fmha_fwd + fmha_bwd, and the same for the three other layouts.
 //
 // The backward functions are ordinary torch::autograd::Function ones, with the node type that goes with them (saved-tensor
-// hooks, compiled autograd and the errors for freed or modified tensors come with it).  Only the forward half of that template
-// is left out: at the sizes where the host sets the pace (a B=2, H=4, S=128 step takes 17 us of GPU time) its argument
-// vectors and output wrapping cost a good part of what the kernels take.
+// hooks, compiled autograd and the errors for freed or modified tensors come with it).  Only the parts of that template that cost a
+// good part of what the kernels take where the host sets the pace (a B=2, H=4, S=128 step takes 17 us of GPU time) are passed by:
+// the argument vectors and output wrapping of its forward half, and the dictionary of saved values, which compiled autograd alone
+// is given.
 // ---------------------------------------------------------------------------------------
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
@@ -651,13 +652,52 @@ c10::TypedOperatorHandle<Ret(Args...)> find_op(const char* name) {
   return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Ret(Args...)>();
 }
 
+// What a call hands to its backward pass beside tensors.
+struct Scalars {
+  int64_t max_seqlen = 0;
+  double p_drop = 0.0;
+  int64_t seed = 0, offset = 0;
+  c10::optional<double> scale;
+};
+
+// F's node.  F::gradients(saved tensors, scalars, gradient of o) does the work of F::backward.  (o: see Recorded.)
+template <typename F>
+struct OpNode final : public torch::autograd::CppNode<F> {
+  Scalars scalars;
+  variable_list apply(variable_list&& grads) override {
+    const std::lock_guard<std::mutex> lock(this->mutex_);
+    const variable_list saved = this->ctx_.get_saved_variables();
+    return F::gradients(saved, scalars, grads[0].defined() ? grads[0] : at::zeros_like(saved[saved.size() - 5]));
+  }
+  // Compiled autograd runs F::backward, which has only the context to go by.
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    auto& data = const_cast<OpNode*>(this)->ctx_.saved_data;
+    data["max_seqlen"] = scalars.max_seqlen;
+    data["p_drop"] = scalars.p_drop;
+    data["seed"] = scalars.seed;
+    data["offset"] = scalars.offset;
+    data["scale"] = scalars.scale;
+    torch::autograd::CppNode<F>::compiled_args(args);
+  }
+};
+template <typename F>
+struct OpFunction : public torch::autograd::Function<F> {
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto& data = ctx->saved_data;
+    return F::gradients(ctx->get_saved_variables(),
+                        {data.at("max_seqlen").toInt(), data.at("p_drop").toDouble(), data.at("seed").toInt(), data.at("offset").toInt(),
+                         data.at("scale").toOptional<double>()},
+                        grads[0]);
+  }
+};
+
 // Runs `forward` (which returns {o, lse}) below the autograd keys and, if a gradient will be wanted, records the node whose
 // backward function is F's.  `inputs`: the differentiable operands; lens: valid lengths or cu_seqlens; offset_tensor: the
 // backward pass must see the value the forward pass saw, even if the caller advances the tensor in between, so it gets a
 // private copy.
 template <typename F, size_t N, typename Forward>
 at::Tensor record(const std::array<TensorRef, N>& inputs, const OptTensor& mask, const OptTensor& lens, const OptTensor& offset_tensor,
-                  int64_t max_seqlen, double p_drop, int64_t seed, int64_t offset, c10::optional<double> scale, Forward forward) {
+                  const Scalars& scalars, Forward forward) {
   // torch.func.grad, vjp and jvp are refused, as by the template: the node knows nothing of their levels
   if (const auto& transforms = at::functorch::functorchTLSAccessor()) transforms->checkSupportsCppAutogradFunction();
   bool wanted = false;
@@ -673,9 +713,9 @@ at::Tensor record(const std::array<TensorRef, N>& inputs, const OptTensor& mask,
     ++n;
   });
   wanted = wanted && at::GradMode::is_enabled();
-  std::shared_ptr<torch::autograd::CppNode<F>> node;
+  std::shared_ptr<OpNode<F>> node;
   if (wanted) {
-    node = std::shared_ptr<torch::autograd::CppNode<F>>(new torch::autograd::CppNode<F>(), torch::autograd::deleteNode);
+    node = std::shared_ptr<OpNode<F>>(new OpNode<F>(), torch::autograd::deleteNode);
     torch::autograd::edge_list edges;
     edges.reserve(n);
     each([&](const at::Tensor& t) { edges.push_back(torch::autograd::impl::gradient_edge(t)); });
@@ -692,33 +732,21 @@ at::Tensor record(const std::array<TensorRef, N>& inputs, const OptTensor& mask,
     torch::autograd::set_history(o, node);
     node->output_info_.emplace_back(o);
     node->set_ctx_grad_fn(node);
-    AutogradContext& ctx = node->ctx_;
+    node->scalars = scalars;
     variable_list save;
     save.reserve(N + 5);
     for (const at::Tensor& t : inputs) save.push_back(t);
     save.insert(save.end(), {o, lse, mask.value_or(at::Tensor()), lens.value_or(at::Tensor()), offset_copy});
-    ctx.save_for_backward(std::move(save));
-    ctx.saved_data["max_seqlen"] = max_seqlen;
-    ctx.saved_data["p_drop"] = p_drop;
-    ctx.saved_data["seed"] = seed;
-    ctx.saved_data["offset"] = offset;
-    ctx.saved_data["scale"] = scale;
+    node->ctx_.save_for_backward(std::move(save));
     node->save_variables_to_ctx();
   }
   return o;
 }
 
-// What `record` saved.
+// The tensors that `record` saved.
 template <size_t N>
 struct Recorded {
-  variable_list t;   // inputs, o, lse, mask, lens, offset_tensor
-  int64_t max_seqlen, seed, offset;
-  double p_drop;
-  c10::optional<double> scale;
-  explicit Recorded(AutogradContext* ctx)
-      : t(ctx->get_saved_variables()), max_seqlen(ctx->saved_data["max_seqlen"].toInt()), seed(ctx->saved_data["seed"].toInt()),
-        offset(ctx->saved_data["offset"].toInt()), p_drop(ctx->saved_data["p_drop"].toDouble()),
-        scale(ctx->saved_data["scale"].toOptional<double>()) {}
+  const variable_list& t;   // inputs, o, lse, mask, lens, offset_tensor
   const at::Tensor& in(size_t i) const { return t[i]; }
   const at::Tensor& o() const { return t[N]; }
   const at::Tensor& lse() const { return t[N + 1]; }
@@ -742,15 +770,15 @@ struct Recorded {
   }
 };
 
-struct FmhaFunction : public torch::autograd::Function<FmhaFunction> {
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+struct FmhaFunction : public OpFunction<FmhaFunction> {
+  static variable_list gradients(const variable_list& saved, const Scalars& c, const at::Tensor& d_o) {
     static auto op = find_op<Triple, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const at::Tensor&, const OptTensor&, const OptTensor&, double, int64_t, int64_t,
                              c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_bwd");
-    const Recorded<3> r(ctx);
+    const Recorded<3> r{saved};
     return r.gradients([&]() -> variable_list {
-      auto [dq, dk, dv] = op.call(grads[0], r.in(0), r.in(1), r.in(2), r.o(), r.lse(), r.mask(), r.lens(), r.p_drop, r.seed, r.offset,
-                                  r.scale, 0, r.offset_tensor());
+      auto [dq, dk, dv] = op.call(d_o, r.in(0), r.in(1), r.in(2), r.o(), r.lse(), r.mask(), r.lens(), c.p_drop, c.seed, c.offset,
+                                  c.scale, 0, r.offset_tensor());
       return {dq, dk, dv};
     });
   }
@@ -761,18 +789,18 @@ at::Tensor fmha_autograd(const at::Tensor& q, const at::Tensor& k, const at::Ten
   // through the dispatcher, so that fake / meta tensors reach the shape-only kernels
   static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, const at::Tensor&, const OptTensor&, const OptTensor&,
                            double, int64_t, int64_t, c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_fwd");
-  return record<FmhaFunction, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset,
-                                 scale, [&] { return op.call(q, k, v, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor); });
+  return record<FmhaFunction, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, mask, seqlens, offset_tensor, {0, p_drop, seed, offset, scale},
+                                 [&] { return op.call(q, k, v, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor); });
 }
 
-struct FmhaQkvPackedFunction : public torch::autograd::Function<FmhaQkvPackedFunction> {
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+struct FmhaQkvPackedFunction : public OpFunction<FmhaQkvPackedFunction> {
+  static variable_list gradients(const variable_list& saved, const Scalars& c, const at::Tensor& d_o) {
     static auto op = find_op<at::Tensor, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const OptTensor&, const OptTensor&, double, int64_t, int64_t, c10::optional<double>, int64_t,
                              const OptTensor&>("mha_manual::fmha_qkvpacked_bwd");
-    const Recorded<1> r(ctx);
+    const Recorded<1> r{saved};
     return r.gradients([&]() -> variable_list {
-      return {op.call(grads[0], r.in(0), r.o(), r.lse(), r.mask(), r.lens(), r.p_drop, r.seed, r.offset, r.scale, 0, r.offset_tensor())};
+      return {op.call(d_o, r.in(0), r.o(), r.lse(), r.mask(), r.lens(), c.p_drop, c.seed, c.offset, c.scale, 0, r.offset_tensor())};
     });
   }
 };
@@ -780,20 +808,20 @@ at::Tensor fmha_qkvpacked_autograd(const at::Tensor& qkv, const OptTensor& mask,
                                    int64_t seed, int64_t offset, c10::optional<double> scale, const OptTensor& offset_tensor) {
   static auto op = find_op<Pair, const at::Tensor&, const OptTensor&, const OptTensor&, double, int64_t, int64_t,
                            c10::optional<double>, int64_t, const OptTensor&>("mha_manual::fmha_qkvpacked_fwd");
-  return record<FmhaQkvPackedFunction, 1>({TensorRef(qkv)}, mask, seqlens, offset_tensor, 0, p_drop, seed, offset, scale, [&] {
+  return record<FmhaQkvPackedFunction, 1>({TensorRef(qkv)}, mask, seqlens, offset_tensor, {0, p_drop, seed, offset, scale}, [&] {
     return op.call(qkv, mask, seqlens, p_drop, seed, offset, scale, 0, offset_tensor);
   });
 }
 
-struct FmhaVarlenFunction : public torch::autograd::Function<FmhaVarlenFunction> {
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+struct FmhaVarlenFunction : public OpFunction<FmhaVarlenFunction> {
+  static variable_list gradients(const variable_list& saved, const Scalars& c, const at::Tensor& d_o) {
     static auto op = find_op<Triple, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
                              const OptTensor&>("mha_manual::fmha_varlen_bwd");
-    const Recorded<3> r(ctx);
+    const Recorded<3> r{saved};
     return r.gradients([&]() -> variable_list {
-      auto [dq, dk, dv] = op.call(grads[0], r.in(0), r.in(1), r.in(2), r.o(), r.lse(), *r.lens(), r.max_seqlen, r.p_drop, r.seed,
-                                  r.offset, r.scale, r.offset_tensor());
+      auto [dq, dk, dv] = op.call(d_o, r.in(0), r.in(1), r.in(2), r.o(), r.lse(), *r.lens(), c.max_seqlen, c.p_drop, c.seed,
+                                  c.offset, c.scale, r.offset_tensor());
       return {dq, dk, dv};
     });
   }
@@ -803,19 +831,19 @@ at::Tensor fmha_varlen_autograd(const at::Tensor& q, const at::Tensor& k, const 
                                 const OptTensor& offset_tensor) {
   static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t, double,
                            int64_t, int64_t, c10::optional<double>, const OptTensor&>("mha_manual::fmha_varlen_fwd");
-  return record<FmhaVarlenFunction, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen,
-                                       p_drop, seed, offset, scale,
+  return record<FmhaVarlenFunction, 3>({TensorRef(q), TensorRef(k), TensorRef(v)}, OptTensor(), cu_seqlens, offset_tensor,
+                                       {max_seqlen, p_drop, seed, offset, scale},
                                        [&] { return op.call(q, k, v, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor); });
 }
 
-struct FmhaVarlenQkvPackedFunction : public torch::autograd::Function<FmhaVarlenQkvPackedFunction> {
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+struct FmhaVarlenQkvPackedFunction : public OpFunction<FmhaVarlenQkvPackedFunction> {
+  static variable_list gradients(const variable_list& saved, const Scalars& c, const at::Tensor& d_o) {
     static auto op = find_op<at::Tensor, const at::Tensor&, const at::Tensor&, const at::Tensor&, const at::Tensor&,
                              const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>, const OptTensor&>(
         "mha_manual::fmha_varlen_qkvpacked_bwd");
-    const Recorded<1> r(ctx);
+    const Recorded<1> r{saved};
     return r.gradients([&]() -> variable_list {
-      return {op.call(grads[0], r.in(0), r.o(), r.lse(), *r.lens(), r.max_seqlen, r.p_drop, r.seed, r.offset, r.scale, r.offset_tensor())};
+      return {op.call(d_o, r.in(0), r.o(), r.lse(), *r.lens(), c.max_seqlen, c.p_drop, c.seed, c.offset, c.scale, r.offset_tensor())};
     });
   }
 };
@@ -824,8 +852,8 @@ at::Tensor fmha_varlen_qkvpacked_autograd(const at::Tensor& qkv, const at::Tenso
                                           const OptTensor& offset_tensor) {
   static auto op = find_op<Pair, const at::Tensor&, const at::Tensor&, int64_t, double, int64_t, int64_t, c10::optional<double>,
                            const OptTensor&>("mha_manual::fmha_varlen_qkvpacked_fwd");
-  return record<FmhaVarlenQkvPackedFunction, 1>({TensorRef(qkv)}, OptTensor(), cu_seqlens, offset_tensor, max_seqlen, p_drop, seed,
-                                                offset, scale,
+  return record<FmhaVarlenQkvPackedFunction, 1>({TensorRef(qkv)}, OptTensor(), cu_seqlens, offset_tensor,
+                                                {max_seqlen, p_drop, seed, offset, scale},
                                                 [&] { return op.call(qkv, cu_seqlens, max_seqlen, p_drop, seed, offset, scale, offset_tensor); });
 }
 

@@ -240,3 +240,24 @@ def test_torch_compile_fullgraph(ops, cuda_device):
     assert torch.equal(outs[0][0], outs[1][0])
     assert torch.equal(outs[0][2], outs[1][2]) and torch.equal(outs[0][3], outs[1][3])     # dK, dV: fixed summation order
     assert (outs[0][1].float() - outs[1][1].float()).abs().max().item() <= 2e-3             # dQ: atomics
+
+
+def test_compiled_autograd_gives_the_same_gradients(ops, cuda_device):
+    from torch._dynamo import compiled_autograd
+
+    x = torch.randn(2, 130, 3, 2, 64, device=cuda_device).half()
+    lens = torch.tensor([130, 70], dtype=torch.int32, device=cuda_device)
+    offset = torch.tensor([3], device=cuda_device)
+    grads = []
+    for compiled in (False, True):
+        leaf = x.clone().requires_grad_()
+        out = ops.fmha_qkvpacked(leaf, None, lens, 0.2, 9, 4, 0.1, offset)
+        if compiled:
+            with compiled_autograd._enable(lambda graph: graph):
+                out.float().square().sum().backward()
+        else:
+            out.float().square().sum().backward()
+        grads.append(leaf.grad)
+    # dK and dV have a fixed order of summation, dQ is summed by atomics
+    assert torch.equal(grads[0][:, :, 1:], grads[1][:, :, 1:])
+    helpers.assert_close(grads[0][:, :, 0], grads[1][:, :, 0], "dq")
