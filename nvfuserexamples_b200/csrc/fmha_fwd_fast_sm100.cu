@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     *philox_off = a.philox_offset + (a.philox_offset_dev != nullptr ? static_cast<uint32_t>(*a.philox_offset_dev) : 0u);
     mbar_init(q_full, 1);
     mbar_init(s_full, 1);
-    mbar_init(p_full, 128);
+    mbar_init(p_full, 4);
     mbar_init(o_full, 1);
     for (int s = 0; s < ST; ++s) {
       mbar_init(k_full + s, 1);
@@ -262,11 +262,12 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   } else if (warp == 0 && MERGED) {
     // ============================ TMA producer + MMA issuer in one warp (D = 64) =====
     // The warp runs convergently; one elected lane issues the loads, MMA bursts go out as in the split version.
-    // Order per key step j: Q K^T(j); then, while the softmax warps work on S(j), wait for that MMA to complete
-    // (a few hundred cycles) and refill what it and the previous P V have released: K of step j+ST and V of step
-    // j-1+ST (the tensor core works in order, so P V(j-1), issued before Q K^T(j), has completed too); then wait
-    // for P(j) and issue P V(j).  No refill ever stands between P V(j) and Q K^T(j+1), the chain the step time
-    // hangs on.
+    // Under the softmax of step j it waits for Q K^T(j) (P V(j-1), issued before it, has completed by then too), refills what
+    // these have released, K of step j+ST and V of step j-1+ST, and makes sure that V(j) and K(j+1) are there.  When P(j) comes,
+    // P V(j) and Q K^T(j+1) go out back to back: a poll between them (some 300 cycles while MMAs with both operands in shared
+    // memory run) or a second one after P(j) would stand in the chain the step time hangs on.
+    // (Polls in between, and 128 arrivals on p_full instead of one per warp: B=4 H=16 S=2048 115.9 us against 101.3, B=64 H=16
+    // S=512 104.8 against 100.5; the split version B=16 H=8 S=512 D=128 with an additive mask 31.3 against 27.7.)
     if constexpr (MERGED) {
       constexpr int KQ = D / 16;     // k-steps of S = Q K^T
       constexpr int KP = TN / 16;    // k-steps of O += P V
@@ -296,38 +297,41 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       uint64_t aq[KQ];
 #pragma unroll
       for (int kk = 0; kk < KQ; ++kk) aq[kk] = dq + kmajor_step(kk, 16384);
-      mbar_wait(q_full, 0, wctx, kFQFull);
-      for (int j = 0; j < n_kv; ++j) {
-        const int s = j % ST;
-        const uint32_t ph = (j / ST) & 1;
-        const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + s * L::kTileBytes), 16, 1024);
-        const uint64_t dv = make_smem_desc_sw128(smem_u32(sV + s * L::kTileBytes), L::kSubTile, 1024);
-        uint64_t bk[KQ], bv[KP];
+      auto issue_qk = [&](int j) {
+        const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + (j % ST) * L::kTileBytes), 16, 1024);
+        uint64_t bk[KQ];
 #pragma unroll
         for (int kk = 0; kk < KQ; ++kk) bk[kk] = dk + kmajor_step(kk, L::kSubTile);
+        umma_ss_x4(tS, aq, bk, kIdescQK, 0u);
+        umma_commit_elect(s_full);
+      };
+      mbar_wait(q_full, 0, wctx, kFQFull);
+      if (n_kv > 0) {
+        mbar_wait(k_full, 0, wctx, kFKFull);
+        tc_fence_after_sync();
+        issue_qk(0);
+      }
+      for (int j = 0; j < n_kv; ++j) {
+        const int s = j % ST;
+        const uint64_t dv = make_smem_desc_sw128(smem_u32(sV + s * L::kTileBytes), L::kSubTile, 1024);
+        uint64_t bv[KP];
 #pragma unroll
         for (int kk = 0; kk < KP; ++kk) bv[kk] = dv + mnmajor_step(kk);
-        mbar_wait(k_full + s, ph, wctx, kFKFull);
-        tc_fence_after_sync();
-        umma_ss_x4(tS, aq, bk, kIdescQK, 0u);
-        umma_commit_elect(k_empty + s);
-        umma_commit_elect(s_full);
-        // refills, under the softmax of this step
-        const bool more_k = j + ST < n_kv, more_v = j >= 1 && j - 1 + ST < n_kv;
+        const bool more_k = j + ST < n_kv, more_v = j >= 1 && j - 1 + ST < n_kv, more = j + 1 < n_kv;
         if (more_k || more_v) {
-          mbar_wait(k_empty + s, ph, wctx, kFKEmpty);       // Q K^T(j) has completed, and P V(j-1) before it
-          if (more_v) mbar_wait(v_empty + ((j - 1) % ST), ((j - 1) / ST) & 1, wctx, kFVEmpty);
+          mbar_wait(s_full, j & 1, wctx, kFKEmpty);
           if (elect_one()) {
             if (more_k) load_k(j + ST);
             if (more_v) load_v(j - 1 + ST);
           }
           __syncwarp();
         }
+        mbar_wait(v_full + s, (j / ST) & 1, wctx, kFVFull);
+        if (more) mbar_wait(k_full + (j + 1) % ST, ((j + 1) / ST) & 1, wctx, kFKFull);
         mbar_wait(p_full, j & 1, wctx, kFPFull);
-        mbar_wait(v_full + s, ph, wctx, kFVFull);
         tc_fence_after_sync();
         umma_ts_x4(tO, tS, 8u, bv, kIdescPV, (j > 0) ? 1u : 0u);
-        umma_commit_elect(v_empty + s);
+        if (more) issue_qk(j + 1);
       }
       umma_commit_elect(o_full);
     }
@@ -345,25 +349,34 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       uint64_t aq[KQ];
 #pragma unroll
       for (int kk = 0; kk < KQ; ++kk) aq[kk] = dq + kmajor_step(kk, 16384);
-      mbar_wait(q_full, 0, wctx, kFQFull);
-      for (int j = 0; j < n_kv; ++j) {
+      auto issue_qk = [&](int j) {
         const int s = j % ST;
-        const uint32_t ph = (j / ST) & 1;
         const uint64_t dk = make_smem_desc_sw128(smem_u32(sK + s * L::kTileBytes), 16, 1024);
-        const uint64_t dv = make_smem_desc_sw128(smem_u32(sV + s * L::kTileBytes), L::kSubTile, 1024);
-        uint64_t bk[KQ], bv[KP];
+        uint64_t bk[KQ];
 #pragma unroll
         for (int kk = 0; kk < KQ; ++kk) bk[kk] = dk + kmajor_step(kk, L::kSubTile);
-#pragma unroll
-        for (int kk = 0; kk < KP; ++kk) bv[kk] = dv + mnmajor_step(kk);
-        mbar_wait(k_full + s, ph, wctx, kFKFull);
-        tc_fence_after_sync();
         if constexpr (KQ == 4) umma_ss_x4(tS, aq, bk, kIdescQK, 0u);
         else umma_ss_x8(tS, aq, bk, kIdescQK, 0u);
-        umma_commit_elect(k_empty + s);
         umma_commit_elect(s_full);
+        umma_commit_elect(k_empty + s);
+      };
+      mbar_wait(q_full, 0, wctx, kFQFull);
+      if (n_kv > 0) {
+        mbar_wait(k_full, 0, wctx, kFKFull);
+        tc_fence_after_sync();
+        issue_qk(0);
+      }
+      for (int j = 0; j < n_kv; ++j) {
+        const int s = j % ST;
+        const uint64_t dv = make_smem_desc_sw128(smem_u32(sV + s * L::kTileBytes), L::kSubTile, 1024);
+        uint64_t bv[KP];
+#pragma unroll
+        for (int kk = 0; kk < KP; ++kk) bv[kk] = dv + mnmajor_step(kk);
+        const bool more = j + 1 < n_kv;
+        // what P V(j) and Q K^T(j+1) need is waited for under the softmax of step j, see the merged version
+        mbar_wait(v_full + s, (j / ST) & 1, wctx, kFVFull);
+        if (more) mbar_wait(k_full + (j + 1) % ST, ((j + 1) / ST) & 1, wctx, kFKFull);
         mbar_wait(p_full, j & 1, wctx, kFPFull);
-        mbar_wait(v_full + s, ph, wctx, kFVFull);
         tc_fence_after_sync();
         const uint32_t acc0 = (j > 0) ? 1u : 0u;
         {
@@ -375,6 +388,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           umma_ts_x4(tO, tS + 32u, 8u, b1, kIdescPV, 1u);
         }
         umma_commit_elect(v_empty + s);
+        if (more) issue_qk(j + 1);
       }
       umma_commit_elect(o_full);
     }
@@ -395,6 +409,11 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     // leaves P and O undefined instead of competing with the others.  (No gain at a ragged last tile of a full grid.)
     const bool warp_idle = SPLIT && q0 + quad * 32 >= q_limit;
 
+    auto arrive_p = [&]() {   // one arrival per warp
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    };
+
     float m_ref = -INFINITY;
     float2 sum2 = make_float2(0.f, 0.f);  // running sum of exp2(t - m_ref), two interleaved partial sums
 
@@ -414,7 +433,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       }
       if (warp_idle) {   // no query row of this warp exists: only keep the step's barriers in phase
         mbar_wait(s_full, j & 1, wctx, kFSFull, 32);
-        mbar_arrive(p_full);
+        arrive_p();
         continue;
       }
       // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
@@ -507,7 +526,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
           for (int c = 0; c < TN / 32; ++c) tmem_st16(tS + c * 16, zero);
           tmem_wait_st();
           tc_fence_before_sync();
-          mbar_arrive(p_full);
+          arrive_p();
           continue;
         }
         if constexpr (DROP) {
@@ -565,7 +584,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(p_full);
+      arrive_p();
     }
 
     // ---- epilogue ------------------------------------------------------------------------
