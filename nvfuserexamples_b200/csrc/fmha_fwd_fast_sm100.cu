@@ -1,6 +1,6 @@
 // fmha_fwd_fast_sm100.cu — the production forward kernel: compact masks only (none, valid
 // lengths, additive [B,S_k] row, or a packed variable-length batch), optional Philox dropout,
-// writes O and the row logsumexp.
+// writes O and the row logsumexp.  (Head dimension 128 without dropout on grids that fill the chip: fmha_fwd_pair_sm100.cu.)
 //
 // CTA organisation as in the general kernel in fmha_fwd_sm100.cu (TMA producer, tcgen05.mma
 // issuer, four softmax warps with one thread per query row; S in tensor memory, P written back
@@ -33,6 +33,7 @@
 
 #include "../../include/fmha_sm100.h"
 #include "fmha_device_utils.cuh"
+#include "fmha_fwd_softmax.cuh"
 #include "fmha_kernel_args.h"
 #include "philox.cuh"
 #include "sm100_ptx.cuh"
@@ -48,19 +49,6 @@ namespace {
 // stores; D = 128 at 168 registers: plain 52, dropout 72, additive 112, both 56).
 constexpr int kThreadsSplit = 192, kThreadsMerged = 160;
 template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged : kThreadsSplit; }
-constexpr float kLog2eF = 1.4426950408889634f;
-constexpr float kLn2F = 0.6931471805599453f;
-
-// Additive key mask, in the log2 domain: a key at or above kDeadMask may matter (scores of N(0,1) rows are a few units,
-// a padding mask is -10000 * log2e), a step with only keys below it is looked at for a shortcut; exp2(x) is zero in fp32,
-// flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.
-constexpr float kDeadMask = -1000.0f;
-constexpr float kZeroExp = -200.0f;
-// Floor of a step's row maximum: the lowest float, not -inf, so that a step or a share whose scores are all -inf (an additive
-// mask of -inf, or of the lowest float, which becomes -inf times log2 e) gives exponentials of zero, not of -inf - (-inf).  No
-// finite score is below it.  (As the start of the running maximum it does the same, but the additive variant at D = 128 then
-// spills more: B=32 H=16 S=512 103.7 -> 107.8 us.)
-constexpr float kNoScore = -3.402823466e+38f;
 constexpr int kMaxKeySplit = 8;   // portable cluster size
 
 enum FastWaitSite {
@@ -90,34 +78,6 @@ struct FastSmem {
   static constexpr int kBytes = kOffMisc + 16;
   static constexpr int kDynBytes = kBytes + 1024;
 };
-
-// 32 columns of a row: t holds their scores; produces 16 packed 16-bit pairs of exp2(t - m_ref) (dropout applied) and
-// adds the undropped values to sum2.
-template <bool BF16, bool KEYADD, bool DROP>
-__device__ __forceinline__ void softmax_chunk(const uint32_t (&t)[32], float sl2, float neg_m, float2& sum2,
-                                              uint32_t (&packed)[16], const uint32_t* keepw) {
-  const float2 sl22 = make_float2(sl2, sl2);
-  const float2 negm2 = make_float2(neg_m, neg_m);
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    float2 x = make_float2(__uint_as_float(t[2 * k]), __uint_as_float(t[2 * k + 1]));
-    if constexpr (KEYADD) x = __fadd2_rn(x, negm2);
-    else x = __ffma2_rn(x, sl22, negm2);
-    float2 p;
-    p.x = fast_exp2(x.x);
-    p.y = fast_exp2(x.y);
-    sum2 = __fadd2_rn(sum2, p);
-    packed[k] = pack2<BF16>(p.x, p.y);
-  }
-  if constexpr (DROP) {
-    // keepw[i]: bit 7 of byte e = keep decision of column 4*i + e; the permutes replicate it over a 16-bit lane
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      packed[2 * i] &= prmt(keepw[i], 0u, 0x9988u);
-      packed[2 * i + 1] &= prmt(keepw[i], 0u, 0xBBAAu);
-    }
-  }
-}
 
 }  // namespace
 
@@ -403,7 +363,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     const uint32_t tS = tmem_base + lane_addr + kColS;
     const uint32_t tO = tmem_base + lane_addr + kColO;
     const float sl2 = a.scale_log2;
-    const uint32_t gbh = static_cast<uint32_t>(a.philox_bh_offset + bh);
+    const DropRow drop_row = {a.philox_keys, philox_off, static_cast<uint32_t>(a.philox_bh_offset + bh), static_cast<uint32_t>(q_row), a.philox_thr};
 
     // Rows past the end are never stored, so with a handful of query rows against long keys a warp that has no row
     // leaves P and O undefined instead of competing with the others.  (No gain at a ragged last tile of a full grid.)
@@ -436,155 +396,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
         arrive_p();
         continue;
       }
-      // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
-      // before they are awaited, while the tensor core is still busy with Q K^T.
-      [[maybe_unused]] uint32_t keepw[DROP ? TN / 4 : 1];
-      auto draw_keep_words = [&]() {
-        const uint32_t kb0 = static_cast<uint32_t>(col0 / 16);
-        const uint32_t poff = *philox_off;
-#pragma unroll
-        for (int d = 0; d < TN / 16; ++d) {
-          const U4 draw = dropout_draw_keys(a.philox_keys, poff, gbh, static_cast<uint32_t>(q_row), kb0 + d);
-          keepw[d * 4 + 0] = (draw.x & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-          keepw[d * 4 + 1] = (draw.y & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-          keepw[d * 4 + 2] = (draw.z & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-          keepw[d * 4 + 3] = (draw.w & 0x7F7F7F7Fu) + (0x80u - a.philox_thr) * 0x01010101u;
-        }
-      };
-    draw_and_look:
-      if constexpr (DROP) {
-        if (live) draw_keep_words();
-      }
-      mbar_wait(s_full, j & 1, wctx, kFSFull, 32);
-      tc_fence_after_sync();
-
-      // ---- scores into registers (raw, or scaled and masked with an additive mask), row maximum --------------------
-      // Without dropout they stay there until they are exponentiated.  With dropout the step's keep words are live as well:
-      // the scores are read a second time, 32 columns at a time (held, they spilled more and cost 57.2 against 55.7 us at B=32
-      // H=12 S=512).
-      constexpr bool HOLD = !DROP;
-      auto finish_scores = [&](int c, uint32_t (&v)[32]) {   // mask added, keys past the end to -inf (exp2 makes them zero)
-        if constexpr (KEYADD) {
-#pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            const float2 mk = *reinterpret_cast<const float2*>(mask_stage + c * 32 + 2 * k);
-            const float2 t = __ffma2_rn(make_float2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1])), make_float2(sl2, sl2), mk);
-            v[2 * k] = __float_as_uint(t.x);
-            v[2 * k + 1] = __float_as_uint(t.y);
-          }
-        }
-        if (n_cols < TN) {
-#pragma unroll
-          for (int k = 0; k < 32; ++k)
-            if (c * 32 + k >= n_cols) v[k] = __float_as_uint(-INFINITY);
-        }
-      };
-      uint32_t sv[TN / 32][32];
-      // The maximum of 32 columns is taken while the next 32 are on their way (D = 128: B=16 H=16 S=1024 163.1 -> 161.6 us,
-      // S=512 with dropout 57.5 -> 56.1; D = 64: 0.5 %).  With an additive mask and the scores held that form spills (B=32 H=16
-      // S=512 D=128 117 -> 121 us), there all are loaded first; with dropout they are not held, and it spares spills (the same
-      // size with dropout: 134.2 -> 121.3 us, D = 64 93.7 -> 89.5).
-      constexpr bool AHEAD = !KEYADD || DROP;
-#pragma unroll
-      for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_ld32(tS + c * 32, sv[c]);
-#pragma unroll
-      for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_wait_ld_dep(sv[c]);
-      if constexpr (!AHEAD) {
-#pragma unroll
-        for (int c = 0; c < TN / 32; ++c) finish_scores(c, sv[c]);
-      }
-      float tile_max = kNoScore;
-#pragma unroll
-      for (int c = 0; c < TN / 32; ++c) {
-        if constexpr (AHEAD) {
-          if (c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
-          finish_scores(c, sv[c]);
-        }
-        auto v = [&](int k) { return __uint_as_float(sv[c][k]); };
-        // with an additive mask a NaN has to show in the maximum, or the shortcut below would step over it
-        auto max3 = [](float x, float y, float z) { return fmax3<KEYADD>(x, y, z); };
-        float m0 = max3(v(0), v(1), v(2));
-        float m1 = max3(v(3), v(4), v(5));
-#pragma unroll
-        for (int k = 6; k + 3 < 32; k += 4) {
-          m0 = max3(m0, v(k), v(k + 1));
-          m1 = max3(m1, v(k + 2), v(k + 3));
-        }
-        tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
-        if constexpr (AHEAD) {
-          if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
-        }
-      }
-      if constexpr (!KEYADD) tile_max = fmaxf(tile_max * sl2, kNoScore);  // scale > 0: the maximum commutes with it
-      // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
-      // the reference maximum that its exponential is zero in fp32, P is zero and nothing else changes.  Decided on the
-      // scores themselves, so the result is the same bits; a third of the steps of a batch with lengths in [S/3, S].
-      if constexpr (KEYADD) {
-        if (!live && __all_sync(0xffffffffu, tile_max - m_ref < kZeroExp)) {
-          const uint32_t zero[16] = {};
-#pragma unroll
-          for (int c = 0; c < TN / 32; ++c) tmem_st16(tS + c * 16, zero);
-          tmem_wait_st();
-          tc_fence_before_sync();
-          arrive_p();
-          continue;
-        }
-        if constexpr (DROP) {
-          if (!live) {   // rare, and a second copy of the draws costs every step (B=2 H=12 S=1024 37.2 -> 36.2 us without it)
-            live = true;
-            goto draw_and_look;
-          }
-        }
-      }
-      // ---- running reference maximum, lazy rescale of O ------------------------------------
-      {
-        float m_new = fmaxf(m_ref, tile_max);
-        if (m_ref != -INFINITY && m_new - m_ref <= 8.0f) m_new = m_ref;  // exponentials stay below 2^8
-        const bool moved = (m_new != m_ref) && (m_ref != -INFINITY);
-        const float alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - m_new);
-        if (j > 0 && __any_sync(0xffffffffu, moved)) {
-#pragma unroll
-          for (int c = 0; c < D / 8; ++c) {   // eight columns at a time: the scores of the step stay in registers meanwhile
-            uint32_t r[8];
-            tmem_ld8(tO + c * 8, r);
-            tmem_wait_ld_dep8(r);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * alpha);
-            tmem_st8(tO + c * 8, r);
-          }
-        }
-        sum2.x *= alpha;
-        sum2.y *= alpha;
-        m_ref = m_new;
-      }
-      // ---- exponentials, dropout, P over S ---------------------------------------------------------------------
-      if constexpr (HOLD) {
-#pragma unroll
-        for (int c = 0; c < TN / 32; ++c) {
-          uint32_t packed[16];
-          softmax_chunk<BF16, KEYADD, DROP>(sv[c], sl2, -m_ref, sum2, packed, keepw);
-          tmem_st16(tS + c * 16, packed);
-        }
-      } else {
-        uint32_t ra[32], rb[32], packed[16];   // chunk c+1 (then c+2) is in flight while chunk c (c+1) is processed
-        tmem_ld32(tS, ra);
-#pragma unroll
-        for (int c = 0; c < TN / 32; c += 2) {
-          tmem_wait_ld_dep(ra);
-          finish_scores(c, ra);
-          tmem_ld32(tS + (c + 1) * 32, rb);
-          softmax_chunk<BF16, KEYADD, DROP>(ra, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
-          tmem_st16(tS + c * 16, packed);
-          tmem_wait_ld_dep(rb);
-          finish_scores(c + 1, rb);
-          if (c + 2 < TN / 32) tmem_ld32(tS + (c + 2) * 32, ra);
-          softmax_chunk<BF16, KEYADD, DROP>(rb, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 + 8 : 0));
-          tmem_st16(tS + c * 16 + 16, packed);
-        }
-      }
-      tmem_wait_st();
-      tc_fence_before_sync();
-      arrive_p();
+      auto wait_s = [&]() { mbar_wait(s_full, j & 1, wctx, kFSFull, 32); };
+      auto arrive = [&](int) { arrive_p(); };
+      softmax_step<D, TN, BF16, KEYADD, DROP, 0>(tS, tO, col0, n_cols, sl2, mask_stage, live, drop_row, m_ref, sum2, wait_s, arrive, [] {}, [] {});
     }
 
     // ---- epilogue ------------------------------------------------------------------------
@@ -623,28 +437,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     // A packed batch's last query tile of a sequence holds rows of the NEXT sequence past q_limit: its rows
     // are written one by one from registers instead of through the tile store.
     const bool partial_rows = packed && (q0 + kTileM > q_limit);
-#pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld32(tO + c * 32, r);
-      tmem_wait_ld_dep(r);
-      uint8_t* tile = sQ + (c / 2) * 16384;  // Q is no longer needed: every QK^T has completed
-      unsigned short* grow = reinterpret_cast<unsigned short*>(a.o_ptr) + static_cast<int64_t>(row_base + q_row) * a.o_ss +
-                             static_cast<int64_t>(h) * a.o_sh + c * 32;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint4 w;
-        w.x = pack2<BF16>(__uint_as_float(r[q * 8 + 0]) * out_scale, __uint_as_float(r[q * 8 + 1]) * out_scale);
-        w.y = pack2<BF16>(__uint_as_float(r[q * 8 + 2]) * out_scale, __uint_as_float(r[q * 8 + 3]) * out_scale);
-        w.z = pack2<BF16>(__uint_as_float(r[q * 8 + 4]) * out_scale, __uint_as_float(r[q * 8 + 5]) * out_scale);
-        w.w = pack2<BF16>(__uint_as_float(r[q * 8 + 6]) * out_scale, __uint_as_float(r[q * 8 + 7]) * out_scale);
-        if (partial_rows) {
-          if (row_ok) *reinterpret_cast<uint4*>(grow + q * 8) = w;
-        } else {
-          *reinterpret_cast<uint4*>(tile + sw128_offset(row, (c % 2) * 4 + q)) = w;
-        }
-      }
-    }
+    // (Q is no longer needed: every Q K^T has completed.)
+    o_tile_out<D, BF16>(tO, out_scale, sQ, row, partial_rows, row_ok,
+                        reinterpret_cast<unsigned short*>(a.o_ptr) + static_cast<int64_t>(row_base + q_row) * a.o_ss + static_cast<int64_t>(h) * a.o_sh);
     fence_proxy_async_smem();
     named_bar_sync(1, 128);
     if (tid == 0) {
@@ -793,6 +588,7 @@ static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream, int n_split =
 }
 
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream) {
+  if (fwd_pair_applies(a, D)) return launch_fwd_pair(a, dtype, stream);
   const bool bf = dtype == FMHA_DTYPE_BF16;
   const bool keyadd = a.mask_kind == FMHA_MASK_KEY_ADDITIVE;
   const bool drop = a.dropout_kind == FMHA_DROPOUT_PHILOX;

@@ -1,0 +1,264 @@
+// fmha_fwd_softmax.cuh — what one softmax thread (one query row) does per key step and at the end of a query tile: shared by
+// the two forward kernels for compact masks (fmha_fwd_fast_sm100.cu, fmha_fwd_pair_sm100.cu).
+#pragma once
+#include "fmha_device_utils.cuh"
+#include "philox.cuh"
+#include "sm100_ptx.cuh"
+
+namespace fmha {
+
+constexpr float kLog2eF = 1.4426950408889634f;
+constexpr float kLn2F = 0.6931471805599453f;
+
+// Additive key mask, in the log2 domain: a key at or above kDeadMask may matter (scores of N(0,1) rows are a few units,
+// a padding mask is -10000 * log2e), a step with only keys below it is looked at for a shortcut; exp2(x) is zero in fp32,
+// flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.
+constexpr float kDeadMask = -1000.0f;
+constexpr float kZeroExp = -200.0f;
+// Floor of a step's row maximum: the lowest float, not -inf, so that a step or a share whose scores are all -inf (an additive
+// mask of -inf, or of the lowest float, which becomes -inf times log2 e) gives exponentials of zero, not of -inf - (-inf).  No
+// finite score is below it.  (As the start of the running maximum it does the same, but the additive variant at D = 128 then
+// spills more: B=32 H=16 S=512 103.7 -> 107.8 us.)
+constexpr float kNoScore = -3.402823466e+38f;
+
+// 32 columns of a row: t holds their scores; produces 16 packed 16-bit pairs of exp2(t - m_ref) (dropout applied) and
+// adds the undropped values to sum2.
+template <bool BF16, bool KEYADD, bool DROP>
+__device__ __forceinline__ void softmax_chunk(const uint32_t (&t)[32], float sl2, float neg_m, float2& sum2,
+                                              uint32_t (&packed)[16], const uint32_t* keepw) {
+  const float2 sl22 = make_float2(sl2, sl2);
+  const float2 negm2 = make_float2(neg_m, neg_m);
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    float2 x = make_float2(__uint_as_float(t[2 * k]), __uint_as_float(t[2 * k + 1]));
+    if constexpr (KEYADD) x = __fadd2_rn(x, negm2);
+    else x = __ffma2_rn(x, sl22, negm2);
+    float2 p;
+    p.x = fast_exp2(x.x);
+    p.y = fast_exp2(x.y);
+    sum2 = __fadd2_rn(sum2, p);
+    packed[k] = pack2<BF16>(p.x, p.y);
+  }
+  if constexpr (DROP) {
+    // keepw[i]: bit 7 of byte e = keep decision of column 4*i + e; the permutes replicate it over a 16-bit lane
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      packed[2 * i] &= prmt(keepw[i], 0u, 0x9988u);
+      packed[2 * i + 1] &= prmt(keepw[i], 0u, 0xBBAAu);
+    }
+  }
+}
+
+// What the keep decisions of a row depend on besides the key.
+struct DropRow {
+  const PhiloxKeys& keys;
+  volatile const uint32_t* offset;   // shared memory: read where a draw starts, so that it holds no register in between
+  uint32_t bh, row, thr;
+};
+
+// One key step of TN keys: scores from tS, the running maximum and sum, P over the scores, O rescaled where the maximum has
+// moved by more than 2^8.  n_cols < TN: the others lie past the end.  KEYADD: mask_stage holds the step's mask in the log2
+// domain; live: some key of the step is not masked away.  wait_s returns when the scores are there; arrive_p(1) hands P to the
+// tensor core, or, with P_FIRST > 0, arrive_p(0) its first P_FIRST chunks of 32 columns and arrive_p(1) the rest.  The exponentials
+// lie between turn_begin and turn_end.
+template <int D, int TN, bool BF16, bool KEYADD, bool DROP, int P_FIRST, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
+__device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, bool live,
+                                             const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,
+                                             const TurnBegin& turn_begin, const TurnEnd& turn_end) {
+  // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
+  // before they are awaited, while the tensor core is still busy with Q K^T.
+  [[maybe_unused]] uint32_t keepw[DROP ? TN / 4 : 1];
+  auto draw_keep_words = [&]() {
+    const uint32_t kb0 = static_cast<uint32_t>(key0 / 16);
+    const uint32_t poff = *dr.offset;
+#pragma unroll
+    for (int d = 0; d < TN / 16; ++d) {
+      const U4 draw = dropout_draw_keys(dr.keys, poff, dr.bh, dr.row, kb0 + d);
+      keepw[d * 4 + 0] = (draw.x & 0x7F7F7F7Fu) + (0x80u - dr.thr) * 0x01010101u;
+      keepw[d * 4 + 1] = (draw.y & 0x7F7F7F7Fu) + (0x80u - dr.thr) * 0x01010101u;
+      keepw[d * 4 + 2] = (draw.z & 0x7F7F7F7Fu) + (0x80u - dr.thr) * 0x01010101u;
+      keepw[d * 4 + 3] = (draw.w & 0x7F7F7F7Fu) + (0x80u - dr.thr) * 0x01010101u;
+    }
+  };
+[[maybe_unused]] draw_and_look:
+  if constexpr (DROP) {
+    if (live) draw_keep_words();
+  }
+  wait_s();
+  tc_fence_after_sync();
+
+  // ---- scores into registers (raw, or scaled and masked with an additive mask), row maximum --------------------
+  // Without dropout they stay there until they are exponentiated.  With dropout the step's keep words are live as well:
+  // the scores are read a second time, 32 columns at a time (held, they spilled more and cost 57.2 against 55.7 us at B=32
+  // H=12 S=512).
+  constexpr bool HOLD = !DROP;
+  auto finish_scores = [&](int c, uint32_t (&v)[32]) {   // mask added, keys past the end to -inf (exp2 makes them zero)
+    if constexpr (KEYADD) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float4 mk = *reinterpret_cast<const float4*>(mask_stage + c * 32 + 4 * k);
+        const float2 sl22 = make_float2(sl2, sl2);
+        const float2 t0 = __ffma2_rn(make_float2(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1])), sl22, make_float2(mk.x, mk.y));
+        const float2 t1 = __ffma2_rn(make_float2(__uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3])), sl22, make_float2(mk.z, mk.w));
+        v[4 * k] = __float_as_uint(t0.x);
+        v[4 * k + 1] = __float_as_uint(t0.y);
+        v[4 * k + 2] = __float_as_uint(t1.x);
+        v[4 * k + 3] = __float_as_uint(t1.y);
+      }
+    }
+    if (n_cols < TN) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k)
+        if (c * 32 + k >= n_cols) v[k] = __float_as_uint(-INFINITY);
+    }
+  };
+  uint32_t sv[TN / 32][32];
+  // The maximum of 32 columns is taken while the next 32 are on their way (D = 128: B=16 H=16 S=1024 163.1 -> 161.6 us,
+  // S=512 with dropout 57.5 -> 56.1; D = 64: 0.5 %).  With an additive mask and the scores held that form spills (B=32 H=16
+  // S=512 D=128 117 -> 121 us), there all are loaded first; with dropout they are not held, and it spares spills (the same
+  // size with dropout: 134.2 -> 121.3 us, D = 64 93.7 -> 89.5).
+    constexpr bool AHEAD = !KEYADD || DROP;
+#pragma unroll
+  for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_ld32(tS + c * 32, sv[c]);
+#pragma unroll
+  for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_wait_ld_dep(sv[c]);
+  if constexpr (!AHEAD) {
+#pragma unroll
+    for (int c = 0; c < TN / 32; ++c) finish_scores(c, sv[c]);
+  }
+  float tile_max = kNoScore;
+#pragma unroll
+  for (int c = 0; c < TN / 32; ++c) {
+    if constexpr (AHEAD) {
+      if (c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
+      finish_scores(c, sv[c]);
+    }
+    auto v = [&](int k) { return __uint_as_float(sv[c][k]); };
+    // with an additive mask a NaN has to show in the maximum, or the shortcut below would step over it
+    auto max3 = [](float x, float y, float z) { return fmax3<KEYADD>(x, y, z); };
+    float m0 = max3(v(0), v(1), v(2));
+    float m1 = max3(v(3), v(4), v(5));
+#pragma unroll
+    for (int k = 6; k + 3 < 32; k += 4) {
+      m0 = max3(m0, v(k), v(k + 1));
+      m1 = max3(m1, v(k + 2), v(k + 3));
+    }
+    tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
+    if constexpr (AHEAD) {
+      if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
+    }
+  }
+  if constexpr (!KEYADD) tile_max = fmaxf(tile_max * sl2, kNoScore);  // scale > 0: the maximum commutes with it
+  // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
+  // the reference maximum that its exponential is zero in fp32, P is zero and nothing else changes.  Decided on the
+  // scores themselves, so the result is the same bits; a third of the steps of a batch with lengths in [S/3, S].
+  if constexpr (KEYADD) {
+    if (!live && __all_sync(0xffffffffu, tile_max - m_ref < kZeroExp)) {
+      turn_begin();
+      turn_end();
+      const uint32_t zero[16] = {};
+#pragma unroll
+      for (int c = 0; c < TN / 32; ++c) tmem_st16(tS + c * 16, zero);
+      tmem_wait_st();
+      tc_fence_before_sync();
+      if (P_FIRST > 0) arrive_p(0);
+      arrive_p(1);
+      return;
+    }
+    if constexpr (DROP) {
+      if (!live) {   // rare, and a second copy of the draws costs every step (B=2 H=12 S=1024 37.2 -> 36.2 us without it)
+        live = true;
+        goto draw_and_look;
+      }
+    }
+  }
+  // ---- running reference maximum, lazy rescale of O ------------------------------------
+  {
+    float m_new = fmaxf(m_ref, tile_max);
+    if (m_ref != -INFINITY && m_new - m_ref <= 8.0f) m_new = m_ref;  // exponentials stay below 2^8
+    const bool moved = (m_new != m_ref) && (m_ref != -INFINITY);
+    const float alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - m_new);
+    if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+      for (int c = 0; c < D / 8; ++c) {   // eight columns at a time: the scores of the step stay in registers meanwhile
+        uint32_t r[8];
+        tmem_ld8(tO + c * 8, r);
+        tmem_wait_ld_dep8(r);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * alpha);
+        tmem_st8(tO + c * 8, r);
+      }
+    }
+    sum2.x *= alpha;
+    sum2.y *= alpha;
+    m_ref = m_new;
+  }
+  turn_begin();
+  // ---- exponentials, dropout, P over S ---------------------------------------------------------------------
+  auto hand_over = [&](int c) {   // after 32-column chunk c
+    if (c + 1 == P_FIRST) {
+      tmem_wait_st();
+      tc_fence_before_sync();
+      arrive_p(0);
+    }
+  };
+  if constexpr (HOLD) {
+#pragma unroll
+    for (int c = 0; c < TN / 32; ++c) {
+      uint32_t packed[16];
+      softmax_chunk<BF16, KEYADD, DROP>(sv[c], sl2, -m_ref, sum2, packed, keepw);
+      tmem_st16(tS + c * 16, packed);
+      hand_over(c);
+    }
+  } else {
+    uint32_t ra[32], rb[32], packed[16];   // chunk c+1 (then c+2) is in flight while chunk c (c+1) is processed
+    tmem_ld32(tS, ra);
+#pragma unroll
+    for (int c = 0; c < TN / 32; c += 2) {
+      tmem_wait_ld_dep(ra);
+      finish_scores(c, ra);
+      tmem_ld32(tS + (c + 1) * 32, rb);
+      softmax_chunk<BF16, KEYADD, DROP>(ra, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
+      tmem_st16(tS + c * 16, packed);
+      hand_over(c);
+      tmem_wait_ld_dep(rb);
+      finish_scores(c + 1, rb);
+      if (c + 2 < TN / 32) tmem_ld32(tS + (c + 2) * 32, ra);
+      softmax_chunk<BF16, KEYADD, DROP>(rb, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 + 8 : 0));
+      tmem_st16(tS + c * 16 + 16, packed);
+      hand_over(c + 1);
+    }
+  }
+  turn_end();
+  tmem_wait_st();
+  tc_fence_before_sync();
+  arrive_p(1);
+}
+
+// O of a finished query tile out of tensor memory, scaled and rounded: into `tile` (shared memory, 128 rows in the swizzled
+// layout of the O tensor map), or, where the tile reaches into rows that are not its own, the valid rows straight to `grow`.
+template <int D, bool BF16>
+__device__ __forceinline__ void o_tile_out(uint32_t tO, float out_scale, uint8_t* tile, int row, bool by_rows, bool row_ok,
+                                           unsigned short* grow) {
+#pragma unroll
+  for (int c = 0; c < D / 32; ++c) {
+    uint32_t r[32];
+    tmem_ld32(tO + c * 32, r);
+    tmem_wait_ld_dep(r);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint4 w;
+      w.x = pack2<BF16>(__uint_as_float(r[q * 8 + 0]) * out_scale, __uint_as_float(r[q * 8 + 1]) * out_scale);
+      w.y = pack2<BF16>(__uint_as_float(r[q * 8 + 2]) * out_scale, __uint_as_float(r[q * 8 + 3]) * out_scale);
+      w.z = pack2<BF16>(__uint_as_float(r[q * 8 + 4]) * out_scale, __uint_as_float(r[q * 8 + 5]) * out_scale);
+      w.w = pack2<BF16>(__uint_as_float(r[q * 8 + 6]) * out_scale, __uint_as_float(r[q * 8 + 7]) * out_scale);
+      if (by_rows) {
+        if (row_ok) *reinterpret_cast<uint4*>(grow + c * 32 + q * 8) = w;
+      } else {
+        *reinterpret_cast<uint4*>(tile + (c / 2) * 16384 + sw128_offset(row, (c % 2) * 4 + q)) = w;
+      }
+    }
+  }
+}
+
+}  // namespace fmha

@@ -39,7 +39,8 @@ struct FwdArgs {
   // tensors; o_ptr / strides serve the row-wise stores of a sequence's last, partial query tile
   int total_rows;
   int zero_uncovered;         // FMHA_FLAG_ZERO_UNCOVERED: 0, or an UncoveredMode
-  int length_class_shift;     // production kernel: -1, or the grid's last axis counts batch elements by (length - 1) >> shift
+  int persist;                // pair kernel: a CTA takes further items of the grid when it has done its own
+  int length_class_shift;     // production kernels: -1, or the grid's last axis counts batch elements by (length - 1) >> shift
   const void* q_ptr;          // the kernel for a handful of query rows reads Q with plain loads
   int64_t q_ss, q_sh, q_sb;
   void* o_ptr;
@@ -122,6 +123,9 @@ struct BwdArgs {
 // Launchers (defined in the .cu files).  Return a cudaError_t as int.
 int launch_fwd(const FwdArgs& a, int D, int dtype, bool legacy, bool p_via_smem, cudaStream_t stream);
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
+// the same for grids that fill the chip: two query tiles per CTA, persistent (fmha_fwd_pair_sm100.cu)
+bool fwd_pair_applies(const FwdArgs& a, int D);
+int launch_fwd_pair(const FwdArgs& a, int dtype, cudaStream_t stream);
 // the kernel for a handful of query rows per head (fmha_fwd_rows_sm100.cu): compact masks, not packed
 bool fwd_rows_applies(int S_q, int S_k, int D, int64_t heads, bool dropout);
 int launch_fwd_rows(const FwdArgs& a, int D, int dtype, cudaStream_t stream);

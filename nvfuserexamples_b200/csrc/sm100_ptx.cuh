@@ -140,6 +140,9 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 // Barrier that also ORs a predicate over its participants: every one of them gets the same answer, which a
 // flag read by each thread on its own cannot promise (used for "has any wait of this CTA been given up?",
 // where threads that disagree would leave each other alone at the next barrier).
@@ -157,6 +160,13 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool pred) {
       : "memory");
   return r != 0;
 }
+
+// Register split of a block of several warpgroups (four aligned warps each; every warp of one executes it): the shares must
+// add up to no more than the block was launched with.
+template <int N>
+__device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ------------------------------------------------------------------------------------
 // thread-block clusters and distributed shared memory
@@ -394,6 +404,34 @@ __device__ __forceinline__ void umma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uin
       "}\n"
       ::"r"(d_tmem), "r"(a_tmem), "r"(a_step), "l"(b[0]), "l"(b[1]), "l"(b[2]), "l"(b[3]), "r"(idesc), "r"(acc_first)
       : "memory");
+}
+// k-steps [K0, K1) of D += A B, A at a_tmem + 8 columns per step, in bursts of four and two.
+__device__ __forceinline__ void umma_ts_x2(uint32_t d_tmem, uint32_t a_tmem, const uint64_t b0, const uint64_t b1, uint32_t idesc,
+                                           uint32_t acc_first) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q, pe;\n\t"
+      ".reg .b32 a1;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 q, 0, 0;\n\t"
+      "add.u32 a1, %1, 8;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, p;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], %3, %4, q;\n\t"
+      "}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b0), "l"(b1), "r"(idesc), "r"(acc_first)
+      : "memory");
+}
+template <int K0, int K1, int N>
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, const uint64_t (&b)[N], uint32_t idesc, uint32_t acc_first) {
+  if constexpr (K1 - K0 >= 4) {
+    const uint64_t y[4] = {b[K0], b[K0 + 1], b[K0 + 2], b[K0 + 3]};
+    umma_ts_x4(d_tmem, a_tmem + K0 * 8, 8u, y, idesc, acc_first);
+    if constexpr (K1 - K0 > 4) umma_ts<K0 + 4, K1>(d_tmem, a_tmem, b, idesc, 1u);
+  } else {
+    static_assert(K1 - K0 == 2, "bursts of four and two");
+    umma_ts_x2(d_tmem, a_tmem + K0 * 8, b[K0], b[K0 + 1], idesc, acc_first);
+  }
 }
 // The same with the four A tiles in two pairs: MMAs 0 and 1 at a0 and a0 + a_step, 2 and 3 at a1 and a1 + a_step.
 __device__ __forceinline__ void umma_ts_2x2(uint32_t d_tmem, uint32_t a0, uint32_t a1, uint32_t a_step, const uint64_t (&b)[4],
