@@ -60,7 +60,7 @@ struct PairSmem {
   static constexpr int kOffClc = kOffItems + kItemSlots * 32;
   static constexpr int kOffBar = kOffClc + 16;
   static constexpr int kNumBars = 2 * kSlots + 2 + 2 + 2 + 4 + 2 + 2 + 2 + 2 * kItemSlots + 1 + 8;
-  static constexpr int kOffMisc = kOffBar + kNumBars * 8;      // tensor-memory base, abort flag, 2 live flags
+  static constexpr int kOffMisc = kOffBar + kNumBars * 8;      // tensor-memory base, abort flag, 2 mask kinds
   static constexpr int kDynBytes = kOffMisc + 16;              // 1024-byte aligned base: checked by the kernel
   static_assert(kDynBytes <= 232448, "shared memory budget exceeded");
 };
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
   uint64_t* turn = clc_full + 1;           // [2][4] by tile and quarter: the other tile's warp has done its exponentials
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 4);
-  volatile int* mask_live = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 8);    // [2]
+  volatile int* mask_kind = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 8);    // [2]
 
   if (smem_u32(smem) & 1023) {
     if (threadIdx.x == 0 && a.status != nullptr) atomicCAS(a.status, 0, kPrSmemBase);
@@ -400,18 +400,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
       for (int k0 = 0; k0 < it.k_limit; k0 += TN, ++t) {
         const int s = t & 1;
         float mk[TN / 32];
-        bool live = false;
+        bool exists[TN / 32];
 #pragma unroll
         for (int i = 0; i < TN / 32; ++i) {
           const int c = k0 + i * 32 + lane;
-          mk[i] = c < a.S_k ? mask[c] * kLog2eF : 0.f;
-          live |= c < a.S_k && !(mk[i] < kDeadMask);
+          exists[i] = c < a.S_k;
+          mk[i] = exists[i] ? mask[c] * kLog2eF : 0.f;
         }
-        live = __any_sync(0xffffffffu, live);
+        const int kind = mask_step_kind(mk, exists);
         if (t >= 2) mbar_wait(mask_empty + s, ((t >> 1) - 1) & 1, wctx, kPrMaskEmpty);
 #pragma unroll
         for (int i = 0; i < TN / 32; ++i) sMask[s * TN + i * 32 + lane] = mk[i];
-        if (lane == 0) mask_live[s] = live;
+        if (lane == 0) mask_kind[s] = kind;
         __syncwarp();
         if (lane == 0) mbar_arrive(mask_full + s);
       }
@@ -457,13 +457,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
         };
         for (int j = 0; j < n_kv; ++j) {
           const float* mask_stage = sMask + (t & 1) * TN;
-          bool live = true;   // additive mask: some key of this step is not masked away
+          int kind = kMaskZero;
           if constexpr (KEYADD) {
             mbar_wait(mask_full + (t & 1), (t >> 1) & 1, wctx, kPrMaskFull, 32);
-            live = mask_live[t & 1] != 0;
-            live = __shfl_sync(0xffffffffu, live, 0);
+            kind = __shfl_sync(0xffffffffu, mask_kind[t & 1], 0);
           }
-          softmax_step<D, TN, BF16, KEYADD, false, PF>(tS, tO, j * TN, min(TN, it.k_limit - j * TN), sl2, mask_stage, live, no_drop, m_ref,
+          softmax_step<D, TN, BF16, KEYADD, false, PF>(tS, tO, j * TN, min(TN, it.k_limit - j * TN), sl2, mask_stage, kind, no_drop, m_ref,
                                                       sum2, wait_s, arrive_p, turn_begin, turn_end);
           s_par ^= 1u;
           if constexpr (KEYADD) {

@@ -12,7 +12,9 @@ constexpr float kLn2F = 0.6931471805599453f;
 
 // Additive key mask, in the log2 domain: a key at or above kDeadMask may matter (scores of N(0,1) rows are a few units,
 // a padding mask is -10000 * log2e), a step with only keys below it is looked at for a shortcut; exp2(x) is zero in fp32,
-// flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.
+// flushed subnormals included, for x < -126: kZeroExp leaves a margin for the rounding of the difference.  A step whose mask is
+// zero throughout is treated like one without a mask.
+enum MaskStep { kMaskZero = 0, kMaskAny = 1, kMaskDead = 2 };
 constexpr float kDeadMask = -1000.0f;
 constexpr float kZeroExp = -200.0f;
 // Floor of a step's row maximum: the lowest float, not -inf, so that a step or a share whose scores are all -inf (an additive
@@ -20,10 +22,21 @@ constexpr float kZeroExp = -200.0f;
 // finite score is below it.  (As the start of the running maximum it does the same, but the additive variant at D = 128 then
 // spills more: B=32 H=16 S=512 103.7 -> 107.8 us.)
 constexpr float kNoScore = -3.402823466e+38f;
+// The kind of a step from its mask values, a whole warp holding them (`exists`: the key does).
+template <int N>
+__device__ __forceinline__ int mask_step_kind(const float (&mk)[N], const bool (&exists)[N]) {
+  bool zero = true, dead = true;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    zero &= !exists[i] || mk[i] == 0.f;
+    dead &= !exists[i] || mk[i] < kDeadMask;
+  }
+  return __all_sync(0xffffffffu, zero) ? kMaskZero : __all_sync(0xffffffffu, dead) ? kMaskDead : kMaskAny;
+}
 
-// 32 columns of a row: t holds their scores; produces 16 packed 16-bit pairs of exp2(t - m_ref) (dropout applied) and
+// 32 columns of a row: t holds their scores; produces 16 packed 16-bit pairs of exp2(t * sl2 - m_ref) (dropout applied) and
 // adds the undropped values to sum2.
-template <bool BF16, bool KEYADD, bool DROP>
+template <bool BF16, bool DROP>
 __device__ __forceinline__ void softmax_chunk(const uint32_t (&t)[32], float sl2, float neg_m, float2& sum2,
                                               uint32_t (&packed)[16], const uint32_t* keepw) {
   const float2 sl22 = make_float2(sl2, sl2);
@@ -31,8 +44,7 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t (&t)[32], float sl2
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
     float2 x = make_float2(__uint_as_float(t[2 * k]), __uint_as_float(t[2 * k + 1]));
-    if constexpr (KEYADD) x = __fadd2_rn(x, negm2);
-    else x = __ffma2_rn(x, sl22, negm2);
+    x = __ffma2_rn(x, sl22, negm2);
     float2 p;
     p.x = fast_exp2(x.x);
     p.y = fast_exp2(x.y);
@@ -57,12 +69,12 @@ struct DropRow {
 };
 
 // One key step of TN keys: scores from tS, the running maximum and sum, P over the scores, O rescaled where the maximum has
-// moved by more than 2^8.  n_cols < TN: the others lie past the end.  KEYADD: mask_stage holds the step's mask in the log2
-// domain; live: some key of the step is not masked away.  wait_s returns when the scores are there; arrive_p(1) hands P to the
+// moved by more than 2^8.  n_cols < TN: the others lie past the end.  KEYADD: `kind` of the step's mask, which mask_stage
+// holds in the log2 domain unless it is zero.  wait_s returns when the scores are there; arrive_p(1) hands P to the
 // tensor core, or, with P_FIRST > 0, arrive_p(0) its first P_FIRST chunks of 32 columns and arrive_p(1) the rest.  The exponentials
 // lie between turn_begin and turn_end.
 template <int D, int TN, bool BF16, bool KEYADD, bool DROP, int P_FIRST, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
-__device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, bool live,
+__device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
                                              const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,
                                              const TurnBegin& turn_begin, const TurnEnd& turn_end) {
   // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
@@ -82,7 +94,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   };
 [[maybe_unused]] draw_and_look:
   if constexpr (DROP) {
-    if (live) draw_keep_words();
+    if (!KEYADD || kind != kMaskDead) draw_keep_words();
   }
   wait_s();
   tc_fence_after_sync();
@@ -92,8 +104,9 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   // the scores are read a second time, 32 columns at a time (held, they spilled more and cost 57.2 against 55.7 us at B=32
   // H=12 S=512).
   constexpr bool HOLD = !DROP;
+  const float mul = KEYADD && kind == kMaskAny ? 1.0f : sl2;   // what takes a score as held to the log2 domain
   auto finish_scores = [&](int c, uint32_t (&v)[32]) {   // mask added, keys past the end to -inf (exp2 makes them zero)
-    if constexpr (KEYADD) {
+    if (KEYADD && kind == kMaskAny) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const float4 mk = *reinterpret_cast<const float4*>(mask_stage + c * 32 + 4 * k);
@@ -113,26 +126,15 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
     }
   };
   uint32_t sv[TN / 32][32];
-  // The maximum of 32 columns is taken while the next 32 are on their way (D = 128: B=16 H=16 S=1024 163.1 -> 161.6 us,
-  // S=512 with dropout 57.5 -> 56.1; D = 64: 0.5 %).  With an additive mask and the scores held that form spills (B=32 H=16
-  // S=512 D=128 117 -> 121 us), there all are loaded first; with dropout they are not held, and it spares spills (the same
-  // size with dropout: 134.2 -> 121.3 us, D = 64 93.7 -> 89.5).
-    constexpr bool AHEAD = !KEYADD || DROP;
-#pragma unroll
-  for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_ld32(tS + c * 32, sv[c]);
-#pragma unroll
-  for (int c = 0; c < (AHEAD ? 1 : TN / 32); ++c) tmem_wait_ld_dep(sv[c]);
-  if constexpr (!AHEAD) {
-#pragma unroll
-    for (int c = 0; c < TN / 32; ++c) finish_scores(c, sv[c]);
-  }
+  // The maximum of 32 columns is taken while the next 32 are on their way (D = 128: B=16 H=16 S=1024 163.1 -> 161.6 us, S=512
+  // with dropout 57.5 -> 56.1; with an additive mask B=64 H=16 S=384 D = 64 67.6 -> 66.7).
+  tmem_ld32(tS, sv[0]);
+  tmem_wait_ld_dep(sv[0]);
   float tile_max = kNoScore;
 #pragma unroll
   for (int c = 0; c < TN / 32; ++c) {
-    if constexpr (AHEAD) {
-      if (c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
-      finish_scores(c, sv[c]);
-    }
+    if (c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
+    finish_scores(c, sv[c]);
     auto v = [&](int k) { return __uint_as_float(sv[c][k]); };
     // with an additive mask a NaN has to show in the maximum, or the shortcut below would step over it
     auto max3 = [](float x, float y, float z) { return fmax3<KEYADD>(x, y, z); };
@@ -144,16 +146,15 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       m1 = max3(m1, v(k + 2), v(k + 3));
     }
     tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
-    if constexpr (AHEAD) {
-      if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
-    }
+    if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
   }
-  if constexpr (!KEYADD) tile_max = fmaxf(tile_max * sl2, kNoScore);  // scale > 0: the maximum commutes with it
+  tile_max *= mul;   // scale > 0: the maximum commutes with it
+  if constexpr (!KEYADD) tile_max = fmaxf(tile_max, kNoScore);
   // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
   // the reference maximum that its exponential is zero in fp32, P is zero and nothing else changes.  Decided on the
   // scores themselves, so the result is the same bits; a third of the steps of a batch with lengths in [S/3, S].
   if constexpr (KEYADD) {
-    if (!live && __all_sync(0xffffffffu, tile_max - m_ref < kZeroExp)) {
+    if (kind == kMaskDead && __all_sync(0xffffffffu, tile_max + kDeadMask - m_ref < kZeroExp)) {   // every mask value is below kDeadMask
       turn_begin();
       turn_end();
       const uint32_t zero[16] = {};
@@ -165,11 +166,9 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       arrive_p(1);
       return;
     }
-    if constexpr (DROP) {
-      if (!live) {   // rare, and a second copy of the draws costs every step (B=2 H=12 S=1024 37.2 -> 36.2 us without it)
-        live = true;
-        goto draw_and_look;
-      }
+    if (kind == kMaskDead) {   // rare, and a second copy of what came before costs every step
+      kind = kMaskAny;
+      goto draw_and_look;
     }
   }
   // ---- running reference maximum, lazy rescale of O ------------------------------------
@@ -206,7 +205,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
 #pragma unroll
     for (int c = 0; c < TN / 32; ++c) {
       uint32_t packed[16];
-      softmax_chunk<BF16, KEYADD, DROP>(sv[c], sl2, -m_ref, sum2, packed, keepw);
+      softmax_chunk<BF16, DROP>(sv[c], mul, -m_ref, sum2, packed, keepw);
       tmem_st16(tS + c * 16, packed);
       hand_over(c);
     }
@@ -218,13 +217,13 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       tmem_wait_ld_dep(ra);
       finish_scores(c, ra);
       tmem_ld32(tS + (c + 1) * 32, rb);
-      softmax_chunk<BF16, KEYADD, DROP>(ra, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
+      softmax_chunk<BF16, DROP>(ra, mul, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
       tmem_st16(tS + c * 16, packed);
       hand_over(c);
       tmem_wait_ld_dep(rb);
       finish_scores(c + 1, rb);
       if (c + 2 < TN / 32) tmem_ld32(tS + (c + 2) * 32, ra);
-      softmax_chunk<BF16, KEYADD, DROP>(rb, sl2, -m_ref, sum2, packed, keepw + (DROP ? c * 8 + 8 : 0));
+      softmax_chunk<BF16, DROP>(rb, mul, -m_ref, sum2, packed, keepw + (DROP ? c * 8 + 8 : 0));
       tmem_st16(tS + c * 16 + 16, packed);
       hand_over(c + 1);
     }
