@@ -190,7 +190,8 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     mbar_fence_init();
     fence_proxy_async_smem();
     // The first product's operands, by the thread that has set up their barriers: the rest of the set-up, tensor memory above all,
-    // takes as long as they do.
+    // takes as long as they do (some 1 000 of a CTA's first 3 500 cycles; B=13 H=12 S=197 10.1 -> 9.2 us, B=64 H=16 S=128 12.6 ->
+    // 11.9, B=32 H=12 S=512 with dropout 51.4 -> 50.4).
     mbar_arrive_expect_tx(q_full, L::kQBytes);
 #pragma unroll
     for (int c = 0; c < D / 64; ++c) tma_load_4d(sQ + c * 16384, &a.tm_q, q_full, c * 64, row_base + q0, h, tb);
