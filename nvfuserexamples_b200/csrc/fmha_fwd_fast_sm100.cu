@@ -47,8 +47,8 @@ namespace {
 // D = 128: 192 threads (TMA producer warp, MMA warp, four softmax warps).  D = 64: 160 threads, one warp issues both
 // the TMA loads and the MMAs.  Registers are allocated per SM sub-partition (16 384 each, warps dealt round-robin):
 // four CTAs of six warps put six warps on a sub-partition (80 registers per thread), four CTAs of five warps put
-// five (96), where the plain variant stays out of local memory, dropout spills 16 bytes and the additive mask 48 to 60 (spill
-// stores; D = 128 at 168 registers: plain 52, dropout 72, additive 112, both 56).
+// five (96), where the plain variant stays out of local memory, dropout spills 16 to 20 bytes, the additive mask 32 to 36 and both
+// 68 to 76 (spill stores; D = 128 at 168 registers: plain 40 to 48, dropout 52 to 76, additive 140 to 148, both 116 to 120).
 constexpr int kThreadsSplit = 192, kThreadsMerged = 160;
 template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged : kThreadsSplit; }
 constexpr int kMaxKeySplit = 8;   // portable cluster size
