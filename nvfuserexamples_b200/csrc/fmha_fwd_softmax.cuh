@@ -148,8 +148,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
     tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
     if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
   }
-  tile_max *= mul;   // scale > 0: the maximum commutes with it
-  if constexpr (!KEYADD) tile_max = fmaxf(tile_max, kNoScore);
+  tile_max = fmax3<KEYADD>(tile_max * mul, kNoScore, kNoScore);   // scale > 0: the maximum commutes with it; the floor may have passed the range
   // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
   // the reference maximum that its exponential is zero in fp32, P is zero and nothing else changes.  Decided on the
   // scores themselves, so the result is the same bits; a third of the steps of a batch with lengths in [S/3, S].

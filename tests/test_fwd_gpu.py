@@ -265,3 +265,30 @@ def test_a_nan_among_masked_keys_is_not_stepped_over(cuda_device, D, p_drop):
     assert torch.isnan(o[3, 2]).all() and torch.isnan(lse.view(B, H, S)[3, 2]).all()
     o[3, 2] = 0
     assert torch.isfinite(o).all()
+
+
+@pytest.mark.parametrize("B,H,S_q,S_k", [
+    (40, 8, 256, 300),    # one CTA per query tile; at D = 128 two tiles per CTA
+    (2, 8, 200, 300),     # one CTA per query tile at both head dimensions
+    (1, 2, 130, 1536),    # keys split over a cluster
+])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("mask", ["none", "zero", "zero_first"])
+def test_scores_of_minus_infinity_under_a_large_scale(cuda_device, B, H, S_q, S_k, D, mask):
+    """Keys whose scores are all -inf contribute zeros, also where they fill a row's first step or a share of the keys and the scale is
+    so large (1, as unscaled attention has it) that the lowest float times scale * log2 e is -inf itself."""
+    q, k, v, _, _ = helpers.randn_like_config(B, H, S_q, S_k, D, torch.float16, seed=D + S_k, device=cuda_device)
+    q, k = q * 0.35, k * 0.35   # scores of unit size, give or take, without the usual 1/sqrt(D)
+    q[..., 0] = q[..., 0].abs() + 0.1
+    n_inf = max(D, S_k // 8)   # at least a whole key step (64 keys at D = 64, 128 at D = 128), or a share of eight
+    k[:, :, :n_inf, 0] = float("-inf")
+    kw, add = {}, None
+    if mask != "none":
+        add = torch.zeros(B, S_k, device=cuda_device)
+        if mask == "zero_first":
+            add[:, n_inf:] = torch.randn(S_k - n_inf, generator=torch.Generator().manual_seed(2)).to(cuda_device)
+        kw["mask"] = add
+    o, lse = api.fmha_forward(q, k, v, scale=1.0, **kw)
+    ref = composite.attention_fp32(q, k, v, add_mask=None if add is None else add.reshape(B, 1, 1, S_k), scale=1.0)
+    helpers.assert_close(o, ref["o"], "o")
+    helpers.assert_close(lse, ref["lse"], "lse", atol=1e-3, rtol=1e-4)
