@@ -55,7 +55,7 @@ constexpr int kMaxKeySplit = 8;   // portable cluster size
 
 enum FastWaitSite {
   kFQFull = 111, kFKEmpty = 112, kFVEmpty = 113, kFKFull = 114, kFVFull = 115, kFPFull = 116, kFSFull = 117,
-  kFOFull = 118
+  kFOFull = 118, kFQkDone = 119
 };
 
 // TN = keys per step.  D = 64 uses 64-key steps: S (64 columns) + O (64 columns) = 128 tensor-memory
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
         for (int kk = 0; kk < KP; ++kk) bv[kk] = dv + mnmajor_step(kk);
         const bool more_k = j + ST < n_kv, more_v = j >= 1 && j - 1 + ST < n_kv, more = j + 1 < n_kv;
         if (more_k || more_v) {
-          mbar_wait(s_full, j & 1, wctx, kFKEmpty);
+          mbar_wait(s_full, j & 1, wctx, kFQkDone);
           if (elect_one()) {
             if (more_k) load_k(j + ST);
             if (more_v) load_v(j - 1 + ST);

@@ -38,8 +38,8 @@ constexpr int kPairThreads = 384;
 constexpr int kItemSlots = 4;
 
 enum PairWaitSite {
-  kPrQFull = 131, kPrQEmpty = 132, kPrKvFull = 133, kPrKvEmpty = 134, kPrSFull = 135, kPrPFull = 136, kPrOFull = 137,
-  kPrMaskFull = 138, kPrMaskEmpty = 139, kPrItem = 140, kPrItemEmpty = 141, kPrClc = 142, kPrSmemBase = 143, kPrTurn = 144
+  kPrQFull = 171, kPrQEmpty = 172, kPrKvFull = 173, kPrKvEmpty = 174, kPrSFull = 175, kPrPFull = 176, kPrOFull = 177,
+  kPrMaskFull = 178, kPrMaskEmpty = 179, kPrItem = 180, kPrItemEmpty = 181, kPrClc = 182, kPrSmemBase = 183, kPrTurn = 184
 };
 
 constexpr int D = 128;

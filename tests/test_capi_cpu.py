@@ -154,3 +154,14 @@ def test_ctypes_layer_rejects_layouts_the_abi_cannot_describe():
         capi._lse_ok(torch.zeros(2, 2, 32)[..., ::2], 64)
     with pytest.raises(ValueError):
         capi._dense_ok(torch.zeros(4, 8).t(), "mask")
+
+
+def test_wait_site_codes_are_unique():
+    """Status word 0 is all that tells which wait of which kernel ran out, so no two sites may share a code."""
+    codes = {}
+    for src in sorted((ROOT / "nvfuserexamples_b200" / "csrc").glob("*.cu*")):
+        for body in re.findall(r"enum \w*WaitSite\s*\{([^}]*)\}", src.read_text()):
+            for name, code in re.findall(r"(\w+)\s*=\s*(\d+)", body):
+                codes.setdefault(int(code), []).append(f"{src.name}: {name}")
+    assert len(codes) > 80 and 900 not in codes   # 900: the self-test's wait
+    assert not {c: sites for c, sites in codes.items() if len(sites) > 1}
