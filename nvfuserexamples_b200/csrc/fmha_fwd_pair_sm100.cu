@@ -520,16 +520,20 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
   }
 }
 
-// Grids of at least two rounds of query tiles on two tiles per SM (the other kernel's capacity), no dropout, three or more key steps:
+// Grids of at least two query tiles per SM (one round of the other kernel's capacity), no dropout, three or more key steps:
 // at one or two steps a CTA's life is its start and its end (S_q=256: S_k=128 12.8 / 12.2 us, S_k=256 16.2 / 16.0, S_k=1024 39.0 /
 // 40.2).  A head with an odd number of tiles leaves half a CTA idle for one item, which takes nearly as long as a whole one: the
 // rounds of pairs over the SMs may be at most 8/7 of the rounds of tiles (H=16: S=384 B=16 34.4 / 33.0 us at 4/3, S=640 68.2 / 69.3 at
 // 6/5, B=8 S=1152 94.1 / 90.1 at 5/4).
-bool fwd_pair_applies(const FwdArgs& a, int head_dim) {
-  if (head_dim != D || a.dropout_kind == FMHA_DROPOUT_PHILOX || a.S_k <= 256) return false;
-  const int64_t sms = sm_count(), n = (a.S_q + kTileM - 1) / kTileM, heads = static_cast<int64_t>(a.H) * a.B;
+bool fwd_pair_pays(int64_t sms, int64_t heads, int64_t S_q, int64_t S_k) {
+  if (sms <= 0 || S_k <= 256) return false;   // no multiprocessors: the query for their number has failed
+  const int64_t n = (S_q + kTileM - 1) / kTileM;
   const int64_t pair_rounds = (heads * ((n + 1) / 2) + sms - 1) / sms, tile_rounds = (heads * n + 2 * sms - 1) / (2 * sms);
   return heads * n >= 2 * sms && 7 * pair_rounds <= 8 * tile_rounds;
+}
+bool fwd_pair_applies(const FwdArgs& a, int head_dim) {
+  if (head_dim != D || a.dropout_kind == FMHA_DROPOUT_PHILOX) return false;
+  return fwd_pair_pays(sm_count(), static_cast<int64_t>(a.H) * a.B, a.S_q, a.S_k);
 }
 
 template <bool BF16, bool KEYADD, bool PACKED>
