@@ -1,21 +1,36 @@
 """The rule on sizes that picks the forward kernel of two query tiles per CTA, called in the built library (no GPU needed)."""
 import ctypes as C
 
+import pytest
+
 from nvfuserexamples_b200 import capi
 
 
-def pair_pays(sms, heads, S_q, S_k):
-    fn = capi.load()["_ZN4fmha13fwd_pair_paysEllll"]   # fmha::fwd_pair_pays(int64_t x 4)
-    fn.argtypes, fn.restype = [C.c_int64] * 4, C.c_bool
-    return fn(sms, heads, S_q, S_k)
+def pair_pays(sms, B, H, S_q, S_k, packed_rows=0):
+    fn = capi.load()["_ZN4fmha13fwd_pair_paysEllllll"]   # fmha::fwd_pair_pays(int64_t x 6)
+    fn.argtypes, fn.restype = [C.c_int64] * 6, C.c_bool
+    return fn(sms, B, H, S_q, S_k, packed_rows)
 
 
 def test_two_tile_rule():
-    assert pair_pays(148, 64, 2048, 2048)       # 4 sequences of 16 heads: the shape the kernel was built for
-    assert not pair_pays(148, 64, 2048, 256)    # two key steps
-    assert not pair_pays(148, 64, 512, 2048)    # fewer than two query tiles per multiprocessor
+    assert pair_pays(148, 4, 16, 2048, 2048)       # 4 sequences of 16 heads: the shape the kernel was built for
+    assert not pair_pays(148, 4, 16, 2048, 256)    # two key steps
+    assert not pair_pays(148, 4, 16, 512, 2048)    # fewer than two query tiles per multiprocessor
+    assert not pair_pays(148, 50, 4, 384, 384)     # three query tiles per head
 
 
 def test_two_tile_rule_without_a_multiprocessor_count():
     """The number of multiprocessors is 0 where its query failed: the one-tile kernel, not a division by zero."""
-    assert not pair_pays(0, 64, 2048, 2048)
+    assert not pair_pays(0, 4, 16, 2048, 2048)
+
+
+@pytest.mark.parametrize("B,H,max_len,rows,pairs", [
+    (10, 8, 512, 153, False), (20, 4, 512, 40, False),    # small grids of short sequences: a tile has its SM to itself
+    (10, 8, 512, 307, False),                             # pairs would need a second round, tiles do not
+    (10, 8, 512, 512, True), (10, 8, 512, 700, True),     # full, and a buffer with rows to spare
+    (64, 16, 512, 102, True), (16, 16, 2048, 50, True),   # large grids of short sequences: pairs spare the empty CTAs
+    (4, 16, 2048, 409, True),
+])
+def test_two_tile_rule_sees_how_full_a_packed_batch_is(B, H, max_len, rows, pairs):
+    assert pair_pays(148, B, H, max_len, max_len)
+    assert pair_pays(148, B, H, max_len, max_len, B * rows) == pairs
