@@ -77,6 +77,12 @@ template <int D, int TN, bool BF16, bool KEYADD, bool DROP, int P_FIRST, class W
 __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
                                              const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,
                                              const TurnBegin& turn_begin, const TurnEnd& turn_end) {
+  // The look at a dead step can only succeed where every row's maximum so far is that of a live key; before the first of them (left
+  // padding) the step is done like any other at once, without a second reading and maximum (lengths U[0.05 S, 0.1 S], padding on the
+  // left: B=64 H=16 S=384 D = 64 89.7 -> 82.7 us, with dropout 130.6 -> 117.2; B=1 H=12 S=2048 D = 128 52.4 -> 47.8).
+  if constexpr (KEYADD) {
+    if (kind == kMaskDead && __any_sync(0xffffffffu, !(m_ref > kDeadMask))) kind = kMaskAny;
+  }
   // Keep decisions of this step's TN columns: Philox does not depend on the scores, so it runs
   // before they are awaited, while the tensor core is still busy with Q K^T.
   [[maybe_unused]] uint32_t keepw[DROP ? TN / 4 : 1];

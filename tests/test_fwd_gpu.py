@@ -292,3 +292,30 @@ def test_scores_of_minus_infinity_under_a_large_scale(cuda_device, B, H, S_q, S_
     ref = composite.attention_fp32(q, k, v, add_mask=None if add is None else add.reshape(B, 1, 1, S_k), scale=1.0)
     helpers.assert_close(o, ref["o"], "o")
     helpers.assert_close(lse, ref["lse"], "lse", atol=1e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("B,H,S_q,S_k,D,dtype", [
+    (3, 2, 200, 333, 64, torch.float16),      # one CTA per query tile
+    (2, 2, 130, 520, 128, torch.bfloat16),
+    (1, 2, 130, 1536, 128, torch.float16),    # keys split over a cluster: whole shares before the first live key
+    (19, 8, 256, 520, 128, torch.float16),    # two query tiles per CTA
+])
+@pytest.mark.parametrize("pad", [-10000.0, float("-inf")])
+@pytest.mark.parametrize("p_drop", [0.0, 0.1])
+def test_additive_mask_that_pads_on_the_left(cuda_device, B, H, S_q, S_k, D, dtype, pad, p_drop):
+    """Whole key steps are masked away before the first live key, and, in the second batch element, between live keys."""
+    if B > 4 and p_drop > 0:
+        B, H = 2, 2   # with dropout the kernel of one tile takes any grid, and the oracle draws on the CPU
+    q, k, v, _, _ = helpers.randn_like_config(B, H, S_q, S_k, D, dtype, seed=S_k, device=cuda_device)
+    add = torch.zeros(B, S_k)
+    for b in range(B):
+        add[b, :S_k - 130 - 7 * b] = pad
+    if B > 1:
+        add[1, :3] = 0.5
+    add = add.to(cuda_device)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    o, lse = api.fmha_forward(q, k, v, mask=add, p_drop=p_drop, seed=8, offset=3, status=status)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    ref, *_ = helpers.oracle_forward(q, k, v, add_mask=add, p_drop=p_drop, seed=8, offset=3)
+    helpers.assert_close(o, ref["o"], "o", dtype)
+    helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
