@@ -110,6 +110,10 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   // the scores are read a second time, 32 columns at a time (held, they spilled more and cost 57.2 against 55.7 us at B=32
   // H=12 S=512).
   constexpr bool HOLD = !DROP;
+  // Mask and dropout, D = 128: the scores with the mask added go back to tensor memory for the second reading, which needs neither the mask
+  // nor the choice then (a mask that is nowhere zero, B=32 H=16 S=512 145.7 -> 137.0 us, S_q=102 S_k=449 18.5 -> 15.3; right padding 126.5 ->
+  // 121.3; at D = 64, four CTAs per SM, the stores cost more than they spare: S=1024 188.8 -> 191.0).
+  constexpr bool REWRITE = KEYADD && DROP && D == 128;
   const float mul = KEYADD && kind == kMaskAny ? 1.0f : sl2;   // what takes a score as held to the log2 domain
   auto finish_scores = [&](int c, uint32_t (&v)[32]) {   // mask added, keys past the end to -inf (exp2 makes them zero)
     if (KEYADD && kind == kMaskAny) {
@@ -133,14 +137,20 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   };
   uint32_t sv[TN / 32][32];
   // The maximum of 32 columns is taken while the next 32 are on their way (D = 128: B=16 H=16 S=1024 163.1 -> 161.6 us, S=512
-  // with dropout 57.5 -> 56.1; with an additive mask B=64 H=16 S=384 D = 64 67.6 -> 66.7).
+  // with dropout 57.5 -> 56.1; with an additive mask B=64 H=16 S=384 D = 64 67.6 -> 66.7).  Not with mask and dropout at D = 64, where the
+  // 96 registers hold one 32 columns beside the keep words (76 -> 24 bytes of spill stores; lengths U[0.4 S, S], B=16 H=16 S=1024 143 -> 130 us,
+  // a mask that is nowhere zero 188.6 -> 170.6).
+  constexpr bool AHEAD = !(KEYADD && DROP && D == 64);
   tmem_ld32(tS, sv[0]);
   tmem_wait_ld_dep(sv[0]);
   float tile_max = kNoScore;
 #pragma unroll
   for (int c = 0; c < TN / 32; ++c) {
-    if (c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
+    if (AHEAD && c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
     finish_scores(c, sv[c]);
+    if constexpr (REWRITE) {
+      if (kind == kMaskAny || n_cols < TN) tmem_st32(tS + c * 32, sv[c]);
+    }
     auto v = [&](int k) { return __uint_as_float(sv[c][k]); };
     // with an additive mask a NaN has to show in the maximum, or the shortcut below would step over it
     auto max3 = [](float x, float y, float z) { return fmax3<KEYADD>(x, y, z); };
@@ -152,7 +162,10 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       m1 = max3(m1, v(k + 2), v(k + 3));
     }
     tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
-    if (c + 1 < TN / 32) tmem_wait_ld_dep(sv[c + 1]);
+    if (c + 1 < TN / 32) {
+      if (!AHEAD) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
+      tmem_wait_ld_dep(sv[c + 1]);
+    }
   }
   tile_max = fmax3<KEYADD>(tile_max * mul, kNoScore, kNoScore);   // scale > 0: the maximum commutes with it; the floor may have passed the range
   // A step whose keys are all masked away (the padded end of a sequence): when every score of it lies so far below
@@ -216,17 +229,18 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
     }
   } else {
     uint32_t ra[32], rb[32], packed[16];   // chunk c+1 (then c+2) is in flight while chunk c (c+1) is processed
+    if constexpr (REWRITE) tmem_wait_st();
     tmem_ld32(tS, ra);
 #pragma unroll
     for (int c = 0; c < TN / 32; c += 2) {
       tmem_wait_ld_dep(ra);
-      finish_scores(c, ra);
+      if constexpr (!REWRITE) finish_scores(c, ra);
       tmem_ld32(tS + (c + 1) * 32, rb);
       softmax_chunk<BF16, DROP>(ra, mul, -m_ref, sum2, packed, keepw + (DROP ? c * 8 : 0));
       tmem_st16(tS + c * 16, packed);
       hand_over(c);
       tmem_wait_ld_dep(rb);
-      finish_scores(c + 1, rb);
+      if constexpr (!REWRITE) finish_scores(c + 1, rb);
       if (c + 2 < TN / 32) tmem_ld32(tS + (c + 2) * 32, ra);
       softmax_chunk<BF16, DROP>(rb, mul, -m_ref, sum2, packed, keepw + (DROP ? c * 8 + 8 : 0));
       tmem_st16(tS + c * 16 + 16, packed);
