@@ -141,12 +141,17 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   // 96 registers hold one 32 columns beside the keep words (76 -> 24 bytes of spill stores; lengths U[0.4 S, S], B=16 H=16 S=1024 143 -> 130 us,
   // a mask that is nowhere zero 188.6 -> 170.6).
   constexpr bool AHEAD = !(KEYADD && DROP && D == 64);
-  tmem_ld32(tS, sv[0]);
-  tmem_wait_ld_dep(sv[0]);
+  // All at once with a mask and the scores held at D = 128 in 168 registers (a mask that is nowhere zero, B=5 H=8 S=528 18.9 -> 18.1 us, B=2 H=12
+  // S=1331 35.4 -> 34.1); the kernel of two tiles per CTA has 216 and is faster without (B=16 H=16 S=2048 475 / 493).
+  constexpr bool ALL = KEYADD && HOLD && D == 128 && P_FIRST == 0;
+#pragma unroll
+  for (int c = 0; c < (ALL ? TN / 32 : 1); ++c) tmem_ld32(tS + c * 32, sv[c]);
+#pragma unroll
+  for (int c = 0; c < (ALL ? TN / 32 : 1); ++c) tmem_wait_ld_dep(sv[c]);
   float tile_max = kNoScore;
 #pragma unroll
   for (int c = 0; c < TN / 32; ++c) {
-    if (AHEAD && c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
+    if (AHEAD && !ALL && c + 1 < TN / 32) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
     finish_scores(c, sv[c]);
     if constexpr (REWRITE) {
       if (kind == kMaskAny || n_cols < TN) tmem_st32(tS + c * 32, sv[c]);
@@ -162,7 +167,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       m1 = max3(m1, v(k + 2), v(k + 3));
     }
     tile_max = max3(tile_max, max3(m0, m1, v(30)), v(31));
-    if (c + 1 < TN / 32) {
+    if (!ALL && c + 1 < TN / 32) {
       if (!AHEAD) tmem_ld32(tS + (c + 1) * 32, sv[c + 1]);
       tmem_wait_ld_dep(sv[c + 1]);
     }
