@@ -520,18 +520,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
   }
 }
 
-// Grids of at least two query tiles per SM (one round of the other kernel's capacity), no dropout, three or more key steps:
+// No dropout, three or more key steps, and grids of at least two query tiles per SM, one round of the other kernel's capacity:
 // at one or two steps a CTA's life is its start and its end (S_q=256: S_k=128 12.8 / 12.2 us, S_k=256 16.2 / 16.0, S_k=1024 39.0 /
 // 40.2).  A head with an odd number of tiles leaves half a CTA idle for one item, which takes nearly as long as a whole one: the
 // rounds of pairs over the SMs may be at most 8/7 of the rounds of tiles (H=16: S=384 B=16 34.4 / 33.0 us at 4/3, S=640 68.2 / 69.3 at
 // 6/5, B=8 S=1152 94.1 / 90.1 at 5/4).  Of three tiles a third is lost, more than the rounds show: one tile per CTA (S=384 H=4
 // B=50 1.06, with lengths U[S/2, S] 1.20, H=12 B=9 1.11 times its time in pairs).
+// One round: where each pair has an SM of its own and single tiles would have to share some, and all are of one length of 1 024 keys or more
+// (S=1024 H=12 B=2 20.9 us one tile per CTA / 20.3, S=2048 36.8 / 34.6, S=2565 46.7 / 44.2; an additive mask, S=1536 H=16 37.3 / 32.2; with
+// lengths U[0.3 S, S] S=1024 19.3 / 20.3).
 // Packed batch: only total_rows tells how full it is.  A sequence below the maximum leaves the other kernel with CTAs that start for
 // nothing (B=64 H=16, maximum 512, 102 rows each: 36.4 us in pairs / 48.9), so two tiles per CTA stay the choice for most of them, except on
 // small grids: with no more than 1.2 tiles of the average length per SM, pairing takes from the tiles the SM of their own (H=8
 // B=10, maximum 512, 153 rows each: 10.7 / 9.7; H=4 B=6, 2048, 165 rows: 10.2 / 9.2), and just above two tiles per SM by the maximum the rounds count
 // that the average length makes (H=8 B=10, 512, 307 rows: 160 pairs take two rounds, 240 tiles one, 18.0 / 11.9).
-bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, int64_t packed_rows) {
+bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, bool lengths, int64_t packed_rows) {
   if (sms <= 0 || S_k <= 256) return false;   // no multiprocessors: the query for their number has failed
   const int64_t heads = B * H;
   auto tiles = [](int64_t rows) { return (rows + kTileM - 1) / kTileM; };
@@ -540,7 +543,9 @@ bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, 
     return 7 * pair_rounds <= 8 * tile_rounds;
   };
   const int64_t n = tiles(S_q);
-  if (n == 3 || heads * n < 2 * sms || !even_rounds(n)) return false;
+  if (n == 3) return false;
+  if (!lengths && S_k >= 1024 && heads * n > sms && heads * ((n + 1) / 2) <= sms) return true;
+  if (heads * n < 2 * sms || !even_rounds(n)) return false;
   if (packed_rows > 0) {
     const int64_t n_avg = tiles(std::min(S_q, (packed_rows + B - 1) / B));
     if (heads * n <= 3 * sms && 5 * heads * n_avg <= 6 * sms) return false;
@@ -550,7 +555,8 @@ bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, 
 }
 bool fwd_pair_applies(const FwdArgs& a, int head_dim) {
   if (head_dim != D || a.dropout_kind == FMHA_DROPOUT_PHILOX) return false;
-  return fwd_pair_pays(sm_count(), a.B, a.H, a.S_q, a.S_k, a.mask_kind == FMHA_MASK_CU_SEQLENS ? a.total_rows : 0);
+  const bool packed = a.mask_kind == FMHA_MASK_CU_SEQLENS;
+  return fwd_pair_pays(sm_count(), a.B, a.H, a.S_q, a.S_k, packed || a.mask_kind == FMHA_MASK_SEQLEN, packed ? a.total_rows : 0);
 }
 
 template <bool BF16, bool KEYADD, bool PACKED>

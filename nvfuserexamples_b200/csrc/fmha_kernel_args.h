@@ -125,8 +125,8 @@ int launch_fwd(const FwdArgs& a, int D, int dtype, bool legacy, bool p_via_smem,
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream);
 // the same for grids that fill the chip: two query tiles per CTA, persistent (fmha_fwd_pair_sm100.cu)
 bool fwd_pair_applies(const FwdArgs& a, int D);
-// its rule on sizes, on a device of `sms` multiprocessors (packed_rows: rows of a packed batch, else 0)
-bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, int64_t packed_rows);
+// its rule on sizes, on a device of `sms` multiprocessors (lengths: sequences may differ; packed_rows: rows of a packed batch, else 0)
+bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, bool lengths, int64_t packed_rows);
 int launch_fwd_pair(const FwdArgs& a, int dtype, cudaStream_t stream);
 // the kernel for a handful of query rows per head (fmha_fwd_rows_sm100.cu): compact masks, not packed
 bool fwd_rows_applies(int S_q, int S_k, int D, int64_t heads, bool dropout);

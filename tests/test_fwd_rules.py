@@ -6,10 +6,10 @@ import pytest
 from nvfuserexamples_b200 import capi
 
 
-def pair_pays(sms, B, H, S_q, S_k, packed_rows=0):
-    fn = capi.load()["_ZN4fmha13fwd_pair_paysEllllll"]   # fmha::fwd_pair_pays(int64_t x 6)
-    fn.argtypes, fn.restype = [C.c_int64] * 6, C.c_bool
-    return fn(sms, B, H, S_q, S_k, packed_rows)
+def pair_pays(sms, B, H, S_q, S_k, packed_rows=0, lengths=True):
+    fn = capi.load()["_ZN4fmha13fwd_pair_paysElllllbl"]   # fmha::fwd_pair_pays(int64_t x 5, bool, int64_t)
+    fn.argtypes, fn.restype = [C.c_int64] * 5 + [C.c_bool, C.c_int64], C.c_bool
+    return fn(sms, B, H, S_q, S_k, lengths, packed_rows)
 
 
 def test_two_tile_rule():
@@ -34,3 +34,12 @@ def test_two_tile_rule_without_a_multiprocessor_count():
 def test_two_tile_rule_sees_how_full_a_packed_batch_is(B, H, max_len, rows, pairs):
     assert pair_pays(148, B, H, max_len, max_len)
     assert pair_pays(148, B, H, max_len, max_len, B * rows) == pairs
+
+
+def test_two_tile_rule_on_one_round():
+    """Pairs that have a multiprocessor each, of long keys and one length; with a pair too many, shorter keys or lengths it is not taken."""
+    assert pair_pays(148, 1, 16, 2048, 2048, lengths=False)        # 256 tiles, 128 pairs
+    assert not pair_pays(148, 1, 16, 2048, 2048, lengths=True)
+    assert not pair_pays(148, 2, 16, 1024, 1023, lengths=False)
+    assert not pair_pays(148, 1, 8, 2048, 2048, lengths=False)     # 128 tiles: each has one of its own
+    assert not pair_pays(148, 1, 15, 2432, 2432, lengths=False)    # 150 pairs
