@@ -157,9 +157,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     const int* cu = reinterpret_cast<const int*>(a.mask);
     row_base = cu[b];
     const int all = cu[b + 1] - row_base;
-    const int len = min(all, a.S_q);   // a sequence longer than the stated maximum is cut there
+    const int len = row_base < 0 ? 0 : min(all, a.S_q);   // a sequence longer than the stated maximum is cut there
     k_limit = len;
-    q_limit = len;
+    q_limit = min(len, a.total_rows - row_base);   // offsets past the tensor, which the host cannot see: no row behind it is written
     tb = 0;
     if (q0 >= len) {   // this sequence has no such query tile (whole CTA, before any barrier)
       if (a.zero_uncovered)

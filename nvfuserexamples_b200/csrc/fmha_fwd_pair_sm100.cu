@@ -249,7 +249,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
       } else if (PACKED) {
         const int* cu = reinterpret_cast<const int*>(a.mask);
         it.row_base = cu[b];
-        it.k_limit = it.q_limit = min(cu[b + 1] - it.row_base, a.S_q);   // a sequence longer than the stated maximum is cut there
+        it.k_limit = it.row_base < 0 ? 0 : min(cu[b + 1] - it.row_base, a.S_q);   // a sequence longer than the stated maximum is cut there
+        it.q_limit = min(it.k_limit, a.total_rows - it.row_base);   // offsets past the tensor, which the host cannot see: no row behind it
       }
       const int rows = it.q_limit - it.q0;
       it.tiles = rows <= 0 ? 0 : rows <= kTileM ? 1 : 2;

@@ -2,6 +2,8 @@
 
 The reference lists padded / irregular shapes as open work (fmha/fmha_manual.cpp:110, :178 of
 shmsong/NvFuserExamples); here a batch is one [total_rows, H, D] tensor per operand plus row offsets."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -336,3 +338,36 @@ def test_uncovered_rows_are_zeroed_inside_the_tensor_only(cuda_device, D):
                     out=tuple(t[:total] for t in outs[1:]), flags=capi.FLAG_ZERO_UNCOVERED)
     for t in outs:
         assert (t[total:] == 7.0).all() and (t[164:total] == 0).all() and (t[64:100] == 0).all() and torch.isfinite(t).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H", [(3, 2), (60, 8)])   # one CTA per query tile; at D = 128 two
+def test_forward_writes_inside_the_tensor_only(cuda_device, B, H, D):
+    """Offsets that reach past the tensor, which the host cannot see: neither O nor logsumexp is written behind its end.  (The tensors are the
+    first rows of larger buffers.)  The rows of the other sequences, and those of the one that is cut, are as they should be."""
+    max_len, spare = 400, 900
+    lens = [300] * (B - 2) + [400, 400]
+    cu_list = [0]
+    for n in lens:
+        cu_list.append(cu_list[-1] + n)
+    total = cu_list[-2] - 260   # the last but one ends 260 rows past the tensor, the last one begins there
+    cu = torch.tensor(cu_list, dtype=torch.int32, device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(7)
+    q, k, v = (torch.randn(total, H, D, device=cuda_device, generator=g).half() for _ in range(3))
+    o = torch.full((total + spare, H, D), 7.0, dtype=torch.half, device=cuda_device)
+    lse = torch.full((H * total + spare,), 7.0, device=cuda_device)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    p = capi.FwdParams()
+    p.struct_bytes, p.dtype = C.sizeof(capi.FwdParams), capi.DTYPE_F16
+    p.B, p.H, p.S_q, p.S_k, p.D, p.scale, p.total_rows = B, H, max_len, max_len, D, D ** -0.5, total
+    p.q, p.k, p.v, p.o = (capi.Tensor4(t.data_ptr(), 0, D, H * D) for t in (q, k, v, o))
+    p.lse, p.mask_kind, p.mask, p.status = lse.data_ptr(), capi.MASK_CU_SEQLENS, cu.data_ptr(), status.data_ptr()
+    assert capi.load().fmha_sm100_fwd(C.byref(p), torch.cuda.current_stream().cuda_stream) == capi.FMHA_OK
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    assert (o[total:] == 7.0).all() and (lse[H * total:] == 7.0).all()
+    for b in (0, B - 3, B - 2):
+        r0, rows = cu_list[b], min(lens[b], total - cu_list[b])
+        qb, kb, vb = (torch.nn.functional.pad(x[r0:r0 + rows], (0, 0, 0, 0, 0, lens[b] - rows)).permute(1, 0, 2) for x in (q, k, v))
+        ref = helpers.composite.attention_fp32(qb, kb, vb)
+        helpers.assert_close(o[r0:r0 + rows].permute(1, 0, 2), ref["o"][:, :rows], f"o of {b}")
+        helpers.assert_close(lse[:H * total].view(H, total)[:, r0:r0 + rows], ref["lse"][:, :rows], f"lse of {b}", atol=1e-3, rtol=1e-4)
