@@ -477,17 +477,20 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
         tc_fence_after_sync();
         it = read_item(n);   // again, instead of in registers through the key steps
         q_row = it.q0 + g * kTileM + row;
-        const bool row_ok = q_row < it.q_limit;
-        const float l_sum = sum2.x + sum2.y;
-        if (a.lse != nullptr && row_ok) {
-          const size_t li = PACKED ? static_cast<size_t>(it.h) * a.total_rows + it.row_base + q_row   // [H, total_rows]
-                                   : static_cast<size_t>(it.b * a.H + it.h) * a.S_q + q_row;          // [B*H, S_q]
-          a.lse[li] = (m_ref + fast_log2(l_sum)) * kLn2F;
+        // After a given-up wait tensor memory holds anything; and the item is this one only if none had been given up when it was read.
+        if (!__any_sync(0xffffffffu, *abort_flag != 0)) {
+          const bool row_ok = q_row < it.q_limit;
+          const float l_sum = sum2.x + sum2.y;
+          if (a.lse != nullptr && row_ok) {
+            const size_t li = PACKED ? static_cast<size_t>(it.h) * a.total_rows + it.row_base + q_row   // [H, total_rows]
+                                     : static_cast<size_t>(it.b * a.H + it.h) * a.S_q + q_row;          // [B*H, S_q]
+            a.lse[li] = (m_ref + fast_log2(l_sum)) * kLn2F;
+          }
+          unsigned short* o_rows = reinterpret_cast<unsigned short*>(a.o_ptr) + static_cast<int64_t>(it.h) * a.o_sh +
+                                   (PACKED ? 0 : it.b * a.o_sb) + static_cast<int64_t>(it.row_base + it.q0 + g * kTileM + quad * 32) * a.o_ss;
+          o_warp_out<BF16>(tO, 1.0f / l_sum, smem_u32(sO) + (warp - 4) * 4096, o_rows, a.o_ss,
+                           it.q_limit - (it.q0 + g * kTileM + quad * 32), lane);
         }
-        unsigned short* o_rows = reinterpret_cast<unsigned short*>(a.o_ptr) + static_cast<int64_t>(it.h) * a.o_sh +
-                                 (PACKED ? 0 : it.b * a.o_sb) + static_cast<int64_t>(it.row_base + it.q0 + g * kTileM + quad * 32) * a.o_ss;
-        o_warp_out<BF16>(tO, 1.0f / l_sum, smem_u32(sO) + (warp - 4) * 4096, o_rows, a.o_ss,
-                         it.q_limit - (it.q0 + g * kTileM + quad * 32), lane);
         tc_fence_before_sync();
       } else if constexpr (KEYADD) {   // the other tile has work, this one does not exist: only keep the mask ring going
         for (int k0 = 0; k0 < it.k_limit; k0 += TN, ++t) {
