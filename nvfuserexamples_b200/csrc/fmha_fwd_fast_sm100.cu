@@ -75,7 +75,7 @@ struct FastSmem {
   static constexpr int kOffV = kOffK + kStages * kTileBytes;
   static constexpr int kOffMask = kOffV + kStages * kTileBytes;  // TN floats per softmax warp
   static constexpr int kOffBar = kOffMask + 4 * TN * 4;
-  static constexpr int kNumBars = 4 + 4 * kStages;
+  static constexpr int kNumBars = 4 + (D == 64 ? 2 : 4) * kStages;   // at D = 64 no buffer has a barrier for being empty
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;
   static constexpr int kBytes = kOffMisc + 16;
   static constexpr int kDynBytes = kBytes + 1024;
@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
   uint64_t* p_full = bars + 2;
   uint64_t* o_full = bars + 3;
   uint64_t* k_full = bars + 4;
-  uint64_t* k_empty = k_full + ST;
-  uint64_t* v_full = k_empty + ST;
-  uint64_t* v_empty = v_full + ST;
+  uint64_t* v_full = k_full + ST;
+  uint64_t* k_empty = v_full + ST;   // D = 128 only
+  uint64_t* v_empty = k_empty + ST;
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 4);
   // Philox offset of this launch: the launch parameter plus the optional device-resident value.  Kept in shared
@@ -183,9 +183,11 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     mbar_init(o_full, 1);
     for (int s = 0; s < ST; ++s) {
       mbar_init(k_full + s, 1);
-      mbar_init(k_empty + s, 1);
       mbar_init(v_full + s, 1);
-      mbar_init(v_empty + s, 1);
+      if constexpr (!MERGED) {
+        mbar_init(k_empty + s, 1);
+        mbar_init(v_empty + s, 1);
+      }
     }
     mbar_fence_init();
     fence_proxy_async_smem();

@@ -140,9 +140,6 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
-__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 // Barrier that also ORs a predicate over its participants: every one of them gets the same answer, which a
 // flag read by each thread on its own cannot promise (used for "has any wait of this CTA been given up?",
 // where threads that disagree would leave each other alone at the next barrier).
