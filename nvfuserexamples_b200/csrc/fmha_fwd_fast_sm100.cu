@@ -16,9 +16,10 @@
 //     sum one packed add;
 //   * without dropout the scores of a step are read from tensor memory once and held in registers between the maximum and
 //     the exponentials; with dropout, whose keep words need registers as well, they are read twice, the load of the next 32
-//     columns in flight while the current 32 are processed;
+//     columns in flight while the current 32 are processed (exceptions with an additive mask: softmax_step);
 //   * with an additive key mask a step whose mask is zero throughout is done like one without a mask, and one whose keys are all
-//     masked away, and would add exact zeros, writes zeros for P (B=64 H=16 S=384, lengths U[S/3, S] as a mask: 76.3 -> 65.2 us);
+//     masked away, and would add exact zeros, writes zeros for P (B=64 H=16 S=384, lengths U[S/3, S] as a mask: 76.3 -> 65.2 us together with the early loads
+//     below);
 //     each softmax warp reads the mask for itself, under the wait for the scores;
 //   * few CTAs against many keys: the key steps of a query tile are dealt out over a cluster (fwd_key_split); many CTAs of
 //     unequal length: the longest sequences first (length_class_shift);
@@ -47,8 +48,8 @@ namespace {
 // D = 128: 192 threads (TMA producer warp, MMA warp, four softmax warps).  D = 64: 160 threads, one warp issues both
 // the TMA loads and the MMAs.  Registers are allocated per SM sub-partition (16 384 each, warps dealt round-robin):
 // four CTAs of six warps put six warps on a sub-partition (80 registers per thread), four CTAs of five warps put
-// five (96), where the plain variant stays out of local memory, dropout spills 16 to 20 bytes, the additive mask 32 to 36 and both
-// 68 to 76 (spill stores; D = 128 at 168 registers: plain 40 to 48, dropout 52 to 76, additive 140 to 148, both 116 to 120).
+// five (96), where the plain variant stays out of local memory, dropout spills 4 to 24 bytes, the additive mask 32 to 36 and both
+// 24 to 28 (spill stores; D = 128 at 168 registers: plain 44 to 48, dropout 52 to 76, additive 140 to 148, both 116 to 120).
 constexpr int kThreadsSplit = 192, kThreadsMerged = 160;
 template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged : kThreadsSplit; }
 constexpr int kMaxKeySplit = 8;   // portable cluster size
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
     mbar_fence_init();
     fence_proxy_async_smem();
     // The first product's operands, by the thread that has set up their barriers: the rest of the set-up, tensor memory above all,
-    // takes as long as they do (some 1 000 of a CTA's first 3 500 cycles; B=13 H=12 S=197 10.1 -> 9.2 us, B=64 H=16 S=128 12.6 ->
+    // takes as long as they do (some 1 000 of a CTA's first 3 500 cycles; back to back in a graph, B=13 H=12 S=197 10.1 -> 9.2 us, B=64 H=16 S=128 12.6 ->
     // 11.9, B=32 H=12 S=512 with dropout 51.4 -> 50.4).
     mbar_arrive_expect_tx(q_full, L::kQBytes);
 #pragma unroll

@@ -1,4 +1,4 @@
-// fmha_fwd_pair_sm100.cu — forward kernel of head dimension 128 for grids that fill the chip: compact masks (none, valid lengths,
+// fmha_fwd_pair_sm100.cu — forward kernel of head dimension 128 for grids that fill the chip (fwd_pair_pays): compact masks (none, valid lengths,
 // additive [B,S_k] row, packed batch), no dropout, O and the row logsumexp.
 //
 // A CTA, one per SM, works on TWO 128-row query tiles of a head at once, which share the K and V tiles it loads, and goes on to the
