@@ -48,8 +48,8 @@ namespace {
 // D = 128: 192 threads (TMA producer warp, MMA warp, four softmax warps).  D = 64: 160 threads, one warp issues both
 // the TMA loads and the MMAs.  Registers are allocated per SM sub-partition (16 384 each, warps dealt round-robin):
 // four CTAs of six warps put six warps on a sub-partition (80 registers per thread), four CTAs of five warps put
-// five (96), where the plain variant stays out of local memory, dropout spills 4 to 24 bytes, the additive mask 32 to 36 and both
-// 24 to 28 (spill stores; D = 128 at 168 registers: plain 44 to 48, dropout 52 to 76, additive 140 to 148, both 116 to 120).
+// five (96), where the plain variant and dropout stay out of local memory (4 bytes with a cluster), the additive mask spills 32 to 36
+// bytes and both 24 to 28 (spill stores; D = 128 at 168 registers: plain 44 to 48, dropout 52 to 76, additive 140 to 148, both 116 to 120).
 constexpr int kThreadsSplit = 192, kThreadsMerged = 160;
 template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged : kThreadsSplit; }
 constexpr int kMaxKeySplit = 8;   // portable cluster size
@@ -422,7 +422,10 @@ __global__ void __launch_bounds__(fast_threads<D>(), FastSmem<D, DROP>::kCtasPer
       }
       auto wait_s = [&]() { mbar_wait(s_full, j & 1, wctx, kFSFull, 32); };
       auto arrive = [&](int) { arrive_p(); };
-      softmax_step<D, TN, BF16, KEYADD, DROP, 0>(tS, tO, col0, n_cols, sl2, mask_stage, kind, drop_row, m_ref, sum2, wait_s, arrive, [] {}, [] {});
+      if constexpr (D == 64)
+        softmax_step_64<BF16, KEYADD, DROP>(tS, tO, col0, n_cols, sl2, mask_stage, kind, drop_row, m_ref, sum2, wait_s, arrive);
+      else
+        softmax_step<D, TN, BF16, KEYADD, DROP, 0, 0, 0>(tS, tO, col0, n_cols, sl2, mask_stage, kind, drop_row, m_ref, sum2, wait_s, arrive, [] {}, [] {});
     }
 
     // ---- epilogue ------------------------------------------------------------------------

@@ -73,7 +73,8 @@ struct DropRow {
 // holds in the log2 domain unless it is zero.  wait_s returns when the scores are there; arrive_p(1) hands P to the
 // tensor core, or, with P_FIRST > 0, arrive_p(0) its first P_FIRST chunks of 32 columns and arrive_p(1) the rest.  The exponentials
 // lie between turn_begin and turn_end.
-template <int D, int TN, bool BF16, bool KEYADD, bool DROP, int P_FIRST, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
+// FROM: at least so many columns exist.  PAD: P of as many further columns is zero.
+template <int D, int TN, bool BF16, bool KEYADD, bool DROP, int P_FIRST, int FROM, int PAD, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
 __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
                                              const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,
                                              const TurnBegin& turn_begin, const TurnEnd& turn_end) {
@@ -129,7 +130,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
         v[4 * k + 3] = __float_as_uint(t1.y);
       }
     }
-    if (n_cols < TN) {
+    if (c * 32 + 32 > FROM && n_cols < TN) {
 #pragma unroll
       for (int k = 0; k < 32; ++k)
         if (c * 32 + k >= n_cols) v[k] = __float_as_uint(-INFINITY);
@@ -182,7 +183,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       turn_end();
       const uint32_t zero[16] = {};
 #pragma unroll
-      for (int c = 0; c < TN / 32; ++c) tmem_st16(tS + c * 16, zero);
+      for (int c = 0; c < (TN + PAD) / 32; ++c) tmem_st16(tS + c * 16, zero);
       tmem_wait_st();
       tc_fence_before_sync();
       if (P_FIRST > 0) arrive_p(0);
@@ -232,6 +233,10 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       tmem_st16(tS + c * 16, packed);
       hand_over(c);
     }
+  } else if constexpr (TN == 32) {
+    uint32_t packed[16];
+    softmax_chunk<BF16, DROP>(sv[0], mul, -m_ref, sum2, packed, keepw);
+    tmem_st16(tS, packed);
   } else {
     uint32_t ra[32], rb[32], packed[16];   // chunk c+1 (then c+2) is in flight while chunk c (c+1) is processed
     if constexpr (REWRITE) tmem_wait_st();
@@ -252,10 +257,29 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
       hand_over(c + 1);
     }
   }
+  if constexpr (PAD > 0) {
+    const uint32_t zero[16] = {};
+#pragma unroll
+    for (int c = TN / 32; c < (TN + PAD) / 32; ++c) tmem_st16(tS + c * 16, zero);
+  }
   turn_end();
   tmem_wait_st();
   tc_fence_before_sync();
   arrive_p(1);
+}
+
+// A 64-key step at head dimension 64.  The last one of a tile may have 32 keys or fewer (one in two, where lengths are spread): then
+// only its first half is read, drawn for and exponentiated, and a longer one looks for keys past the end in its second half alone
+// (B=32 H=12 S=512 with dropout, lengths U[256, 512] 53.3 -> 49.4 us, B=16 H=8 S=160 8.6 -> 7.4, B=13 H=12 S=197 without 9.2 -> 8.8).  Not with an
+// additive mask, which has such a step only where S_k is no multiple of 64, and registers to spare for a second copy nowhere (B=64 H=16 S=384
+// 65.8 -> 67.7).
+template <bool BF16, bool KEYADD, bool DROP, class WaitS, class ArriveP>
+__device__ __forceinline__ void softmax_step_64(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
+                                                const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p) {
+  auto none = [] {};
+  if constexpr (KEYADD) softmax_step<64, 64, BF16, KEYADD, DROP, 0, 0, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, none, none);
+  else if (n_cols > 32) softmax_step<64, 64, BF16, KEYADD, DROP, 0, 32, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, none, none);
+  else softmax_step<64, 32, BF16, KEYADD, DROP, 0, 0, 32>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, none, none);
 }
 
 // O of a finished query tile out of tensor memory, scaled and rounded: into `tile` (shared memory, 128 rows in the swizzled

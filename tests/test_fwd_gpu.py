@@ -319,3 +319,23 @@ def test_additive_mask_that_pads_on_the_left(cuda_device, B, H, S_q, S_k, D, dty
     ref, *_ = helpers.oracle_forward(q, k, v, add_mask=add, p_drop=p_drop, seed=8, offset=3)
     helpers.assert_close(o, ref["o"], "o", dtype)
     helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("p", [0.0, 0.2])
+@pytest.mark.parametrize("mask", ["none", "seqlen", "key"])
+@pytest.mark.parametrize("S_k", [31, 32, 33, 63, 65, 95, 96, 97])
+def test_last_key_step_around_half_a_step(cuda_device, S_k, mask, p):
+    """Head dimension 64: a last step of up to 32 keys is done by halves; lengths around it, and whole steps past a length."""
+    B, H, S_q, dtype = 4, 2, 130, torch.float16
+    q, k, v, _, _ = helpers.randn_like_config(B, H, S_q, S_k, 64, dtype, seed=S_k, device=cuda_device)
+    lens = torch.tensor([S_k, max(1, S_k - 1), max(1, S_k - 31), max(1, S_k - 33)], dtype=torch.int32, device=cuda_device)
+    kw, okw = {}, {}
+    if mask == "seqlen":
+        kw["seqlens"], okw["lens"] = lens, lens
+    elif mask == "key":
+        add = composite.padding_add_mask(lens.cpu(), S_k).reshape(B, S_k).to(cuda_device)
+        kw["mask"], okw["add_mask"] = add, add
+    o, lse = api.fmha_forward(q, k, v, p_drop=p, seed=4, offset=9, **kw)
+    ref, *_ = helpers.oracle_forward(q, k, v, p_drop=p, seed=4, offset=9, **okw)
+    helpers.assert_close(o, ref["o"], "o", dtype)
+    helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
