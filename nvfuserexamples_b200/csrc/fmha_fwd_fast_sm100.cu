@@ -580,7 +580,7 @@ static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, bool long_step
 // 35.2 -> 33.3, B=32 H=12 S=512 with dropout 57.0 -> 54.2); beyond it does not (B=64 H=16 S=384 62.3 -> 64.9 us, with two
 // elements per lane), nor at D = 128, where a CTA's start is the longer chain (B=16 H=12 S=512 37.1 -> 38.4 us), and with no
 // more CTAs than SMs the order does not matter.
-static int length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_lengths) {
+int fwd_length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_lengths) {
   const int64_t sms = sm_count();
   if (no_lengths || D != 64 || (a.mask_kind != FMHA_MASK_SEQLEN && a.mask_kind != FMHA_MASK_CU_SEQLENS) || a.B < 2 ||
       a.B > kMaxOrdered || ctas <= sms || ctas > 4 * FastSmem<64>::kCtasPerSm * sms)
@@ -609,13 +609,14 @@ static int launch_fast_impl(const FwdArgs& a, cudaStream_t stream, int n_split =
   }
   dim3 grid((a.S_q + kTileM - 1) / kTileM * n_split, a.H, a.B);
   FwdArgs args = a;
-  args.length_class_shift = length_class_shift(a, D, static_cast<int64_t>(grid.x) * grid.y * grid.z, KEYADD || SPLIT);
+  args.length_class_shift = fwd_length_class_shift(a, D, static_cast<int64_t>(grid.x) * grid.y * grid.z, KEYADD || SPLIT);
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(fast_threads<D>()), L::kDynBytes, stream, args, SPLIT ? n_split : 0);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 int launch_fwd_fast(const FwdArgs& a, int D, int dtype, cudaStream_t stream) {
   if (fwd_pair_applies(a, D)) return launch_fwd_pair(a, dtype, stream);
+  if (fwd_chain_applies(a, D)) return launch_fwd_chain(a, dtype, stream);
   const bool bf = dtype == FMHA_DTYPE_BF16;
   const bool keyadd = a.mask_kind == FMHA_MASK_KEY_ADDITIVE;
   const bool drop = a.dropout_kind == FMHA_DROPOUT_PHILOX;

@@ -128,6 +128,13 @@ bool fwd_pair_applies(const FwdArgs& a, int D);
 // its rule on sizes, on a device of `sms` multiprocessors (lengths: sequences may differ; packed_rows: rows of a packed batch, else 0)
 bool fwd_pair_pays(int64_t sms, int64_t B, int64_t H, int64_t S_q, int64_t S_k, bool lengths, int64_t packed_rows);
 int launch_fwd_pair(const FwdArgs& a, int dtype, cudaStream_t stream);
+// the one-tile kernel's choice of order: a shift that puts the lengths into classes, or -1
+int fwd_length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_lengths);
+// the same at head dimension 64 for grids of more tiles than the chip holds: a CTA takes one tile after the other (fmha_fwd_chain_sm100.cu)
+bool fwd_chain_applies(const FwdArgs& a, int D);
+// its rule on sizes, on a device of `sms` multiprocessors
+bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool dropout);
+int launch_fwd_chain(const FwdArgs& a, int dtype, cudaStream_t stream);
 // the kernel for a handful of query rows per head (fmha_fwd_rows_sm100.cu): compact masks, not packed
 bool fwd_rows_applies(int S_q, int S_k, int D, int64_t heads, bool dropout);
 int launch_fwd_rows(const FwdArgs& a, int D, int dtype, cudaStream_t stream);

@@ -1,0 +1,66 @@
+"""The forward kernel whose CTAs go from query tile to query tile (head dimension 64, large grids) against the kernel of one tile per
+CTA, bit for bit, on the same batch in pieces too small for it, and against the fp32 composite: one key step and several, last
+steps of up to and more than half a step, ragged query tiles, each mask kind, dropout.  Tolerances: helpers.assert_close."""
+import pytest
+import torch
+
+import mha_manual  # noqa: F401  registers torch.ops.mha_manual.*
+from nvfuserexamples_b200 import api, capi
+from oracle import composite
+from tests import helpers
+from tests.test_fwd_rules import chain_pays
+
+pytestmark = pytest.mark.gpu
+
+B, H, PIECE = 75, 12, 15   # two query tiles per head: 1 800 tiles; 360 in a piece, where the keys of a tile are not split over a cluster either
+
+
+def batch(S_q, S_k, dtype, kind, dev):
+    g = torch.Generator(device=dev).manual_seed(S_q + S_k)
+    q, k, v = (torch.randn(B, H, S, 64, device=dev, generator=g).to(dtype) for S in (S_q, S_k, S_k))
+    lens = (torch.arange(B, device=dev, dtype=torch.int32) * 7919) % S_k + 1
+    if kind == "seqlen":
+        return q, k, v, dict(seqlens=lens), composite.padding_add_mask(lens, S_k)
+    if kind == "key":   # padding at the end, at the start, -inf, and none
+        add = composite.padding_add_mask(lens, S_k, -10000.0).reshape(B, S_k)
+        add[1::4] = add[1::4].flip(-1)
+        add[2::4] = torch.where(add[2::4] < 0, float("-inf"), 0.0)
+        add[3::4] = 0.0
+        return q, k, v, dict(mask=add), add.reshape(B, 1, 1, S_k)
+    return q, k, v, {}, None
+
+
+@pytest.mark.parametrize("p", [0.0, 0.2])
+@pytest.mark.parametrize("kind", ["none", "seqlen", "key"])
+@pytest.mark.parametrize("S_q,S_k", [(129, 1), (200, 32), (129, 33), (256, 64), (129, 65), (140, 97), (129, 160), (255, 250)])
+def test_same_bits_as_a_tile_per_cta(cuda_device, S_q, S_k, kind, p):
+    dtype = torch.float16 if (S_q + S_k) % 2 else torch.bfloat16
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert chain_pays(sms, B * H * 2, S_k, kind == "key", p > 0) and not chain_pays(sms, PIECE * H * 2, S_k, kind == "key", p > 0)
+    q, k, v, kw, add = batch(S_q, S_k, dtype, kind, cuda_device)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    o, lse = api.fmha_forward(q, k, v, p_drop=p, seed=5, offset=2, status=status, **kw)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    for b in range(0, B, PIECE):
+        s = slice(b, b + PIECE)
+        op, lp = api.fmha_forward(q[s], k[s], v[s], p_drop=p, seed=5, offset=2, bh_offset=b * H, **{n: t[s] for n, t in kw.items()})
+        assert torch.equal(o[s], op) and torch.equal(lse[s], lp)
+    if p == 0.0 and dtype == torch.float16:
+        ref = composite.attention_fp32(q, k, v, add_mask=add)
+        helpers.assert_close(o, ref["o"], "o", dtype)
+        helpers.assert_close(lse, ref["lse"], "lse", torch.float16, atol=1e-3, rtol=1e-4)
+
+
+def test_repeated_and_concurrent_calls(cuda_device):
+    """Calls on two streams share the SMs, so that a call's CTAs start at any time; every result is the same."""
+    q, k, v, kw, _ = batch(256, 128, torch.float16, "seqlen", cuda_device)
+    first = api.fmha_forward(q, k, v, p_drop=0.1, seed=1, offset=1, **kw)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for i in range(6):
+        with torch.cuda.stream(streams[i % 2]):
+            got.append(api.fmha_forward(q, k, v, p_drop=0.1, seed=1, offset=1, **kw))
+    torch.cuda.synchronize()
+    for o, lse in got:
+        assert torch.equal(o, first[0]) and torch.equal(lse, first[1])

@@ -43,3 +43,19 @@ def test_two_tile_rule_on_one_round():
     assert not pair_pays(148, 2, 16, 1024, 1023, lengths=False)
     assert not pair_pays(148, 1, 8, 2048, 2048, lengths=False)     # 128 tiles: each has one of its own
     assert not pair_pays(148, 1, 15, 2432, 2432, lengths=False)    # 150 pairs
+
+
+def chain_pays(sms, tiles, S_k, keyadd, dropout):
+    fn = capi.load()["_ZN4fmha14fwd_chain_paysElllbb"]   # fmha::fwd_chain_pays(int64_t x 3, bool, bool)
+    fn.argtypes, fn.restype = [C.c_int64] * 3 + [C.c_bool] * 2, C.c_bool
+    return fn(sms, tiles, S_k, keyadd, dropout)
+
+
+def test_rule_of_the_kernel_that_goes_from_tile_to_tile():
+    assert chain_pays(148, 593, 256, False, False) and not chain_pays(148, 592, 256, False, False)   # one tile more than are resident
+    assert chain_pays(148, 593, 384, True, False) and not chain_pays(148, 593, 384, False, False)    # six key steps want three rounds
+    assert chain_pays(148, 1776, 384, False, False) and not chain_pays(148, 9999, 385, True, False)
+    assert chain_pays(148, 1480, 640, False, True) and not chain_pays(148, 1479, 640, False, True)   # dropout: two and a half
+    assert chain_pays(148, 1776, 640, True, True) and not chain_pays(148, 1775, 640, True, True)
+    assert not chain_pays(148, 9999, 641, False, True)
+    assert not chain_pays(0, 0, 64, False, False)
