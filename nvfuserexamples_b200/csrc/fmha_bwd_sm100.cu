@@ -5,7 +5,7 @@
 // (fmha/fmha_manual.cpp:891-897).  This backward needs neither: it recomputes the
 // probabilities from Q, K and the per-row logsumexp the forward kernel wrote.
 //
-// Head dimension 64, three kernels per call:
+// Head dimension 64, three kernels per call (one where there is a single key tile, see ONE_KV):
 //   1. bwd_prepare : delta[row] = sum_d dO[row,d] * O[row,d], and zero the fp32 dQ accumulator
 //   2. bwd_main    : persistent CTAs (one per SM) draw (128-key tile, head, batch) work items from a
 //                    counter and loop over the 128-row query tiles of each
@@ -135,6 +135,22 @@ __device__ __forceinline__ uint32_t keep_word_32x32(const PhiloxKeys& keys, uint
   return __shfl_sync(0xffffffffu, keep, 8 * (lane & 3) + (lane >> 2));
 }
 
+// A row's 64 products, eight lanes with eight each: the sum in all of them.
+template <bool BF16>
+__device__ __forceinline__ float row_dot(const uint4& x, const uint4& y) {
+  const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+  float sum = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    sum = fmaf(unpack_lo<BF16>(xs[k]), unpack_lo<BF16>(ys[k]), sum);
+    sum = fmaf(unpack_hi<BF16>(xs[k]), unpack_hi<BF16>(ys[k]), sum);
+  }
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+  return sum;
+}
+
 // 32 registers, so that eight blocks share an SM: the rare zeroing of uncovered rows had taken 48 (20.2 -> 24.6 us at 16 384
 // rows, 16 heads).
 template <bool BF16>
@@ -177,17 +193,7 @@ __global__ void __launch_bounds__(256, 8) bwd_prepare_kernel(const __grid_consta
   float4* acc = reinterpret_cast<float4*>(m.dq_accum + (static_cast<int64_t>(bh) * m.S_q_pad + r) * D + part * per);
 #pragma unroll
   for (int i = 0; i < per / 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const uint32_t xo[4] = {wo.x, wo.y, wo.z, wo.w};
-  const uint32_t xd[4] = {wd.x, wd.y, wd.z, wd.w};
-  float sum = 0.f;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    sum = fmaf(unpack_lo<BF16>(xo[k]), unpack_lo<BF16>(xd[k]), sum);
-    sum = fmaf(unpack_hi<BF16>(xo[k]), unpack_hi<BF16>(xd[k]), sum);
-  }
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+  const float sum = row_dot<BF16>(wo, wd);
   if (part == 0 && r < q_limit) m.delta[static_cast<int64_t>(bh) * m.S_q + r] = sum;
 }
 
@@ -288,7 +294,11 @@ struct BwdItem {
 };
 
 // PACKED: FMHA_MASK_CU_SEQLENS; a template parameter so that the padded kernels carry none of its bookkeeping.
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
+// ONE_KV: D = 64 and a single key tile (bwd_one_kv).  Nothing is added up for dQ then, so its tiles are written as they come; delta is formed
+// here, by the compute warps, 8 rows each, with the loads under the draws and the wait for S; and work items are equal and need no
+// counter.  The accumulator, its clearing and conversion and the two launches around this one took a quarter of the time (whole backward
+// B=2 H=4 S=128 with dropout 11.3 -> 8.6 us, B=13 H=12 S=100 15.4 -> 11.5, B=32 H=16 S=128 27.9 -> 20.1, B=128 H=16 93.0 -> 71.9).
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool ONE_KV = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
   griddep_wait();
   using L = BwdSmem<D>;
@@ -373,7 +383,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       mbar_init(do_empty + s, 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(stat_full + s, 1);
+      mbar_init(stat_full + s, ONE_KV ? 1 + kComputeThreads / 32 : 1);
       mbar_init(stat_empty + s, kComputeThreads / 32);
       mbar_init(item_full + s, 1);
       mbar_init(item_empty + s, 2 + kComputeThreads / 32);   // MMA warp, statistics warp, every compute warp
@@ -465,7 +475,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
                static_cast<uint32_t>(it.row_base));
         mbar_arrive(item_full + slot);
         if (it.id < 0) break;
-        next = atomicAdd(a.work_counter, 1) + static_cast<int>(gridDim.x);   // not looked at before this item's loads are out
+        if constexpr (ONE_KV) next += static_cast<int>(gridDim.x);
+        else next = atomicAdd(a.work_counter, 1) + static_cast<int>(gridDim.x);   // not looked at before this item's loads are out
         const int tb = packed ? 0 : it.b;
         if (it.n_cols <= 0) continue;
         const int kvb = w % KV;
@@ -666,7 +677,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           d[k] = 0.f;
           if (r < cur.q_limit) {
             x[k] = lse[r];
-            d[k] = delta[r];
+            if (!ONE_KV) d[k] = delta[r];
           }
         }
         const int slot = t & 1;
@@ -675,7 +686,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           st[k * 32 + lane] = -x[k] * kLog2eB;
-          st[kTileM + k * 32 + lane] = d[k] * inv_c;
+          if (!ONE_KV) st[kTileM + k * 32 + lane] = d[k] * inv_c;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(stat_full + slot);
@@ -721,6 +732,18 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       tmem_wait_ld();
       tc_fence_before_sync();
       mbar_arrive(dq_free);                          // the dQ columns may be overwritten
+      if constexpr (ONE_KV) {
+        const int q_tiles = n_q_all, q = tile % q_tiles * kTileM + row, h = tile / q_tiles % a.H, b = tile / q_tiles / a.H;
+        if (q < a.S_q && *abort_flag == 0) {
+          const float mul = a.scale * dscale;
+          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.dq_ptr) + b * a.dq_sb + h * a.dq_sh +
+                                                static_cast<int64_t>(q) * a.dq_ss + cq * DQ);
+          auto pair = [&](int k) { return pack2<BF16>(__uint_as_float(r[k]) * mul, __uint_as_float(r[k + 1]) * mul); };
+#pragma unroll
+          for (int k = 0; k < DQ / 8; ++k) dst[k] = make_uint4(pair(8 * k), pair(8 * k + 2), pair(8 * k + 4), pair(8 * k + 6));
+        }
+        return;
+      }
       float* dst = a.dq_accum + static_cast<int64_t>(tile) * (kTileM * D) + dq_accum_index<D>(row, cq * DQ);
 #pragma unroll
       for (int q = 0; q < DQ / 4; ++q)
@@ -817,6 +840,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       }
 
       for (int i = 0; i < n_q; ++i, ++t) {
+        // ONE_KV: O and dO for delta of rows [8 cw, +8) of the tile, eight lanes a row, four rows an instruction.  (Its place among the
+        // statistics is free: every warp has passed the barriers of the tile before.)
+        [[maybe_unused]] uint4 wo[2], wd[2];
+        if constexpr (ONE_KV) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int64_t r = i * kTileM + cw * 8 + k * 4 + (lane >> 3);
+            wo[k] = wd[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < a.S_q) {
+              wo[k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.o_ptr) + cur.b * a.o_sb + cur.h * a.o_sh + r * a.o_ss) + (lane & 7));
+              wd[k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.do_ptr) + cur.b * a.do_sb + cur.h * a.do_sh + r * a.do_ss) + (lane & 7));
+            }
+          }
+        }
         // Keep decisions of this thread's key and 32 query columns, drawn before S is needed.  (Measured and not better: after P
         // or dS has been handed on, a tile ahead; among the exponentials; half of the warps ahead of the others; one bit per score
         // from the pass before, whose draws cost there what they save here - B=16 H=16 S=1024 320 us for the backward against 319 -
@@ -825,6 +862,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         if constexpr (DROP) {
           keep = keep_word_32x32(a.philox_keys, *philox_off, gbh, static_cast<uint32_t>(i * kTileM + cq * 32),
                                  static_cast<uint32_t>((cur.k0 + quad * 32) / 16), a.philox_thr, lane);
+        }
+        if constexpr (ONE_KV) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float sum = row_dot<BF16>(wo[k], wd[k]);
+            if ((lane & 7) == 0) sStats[(t & 1) * 2 * kTileM + kTileM + cw * 8 + k * 4 + (lane >> 3)] = sum * (DROP ? 1.0f / a.dropout_scale : 1.0f);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(stat_full + (t & 1));
         }
         const uint32_t stats = smem_u32(sStats + (t & 1) * 2 * kTileM + cq * 32);
         {   // both polls go out before either answer is looked at
@@ -953,10 +999,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
-template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false>
+template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool ONE_KV = false>
 static int launch_bwd_impl(const BwdArgs& a, cudaStream_t stream) {
   using L = BwdSmem<D>;
-  auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED>;
+  auto kfn = fmha_bwd_kernel<D, BF16, KEYADD, DROP, PACKED, ONE_KV>;
   static std::atomic<bool> configured[64] = {};   // per device; set after the attribute call succeeded
   int dev = 0;
   cudaGetDevice(&dev);
@@ -988,6 +1034,19 @@ int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream) {
     FMHA_BWD_PACKED(128, true, true)
 #undef FMHA_BWD_PACKED
     return static_cast<int>(cudaErrorInvalidValue);
+  }
+  if (bwd_one_kv(D, static_cast<int64_t>(a.B) * a.H, a.S_q, a.S_k, false)) {
+#define FMHA_BWD_ONE(BF, KA, DR) \
+  if (bf == BF && keyadd == KA && drop == DR) return launch_bwd_impl<64, BF, KA, DR, false, true>(a, stream);
+    FMHA_BWD_ONE(false, false, false)
+    FMHA_BWD_ONE(false, false, true)
+    FMHA_BWD_ONE(false, true, false)
+    FMHA_BWD_ONE(false, true, true)
+    FMHA_BWD_ONE(true, false, false)
+    FMHA_BWD_ONE(true, false, true)
+    FMHA_BWD_ONE(true, true, false)
+    FMHA_BWD_ONE(true, true, true)
+#undef FMHA_BWD_ONE
   }
 #define FMHA_BWD_CASE(DD, BF, KA, DR) \
   if (D == DD && bf == BF && keyadd == KA && drop == DR) return launch_bwd_impl<DD, BF, KA, DR>(a, stream);

@@ -414,17 +414,21 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
     a.zero = {{tdq, tdk, tdv}, p->total_rows, uncovered_mode(p->B, p->S_q, p->total_rows)};
     if (const int e0 = zero_outside_rows(a.zero, p->B, p->H, p->D, cu_seqlens, stream)) return cuda_fail(static_cast<cudaError_t>(e0));
   }
+  a.o_ptr = to.ptr; a.o_sb = to.stride_b; a.o_sh = to.stride_h; a.o_ss = to.stride_s;
+  a.do_ptr = tdo.ptr; a.do_sb = tdo.stride_b; a.do_sh = tdo.stride_h; a.do_ss = tdo.stride_s;
+  a.dq_ptr = tdq.ptr; a.dq_ss = tdq.stride_s; a.dq_sh = tdq.stride_h; a.dq_sb = tdq.stride_b;
   const bool two_pass = p->D == 128;   // dQ (and delta) in a kernel of its own; see fmha_bwd_dq_sm100.cu
   int e = 0;
+  if (bwd_one_kv(p->D, static_cast<int64_t>(p->B) * p->H, p->S_q, p->S_k, packed)) {
+    e = launch_bwd(a, p->D, p->dtype, stream);
+    return e != 0 ? cuda_fail(static_cast<cudaError_t>(e)) : FMHA_OK;
+  }
   if (p->flags & FMHA_FLAG_BWD_SKIP_PREPARE) {
     // the caller prepared delta and the accumulator itself; the work counter is still ours to clear
     cudaError_t ce = cudaMemsetAsync(work_counter, 0, sizeof(int), stream);
     if (ce != cudaSuccess) return cuda_fail(ce);
   } else if (two_pass) {
     if ((rc = make_tmap(&a.tm_dq, tdq, p->dtype, mB, p->H, mSq, p->D, 32, 16))) return rc;
-    a.o_ptr = to.ptr; a.o_sb = to.stride_b; a.o_sh = to.stride_h; a.o_ss = to.stride_s;
-    a.do_ptr = tdo.ptr; a.do_sb = tdo.stride_b; a.do_sh = tdo.stride_h; a.do_ss = tdo.stride_s;
-    a.dq_ptr = tdq.ptr; a.dq_ss = tdq.stride_s; a.dq_sh = tdq.stride_h;
     e = launch_bwd_dq(a, p->dtype, stream);
     if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   } else {

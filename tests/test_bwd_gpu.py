@@ -341,3 +341,35 @@ def test_additive_mask_down_to_minus_infinity(cuda_device, B, H, S_q, S_k, D, va
     for got, want, name in zip(grads, helpers.oracle_backward(q, k, v, d_o, add=add_, keep=keep, ks=ks), ("dq", "dk", "dv")):
         helpers.assert_close(got, want, name, torch.float16)
     assert all((g[:, :, ~live.to(cuda_device)] == 0).all() for g in grads[1:])
+
+
+@pytest.mark.parametrize("p", [0.0, 0.2])
+@pytest.mark.parametrize("mask", ["none", "seqlen", "key"])
+@pytest.mark.parametrize("B,H,S_q,S_k", [(2, 3, 127, 16), (3, 2, 129, 128), (2, 2, 384, 100), (2, 2, 385, 100), (40, 8, 128, 127), (38, 4, 600, 33)])
+def test_one_key_tile_without_the_passes(cuda_device, B, H, S_q, S_k, mask, p):
+    """Head dimension 64 and up to 128 keys: delta and dQ in the main kernel alone (a few heads of more than three query tiles keep the
+    passes), ragged rows and keys, more heads than SMs, rows of a [B,S,H,D] layout.  The first and the last head against the oracle."""
+    dtype = torch.float16
+    q, k, v, d_o, lens = helpers.randn_like_config(B, H, S_q, S_k, 64, dtype, seed=S_q + S_k, device=cuda_device)
+    d_o = d_o.transpose(1, 2).contiguous().transpose(1, 2)
+    kw, one = {}, lambda b: {}
+    if mask == "seqlen":
+        kw["seqlens"], one = lens, lambda b: dict(lens=lens[b:b + 1])
+    elif mask == "key":
+        add = composite.padding_add_mask(lens.cpu(), S_k).reshape(B, S_k).to(cuda_device)
+        kw["mask"], one = add, lambda b: dict(add_mask=add[b:b + 1])
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    o, lse = api.fmha_forward(q, k, v, p_drop=p, seed=6, offset=3, status=status, **kw)
+    out = tuple(torch.full(t.shape, 7.0, dtype=dtype, device=cuda_device) for t in (q, k, v))
+    dq, dk, dv = api.fmha_backward(d_o, q, k, v, o, lse, p_drop=p, seed=6, offset=3, status=status, out=out, **kw)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    for b, h in ((0, 0), (B - 1, H - 1)):
+        sl = (slice(b, b + 1), slice(h, h + 1))
+        ref, add_, keep, ks = helpers.oracle_forward(q[sl], k[sl], v[sl], p_drop=p, seed=6, offset=3, bh_offset=b * H + h, **one(b))
+        # A few keys have probabilities near 1, rounded to 2^-12 of that, and a gradient of 0.125 times the sum of up to 600 such
+        # terms: 0.125 * sqrt(600) * 2^-12 * |dS| ~ 1e-3 at one standard deviation, the whole of the elementwise bar.  So the
+        # yardstick of short sums, twice the 16-bit composite's error.
+        refs = helpers.oracle_backward(q[sl], k[sl], v[sl], d_o[sl], add=add_, keep=keep, ks=ks)
+        eager = helpers.eager_16bit(q[sl], k[sl], v[sl], d_o[sl], add=add_, keep=keep, ks=ks)[1:]
+        for got, want, e, name in zip((dq, dk, dv), refs, eager, ("dq", "dk", "dv")):
+            helpers.assert_no_worse_than_eager(got[sl], want, e, f"{name}[{b},{h}]")
