@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fmha_fwd_pair_kernel(const __
             mbar_wait(mask_full + (t & 1), (t >> 1) & 1, wctx, kPrMaskFull, 32);
             kind = __shfl_sync(0xffffffffu, mask_kind[t & 1], 0);
           }
-          softmax_step<D, TN, BF16, KEYADD, false, PF, 0, 0>(tS, tO, j * TN, min(TN, it.k_limit - j * TN), sl2, mask_stage, kind, no_drop, m_ref,
+          softmax_step_128<BF16, KEYADD, false, PF>(tS, tO, j * TN, min(TN, it.k_limit - j * TN), sl2, mask_stage, kind, no_drop, m_ref,
                                                       sum2, wait_s, arrive_p, turn_begin, turn_end);
           s_par ^= 1u;
           if constexpr (KEYADD) {

@@ -219,7 +219,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   turn_begin();
   // ---- exponentials, dropout, P over S ---------------------------------------------------------------------
   auto hand_over = [&](int c) {   // after 32-column chunk c
-    if (c + 1 == P_FIRST) {
+    if (PAD == 0 && c + 1 == P_FIRST) {
       tmem_wait_st();
       tc_fence_before_sync();
       arrive_p(0);
@@ -265,6 +265,7 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
   turn_end();
   tmem_wait_st();
   tc_fence_before_sync();
+  if (PAD > 0 && P_FIRST > 0) arrive_p(0);
   arrive_p(1);
 }
 
@@ -280,6 +281,21 @@ __device__ __forceinline__ void softmax_step_64(uint32_t tS, uint32_t tO, int ke
   if constexpr (KEYADD) softmax_step<64, 64, BF16, KEYADD, DROP, 0, 0, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, none, none);
   else if (n_cols > 32) softmax_step<64, 64, BF16, KEYADD, DROP, 0, 32, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, none, none);
   else softmax_step<64, 32, BF16, KEYADD, DROP, 0, 0, 32>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, none, none);
+}
+
+// The same at head dimension 128, 128 keys a step and 64 to the half (kernel times: S=64 without a mask B=8 H=12 5.3 -> 4.5 us, with dropout
+// B=36 H=16 14.1 -> 10.2; lengths with dropout B=16 H=8 S=640 packed 37.5 -> 33.8, B=10 H=8 S=2048 140 -> 134; without, two tiles per CTA,
+// B=16 H=16 S=300 25.8 -> 24.0, B=12 H=12 S=2048 212 -> 210; of 90 sizes none slower).
+template <bool BF16, bool KEYADD, bool DROP, int P_FIRST, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
+__device__ __forceinline__ void softmax_step_128(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
+                                                 const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,
+                                                 const TurnBegin& turn_begin, const TurnEnd& turn_end) {
+  if constexpr (KEYADD)
+    softmax_step<128, 128, BF16, KEYADD, DROP, P_FIRST, 0, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, turn_begin, turn_end);
+  else if (n_cols > 64)
+    softmax_step<128, 128, BF16, KEYADD, DROP, P_FIRST, 64, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, turn_begin, turn_end);
+  else
+    softmax_step<128, 64, BF16, KEYADD, DROP, P_FIRST, 0, 64>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, turn_begin, turn_end);
 }
 
 // O of a finished query tile out of tensor memory, scaled and rounded: into `tile` (shared memory, 128 rows in the swizzled

@@ -323,12 +323,13 @@ def test_additive_mask_that_pads_on_the_left(cuda_device, B, H, S_q, S_k, D, dty
 
 @pytest.mark.parametrize("p", [0.0, 0.2])
 @pytest.mark.parametrize("mask", ["none", "seqlen", "key"])
-@pytest.mark.parametrize("S_k", [31, 32, 33, 63, 65, 95, 96, 97])
-def test_last_key_step_around_half_a_step(cuda_device, S_k, mask, p):
-    """Head dimension 64: a last step of up to 32 keys is done by halves; lengths around it, and whole steps past a length."""
+@pytest.mark.parametrize("S_k,D", [(31, 64), (32, 64), (33, 64), (63, 64), (65, 64), (95, 64), (96, 64), (97, 64),
+                                   (63, 128), (64, 128), (65, 128), (127, 128), (129, 128), (191, 128), (192, 128), (193, 128)])
+def test_last_key_step_around_half_a_step(cuda_device, S_k, D, mask, p):
+    """A last step of up to 32 keys (64 at head dimension 128) is done by halves; lengths around it, and whole steps past a length."""
     B, H, S_q, dtype = 4, 2, 130, torch.float16
-    q, k, v, _, _ = helpers.randn_like_config(B, H, S_q, S_k, 64, dtype, seed=S_k, device=cuda_device)
-    lens = torch.tensor([S_k, max(1, S_k - 1), max(1, S_k - 31), max(1, S_k - 33)], dtype=torch.int32, device=cuda_device)
+    q, k, v, _, _ = helpers.randn_like_config(B, H, S_q, S_k, D, dtype, seed=S_k, device=cuda_device)
+    lens = torch.tensor([S_k, max(1, S_k - 1), max(1, S_k - D // 2 + 1), max(1, S_k - D // 2 - 1)], dtype=torch.int32, device=cuda_device)
     kw, okw = {}, {}
     if mask == "seqlen":
         kw["seqlens"], okw["lens"] = lens, lens
