@@ -49,7 +49,7 @@ namespace {
 // the TMA loads and the MMAs.  Registers are allocated per SM sub-partition (16 384 each, warps dealt round-robin):
 // four CTAs of six warps put six warps on a sub-partition (80 registers per thread), four CTAs of five warps put
 // five (96), where the plain variant and dropout stay out of local memory (4 bytes with a cluster), the additive mask spills 32 to 36
-// bytes and both 24 to 28 (spill stores; D = 128 at 168 registers: plain 36 to 44, dropout 20 to 24, additive 140 to 148, both 116 to 120).
+// bytes and both 24 to 28 (spill stores; D = 128 at 168 registers: plain 36 to 44, dropout 20 to 24, additive 112 to 116, both 140 to 144).
 constexpr int kThreadsSplit = 192, kThreadsMerged = 160;
 template <int D> constexpr int fast_threads() { return D == 64 ? kThreadsMerged : kThreadsSplit; }
 constexpr int kMaxKeySplit = 8;   // portable cluster size

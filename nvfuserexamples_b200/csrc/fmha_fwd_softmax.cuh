@@ -285,14 +285,13 @@ __device__ __forceinline__ void softmax_step_64(uint32_t tS, uint32_t tO, int ke
 
 // The same at head dimension 128, 128 keys a step and 64 to the half (kernel times: S=64 without a mask B=8 H=12 5.3 -> 4.5 us, with dropout
 // B=36 H=16 14.1 -> 10.2; lengths with dropout B=16 H=8 S=640 packed 37.5 -> 33.8, B=10 H=8 S=2048 140 -> 134; without, two tiles per CTA,
-// B=16 H=16 S=300 25.8 -> 24.0, B=12 H=12 S=2048 212 -> 210; of 90 sizes none slower).
+// B=16 H=16 S=300 25.8 -> 24.0, B=12 H=12 S=2048 212 -> 210; of 90 sizes none slower).  With an additive mask as well, which gains here even
+// where no last step is short: B=98 H=16 S=256 108 -> 104, B=64 H=16 S=384 133 -> 127, S=160 B=34 H=8 18.0 -> 15.8.
 template <bool BF16, bool KEYADD, bool DROP, int P_FIRST, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
 __device__ __forceinline__ void softmax_step_128(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
                                                  const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,
                                                  const TurnBegin& turn_begin, const TurnEnd& turn_end) {
-  if constexpr (KEYADD)
-    softmax_step<128, 128, BF16, KEYADD, DROP, P_FIRST, 0, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, turn_begin, turn_end);
-  else if (n_cols > 64)
+  if (n_cols > 64)
     softmax_step<128, 128, BF16, KEYADD, DROP, P_FIRST, 64, 0>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, turn_begin, turn_end);
   else
     softmax_step<128, 64, BF16, KEYADD, DROP, P_FIRST, 0, 64>(tS, tO, key0, n_cols, sl2, mask_stage, kind, dr, m_ref, sum2, wait_s, arrive_p, turn_begin, turn_end);
