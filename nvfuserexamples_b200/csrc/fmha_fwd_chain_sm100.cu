@@ -410,9 +410,9 @@ bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool d
   return S_k <= 384 && (keyadd || S_k <= 256 || tiles >= 3 * round);
 }
 bool fwd_chain_applies(const FwdArgs& a, int head_dim) {
+  const int64_t tiles = static_cast<int64_t>((a.S_q + kTileM - 1) / kTileM) * a.H * a.B;
   return head_dim == D && a.mask_kind != FMHA_MASK_CU_SEQLENS &&
-         fwd_chain_pays(sm_count(), static_cast<int64_t>((a.S_q + kTileM - 1) / kTileM) * a.H * a.B, a.S_k, a.mask_kind == FMHA_MASK_KEY_ADDITIVE,
-                        a.dropout_kind == FMHA_DROPOUT_PHILOX);
+         fwd_chain_pays(sm_count(), tiles, a.S_k, a.mask_kind == FMHA_MASK_KEY_ADDITIVE, a.dropout_kind == FMHA_DROPOUT_PHILOX);
 }
 
 template <bool BF16, bool KEYADD, bool DROP>

@@ -581,10 +581,10 @@ static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, bool long_step
 // elements per lane), nor at D = 128, where a CTA's start is the longer chain (B=16 H=12 S=512 37.1 -> 38.4 us), and with no
 // more CTAs than SMs the order does not matter.
 int fwd_length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_lengths) {
-  const int64_t sms = sm_count();
-  if (no_lengths || D != 64 || (a.mask_kind != FMHA_MASK_SEQLEN && a.mask_kind != FMHA_MASK_CU_SEQLENS) || a.B < 2 ||
-      a.B > kMaxOrdered || ctas <= sms || ctas > 4 * FastSmem<64>::kCtasPerSm * sms)
+  if (no_lengths || D != 64 || (a.mask_kind != FMHA_MASK_SEQLEN && a.mask_kind != FMHA_MASK_CU_SEQLENS) || a.B < 2 || a.B > kMaxOrdered)
     return -1;
+  const int64_t sms = sm_count();
+  if (ctas <= sms || ctas > 4 * FastSmem<64>::kCtasPerSm * sms) return -1;
   int shift = 0;
   while ((a.S_k - 1) >> shift > 7) ++shift;
   return shift;
