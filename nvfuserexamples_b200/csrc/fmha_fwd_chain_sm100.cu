@@ -34,8 +34,8 @@ constexpr int kChThreads = 160;
 constexpr int kChCtasPerSm = 4;
 
 enum ChainWaitSite {
-  kChQFull = 131, kChKFull = 132, kChVFull = 133, kChPFull = 134, kChSFull = 135, kChQkDone = 136, kChOFull = 137, kChOStaged = 138,
-  kChItem = 139, kChItemEmpty = 140, kChClc = 141, kChSmemBase = 142
+  kChQFull = 121, kChKFull = 122, kChVFull = 123, kChPFull = 124, kChSFull = 125, kChQkDone = 126, kChOFull = 127, kChOStaged = 128,
+  kChItem = 129, kChItemEmpty = 130, kChClc = 131, kChSmemBase = 132
 };
 
 constexpr int D = 64;
