@@ -131,7 +131,7 @@ enum {
   /* backward, measurement aids: launch only part of the kernel sequence so that the main kernel (dK and dV; at D = 64 also
      dQ) can be timed alone: without what comes before it (D = 64: row statistics, accumulator clearing; D = 128:
      dQ and the row statistics), without the dQ conversion that follows it (D = 64).  No effect where there is nothing before and
-     after it (D = 64 and up to 128 keys, as a rule).  The workspace must have been prepared by
+     after it (D = 64 and up to 128 keys, as a rule; FMHA_FLAG_ZERO_UNCOVERED of a packed batch is before it there too).  The workspace must have been prepared by
      an earlier full call; results of such partial calls are not meaningful. */
   FMHA_FLAG_BWD_SKIP_PREPARE = 2,
   FMHA_FLAG_BWD_SKIP_FINISH = 4,

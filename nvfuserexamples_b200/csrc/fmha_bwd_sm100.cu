@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256, PACKED ? 4 : 8) bwd_prepare_kernel(const 
         zero_uncovered_rows(m.zero.grad[t].ptr, m.zero.grad[t].stride_s, m.zero.grad[t].stride_h, h, b, m.B, cu, m.S_q, m.total_rows, D,
                             r0, r0 + 32 * R, m.zero.mode == kUncoveredAll, threadIdx.x, blockDim.x);
     }
-    if (r0 >= q_limit) return;   // nothing of the accumulator there is added to or read
+    if (r0 >= q_limit || m.dq_accum == nullptr) return;   // nothing of the accumulator there is added to or read; or rows to zero are all there is to do
     row_o = static_cast<int64_t>(base + r) * a.o_ss;
     row_do = static_cast<int64_t>(base + r) * a.do_ss;
   }
@@ -306,7 +306,8 @@ struct BwdItem {
 // PACKED: FMHA_MASK_CU_SEQLENS; a template parameter so that the padded kernels carry none of its bookkeeping.
 // ONE_KV: D = 64 and a single key tile (bwd_one_kv).  Nothing is added up for dQ then, so its tiles are written as they come; delta is formed
 // here, by the compute warps, 8 rows each, with the loads under the draws and the wait for S; and work items are equal and need no
-// counter.  The accumulator, its clearing and conversion and the two launches around this one took a quarter of the time (whole backward
+// counter.  A packed batch has the pass before it, to zero rows.  The accumulator, its clearing and conversion and the launches around
+// this one took a quarter of the time (packed B=32 H=16, up to 128 rows each, 34.6 -> 29.3 us; whole backward of padded batches
 // B=2 H=4 S=128 with dropout 11.3 -> 8.6 us, B=13 H=12 S=100 15.4 -> 11.5, B=32 H=16 S=128 27.9 -> 20.1, B=128 H=16 93.0 -> 71.9).
 template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool ONE_KV = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
@@ -743,8 +744,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       tc_fence_before_sync();
       mbar_arrive(dq_free);                          // the dQ columns may be overwritten
       if constexpr (ONE_KV) {
-        const int q_tiles = n_q_all, q = tile % q_tiles * kTileM + row, h = tile / q_tiles % a.H, b = tile / q_tiles / a.H;
-        if (q < a.S_q && *abort_flag == 0) {
+        const int q_tiles = n_q_all, h = tile / q_tiles % a.H;
+        int q = tile % q_tiles * kTileM + row, b = tile / q_tiles / a.H, rows = a.S_q;
+        if constexpr (PACKED) {
+          const int* cu = reinterpret_cast<const int*>(a.mask);
+          const int first = cu[b];
+          rows = min(min(cu[b + 1] - first, a.S_q), a.total_rows - first);   // offsets past the tensor, which the host cannot see: no row behind it
+          rows += first;
+          q += first;
+          b = 0;
+        }
+        if (q < rows && *abort_flag == 0) {
           const float mul = a.scale * dscale;
           uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.dq_ptr) + b * a.dq_sb + h * a.dq_sh +
                                                 static_cast<int64_t>(q) * a.dq_ss + cq * DQ);
@@ -858,9 +868,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
           for (int k = 0; k < 2; ++k) {
             const int64_t r = i * kTileM + cw * 8 + k * 4 + (lane >> 3);
             wo[k] = wd[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (r < a.S_q) {
-              wo[k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.o_ptr) + cur.b * a.o_sb + cur.h * a.o_sh + r * a.o_ss) + (lane & 7));
-              wd[k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.do_ptr) + cur.b * a.do_sb + cur.h * a.do_sh + r * a.do_ss) + (lane & 7));
+            if (r < (packed ? cur.q_limit : a.S_q)) {
+              const int64_t at = packed ? cur.row_base + r : r, b = packed ? 0 : cur.b;
+              wo[k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.o_ptr) + b * a.o_sb + cur.h * a.o_sh + at * a.o_ss) + (lane & 7));
+              wd[k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(a.do_ptr) + b * a.do_sb + cur.h * a.do_sh + at * a.do_ss) + (lane & 7));
             }
           }
         }
@@ -1031,7 +1042,15 @@ int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream) {
   const bool bf = dtype == FMHA_DTYPE_BF16;
   const bool keyadd = a.mask_kind == FMHA_MASK_KEY_ADDITIVE;
   const bool drop = a.dropout_kind == FMHA_DROPOUT_PHILOX;
+  const bool one_kv = bwd_one_kv(D, static_cast<int64_t>(a.B) * a.H, a.S_q, a.S_k);
   if (a.mask_kind == FMHA_MASK_CU_SEQLENS) {
+#define FMHA_BWD_ONE_PACKED(BF, DR) \
+  if (one_kv && bf == BF && drop == DR) return launch_bwd_impl<64, BF, false, DR, true, true>(a, stream);
+    FMHA_BWD_ONE_PACKED(false, false)
+    FMHA_BWD_ONE_PACKED(false, true)
+    FMHA_BWD_ONE_PACKED(true, false)
+    FMHA_BWD_ONE_PACKED(true, true)
+#undef FMHA_BWD_ONE_PACKED
 #define FMHA_BWD_PACKED(DD, BF, DR) \
   if (D == DD && bf == BF && drop == DR) return launch_bwd_impl<DD, BF, false, DR, true>(a, stream);
     FMHA_BWD_PACKED(64, false, false)
@@ -1045,7 +1064,7 @@ int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream) {
 #undef FMHA_BWD_PACKED
     return static_cast<int>(cudaErrorInvalidValue);
   }
-  if (bwd_one_kv(D, static_cast<int64_t>(a.B) * a.H, a.S_q, a.S_k, false)) {
+  if (one_kv) {
 #define FMHA_BWD_ONE(BF, KA, DR) \
   if (bf == BF && keyadd == KA && drop == DR) return launch_bwd_impl<64, BF, KA, DR, false, true>(a, stream);
     FMHA_BWD_ONE(false, false, false)

@@ -419,8 +419,10 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
   a.dq_ptr = tdq.ptr; a.dq_ss = tdq.stride_s; a.dq_sh = tdq.stride_h; a.dq_sb = tdq.stride_b;
   const bool two_pass = p->D == 128;   // dQ (and delta) in a kernel of its own; see fmha_bwd_dq_sm100.cu
   int e = 0;
-  if (bwd_one_kv(p->D, static_cast<int64_t>(p->B) * p->H, p->S_q, p->S_k, packed)) {
-    e = launch_bwd(a, p->D, p->dtype, stream);
+  if (bwd_one_kv(p->D, static_cast<int64_t>(p->B) * p->H, p->S_q, p->S_k)) {
+    a.dq_accum = nullptr;
+    if (a.zero.grad[0].ptr != nullptr && !(p->flags & FMHA_FLAG_BWD_SKIP_PREPARE)) e = launch_bwd_prepare(to, tdo, a, p->dtype, stream);
+    if (e == 0) e = launch_bwd(a, p->D, p->dtype, stream);
     return e != 0 ? cuda_fail(static_cast<cudaError_t>(e)) : FMHA_OK;
   }
   if (p->flags & FMHA_FLAG_BWD_SKIP_PREPARE) {

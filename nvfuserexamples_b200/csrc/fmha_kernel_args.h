@@ -98,7 +98,7 @@ struct BwdArgs {
   float scale_log2;  // softmax scale * log2(e)
   const float* lse;  // [B*H, S_q] natural log
   float* delta;        // [B*H, S_q] rowsum(dO * O)
-  float* dq_accum;     // head dimension 64: [B*H, S_q_pad, D] fp32 in the blocked order of dq_accum_index, zero on entry
+  float* dq_accum;     // head dimension 64: [B*H, S_q_pad, D] fp32 in the blocked order of dq_accum_index, zero on entry; null: not used
   int* work_counter;   // zero on entry; the persistent CTAs draw their work items from it
   // FMHA_MASK_CU_SEQLENS: mask = int32 [B+1] row offsets into the packed [total_rows, H, D] tensors; the raw
   // dK / dV pointers serve the row-wise stores of a sequence's last, partial key tile
@@ -143,12 +143,12 @@ bool fwd_dense_applies(const FwdArgs& a, int D);
 int launch_fwd_dense(const FwdArgs& a, int dtype, cudaStream_t stream);
 int launch_bwd_dq(const BwdArgs& a, int dtype, cudaStream_t stream);   // head dimension 128: dQ, delta, work counter
 int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream);
-// Head dimension 64, one key tile: whether the main kernel is all there is (ONE_KV in fmha_bwd_sm100.cu).  A packed batch keeps its passes,
-// which also zero rows; and so do a few heads of many query tiles: delta formed within an item costs each of its tiles 0.6 us, in a
+// Head dimension 64, one key tile: whether the main kernel is all there is (ONE_KV in fmha_bwd_sm100.cu), in a packed batch after the
+// pass before it has zeroed rows, and nothing else.  Not for a few heads of many query tiles: delta formed within an item costs each of its tiles 0.6 us, in a
 // pass of its own it has the whole chip (8 heads, S_k=50, alone / with the passes: S_q=256 10.7 / 12.3 us, 384 13.7 / 13.9, 512 17.0 / 15.4; 96
 // heads 512 17.4 / 20.5, 1024 30.5 / 32.4; 512 heads 1024 138 / 153).
-constexpr bool bwd_one_kv(int D, int64_t heads, int S_q, int S_k, bool packed) {
-  return D == 64 && S_k <= kTileN && !packed && (S_q <= 3 * kTileM || heads >= 12 * ((S_q + kTileM - 1) / kTileM));
+constexpr bool bwd_one_kv(int D, int64_t heads, int S_q, int S_k) {
+  return D == 64 && S_k <= kTileN && (S_q <= 3 * kTileM || heads >= 12 * ((S_q + kTileM - 1) / kTileM));
 }
 // head dimension 64: the passes before and after the main kernel
 // `m`: the main kernel's arguments (sizes, mask, Philox, workspace)

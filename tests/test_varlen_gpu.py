@@ -371,3 +371,31 @@ def test_forward_writes_inside_the_tensor_only(cuda_device, B, H, D):
         ref = helpers.composite.attention_fp32(qb, kb, vb)
         helpers.assert_close(o[r0:r0 + rows].permute(1, 0, 2), ref["o"][:, :rows], f"o of {b}")
         helpers.assert_close(lse[:H * total].view(H, total)[:, r0:r0 + rows], ref["lse"][:, :rows], f"lse of {b}", atol=1e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("p", [0.0, 0.2])
+@pytest.mark.parametrize("lens,max_len", [([128, 1, 77, 0, 128], 128), ([100, 33, 140, 64], 128), ([20] * 60, 64)])
+def test_backward_of_one_key_tile_like_the_padded_batch(cuda_device, lens, max_len, p):
+    """Head dimension 64 and up to 128 rows a sequence: one pass zeroes rows, the main kernel does the rest.  The same bits as a sequence on
+    its own gives in a padded call (which has no pass at all), zeros in the rows a sequence is cut by and behind the last one."""
+    H, D, dtype = 3, 64, torch.float16
+    q, k, v, d_o, cu = packed_batch(lens, H, D, dtype, seed=sum(lens), device=cuda_device)
+    pad = lambda t: torch.cat([t, torch.ones(9, H, D, dtype=dtype, device=cuda_device)])
+    q, k, v, d_o = map(pad, (q, k, v, d_o))
+    res = capi.fwd_varlen(q, k, v, cu, max_len, p_drop=p, seed=8, offset=4)
+    out = tuple(torch.full_like(q, 7.0) for _ in range(3))
+    grads = capi.bwd_varlen(d_o, q, k, v, res["o"], res["lse"], cu, max_len, p_drop=p, seed=8, offset=4, out=out, flags=capi.FLAG_ZERO_UNCOVERED)
+    first = cu.tolist()
+    for b, n in enumerate(lens):
+        n = min(n, max_len)
+        if n == 0:
+            continue
+        rows = slice(first[b], first[b] + n)
+        one = [t[rows].transpose(0, 1).unsqueeze(0).contiguous() for t in (d_o, q, k, v, res["o"])]
+        lse = res["lse"][:, rows].unsqueeze(0).contiguous()
+        kw = dict(p_drop=p, seed=8, offset=4, bh_offset=b * H)
+        for got, want in zip(grads, capi.bwd(*one, lse, **kw)):
+            assert torch.equal(got[rows], want[0].transpose(0, 1))
+        for got in grads:
+            assert (got[first[b] + n:first[b + 1]] == 0).all()
+    assert all((got[first[-1]:] == 0).all() for got in grads)
