@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) fmha_bwd_dq_kernel(const __grid
     } else if (packed) {
       const int* cu = reinterpret_cast<const int*>(a.mask);
       it.row_base = cu[z];
-      it.k_limit = it.q_limit = min(cu[z + 1] - it.row_base, a.S_q);   // cut at the stated maximum
+      it.k_limit = it.q_limit = packed_rows(it.row_base, cu[z + 1], a.S_q, a.total_rows);
       it.tb = 0;
     }
     it.n_kv = (it.k_limit + kTileN - 1) / kTileN;
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(256) bwd_delta_kernel(const __grid_constant__ 
   int64_t base_o = static_cast<int64_t>(b) * a.o_sb, base_do = static_cast<int64_t>(b) * a.do_sb;
   if (a.mask_kind == FMHA_MASK_CU_SEQLENS) {
     const int* cu = static_cast<const int*>(a.mask);
-    q_limit = min(cu[b + 1] - cu[b], a.S_q);
+    q_limit = packed_rows(cu[b], cu[b + 1], a.S_q, a.total_rows);
     base_o = static_cast<int64_t>(cu[b]) * a.o_ss;
     base_do = static_cast<int64_t>(cu[b]) * a.do_ss;
   }

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256, PACKED ? 4 : 8) bwd_prepare_kernel(const 
     const int* cu = static_cast<const int*>(m.mask);
     const int base = cu[b];
     const int len = cu[b + 1] - base;
-    q_limit = min(len, m.S_q);   // rows past the stated maximum length take no part
+    q_limit = packed_rows(base, cu[b + 1], m.S_q, m.total_rows);
     if (m.zero.grad[0].ptr != nullptr && (r0 + 32 * R > q_limit || len > q_limit)) {
       for (int t = 0; t < 3; ++t)
         zero_uncovered_rows(m.zero.grad[t].ptr, m.zero.grad[t].stride_s, m.zero.grad[t].stride_h, h, b, m.B, cu, m.S_q, m.total_rows, D,
@@ -217,6 +217,7 @@ struct FinishArgs {
   int B, H, S_q, S_q_pad;
   float scale;
   const int* cu_seqlens;  // packed batch: row offsets into the [total_rows, H, D] dQ (sb unused), else null
+  int total_rows;
 };
 
 // A block converts 128 rows of a head: coalesced 16-byte reads of the accumulator (eight in flight per thread),
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishArgs a) {
   int q_limit = a.S_q;
   if (a.cu_seqlens != nullptr) {
     const int first = a.cu_seqlens[b];
-    q_limit = min(a.cu_seqlens[b + 1] - first, a.S_q);   // rows past the stated maximum length take no part
+    q_limit = packed_rows(first, a.cu_seqlens[b + 1], a.S_q, a.total_rows);
     base = static_cast<int64_t>(first) * a.ss;
   }
   if (r0 >= q_limit) return;
@@ -442,10 +443,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         it.row_base = cu[it.b];
         // a sequence longer than the stated maximum is cut there: its tiles would otherwise run into the next
         // head's rows of the dQ accumulator and of delta
-        const int len = min(cu[it.b + 1] - it.row_base, a.S_q);
-        k_limit = len;
-        it.q_limit = len;
-        it.n_q = (len + kTileM - 1) / kTileM;
+        k_limit = it.q_limit = packed_rows(it.row_base, cu[it.b + 1], a.S_q, a.total_rows);
+        it.n_q = (it.q_limit + kTileM - 1) / kTileM;
       }
       it.n_cols = min(kTileN, k_limit - it.k0);
     }
@@ -725,6 +724,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       mbar_wait(bar, parity, wctx, site, kComputeSleepNs);
       tc_fence_after_sync();
     };
+    // What the write-outs of an item done during the next one (dK and dV, ONE_KV: its last dQ tile) need to know of it waits in shared memory.
+    const uint32_t rec = smem_u32(smem + L::kOffRec) + cw * 32;
     // Frees the warp's staging tile (its previous TMA copies have been read).
     auto stage_free = [&]() {
       if (lane == 0) tma_store_wait_read();
@@ -734,6 +735,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     // accumulator is laid out so that a warp's instruction covers 512 consecutive bytes (dq_accum_index), which keeps the
     // tile out of shared memory: staged there for TMA reduce-adds it cost 32 (D = 64) or 64 KB written and read again per
     // tile, a fifth of all shared-memory traffic.
+    // `tile` is its place there; ONE_KV: twice its number within the item, and the parity of the item's.
     [[maybe_unused]] auto dq_readout = [&](int tt, int tile) {   // D = 64
       wait_all(dq_full, tt & 1, kSiteDqFull);
       uint32_t r[DQ];
@@ -744,20 +746,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
       tc_fence_before_sync();
       mbar_arrive(dq_free);                          // the dQ columns may be overwritten
       if constexpr (ONE_KV) {
-        const int q_tiles = n_q_all, h = tile / q_tiles % a.H;
-        int q = tile % q_tiles * kTileM + row, b = tile / q_tiles / a.H, rows = a.S_q;
-        if constexpr (PACKED) {
-          const int* cu = reinterpret_cast<const int*>(a.mask);
-          const int first = cu[b];
-          rows = min(min(cu[b + 1] - first, a.S_q), a.total_rows - first);   // offsets past the tensor, which the host cannot see: no row behind it
-          rows += first;
-          q += first;
-          b = 0;
-        }
-        if (q < rows && *abort_flag == 0) {
+        const uint4 x = lds128(rec + (tile & 1) * 16);
+        const int64_t h = x.x & 0xffffu, b = packed ? 0u : x.x >> 16;
+        const int q = (tile >> 1) * kTileM + row;
+        if (q < static_cast<int>(x.w) && *abort_flag == 0) {
           const float mul = a.scale * dscale;
           uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.dq_ptr) + b * a.dq_sb + h * a.dq_sh +
-                                                static_cast<int64_t>(q) * a.dq_ss + cq * DQ);
+                                                static_cast<int64_t>(static_cast<int>(x.z) + q) * a.dq_ss + cq * DQ);
           auto pair = [&](int k) { return pack2<BF16>(__uint_as_float(r[k]) * mul, __uint_as_float(r[k + 1]) * mul); };
 #pragma unroll
           for (int k = 0; k < DQ / 8; ++k) dst[k] = make_uint4(pair(8 * k), pair(8 * k + 2), pair(8 * k + 4), pair(8 * k + 6));
@@ -827,8 +822,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     };
 
     int n = 0, w = 0, t = 0;      // items fetched, items with work, query tiles so far
-    // What the write-out of an item's dK and dV, done during the next item, needs to know of it waits in shared memory.
-    const uint32_t rec = smem_u32(smem + L::kOffRec) + cw * 32;
     bool pending = false;         // dK and dV of item number w-1 (with work) are still in tensor memory
     auto store_pending = [&]() {
       const uint4 r = lds128(rec + ((w - 1) & 1) * 16);
@@ -836,7 +829,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
                  static_cast<int>(r.w), true);
       pending = false;
     };
-    [[maybe_unused]] int prev_tile = 0;       // D = 64: accumulator tile of tile t-1,
+    [[maybe_unused]] int prev_tile = 0;       // D = 64: tile t-1 as dq_readout wants it,
     [[maybe_unused]] bool dq_out = true;      // and whether its dQ has been read out
 
     while (true) {
@@ -988,7 +981,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
         if constexpr (D == 64) {
           if (!dq_out) dq_readout(t - 1, prev_tile);
           dq_out = false;
-          prev_tile = bh * n_q_all + i;
+          prev_tile = ONE_KV ? 2 * i + (w & 1) : bh * n_q_all + i;
         }
       }
       pending = true;
@@ -1114,11 +1107,12 @@ int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const Bw
 }
 
 int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int dtype, float scale,
-                      const int* cu_seqlens, cudaStream_t stream) {
+                      const int* cu_seqlens, int total_rows, cudaStream_t stream) {
   FinishArgs f;
   f.dq_accum = dq_accum; f.dq = dq.ptr;
   f.sb = dq.stride_b; f.sh = dq.stride_h; f.ss = dq.stride_s;
-  f.B = B; f.H = H; f.S_q = S_q; f.S_q_pad = S_q_pad; f.scale = scale; f.cu_seqlens = cu_seqlens;
+  f.B = B; f.H = H; f.S_q = S_q; f.S_q_pad = S_q_pad; f.scale = scale;
+  f.cu_seqlens = cu_seqlens; f.total_rows = total_rows;
   const dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((S_q + kFinishRows - 1) / kFinishRows));
   auto kfn = dtype == FMHA_DTYPE_BF16 ? bwd_finish_kernel<true> : bwd_finish_kernel<false>;
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(256), 0, stream, f);

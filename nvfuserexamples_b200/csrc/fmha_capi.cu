@@ -441,7 +441,7 @@ int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream_) {
   if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   if (!two_pass && !(p->flags & FMHA_FLAG_BWD_SKIP_FINISH)) {
     // the main kernel leaves the dropout factor 1/(1-p) out of dS; it is applied here (and to dK, dV in its epilogue)
-    e = launch_bwd_finish(dq_accum, tdq, p->B, p->H, p->S_q, s_q_pad, p->dtype, p->scale * a.dropout_scale, cu_seqlens, stream);
+    e = launch_bwd_finish(dq_accum, tdq, p->B, p->H, p->S_q, s_q_pad, p->dtype, p->scale * a.dropout_scale, cu_seqlens, p->total_rows, stream);
     if (e != 0) return cuda_fail(static_cast<cudaError_t>(e));
   }
   return FMHA_OK;

@@ -107,6 +107,13 @@ __device__ __forceinline__ int batch_of_rank(int rank, int B, uint32_t cls) {
   return __ffs(__ballot_sync(0xffffffffu, (in >> lane & 1u) && __popc(in & ((1u << lane) - 1u)) == rank)) - 1;
 }
 
+// Packed batch, backward: the rows of the sequence whose offsets are `first` and `next`.  It is cut at the stated maximum length, and at the end of
+// the tensor where its offset reaches past that, which the host cannot see; one that begins before the tensor has none.  (The forward counts keys
+// behind the tensor as zeros, which are in the logsumexp and add nothing to any gradient.)
+__device__ __forceinline__ int packed_rows(int first, int next, int max_len, int total_rows) {
+  return first < 0 ? 0 : min(min(next - first, max_len), total_rows - first);
+}
+
 // Packed batch, FMHA_FLAG_ZERO_UNCOVERED: zeroes, in head h of a [total_rows, H, D] tensor, the caller's share of the rows that no
 // tile covers.  The caller stands for rows [r0, r1) of sequence b, as if every sequence had max_len rows; all callers together
 // stand for all of them.  A sequence past max_len: its callers share the rows it is cut by.  Rows outside all sequences (`outside`;

@@ -154,7 +154,7 @@ constexpr bool bwd_one_kv(int D, int64_t heads, int S_q, int S_k) {
 // `m`: the main kernel's arguments (sizes, mask, Philox, workspace)
 int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const BwdArgs& m, int dtype, cudaStream_t stream);
 int launch_bwd_finish(const float* dq_accum, const fmha_tensor4& dq, int B, int H, int S_q, int S_q_pad, int dtype, float scale,
-                      const int* cu_seqlens, cudaStream_t stream);
+                      const int* cu_seqlens, int total_rows, cudaStream_t stream);
 
 // Multiprocessors of the current device, asked for once per device.
 inline int sm_count() {

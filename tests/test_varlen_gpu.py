@@ -373,6 +373,41 @@ def test_forward_writes_inside_the_tensor_only(cuda_device, B, H, D):
         helpers.assert_close(lse[:H * total].view(H, total)[:, r0:r0 + rows], ref["lse"][:, :rows], f"lse of {b}", atol=1e-3, rtol=1e-4)
 
 
+@pytest.mark.parametrize("B,H", [(3, 2), (60, 8)])   # fewer work items than SMs, and several per SM
+@pytest.mark.parametrize("max_len", [128, 400])      # at D = 64 one key tile, and the passes around the main kernel
+@pytest.mark.parametrize("D", [64, 128])
+def test_backward_writes_inside_the_tensor_only(cuda_device, D, max_len, B, H):
+    """Offsets that reach past the tensor at either end, which the host cannot see: no gradient row is written before or behind it.  (All
+    tensors lie within larger buffers.)  The sequence that is cut has the gradients of one whose further keys are zeros, as its forward has."""
+    spare = 2 * max_len + 100
+    lens = [max_len - 38] * (B - 2) + [max_len, max_len]
+    cu_list = [0]
+    for n in lens:
+        cu_list.append(cu_list[-1] + n)
+    total = cu_list[-2] - (max_len - 70)   # the last but one has 70 of its rows, the last one begins behind the tensor
+    cu = torch.tensor([-40] + cu_list, dtype=torch.int32, device=cuda_device)   # and one before all of them begins before it
+    g = torch.Generator(device=cuda_device).manual_seed(7)
+    big = [torch.randn(spare + total + spare, H, D, device=cuda_device, generator=g).half() for _ in range(5)]
+    q, k, v, d_o, o = (t[spare:spare + total] for t in big)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    lse = torch.full((spare + H * total + spare,), 7.0, device=cuda_device)
+    inside = lse[spare:spare + H * total].view(H, total)
+    res = capi.fwd_varlen(q, k, v, cu, max_len, out=o, status=status)
+    inside.copy_(res["lse"])
+    outs = [torch.full_like(big[0], 7.0) for _ in range(3)]
+    grads = [t[spare:spare + total] for t in outs]
+    capi.bwd_varlen(d_o, q, k, v, o, inside, cu, max_len, out=tuple(grads), status=status)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    for t in outs:
+        assert (t[:spare] == 7.0).all() and (t[spare + total:] == 7.0).all() and torch.isfinite(t).all()
+    for b in (0, B - 3, B - 2):
+        r0, rows = cu_list[b], min(lens[b], total - cu_list[b])
+        one = [torch.nn.functional.pad(x[r0:r0 + rows], (0, 0, 0, 0, 0, lens[b] - rows)).permute(1, 0, 2).unsqueeze(0).cpu() for x in (q, k, v, d_o)]
+        refs = helpers.composite.attention_grads_fp32(*one, add_mask=None, keep=None, keep_scale=1.0)
+        for got, want, name in zip(grads, refs, ("dq", "dk", "dv")):
+            helpers.assert_close(got[r0:r0 + rows].permute(1, 0, 2), want[0][:, :rows], f"{name} of {b}")
+
+
 @pytest.mark.parametrize("p", [0.0, 0.2])
 @pytest.mark.parametrize("lens,max_len", [([128, 1, 77, 0, 128], 128), ([100, 33, 140, 64], 128), ([20] * 60, 64)])
 def test_backward_of_one_key_tile_like_the_padded_batch(cuda_device, lens, max_len, p):
