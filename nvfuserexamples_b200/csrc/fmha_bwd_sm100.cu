@@ -152,15 +152,17 @@ __device__ __forceinline__ float row_dot(const uint4& x, const uint4& y) {
 }
 
 // Bound by memory: O and dO in, the accumulator out (B=32 H=16 S=512: 134 MB in 18.4 us, 7.3 TB/s; with each thread clearing the 32 bytes
-// of its own eight columns, half a sector an instruction, 19.8).  PACKED: a block waits for the row offsets before it can load, so it takes
-// four times the rows, their loads in flight together, and four blocks an SM leave the rare zeroing of uncovered rows its registers
-// (12 288 rows, 16 heads 20.6 -> 15.3 us; twice the rows 15.9, in 32 registers 17.4).
-template <bool BF16, bool PACKED>
+// of its own eight columns, half a sector an instruction, 19.8).  PACKED: a block waits for the row offsets before it can load, so on large grids it
+// takes four times the rows (R), their loads in flight together, and four blocks an SM leave the rare zeroing of uncovered rows its registers
+// (12 288 rows, 16 heads 20.6 -> 15.3 us; twice the rows 15.9, in 32 registers 17.4).  Where that leaves less than 1.5 blocks per multiprocessor there is
+// nothing to hide the wait behind, and blocks of 32 rows are done sooner (whole backward with four / one times 32 rows: 4 blocks of 128 rows
+// 14.2 / 13.9 us, 48 18.4 / 17.9, 96 17.3 / 16.8, 192 21.7 / 21.3 and with short sequences 16.4 / 16.7, 288 24.3 / 24.7 and 17.4 / 18.5).
+template <bool BF16, bool PACKED, int R>
 __global__ void __launch_bounds__(256, PACKED ? 4 : 8) bwd_prepare_kernel(const __grid_constant__ PrepArgs a) {
   griddep_wait();
   // grid = (B*H, blocks of 32 R rows); 8 threads per row, 8 elements each.
   // The head index comes from the grid, so no thread divides 64-bit indices.
-  constexpr int D = kAccumD, per = D / 8, R = PACKED ? 4 : 1;
+  constexpr int D = kAccumD, per = D / 8;
   const BwdArgs& m = a.m;
   const int part = threadIdx.x & 7;
   const int bh = blockIdx.x;
@@ -1099,9 +1101,11 @@ int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const Bw
   p.do_sb = dot.stride_b; p.do_sh = dot.stride_h; p.do_ss = dot.stride_s;
   p.m = m;
   const bool packed = m.mask_kind == FMHA_MASK_CU_SEQLENS, bf = dtype == FMHA_DTYPE_BF16;
-  const dim3 grid(static_cast<unsigned>(m.B) * m.H, static_cast<unsigned>(m.S_q_pad / (packed ? 128 : 32)));
-  auto kfn = packed ? (bf ? bwd_prepare_kernel<true, true> : bwd_prepare_kernel<false, true>)
-                    : (bf ? bwd_prepare_kernel<true, false> : bwd_prepare_kernel<false, false>);
+  const bool four = packed && static_cast<int64_t>(m.B) * m.H * (m.S_q_pad / 128) * 2 >= 3 * static_cast<int64_t>(sm_count());
+  const dim3 grid(static_cast<unsigned>(m.B) * m.H, static_cast<unsigned>(m.S_q_pad / (four ? 128 : 32)));
+  auto kfn = four     ? (bf ? bwd_prepare_kernel<true, true, 4> : bwd_prepare_kernel<false, true, 4>)
+             : packed ? (bf ? bwd_prepare_kernel<true, true, 1> : bwd_prepare_kernel<false, true, 1>)
+                      : (bf ? bwd_prepare_kernel<true, false, 1> : bwd_prepare_kernel<false, false, 1>);
   const cudaError_t e = launch_overlapped(kfn, grid, dim3(256), 0, stream, p);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

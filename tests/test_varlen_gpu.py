@@ -408,6 +408,31 @@ def test_backward_writes_inside_the_tensor_only(cuda_device, D, max_len, B, H):
             helpers.assert_close(got[r0:r0 + rows].permute(1, 0, 2), want[0][:, :rows], f"{name} of {b}")
 
 
+def test_backward_pass_of_large_and_small_blocks(cuda_device):
+    """Head dimension 64: the pass before the main kernel takes blocks of 128 rows on grids of at least 1.5 of them per SM, blocks of 32 below.  The same
+    gradients, bit for bit (two key tiles: either order of adding them to dQ's zeros gives the same sum), and zeros in the rows no tile covers."""
+    H, D, max_len, tail = 3, 64, 200, 77
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = (3 * sms + 4 * H - 1) // (4 * H)   # the first batch with 2 * (B * H * 2 blocks of 128 rows) >= 3 * sms
+    lens = [(37 * b) % 260 for b in range(B)]   # empty ones, ones past max_len
+    q, k, v, d_o, cu = packed_batch(lens + [tail], H, D, torch.float16, seed=9, device=cuda_device)
+    got = []
+    for n in (B, B - 1):   # the rows behind the last sequence belong to none
+        rows = int(cu[n]) + tail if n == B else int(cu[n]) + lens[-1]
+        x = [t[:rows] for t in (q, k, v, d_o)]
+        res = capi.fwd_varlen(*x[:3], cu[:n + 1].contiguous(), max_len, flags=capi.FLAG_ZERO_UNCOVERED)
+        out = tuple(torch.full_like(x[0], float("nan")) for _ in range(3))
+        got.append(capi.bwd_varlen(x[3], *x[:3], res["o"], res["lse"], cu[:n + 1].contiguous(), max_len, out=out, flags=capi.FLAG_ZERO_UNCOVERED))
+        covered = torch.zeros(rows, dtype=torch.bool, device=cuda_device)
+        for b in range(n):
+            covered[int(cu[b]):int(cu[b]) + min(lens[b], max_len)] = True
+        for t in out:
+            assert (t[~covered] == 0).all() and torch.isfinite(t).all()
+    end = int(cu[B - 1])
+    for large, small in zip(*got):
+        assert torch.equal(large[:end], small[:end])
+
+
 @pytest.mark.parametrize("p", [0.0, 0.2])
 @pytest.mark.parametrize("lens,max_len", [([128, 1, 77, 0, 128], 128), ([100, 33, 140, 64], 128), ([20] * 60, 64)])
 def test_backward_of_one_key_tile_like_the_padded_batch(cuda_device, lens, max_len, p):
