@@ -409,10 +409,19 @@ bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool d
   if (dropout) return S_k <= 640 && 2 * tiles >= (keyadd ? 6 : 5) * round;
   return S_k <= 384 && (keyadd || S_k <= 256 || tiles >= 3 * round);
 }
+// The same where it is known whether sequences may differ in length.  Without lengths, dropout or mask a second round that is nearly full of four whole key
+// steps does not pay (S_k=256, 1.6 and 1.7 rounds 0.98 to 0.99, 1.8 to 2.0 rounds 1.03 to 1.045, 2.05 0.97; 1.8 to 2.0 rounds with lengths 0.95 to 0.98,
+// S_k=240 0.98 to 1.00, 224 and 208 0.95 to 0.97, 192 1.00 to 1.01).
+bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool dropout, bool lengths) {
+  const int64_t round = kChCtasPerSm * sms;
+  if (!keyadd && !dropout && !lengths && S_k > 240 && 10 * tiles > 17 * round && tiles <= 2 * round) return false;
+  return fwd_chain_pays(sms, tiles, S_k, keyadd, dropout);
+}
 bool fwd_chain_applies(const FwdArgs& a, int head_dim) {
   const int64_t tiles = static_cast<int64_t>((a.S_q + kTileM - 1) / kTileM) * a.H * a.B;
   return head_dim == D && a.mask_kind != FMHA_MASK_CU_SEQLENS &&
-         fwd_chain_pays(sm_count(), tiles, a.S_k, a.mask_kind == FMHA_MASK_KEY_ADDITIVE, a.dropout_kind == FMHA_DROPOUT_PHILOX);
+         fwd_chain_pays(sm_count(), tiles, a.S_k, a.mask_kind == FMHA_MASK_KEY_ADDITIVE, a.dropout_kind == FMHA_DROPOUT_PHILOX,
+                        a.mask_kind == FMHA_MASK_SEQLEN);
 }
 
 template <bool BF16, bool KEYADD, bool DROP>

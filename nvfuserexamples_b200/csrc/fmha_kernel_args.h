@@ -134,6 +134,7 @@ int fwd_length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_length
 bool fwd_chain_applies(const FwdArgs& a, int D);
 // its rule on sizes, on a device of `sms` multiprocessors
 bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool dropout);
+bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool dropout, bool lengths);   // lengths: sequences may differ
 int launch_fwd_chain(const FwdArgs& a, int dtype, cudaStream_t stream);
 // the kernel for a handful of query rows per head (fmha_fwd_rows_sm100.cu): compact masks, not packed
 bool fwd_rows_applies(int S_q, int S_k, int D, int64_t heads, bool dropout);

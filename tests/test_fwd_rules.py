@@ -59,3 +59,13 @@ def test_rule_of_the_kernel_that_goes_from_tile_to_tile():
     assert chain_pays(148, 1776, 640, True, True) and not chain_pays(148, 1775, 640, True, True)
     assert not chain_pays(148, 9999, 641, False, True)
     assert not chain_pays(0, 0, 64, False, False)
+
+
+def test_rule_of_the_kernel_that_goes_from_tile_to_tile_without_lengths():
+    """One length of four whole key steps: not where the second round is nearly full."""
+    fn = capi.load()["_ZN4fmha14fwd_chain_paysElllbbb"]   # fmha::fwd_chain_pays(int64_t x 3, bool x 3)
+    fn.argtypes, fn.restype = [C.c_int64] * 3 + [C.c_bool] * 3, C.c_bool
+    assert fn(148, 1006, 256, False, False, False) and not fn(148, 1007, 256, False, False, False)
+    assert not fn(148, 1184, 241, False, False, False) and fn(148, 1185, 256, False, False, False)
+    assert fn(148, 1184, 240, False, False, False) and fn(148, 1184, 256, False, False, True) and fn(148, 1184, 256, True, False, False)
+    assert not fn(148, 1184, 256, False, True, False) and not fn(148, 592, 64, False, False, False)
