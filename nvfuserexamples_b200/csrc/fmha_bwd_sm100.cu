@@ -1015,6 +1015,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
+// Head dimension 64, one key tile: whether the main kernel is all there is (ONE_KV), in a packed batch after the pass before it has zeroed rows, and nothing
+// else.  Not for a few heads of many query tiles: delta formed within an item costs each of its tiles 0.6 us, in a pass of its own it has the whole chip
+// (8 heads, S_k=50, alone / with the passes: S_q=256 10.7 / 12.3 us, 384 13.7 / 13.9, 512 17.0 / 15.4).  Where it is taken, S_k=100: 1 to 1024 heads,
+// S_q=128 0.67 to 0.84 of the passes' time, 384 0.69 to 1.00, 48 heads and more S_q=512 0.71 to 0.98, 96 and more 1024 0.69 to 1.00 (1.02 at 160 heads).
+bool bwd_one_kv(int D, int64_t heads, int S_q, int S_k) {
+  return D == 64 && S_k <= kTileN && (S_q <= 3 * kTileM || heads >= 12 * ((S_q + kTileM - 1) / kTileM));
+}
+
 template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool ONE_KV = false>
 static int launch_bwd_impl(const BwdArgs& a, cudaStream_t stream) {
   using L = BwdSmem<D>;

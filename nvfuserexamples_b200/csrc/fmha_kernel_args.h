@@ -144,13 +144,8 @@ bool fwd_dense_applies(const FwdArgs& a, int D);
 int launch_fwd_dense(const FwdArgs& a, int dtype, cudaStream_t stream);
 int launch_bwd_dq(const BwdArgs& a, int dtype, cudaStream_t stream);   // head dimension 128: dQ, delta, work counter
 int launch_bwd(const BwdArgs& a, int D, int dtype, cudaStream_t stream);
-// Head dimension 64, one key tile: whether the main kernel is all there is (ONE_KV in fmha_bwd_sm100.cu), in a packed batch after the
-// pass before it has zeroed rows, and nothing else.  Not for a few heads of many query tiles: delta formed within an item costs each of its tiles 0.6 us, in a
-// pass of its own it has the whole chip (8 heads, S_k=50, alone / with the passes: S_q=256 10.7 / 12.3 us, 384 13.7 / 13.9, 512 17.0 / 15.4; 96
-// heads 512 17.4 / 20.5, 1024 30.5 / 32.4; 512 heads 1024 138 / 153).
-constexpr bool bwd_one_kv(int D, int64_t heads, int S_q, int S_k) {
-  return D == 64 && S_k <= kTileN && (S_q <= 3 * kTileM || heads >= 12 * ((S_q + kTileM - 1) / kTileM));
-}
+// head dimension 64, one key tile: whether the main kernel is all there is (ONE_KV in fmha_bwd_sm100.cu)
+bool bwd_one_kv(int D, int64_t heads, int S_q, int S_k);
 // head dimension 64: the passes before and after the main kernel
 // `m`: the main kernel's arguments (sizes, mask, Philox, workspace)
 int launch_bwd_prepare(const fmha_tensor4& ot, const fmha_tensor4& dot, const BwdArgs& m, int dtype, cudaStream_t stream);

@@ -8,6 +8,7 @@ import torch
 from nvfuserexamples_b200 import api, capi, sharding
 from oracle import composite
 from tests import helpers
+from tests.test_fwd_rules import one_kv
 
 pytestmark = pytest.mark.gpu
 
@@ -373,3 +374,67 @@ def test_one_key_tile_without_the_passes(cuda_device, B, H, S_q, S_k, mask, p):
         eager = helpers.eager_16bit(q[sl], k[sl], v[sl], d_o[sl], add=add_, keep=keep, ks=ks)[1:]
         for got, want, e, name in zip((dq, dk, dv), refs, eager, ("dq", "dk", "dv")):
             helpers.assert_no_worse_than_eager(got[sl], want, e, f"{name}[{b},{h}]")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("p", [0.0, 0.2])
+@pytest.mark.parametrize("mask", ["none", "seqlen", "key"])
+def test_one_key_tile_same_bits_as_with_the_passes(cuda_device, mask, p, dtype):
+    """Head dimension 64 and one key tile: the main kernel alone against the three kernels, which the same batch takes in pieces of few heads.
+    There dQ is one addition to zero, so every bit is the same, in all heads.  All tensors are rows of [B,S,H,D] layouts, the gradients
+    views of larger buffers."""
+    B, H, S_q, S_k, D, piece = 19, 4, 600, 100, 64, 10
+    assert one_kv(D, B * H, S_q, S_k) and not one_kv(D, piece * H, S_q, S_k)
+    q, k, v, d_o, lens = (t.to(cuda_device) for t in helpers.randn_like_config(B, H, S_q, S_k, D, dtype, seed=4, device="cpu"))
+    q, k, v, d_o = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v, d_o))
+    kw = {"none": {}, "seqlen": dict(seqlens=lens), "key": dict(mask=composite.padding_add_mask(lens, S_k).reshape(B, S_k))}[mask]
+    fwd = torch.full((B, S_q, H, D), float("nan"), dtype=dtype, device=cuda_device).transpose(1, 2)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    o, lse = api.fmha_forward(q, k, v, p_drop=p, seed=3, offset=1, out=fwd, status=status, **kw)
+
+    def gradients():
+        return tuple(torch.full((B, S, H + 1, D + 8), float("nan"), dtype=dtype, device=cuda_device)[:, :, :H, :D].transpose(1, 2) for S in (S_q, S_k, S_k))
+    whole, pieces = gradients(), gradients()
+    api.fmha_backward(d_o, q, k, v, o, lse, p_drop=p, seed=3, offset=1, out=whole, status=status, **kw)
+    for b in range(0, B, piece):
+        s = slice(b, b + piece)
+        api.fmha_backward(d_o[s], q[s], k[s], v[s], o[s], lse[s].contiguous(), p_drop=p, seed=3, offset=1, bh_offset=b * H, status=status,
+                          out=tuple(t[s] for t in pieces), **{n: t[s].contiguous() for n, t in kw.items()})
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    for x, y in zip(whole, pieces):
+        assert torch.isfinite(x).all() and torch.equal(x, y)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("p", [0.0, 0.2])
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("B,H,S", [(2, 3, 77), (57, 3, 128)])   # 171 work items: more than SMs
+def test_one_key_tile_on_the_fused_projection_layout(cuda_device, B, H, S, packed, p, dtype):
+    """One [B,S,3,H,D] (packed: [rows,3,H,D]) gradient, written around what the buffer held before, with the bits of the call on contiguous tensors."""
+    D = 64
+    g = torch.Generator(device=cuda_device).manual_seed(S + B)
+    lens = (torch.arange(B, device=cuda_device) * 31 % S + 1).int()
+    lead = (int(lens.sum()),) if packed else (B, S)
+    qkv = torch.randn(*lead, 3, H, D, device=cuda_device, generator=g).to(dtype)
+    d_o = torch.randn(*lead, H, D, device=cuda_device, generator=g).to(dtype)
+    grad = torch.full((*lead, 4, H, D), float("nan"), dtype=dtype, device=cuda_device)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    kw = dict(p_drop=p, seed=7, offset=5, status=status)
+    if packed:
+        cu = torch.cat([torch.zeros(1, device=cuda_device, dtype=torch.int32), lens.cumsum(0).int()])
+        q, k, v = (qkv[:, i] for i in range(3))
+        r = capi.fwd_varlen(q, k, v, cu, S, **kw)
+        capi.bwd_varlen(d_o, q, k, v, r["o"], r["lse"], cu, S, out=tuple(grad[:, i] for i in range(3)), **kw)
+        want = capi.bwd_varlen(d_o, q.contiguous(), k.contiguous(), v.contiguous(), r["o"], r["lse"], cu, S, **kw)
+        got = [grad[:, i] for i in range(3)]
+    else:
+        q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
+        kw["seqlens"], dt = lens, d_o.transpose(1, 2)
+        o, lse = api.fmha_forward(q, k, v, out=torch.full_like(d_o, float("nan")).transpose(1, 2), **kw)
+        got = [grad[:, :, i].transpose(1, 2) for i in range(3)]
+        api.fmha_backward(dt, q, k, v, o, lse, out=tuple(got), **kw)
+        want = api.fmha_backward(dt.contiguous(), q.contiguous(), k.contiguous(), v.contiguous(), o.contiguous(), lse, **kw)
+    assert capi.check_status(status) == [0, 0, 0, 0]
+    for x, y in zip(got, want):
+        assert torch.isfinite(x).all() and torch.equal(x, y)
+    assert torch.isnan(grad[..., 3, :, :]).all()

@@ -64,3 +64,38 @@ def test_repeated_and_concurrent_calls(cuda_device):
     torch.cuda.synchronize()
     for o, lse in got:
         assert torch.equal(o, first[0]) and torch.equal(lse, first[1])
+
+
+@pytest.mark.parametrize("kind,p", [("none", 0.0), ("seqlen", 0.2), ("key", 0.0)])
+def test_fused_projection_layout_and_strided_out(cuda_device, kind, p):
+    """q, k and v as views of one [B,S,3,H,D] tensor, O into a view of a larger buffer: the bits of the call on contiguous tensors, and nothing beside them."""
+    S = 140
+    q, k, v, kw, _ = batch(S, S, torch.bfloat16, kind, cuda_device)
+    want = api.fmha_forward(q, k, v, p_drop=p, seed=5, offset=2, **kw)
+    qkv = torch.stack([t.transpose(1, 2) for t in (q, k, v)], dim=2)
+    buf = torch.full((B, S + 9, H + 1, 64), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    o, lse = api.fmha_forward(*(qkv[:, :, i].transpose(1, 2) for i in range(3)), p_drop=p, seed=5, offset=2, out=buf[:, :S, :H].transpose(1, 2), **kw)
+    assert torch.equal(o, want[0]) and torch.equal(lse, want[1])
+    assert (buf[:, S:] == 7.0).all() and (buf[:, :, H] == 7.0).all()
+
+
+def test_replayed_graph_and_device_resident_offset(cuda_device):
+    """A captured call replays with the bits of an eager one, the Philox offset from the value the tensor holds then."""
+    ops = torch.ops.mha_manual
+    q, k, v, kw, _ = batch(256, 128, torch.float16, "seqlen", cuda_device)
+    lens, off = kw["seqlens"], torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    eager = {value: ops.fmha_fwd(q, k, v, None, lens, 0.2, 3, 10 + value) for value in (0, 5)}
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream(device=cuda_device)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            o, lse = ops.fmha_fwd(q, k, v, None, lens, 0.2, 3, 10, None, 0, off)
+    torch.cuda.current_stream().wait_stream(side)
+    for value in (0, 5, 0):
+        off.fill_(value)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(o, eager[value][0]) and torch.equal(lse, eager[value][1])
+    assert not torch.equal(eager[0][0], eager[5][0])
+    ops.check_status()

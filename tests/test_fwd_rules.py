@@ -1,4 +1,4 @@
-"""The rule on sizes that picks the forward kernel of two query tiles per CTA, called in the built library (no GPU needed)."""
+"""The rules on sizes that pick a kernel, called in the built library (no GPU needed)."""
 import ctypes as C
 
 import pytest
@@ -69,3 +69,15 @@ def test_rule_of_the_kernel_that_goes_from_tile_to_tile_without_lengths():
     assert not fn(148, 1184, 241, False, False, False) and fn(148, 1185, 256, False, False, False)
     assert fn(148, 1184, 240, False, False, False) and fn(148, 1184, 256, False, False, True) and fn(148, 1184, 256, True, False, False)
     assert not fn(148, 1184, 256, False, True, False) and not fn(148, 592, 64, False, False, False)
+
+
+def one_kv(D, heads, S_q, S_k):
+    fn = capi.load()["_ZN4fmha10bwd_one_kvEilii"]   # fmha::bwd_one_kv(int, int64_t, int, int)
+    fn.argtypes, fn.restype = [C.c_int, C.c_int64, C.c_int, C.c_int], C.c_bool
+    return fn(D, heads, S_q, S_k)
+
+
+def test_rule_of_the_backward_of_one_key_tile():
+    assert one_kv(64, 1, 384, 128) and not one_kv(64, 1, 384, 129) and not one_kv(128, 512, 128, 128)
+    assert not one_kv(64, 47, 385, 100) and one_kv(64, 48, 385, 100)      # four query tiles
+    assert not one_kv(64, 59, 600, 100) and one_kv(64, 60, 600, 100)      # five
