@@ -99,3 +99,17 @@ def test_replayed_graph_and_device_resident_offset(cuda_device):
         assert torch.equal(o, eager[value][0]) and torch.equal(lse, eager[value][1])
     assert not torch.equal(eager[0][0], eager[5][0])
     ops.check_status()
+
+
+@pytest.mark.parametrize("p", [0.0, 0.2])
+def test_a_nan_among_masked_keys_is_not_stepped_over(cuda_device, p):
+    """As in the kernel of one tile per CTA: a key whose score is NaN makes its head's rows NaN, masked away or not, and no other head's."""
+    S = 250
+    q, k, v, _, _ = batch(S, S, torch.float16, "none", cuda_device)
+    mask = torch.where(torch.arange(S, device=cuda_device) < 50, 0.0, -1e4).repeat(B, 1)
+    want, _ = api.fmha_forward(q, k, v, mask=mask, p_drop=p, seed=1)
+    k[30, 5, 200] = float("nan")
+    o, lse = api.fmha_forward(q, k, v, mask=mask, p_drop=p, seed=1)
+    assert torch.isnan(o[30, 5]).all() and torch.isnan(lse.view(B, H, S)[30, 5]).all()
+    o[30, 5] = want[30, 5]
+    assert torch.isfinite(want).all() and torch.equal(o, want)
