@@ -418,7 +418,7 @@ def run_ours(args, rank, world, local_rank):
                 "peak_source": f"{pk['source']} bf16 burst", "ms_per_launch": bwd_main_ms,
                 "algorithmic_flops_per_launch": exe_b}
     ach_f = exe_f / (fwd_ms * 1e-3) / 1e12
-    roofline_fwd = {"kernel": "fmha_fwd_fast_kernel<64,fp16,seqlen,dropout>", "bound": "tensor", "achieved": ach_f,
+    roofline_fwd = {"kernel": "fmha_fwd_chain_kernel<fp16,seqlen,dropout>", "bound": "tensor", "achieved": ach_f,
                     "peak": pk["tflops"], "unit": "TFLOP/s", "frac": ach_f / pk["tflops"], "ms_per_launch": fwd_ms,
                     "dense_equiv_frac": dense_f / (fwd_ms * 1e-3) / 1e12 / pk["tflops"]}
 

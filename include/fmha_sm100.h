@@ -172,7 +172,8 @@ int fmha_sm100_fwd(const fmha_fwd_params* p, void* stream);
 int fmha_sm100_bwd(const fmha_bwd_params* p, void* stream);
 
 /* Bytes of device scratch fmha_sm100_bwd needs for these sizes: the row term delta = rowsum(dO * O) and, at D = 64, an fp32 dQ
-   accumulator. */
+   accumulator.  Where the main kernel alone does the backward (D = 64, up to 128 keys, as a rule) they are counted as well, although it
+   does not touch them: fewer heads of the same lengths may not be done that way, and a workspace of the largest batch serves the smaller ones. */
 int fmha_sm100_bwd_workspace_bytes(const fmha_bwd_params* p, size_t* bytes);
 
 /* Backward for callers that cannot hand over a workspace (this entry point has no counterpart

@@ -44,7 +44,7 @@ namespace {
 #endif
 constexpr uint32_t kComputeSleepNs = FMHA_BWD_POLL_SLEEP_NS;  // pause between barrier polls of the compute warps
 constexpr int kComputeThreads = 512;               // 16 compute warps
-constexpr int kBwdStatWarp = 2 + kComputeThreads / 32;   // the warp that fetches lse and delta
+constexpr int kBwdStatWarp = 2 + kComputeThreads / 32;   // the warp that fetches lse and delta (ONE_KV: lse)
 constexpr int kBwdThreads = 64 + kComputeThreads + 32;   // + producer warp + MMA warp + statistics warp
 constexpr float kLog2eB = 1.4426950408889634f;
 
@@ -151,8 +151,8 @@ __device__ __forceinline__ float row_dot(const uint4& x, const uint4& y) {
   return sum;
 }
 
-// Bound by memory: O and dO in, the accumulator out (B=32 H=16 S=512: 134 MB in 18.4 us, 7.3 TB/s; with each thread clearing the 32 bytes
-// of its own eight columns, half a sector an instruction, 19.8).  PACKED: a block waits for the row offsets before it can load, so on large grids it
+// Bound by memory: O and dO in, the accumulator out (B=32 H=16 S=512: 134 MB in 18.4 us, 7.3 TB/s, above the card's copy rate, because a part
+// of the accumulator stays in the L2 cache; with each thread clearing the 32 bytes of its own eight columns, half a sector an instruction, 19.8).  PACKED: a block waits for the row offsets before it can load, so on large grids it
 // takes four times the rows (R), their loads in flight together, and four blocks an SM leave the rare zeroing of uncovered rows its registers
 // (12 288 rows, 16 heads 20.6 -> 15.3 us; twice the rows 15.9, in 32 registers 17.4).  Where that leaves less than 1.5 blocks per multiprocessor there is
 // nothing to hide the wait behind, and blocks of 32 rows are done sooner (whole backward with four / one times 32 rows: 4 blocks of 128 rows
@@ -310,8 +310,8 @@ struct BwdItem {
 // ONE_KV: D = 64 and a single key tile (bwd_one_kv).  Nothing is added up for dQ then, so its tiles are written as they come; delta is formed
 // here, by the compute warps, 8 rows each, with the loads under the draws and the wait for S; and work items are equal and need no
 // counter.  A packed batch has the pass before it, to zero rows.  The accumulator, its clearing and conversion and the launches around
-// this one took a quarter of the time (packed B=32 H=16, up to 128 rows each, 34.6 -> 29.3 us; whole backward of padded batches
-// B=2 H=4 S=128 with dropout 11.3 -> 8.6 us, B=13 H=12 S=100 15.4 -> 11.5, B=32 H=16 S=128 27.9 -> 20.1, B=128 H=16 93.0 -> 71.9).
+// this one took 14 to 30 % of the time (whole backward, without / with dropout: B=2 H=4 S=128 10.6 -> 7.8 / 10.9 -> 8.4 us, B=13 H=12 S=100 15.1 -> 11.2 /
+// 16.6 -> 13.0, B=32 H=16 S=128 27.8 -> 19.5 / 29.1 -> 23.0, B=128 H=16 94.4 -> 68.3 / 97.8 -> 75.7; packed, B=32 H=16 of 64 to 128 rows 34.2 -> 27.7 / 36.1 -> 31.2).
 template <int D, bool BF16, bool KEYADD, bool DROP, bool PACKED = false, bool ONE_KV = false>
 __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_constant__ BwdArgs a) {
   griddep_wait();
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fmha_bwd_kernel(const __grid_c
     }
   } else if (warp == kBwdStatWarp) {
     // ============================ row statistics =====================================
-    // lse and delta of a tile's 128 query rows, in the form the compute warps use them, one to two tiles ahead.
+    // lse and delta of a tile's 128 query rows (ONE_KV: lse alone), in the form the compute warps use them, one to two tiles ahead.
     const float inv_c = DROP ? 1.0f / a.dropout_scale : 1.0f;
     int n = 0, t = 0;
     while (true) {

@@ -10,7 +10,8 @@
 // dropout 1 650), four of which run at a time per scheduler against 512 of exponentials each; a CTA per tile added its start (launch, tensor
 // memory, first loads, first product: 3 500 cycles) and its end (2 500), here a tile ends in 1 800 (P V 500, O 800, the next item 400).
 // Four CTAs per SM hide part of either: B=64 H=16 S=384 with an additive mask 65.8 -> 62.9 us, B=32 H=12 S=512 with dropout 49.4 -> 47.7,
-// B=228 H=12 S=64 with a mask 23.1 -> 17.8.  The additive mask of a step brought into shared memory a step ahead took its 600 cycles
+// B=228 H=12 S=64 with a mask 23.1 -> 17.8 (kernel times).  With an additive mask it spills 68 bytes where the other kernel spills 32 (with dropout as well 8, 24
+// there; without either 4, none there).  The additive mask of a step brought into shared memory a step ahead took its 600 cycles
 // out of the chain and left the time as it was (62.9 / 64.3).  A packed batch is left to the other kernel: each tile past the end of its
 // sequence costs a question and an answer here (the tracked unpadded batch 62.2 -> 68.3).
 #include <cuda_bf16.h>
@@ -402,7 +403,9 @@ __global__ void __launch_bounds__(kChThreads, kChCtasPerSm) fmha_fwd_chain_kerne
 // this kernel / a CTA per tile: without dropout or mask S=48 0.80 to 0.94, 128 0.90 to 0.96, 256 0.93 to 1.00, 384 0.96 to 0.99 from three
 // rounds on and 1.03 at 1.8, 449 1.01 to 1.05, 849 and 2048 1.02 to 1.06; additive mask S=64 0.77, 128 0.88 to 0.97, 384 0.96, 449 0.93 to
 // 1.05; dropout S=128 0.90 to 0.98 from 2.3 rounds on and up to 1.04 below, 197 1.07 at 1.2 rounds and 0.94 at 5.5, 512 0.97 to 1.00, 849 and
-// more 0.98 to 1.06; both, S=197 1.03 at 1.6 rounds and 0.94 to 0.99 from three on.
+// more 0.98 to 1.06; both, S=197 1.03 at 1.6 rounds and 0.94 to 0.99 from three on.  Between one and two rounds of five and six key steps with a mask
+// it depends on the padding and on how the last tiles fall (300 and 384 keys, 1.0 to 2.0 rounds: 0.96 to 1.04 with lengths U[0.4 S, S], 0.96 to 1.07 with a mask that
+// masks nothing, 0.95 to 1.00 with one that is nowhere zero).
 bool fwd_chain_pays(int64_t sms, int64_t tiles, int64_t S_k, bool keyadd, bool dropout) {
   const int64_t round = kChCtasPerSm * sms;
   if (tiles <= round) return false;

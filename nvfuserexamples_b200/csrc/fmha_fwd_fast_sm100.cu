@@ -579,7 +579,9 @@ static int fwd_key_split(int64_t ctas, int steps, int S_q, int D, bool long_step
 // the last ones to finish leave SMs idle (lengths U[S/2, S]: B=8 H=12 S=512 16.2 -> 14.9 us, B=16 H=8 S=640 with dropout
 // 35.2 -> 33.3, B=32 H=12 S=512 with dropout 57.0 -> 54.2); beyond it does not (B=64 H=16 S=384 62.3 -> 64.9 us, with two
 // elements per lane), nor at D = 128, where a CTA's start is the longer chain (B=16 H=12 S=512 37.1 -> 38.4 us), and with no
-// more CTAs than SMs the order does not matter.
+// more CTAs than SMs the order does not matter.  These figures are of a CTA per tile.  The kernel that goes from tile to tile keeps the rule, and gains
+// as much: B=32 S=512 with dropout, lengths U[256, 512] 12 heads 48.3 -> 45.1 us, 16 heads 64.7 -> 58.8, U[128, 512] 45.3 -> 39.2 and 57.1 -> 51.2, B=32
+// H=16 S=256 without 16.8 -> 15.8.
 int fwd_length_class_shift(const FwdArgs& a, int D, int64_t ctas, bool no_lengths) {
   if (no_lengths || D != 64 || (a.mask_kind != FMHA_MASK_SEQLEN && a.mask_kind != FMHA_MASK_CU_SEQLENS) || a.B < 2 || a.B > kMaxOrdered)
     return -1;

@@ -1,5 +1,5 @@
 // fmha_fwd_softmax.cuh — what one softmax thread (one query row) does per key step and at the end of a query tile: shared by
-// the two forward kernels for compact masks (fmha_fwd_fast_sm100.cu, fmha_fwd_pair_sm100.cu).
+// the three forward kernels for compact masks and any number of rows (fmha_fwd_fast_sm100.cu, fmha_fwd_pair_sm100.cu, fmha_fwd_chain_sm100.cu).
 #pragma once
 #include "fmha_device_utils.cuh"
 #include "philox.cuh"
@@ -271,7 +271,8 @@ __device__ __forceinline__ void softmax_step(uint32_t tS, uint32_t tO, int key0,
 
 // A 64-key step at head dimension 64.  The last one of a tile may have 32 keys or fewer (one in two, where lengths are spread): then
 // only its first half is read, drawn for and exponentiated, and a longer one looks for keys past the end in its second half alone
-// (B=32 H=12 S=512 with dropout, lengths U[256, 512] 53.3 -> 49.4 us, B=16 H=8 S=160 8.6 -> 7.4, B=13 H=12 S=197 without 9.2 -> 8.8).  Not with an
+// (kernel times, a CTA per tile: B=32 S=512 with dropout, lengths U[256, 512] 12 heads 50.1 -> 46.9 us, 16 heads 64.0 -> 59.8, B=16 H=8 S=160 8.3 -> 7.1,
+// B=13 H=12 S=197 without 8.6 -> 8.3; few keys split over a cluster, 449 with lengths 7.20 -> 7.34).  Not with an
 // additive mask, which has such a step only where S_k is no multiple of 64, and registers to spare for a second copy nowhere (B=64 H=16 S=384
 // 65.8 -> 67.7).
 template <bool BF16, bool KEYADD, bool DROP, class WaitS, class ArriveP>
@@ -286,7 +287,9 @@ __device__ __forceinline__ void softmax_step_64(uint32_t tS, uint32_t tO, int ke
 // The same at head dimension 128, 128 keys a step and 64 to the half (kernel times: S=64 without a mask B=8 H=12 5.3 -> 4.5 us, with dropout
 // B=36 H=16 14.1 -> 10.2; lengths with dropout B=16 H=8 S=640 packed 37.5 -> 33.8, B=10 H=8 S=2048 140 -> 134; without, two tiles per CTA,
 // B=16 H=16 S=300 25.8 -> 24.0, B=12 H=12 S=2048 212 -> 210; of 90 sizes none slower).  With an additive mask as well, which gains here even
-// where no last step is short: B=98 H=16 S=256 108 -> 104, B=64 H=16 S=384 133 -> 127, S=160 B=34 H=8 18.0 -> 15.8.
+// where no last step is short: B=98 H=16 S=256 108 -> 104, B=64 H=16 S=384 133 -> 127, S=160 B=34 H=8 18.0 -> 15.8.  With mask and dropout, whose spills
+// it raises from 116 to 140 bytes: B=36 H=16 S=64 15.7 -> 11.6, S=160 B=34 H=8 21.2 -> 18.1, S=300 B=12 H=12 25.6 -> 23.9, S=384 and more 0.94 to 1.00 of the time,
+// one whole step on a small grid 6.03 -> 6.15, keys split over a cluster 0.91 to 1.04.
 template <bool BF16, bool KEYADD, bool DROP, int P_FIRST, class WaitS, class ArriveP, class TurnBegin, class TurnEnd>
 __device__ __forceinline__ void softmax_step_128(uint32_t tS, uint32_t tO, int key0, int n_cols, float sl2, const float* mask_stage, int kind,
                                                  const DropRow& dr, float& m_ref, float2& sum2, const WaitS& wait_s, const ArriveP& arrive_p,

@@ -84,8 +84,9 @@ struct BwdArgs {
   alignas(64) CUtensorMap tm_do;
   alignas(64) CUtensorMap tm_dk;  // 16-bit outputs, {D/4 x 32} boxes (one per compute warp), no swizzle
   alignas(64) CUtensorMap tm_dv;
-  // Head dimension 128, dQ kernel (fmha_bwd_dq_sm100.cu): 16-bit dQ in {16 x 32} boxes; O and dO for the row term delta
-  alignas(64) CUtensorMap tm_dq;
+  alignas(64) CUtensorMap tm_dq;   // head dimension 128, dQ kernel (fmha_bwd_dq_sm100.cu): 16-bit dQ in {16 x 32} boxes
+  // O and dO for the row term delta, in the kernel that forms it, and dQ where it is written row by row: the dQ kernel, and the main kernel
+  // with a single key tile at head dimension 64 (ONE_KV)
   const void* o_ptr;
   const void* do_ptr;
   int64_t o_sb, o_sh, o_ss, do_sb, do_sh, do_ss;
@@ -97,9 +98,9 @@ struct BwdArgs {
   float scale;       // softmax scale
   float scale_log2;  // softmax scale * log2(e)
   const float* lse;  // [B*H, S_q] natural log
-  float* delta;        // [B*H, S_q] rowsum(dO * O)
+  float* delta;        // [B*H, S_q] rowsum(dO * O); not used with ONE_KV
   float* dq_accum;     // head dimension 64: [B*H, S_q_pad, D] fp32 in the blocked order of dq_accum_index, zero on entry; null: not used
-  int* work_counter;   // zero on entry; the persistent CTAs draw their work items from it
+  int* work_counter;   // zero on entry; the persistent CTAs draw their work items from it (not with ONE_KV: every grid-th item)
   // FMHA_MASK_CU_SEQLENS: mask = int32 [B+1] row offsets into the packed [total_rows, H, D] tensors; the raw
   // dK / dV pointers serve the row-wise stores of a sequence's last, partial key tile
   int total_rows;

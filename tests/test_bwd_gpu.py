@@ -349,7 +349,7 @@ def test_additive_mask_down_to_minus_infinity(cuda_device, B, H, S_q, S_k, D, va
 @pytest.mark.parametrize("B,H,S_q,S_k", [(2, 3, 127, 16), (3, 2, 129, 128), (2, 2, 384, 100), (2, 2, 385, 100), (40, 8, 128, 127), (38, 4, 600, 33)])
 def test_one_key_tile_without_the_passes(cuda_device, B, H, S_q, S_k, mask, p):
     """Head dimension 64 and up to 128 keys: delta and dQ in the main kernel alone (a few heads of more than three query tiles keep the
-    passes), ragged rows and keys, more heads than SMs, rows of a [B,S,H,D] layout.  The first and the last head against the oracle."""
+    passes), ragged rows and keys, more heads than SMs, dO with the rows of a [B,S,H,D] layout.  The first and the last head against the oracle."""
     dtype = torch.float16
     q, k, v, d_o, lens = helpers.randn_like_config(B, H, S_q, S_k, 64, dtype, seed=S_q + S_k, device=cuda_device)
     d_o = d_o.transpose(1, 2).contiguous().transpose(1, 2)

@@ -268,7 +268,7 @@ def test_a_nan_among_masked_keys_is_not_stepped_over(cuda_device, D, p_drop):
 
 
 @pytest.mark.parametrize("B,H,S_q,S_k", [
-    (40, 8, 256, 300),    # one CTA per query tile; at D = 128 two tiles per CTA
+    (40, 8, 256, 300),    # one CTA per query tile, with a mask from tile to tile; at D = 128 two tiles per CTA
     (2, 8, 200, 300),     # one CTA per query tile at both head dimensions
     (1, 2, 130, 1536),    # keys split over a cluster
 ])
